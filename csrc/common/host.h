@@ -63,6 +63,24 @@ inline int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, 
   return 0;
 }
 
+// 2-D output tensor (bf16 or fp32, row stride `ld` elements) read and written in boxes of 128 bytes x `box_rows` rows,
+// 128-byte swizzle.
+inline int make_tmap_2d_out(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, bool f32,
+                            uint32_t box_rows) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) ZB_FAIL(-3, "cuTensorMapEncodeTiled entry point not available");
+  const uint64_t es = f32 ? 4 : 2;
+  cuuint64_t dims[2] = {cols, rows};
+  cuuint64_t strides[1] = {ld * es};
+  cuuint32_t box[2] = {cuuint32_t(128 / es), box_rows};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base),
+                  dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) ZB_FAIL(-5, "cuTensorMapEncodeTiled failed with %d", int(r));
+  return 0;
+}
+
 // General N-d bf16 tensor map (innermost dimension first), 128-byte swizzle.
 inline int make_tmap_nd_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
                              const uint64_t* strides_bytes /* rank-1 */, const uint32_t* box) {

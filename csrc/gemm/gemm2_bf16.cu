@@ -92,12 +92,31 @@ struct Gemm2Cfg {
   static constexpr int A_BYTES = 128 * BK * 2;
   static constexpr int B_BYTES = 128 * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = 6;
   static constexpr int TMEM_COLS = 512;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
+  static constexpr int EP_BYTES = 32 * 128;    // epilogue box: 32 rows x 128 bytes
+  // Shared memory is split at launch: 6 operand stages and 2 epilogue boxes per epilogue warp, or 5 and 4.  The sixth
+  // stage is worth 3 - 5 % of the main loop (4096 x 22016 x 4096: 486 -> 472 us), two more boxes shorten the epilogue
+  // of a tile whose old C tile has to be read (load, add, store in flight at once).  The epilogue of a tile runs under
+  // the main loop of the next one, so the boxes only count where that loop is short: K < 2048.
+  static constexpr int MAX_STAGES = 6, MAX_EP_BUFS = 4;
+  static constexpr int RING_BYTES = 6 * STAGE_BYTES + 4 * 2 * EP_BYTES;
+  static_assert(RING_BYTES == 5 * STAGE_BYTES + 4 * 4 * EP_BYTES, "both splits fill the same space");
+  static constexpr int SMEM_BYTES = RING_BYTES + 1024 + 512;
 };
 
+// How the accumulators leave the SM.  DIRECT: one output row per thread, loads and stores straight to global memory
+// (any alignment, any combination of options).  BF16 / F32: 32 x 128-byte boxes through shared memory and TMA; the old
+// C tile or the addend of a bf16 output arrives by TMA as well, two boxes ahead; an accumulating fp32 output is added
+// in L2 (cp.reduce), so it is never read into the SM.  The direct form issues 16-byte accesses of 32 different rows per
+// instruction and waits for the old C values chunk by chunk: about 20 us per 256 x 256 tile that accumulates, longer
+// than the tile's main loop below K = 4096.  Weight gradients with the boxes: 3072 x 768 x 2048 fp32 34.7 -> 17.9 us,
+// 20480 x 5120 x 2048 bf16 432 -> 335 us; plain bf16 outputs 1018 x 49152 x 512 61 -> 48 us.
+enum : int { EP_DIRECT = 0, EP_BF16 = 1, EP_F32 = 2 };
+
 struct Gemm2Extra {
+  TileOrder order;
+  int ep;          // EP_*
+  int ep_load;     // EP_BF16: add the tensor behind tmap_x (old C or addend)
   int a_3d, b_3d;  // MN-major operand fetched with one 3-D TMA box {64, BK, 2} instead of two 2-D boxes
 };
 
@@ -107,32 +126,33 @@ struct Gemm2Extra {
 // FUSED_AG (Params = GemmAgParams): four more warps per CTA pull the peers' parameter shards into the local
 // unsharded buffer while the tiles whose B rows are already present run; each CTA's producer waits for the
 // chunks that cover its own 128 rows of B.
-template <bool A_MN, bool B_MN, typename Params = GemmParams>
+template <bool A_MN, bool B_MN, typename Params, int STAGES>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(std::is_same<Params, GemmAgParams>::value ? 320 : 192, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                  const Params p, const Gemm2Extra ex) {
+                  const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_x, const Params p,
+                  const Gemm2Extra ex) {
   using Cfg = Gemm2Cfg;
   constexpr bool SCATTER = std::is_same<Params, GemmScatterParams>::value;
-  constexpr bool ACCPF = std::is_same<Params, GemmAccPrefetchParams>::value;
   constexpr bool FUSED_AG = std::is_same<Params, GemmAgParams>::value;
-  constexpr int BK = Cfg::BK, STAGES = Cfg::STAGES, BN = Cfg::BN;
+  constexpr int BK = Cfg::BK, MAXS = Cfg::MAX_STAGES, BN = Cfg::BN;
+  constexpr int EP_BUFS = STAGES == 6 ? 2 : 4;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES);
+  uint8_t* sE = smem + STAGES * Cfg::STAGE_BYTES;   // epilogue boxes, EP_BUFS per epilogue warp
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::RING_BYTES);
   uint64_t* full = bars;                          // leader's copy is the one in use
-  uint64_t* empty = bars + STAGES;                // each CTA waits on its own
-  uint64_t* tmem_full = bars + 2 * STAGES;        // [2], each CTA waits on its own
-  uint64_t* tmem_empty = bars + 2 * STAGES + 2;   // [2], leader's copy, 8 arrivals
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
+  uint64_t* empty = bars + MAXS;                  // each CTA waits on its own
+  uint64_t* tmem_full = bars + 2 * MAXS;          // [2], each CTA waits on its own
+  uint64_t* tmem_empty = bars + 2 * MAXS + 2;     // [2], leader's copy, 8 arrivals
+  uint64_t* x_full = bars + 2 * MAXS + 4;         // [4 warps][MAX_EP_BUFS]: a box of tmap_x has landed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(x_full + 4 * Cfg::MAX_EP_BUFS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();
   const bool leader = cta == 0;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  const int tiles_m = (p.M + Cfg::BM - 1) / Cfg::BM;
-  const int tiles_n = (p.N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n;
+  const int num_tiles = ex.order.tiles_m * ex.order.tiles_n;
   const int num_kb = (p.K + BK - 1) / BK;
   WaitCtx wctx{abort_flag, p.status};
 
@@ -146,6 +166,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       mbar_init(&tmem_full[i], 1);
       mbar_init(&tmem_empty[i], 8);
     }
+    for (int i = 0; i < 4 * Cfg::MAX_EP_BUFS; ++i) mbar_init(&x_full[i], 1);
     mbar_fence_init();
   }
   if (warp == 1) {
@@ -159,15 +180,20 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
-    if (lane == 0) {
-      tma_prefetch_desc(&tmap_a);
-      tma_prefetch_desc(&tmap_b);
+    {
+      const bool elected = elect_one();
+      if (elected) {
+        tma_prefetch_desc(&tmap_a);
+        tma_prefetch_desc(&tmap_b);
+      }
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        const int m0 = (tile % tiles_m) * Cfg::BM + int(cta) * 128;
-        const int n0 = (tile / tiles_m) * BN + int(cta) * 128;
+        int tm, tn;
+        tile_at(ex.order, tile, tm, tn);
+        const int m0 = tm * Cfg::BM + int(cta) * 128;
+        const int n0 = tn * BN + int(cta) * 128;
         // (the second CTA's half may start past the edge of a ragged tile: its loads then read the fill value)
         if (!zb_in_bounds(m0 - int(cta) * 128 < p.M && n0 - int(cta) * 128 < p.N && tile >= 0, p.status, 1)) break;
         if constexpr (FUSED_AG) {
@@ -189,22 +215,24 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (!mbar_wait(&empty[stage], phase ^ 1, wctx, ST_TIMEOUT_EMPTY)) { ok = false; break; }
           uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
           uint8_t* sb = sa + Cfg::A_BYTES;
-          if (leader) mbar_expect_tx(&full[stage], 2 * Cfg::STAGE_BYTES);
-          if (!A_MN) {
-            tma_load_2d_pair(sa, &tmap_a, &full[stage], kb * BK, m0);
-          } else if (ex.a_3d) {
-            tma_load_3d_pair(sa, &tmap_a, &full[stage], 0, kb * BK, m0 >> 6);
-          } else {
-            tma_load_2d_pair(sa, &tmap_a, &full[stage], m0, kb * BK);
-            tma_load_2d_pair(sa + BK * 128, &tmap_a, &full[stage], m0 + 64, kb * BK);
-          }
-          if (!B_MN) {
-            tma_load_2d_pair(sb, &tmap_b, &full[stage], kb * BK, n0);
-          } else if (ex.b_3d) {
-            tma_load_3d_pair(sb, &tmap_b, &full[stage], 0, kb * BK, n0 >> 6);
-          } else {
-            tma_load_2d_pair(sb, &tmap_b, &full[stage], n0, kb * BK);
-            tma_load_2d_pair(sb + BK * 128, &tmap_b, &full[stage], n0 + 64, kb * BK);
+          if (elected) {
+            if (leader) mbar_expect_tx(&full[stage], 2 * Cfg::STAGE_BYTES);
+            if (!A_MN) {
+              tma_load_2d_pair(sa, &tmap_a, &full[stage], kb * BK, m0);
+            } else if (ex.a_3d) {
+              tma_load_3d_pair(sa, &tmap_a, &full[stage], 0, kb * BK, m0 >> 6);
+            } else {
+              tma_load_2d_pair(sa, &tmap_a, &full[stage], m0, kb * BK);
+              tma_load_2d_pair(sa + BK * 128, &tmap_a, &full[stage], m0 + 64, kb * BK);
+            }
+            if (!B_MN) {
+              tma_load_2d_pair(sb, &tmap_b, &full[stage], kb * BK, n0);
+            } else if (ex.b_3d) {
+              tma_load_3d_pair(sb, &tmap_b, &full[stage], 0, kb * BK, n0 >> 6);
+            } else {
+              tma_load_2d_pair(sb, &tmap_b, &full[stage], n0, kb * BK);
+              tma_load_2d_pair(sb + BK * 128, &tmap_b, &full[stage], n0 + 64, kb * BK);
+            }
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -212,8 +240,12 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA only) ------------------------------
-    if (leader && lane == 0) {
+    // The whole warp walks the loop and one elected lane issues: addresses and descriptors stay warp-uniform.  With the
+    // loop inside `if (lane == 0)` issuing the four products of a k-block took longer than the tensor core needs for
+    // them (4096 x 22016 x 4096: 519 -> 494 us).
+    if (leader) {
       constexpr uint32_t idesc = umma_idesc_bf16(256, BN, A_MN, B_MN);
+      const bool elected = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       int local = 0;
@@ -229,66 +261,128 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE_BYTES);
           const uint32_t sb = sa + Cfg::A_BYTES;
+          if (elected) {
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) {
-            uint64_t da = A_MN ? umma_desc_mnmajor(sa + kk * 16 * 128, BK * 128) : umma_desc_kmajor(sa + kk * 32);
-            uint64_t db = B_MN ? umma_desc_mnmajor(sb + kk * 16 * 128, BK * 128) : umma_desc_kmajor(sb + kk * 32);
-            umma_f16_ss_pair(d_tmem, da, db, idesc, (kb | kk) != 0 ? 1u : 0u);
+            for (int kk = 0; kk < BK / 16; ++kk) {
+              uint64_t da = A_MN ? umma_desc_mnmajor(sa + kk * 16 * 128, BK * 128) : umma_desc_kmajor(sa + kk * 32);
+              uint64_t db = B_MN ? umma_desc_mnmajor(sb + kk * 16 * 128, BK * 128) : umma_desc_kmajor(sb + kk * 32);
+              umma_f16_ss_pair(d_tmem, da, db, idesc, (kb | kk) != 0 ? 1u : 0u);
+            }
+            umma_commit_pair(&empty[stage]);
           }
-          umma_commit_pair(&empty[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
-        if (ok) umma_commit_pair(&tmem_full[buf]);
+        if (ok && elected) umma_commit_pair(&tmem_full[buf]);
       }
     }
   } else if (warp < 6) {
     // ------------------------------ epilogue (own 128 rows) ------------------------------
     const int q = warp & 3;
     const EpilogueCfg ecfg = epilogue_cfg(p);
+    uint8_t* my_boxes = sE + q * EP_BUFS * Cfg::EP_BYTES;
+    uint64_t* my_full = x_full + q * Cfg::MAX_EP_BUFS;
+    const uint32_t slot_mask = uint32_t(EP_BUFS) - 1, phase_shift = EP_BUFS == 4 ? 2 : 1;
+    const int ahead = EP_BUFS == 4 ? 2 : 1;   // boxes of tmap_x requested ahead of the one being added
+    uint32_t ep_count = 0;   // boxes this warp has stored: slot and barrier phase of the next one
     int local = 0;
     for (int tile = pair; tile < num_tiles; tile += num_pairs, ++local) {
-      const int m0 = (tile % tiles_m) * Cfg::BM + int(cta) * 128;
-      const int n0 = (tile / tiles_m) * BN;
+      int tm, tn;
+      tile_at(ex.order, tile, tm, tn);
+      const int m0 = tm * Cfg::BM + int(cta) * 128;
+      const int n0 = tn * BN;
       const int buf = local & 1;
       const uint32_t use = uint32_t(local >> 1);
-      if constexpr (ACCPF) {
-        // bf16 C += result without bias / addend / activation (checked on the host): request this thread's whole
-        // old C row of the tile now; the loads complete while the tile's main loop is still running
-        const int row = m0 + q * 32 + lane;
-        const bool row_ok = row < p.M;
-        const bool fast = row_ok && ecfg.vec_ok && n0 + BN <= p.N;
-        uint4 oldc[BN / 8];
-        __nv_bfloat16* crow = static_cast<__nv_bfloat16*>(p.C) + size_t(row_ok ? row : 0) * p.ldc + n0;
-        if (fast) {
-#pragma unroll
-          for (int j = 0; j < BN / 8; ++j) oldc[j] = reinterpret_cast<const uint4*>(crow)[j];
+      if (!SCATTER && ex.ep != EP_DIRECT) {
+        const int row0 = m0 + q * 32;
+        const int wide = ex.ep == EP_F32 ? 32 : 64;                    // columns of a box
+        const int boxes = row0 < p.M ? min(BN / wide, (p.N - n0 + wide - 1) / wide) : 0;
+        auto load_box = [&](int c) {   // box c of this tile -> its ring slot (lane 0)
+          const uint32_t k = ep_count + uint32_t(c);
+          mbar_expect_tx(&my_full[k & slot_mask], Cfg::EP_BYTES);
+          tma_load_2d(my_boxes + (k & slot_mask) * Cfg::EP_BYTES, &tmap_x, &my_full[k & slot_mask], n0 + c * 64, row0);
+        };
+        if (ex.ep_load && lane == 0) {
+          bulk_wait_read<0>();   // stores of earlier boxes (issued a main loop ago) still hold the slots of boxes 0 and 1
+          if (boxes > 0) load_box(0);
+          if (boxes > 1) load_box(1);
         }
         if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full[buf], use & 1, wctx, ST_TIMEOUT_TMEM_FULL))) break;
         tc_fence_after();
-#pragma unroll
-        for (int c = 0; c < BN / 32; ++c) {
-          const int col0 = n0 + c * 32;
-          if (col0 < p.N) {
+        auto release_tmem = [&] {   // this warp has read its part of the accumulators
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(&tmem_empty[buf], 0);
+        };
+        auto wait_slot = [&] {      // the store of box k - EP_BUFS has left the slot of box k
+          if (EP_BUFS == 4) bulk_wait_read<3>();
+          else bulk_wait_read<1>();
+        };
+        bool ok = true;
+        if (boxes == 0) release_tmem();
+        for (int c = 0; c < boxes; ++c) {
+          const uint32_t k = ep_count + uint32_t(c);
+          const uint32_t box = smem_u32(my_boxes + (k & slot_mask) * Cfg::EP_BYTES) + uint32_t(lane) * 128;
+          const int col0 = n0 + c * wide;
+          const uint32_t t_addr = tmem_base + (uint32_t(q * 32) << 16) + uint32_t(buf * BN + c * wide);
+          if (ex.ep == EP_F32) {
             uint32_t r[32];
-            tmem_ld32(tmem_base + (uint32_t(q * 32) << 16) + uint32_t(buf * BN + c * 32), r);
+            tmem_ld32(t_addr, r);
+            if (lane == 0) wait_slot();
             tmem_wait_ld();
-            if (fast) {
+            if (c == boxes - 1) release_tmem();
+            epilogue_bias_act(p, col0, r);
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              st_shared_v4(box + uint32_t((j ^ (lane & 7)) << 4), r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          } else {
+            uint32_t r[32], s[32];
+            tmem_ld32(t_addr, r);
+            tmem_ld32(t_addr + 32u, s);
+            if (lane == 0) {
+              if (!ex.ep_load) {
+                wait_slot();
+              } else if (c + ahead >= 2 && c + ahead < boxes) {
+                // box k + ahead takes the slot of box k - ahead, which has to have left
+                if (ahead == 2) bulk_wait_read<1>();
+                else bulk_wait_read<0>();
+                load_box(c + ahead);
+              }
+            }
+            tmem_wait_ld();
+            if (c == boxes - 1) release_tmem();
+            epilogue_bias_act(p, col0, r);
+            epilogue_bias_act(p, col0 + 32, s);
+            __syncwarp();
+            if (ex.ep_load) {
+              ok = __all_sync(0xffffffffu, mbar_wait(&my_full[k & slot_mask], (k >> phase_shift) & 1, wctx, ST_TIMEOUT_FULL));
+              if (!ok) break;
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                const uint4 a = oldc[c * 4 + j];
-                const float2 f0 = unpack_bf16x2(a.x), f1 = unpack_bf16x2(a.y), f2 = unpack_bf16x2(a.z), f3 = unpack_bf16x2(a.w);
-                uint4 o;
-                o.x = pack_bf16x2(__uint_as_float(r[j * 8 + 0]) + f0.x, __uint_as_float(r[j * 8 + 1]) + f0.y);
-                o.y = pack_bf16x2(__uint_as_float(r[j * 8 + 2]) + f1.x, __uint_as_float(r[j * 8 + 3]) + f1.y);
-                o.z = pack_bf16x2(__uint_as_float(r[j * 8 + 4]) + f2.x, __uint_as_float(r[j * 8 + 5]) + f2.y);
-                o.w = pack_bf16x2(__uint_as_float(r[j * 8 + 6]) + f3.x, __uint_as_float(r[j * 8 + 7]) + f3.y);
-                reinterpret_cast<uint4*>(crow)[c * 4 + j] = o;
+                add_bf16x8(r, 8 * j, ld_shared_v4(box + uint32_t((j ^ (lane & 7)) << 4)));
+                add_bf16x8(s, 8 * j, ld_shared_v4(box + uint32_t(((j + 4) ^ (lane & 7)) << 4)));
               }
-            } else if (row_ok) {
-              epilogue_store_chunk(p, ecfg, row, col0, r);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const uint4 a = pack_f32x8(r, 8 * j), b = pack_f32x8(s, 8 * j);
+              st_shared_v4(box + uint32_t((j ^ (lane & 7)) << 4), a.x, a.y, a.z, a.w);
+              st_shared_v4(box + uint32_t(((j + 4) ^ (lane & 7)) << 4), b.x, b.y, b.z, b.w);
             }
           }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            const void* src = my_boxes + (k & slot_mask) * Cfg::EP_BYTES;
+            if (zb_in_bounds(row0 >= 0 && row0 < p.M && col0 >= 0 && col0 < p.N, p.status, 2)) {
+              if (ex.ep == EP_F32 && ecfg.accum) tma_reduce_add_2d(&tmap_c, src, col0, row0);
+              else tma_store_2d(&tmap_c, src, col0, row0);
+            }
+            bulk_commit();
+          }
         }
+        ep_count += uint32_t(boxes);
+        if (!ok) break;
       } else {
       if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full[buf], use & 1, wctx, ST_TIMEOUT_TMEM_FULL))) break;
       tc_fence_after();
@@ -310,11 +404,12 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         if constexpr (SCATTER) epilogue_scatter_chunk(crow, col0, p.N, ecfg.vec_ok, r);
         else epilogue_store_chunk(p, ecfg, row, col0, r);
       }
-      }
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(&tmem_empty[buf], 0);
+      }
     }
+    if (lane == 0) bulk_wait_all();
     if constexpr (SCATTER) __threadfence_system();   // this thread's rows are visible to their owners before the flags
   }
 
@@ -411,12 +506,49 @@ static int make_tmap_mn3d(CUtensorMap* out, const void* base, uint64_t krows, ui
   return make_tmap_nd_bf16(out, base, 3, dims, strides, box);
 }
 
+// Tile order.  The operand of the band (the one with fewer tiles) is read from DRAM once per band and stays in L2 while
+// the other operand streams through once per band, so a band as wide as that dimension reads both operands once.  It
+// has to fit: with a band of more than BAND_BYTES (about a third of L2, each die keeps its own copy of what its SMs
+// read) every wave reads the band again, and then the narrower bands win whose waves are close to square (74 pairs:
+// 8 - 10 tiles).  The all-gather kernel keeps rows of B ascending, the order in which its chunks arrive.
+// Weight gradient 22016 x 4096 x 4096 (fp32 bucket): 826 us with rows fastest, which read dY^T once per 256 columns,
+// 674 us so.
+template <typename Params>
+static TileOrder gemm2_tile_order(int M, int N, int K) {
+  constexpr long BAND_BYTES = 40l << 20;
+  TileOrder o;
+  o.tiles_m = (M + Gemm2Cfg::BM - 1) / Gemm2Cfg::BM;
+  o.tiles_n = (N + Gemm2Cfg::BN - 1) / Gemm2Cfg::BN;
+  o.n_fast = !std::is_same<Params, GemmAgParams>::value && o.tiles_n < o.tiles_m;
+  const int nf = o.n_fast ? o.tiles_n : o.tiles_m;
+  o.band = nf;
+  if (!std::is_same<Params, GemmAgParams>::value && (nf > 16 || long(nf) * 256 * K * 2 > BAND_BYTES)) {
+    const int bands = (nf + 9) / 10;
+    o.band = (nf + bands - 1) / bands;
+  }
+  return o;
+}
+
 template <bool A_MN, bool B_MN, typename Params = GemmParams>
 static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, int ldb, int max_ctas,
                         cudaStream_t stream) {
   using Cfg = Gemm2Cfg;
   CUtensorMap ta, tb;
-  Gemm2Extra ex = {0, 0};
+  Gemm2Extra ex = {};
+  // TMA epilogue: 16-byte aligned rows, and at most one tensor to add to a bf16 output
+  CUtensorMap tc = {}, tx = {};
+  const bool f32 = (p.flags & GEMM_OUT_F32) != 0, acc = (p.flags & GEMM_ACCUMULATE) != 0, add = p.addend != nullptr;
+  auto rows_ok = [](const void* base, long ld_bytes) { return (reinterpret_cast<uintptr_t>(base) & 15) == 0 && ld_bytes % 16 == 0; };
+  if (std::is_same<Params, GemmParams>::value && rows_ok(p.C, long(p.ldc) * (f32 ? 4 : 2)) &&
+      !(f32 ? add : (add && acc)) && (!add || rows_ok(p.addend, long(p.ld_addend) * 2))) {
+    ex.ep = f32 ? EP_F32 : EP_BF16;
+    ex.ep_load = !f32 && (acc || add);
+    int rc_ep = make_tmap_2d_out(&tc, p.C, p.M, p.N, p.ldc, f32, 32);
+    if (rc_ep) return rc_ep;
+    if (add) rc_ep = make_tmap_2d_out(&tx, p.addend, p.M, p.N, p.ld_addend, false, 32);
+    else tx = tc;
+    if (rc_ep) return rc_ep;
+  }
   int rc;
   if (!A_MN) rc = make_tmap_2d_bf16(&ta, A, p.M, p.K, lda, 128, 64);
   else if (p.M % 64 == 0) { rc = make_tmap_mn3d(&ta, A, p.K, p.M, lda); ex.a_3d = 1; }
@@ -426,17 +558,23 @@ static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, 
   else if (p.N % 64 == 0) { rc = make_tmap_mn3d(&tb, B, p.K, p.N, ldb); ex.b_3d = 1; }
   else rc = make_tmap_2d_bf16(&tb, B, p.K, p.N, ldb, 64, 64);
   if (rc) return rc;
-  auto kern = gemm2_bf16_kernel<A_MN, B_MN, Params>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    ZB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
-    attr_set = true;
+  // five stages and four boxes where the tile's epilogue is not hidden by a long main loop (comment at Gemm2Cfg)
+  const bool short_k = std::is_same<Params, GemmParams>::value && ex.ep != EP_DIRECT && p.K < 2048;
+  auto kern = gemm2_bf16_kernel<A_MN, B_MN, Params, 6>;
+  if constexpr (std::is_same<Params, GemmParams>::value) {
+    if (short_k) kern = gemm2_bf16_kernel<A_MN, B_MN, Params, 5>;
   }
-  const int tiles = ((p.M + Cfg::BM - 1) / Cfg::BM) * ((p.N + Cfg::BN - 1) / Cfg::BN);
+  static bool attr_set[2] = {false, false};
+  if (!attr_set[short_k]) {
+    ZB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+    attr_set[short_k] = true;
+  }
+  ex.order = gemm2_tile_order<Params>(p.M, p.N, p.K);
+  const int tiles = ex.order.tiles_m * ex.order.tiles_n;
   int pairs = num_sms() / 2;
   if (max_ctas > 0 && max_ctas / 2 < pairs) pairs = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
   if (tiles < pairs) pairs = tiles;
-  kern<<<2 * pairs, std::is_same<Params, GemmAgParams>::value ? 320 : 192, Cfg::SMEM_BYTES, stream>>>(ta, tb, p, ex);
+  kern<<<2 * pairs, std::is_same<Params, GemmAgParams>::value ? 320 : 192, Cfg::SMEM_BYTES, stream>>>(ta, tb, tc, tx, p, ex);
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -499,32 +637,12 @@ extern "C" int zb_gemm2_rs_bf16(const void* A, const void* B, int M, int N, int 
   return launch_gemm2<false, false, GemmScatterParams>(A, B, p, lda, ldb, max_ctas, stream);
 }
 
-// C (bf16) += A @ B^T with the old C tile requested before the tile's accumulators are ready (candidate for the
-// weight-gradient GEMMs).  Same operand conventions as zb_gemm2_bf16; only bf16 accumulation without bias,
-// addend or activation takes the prefetching kernel, anything else is forwarded to zb_gemm2_bf16.
+// Another name of zb_gemm2_bf16: its epilogue requests the old C tile of a bf16 accumulation ahead of the accumulators.
 extern "C" int zb_gemm2_accpf_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
                                    int ldc, int a_mn_major, int b_mn_major, const void* bias, const void* addend,
                                    int ld_addend, int flags, int max_ctas, int* status, cudaStream_t stream) {
-  using namespace zb;
-  if (flags != GEMM_ACCUMULATE || bias != nullptr || addend != nullptr)
-    return zb_gemm2_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, bias, addend, ld_addend, flags,
-                         max_ctas, status, stream);
-  if (M <= 0 || N <= 0 || K <= 0) ZB_FAIL(-1, "gemm2: empty problem %d x %d x %d", M, N, K);
-  GemmAccPrefetchParams p;
-  p.C = C;
-  p.bias = nullptr; p.addend = nullptr;
-  p.M = M; p.N = N; p.K = K;
-  p.ldc = ldc; p.ld_addend = 0;
-  p.flags = flags;
-  p.status = status;
-  p.gate_flags = nullptr;
-  p.gate_epoch = 0;
-  p.gate_base = 0; p.gate_row_bytes = 0; p.gate_shard_bytes = 1;
-  p.gate_chunk_bytes = 1; p.gate_cps = 1; p.gate_self = -1;
-  if (!a_mn_major && !b_mn_major) return launch_gemm2<false, false, GemmAccPrefetchParams>(A, B, p, lda, ldb, max_ctas, stream);
-  if (!a_mn_major && b_mn_major) return launch_gemm2<false, true, GemmAccPrefetchParams>(A, B, p, lda, ldb, max_ctas, stream);
-  if (a_mn_major && b_mn_major) return launch_gemm2<true, true, GemmAccPrefetchParams>(A, B, p, lda, ldb, max_ctas, stream);
-  return launch_gemm2<true, false, GemmAccPrefetchParams>(A, B, p, lda, ldb, max_ctas, stream);
+  return zb_gemm2_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, bias, addend, ld_addend, flags, max_ctas,
+                       status, stream);
 }
 
 

@@ -69,15 +69,83 @@ struct GemmAgParams : GemmParams {
 };
 
 
-// Selects the kernels whose accumulate epilogue (C += result, bf16) reads the old C tile before the tile's
-// accumulators are ready, so that the read latency hides behind the main loop (weight gradients).
-struct GemmAccPrefetchParams : GemmParams {};
-
-
 __device__ __forceinline__ float gelu_tanh(float x) {
   const float k0 = 0.7978845608028654f, k1 = 0.044715f;
   float u = k0 * (x + k1 * x * x * x);
   return 0.5f * x * (1.f + tanhf(u));
+}
+
+
+// Order in which the output tiles are handed to the persistent CTA pairs: bands of `band` tiles of the dimension with
+// fewer tiles, walked fastest, while the other dimension advances; one band after the other.
+struct TileOrder {
+  int tiles_m, tiles_n, band;
+  bool n_fast;
+};
+__host__ __device__ __forceinline__ void tile_at(const TileOrder& o, int tile, int& tm, int& tn) {
+  const int nf = o.n_fast ? o.tiles_n : o.tiles_m, ns = o.n_fast ? o.tiles_m : o.tiles_n;
+  int b = 0, r = tile, w = o.band;
+  if (o.band < nf) {
+    b = tile / (o.band * ns);
+    r = tile - b * o.band * ns;
+    w = min(o.band, nf - b * o.band);   // the last band may be narrower
+  }
+  const int slow = r / w, fast = b * o.band + (r - slow * w);
+  tm = o.n_fast ? slow : fast;
+  tn = o.n_fast ? fast : slow;
+}
+
+
+// bias and activation on 32 accumulator columns [col0, col0 + 32) of one row
+__device__ __forceinline__ void epilogue_bias_act(const GemmParams& p, int col0, uint32_t (&r)[32]) {
+  if (p.bias != nullptr) {
+    if (col0 + 32 <= p.N && (reinterpret_cast<uintptr_t>(p.bias + col0) & 15) == 0) {
+      const uint4* bp = reinterpret_cast<const uint4*>(p.bias + col0);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint4 b = __ldg(bp + j);
+        const float2 f0 = unpack_bf16x2(b.x), f1 = unpack_bf16x2(b.y), f2 = unpack_bf16x2(b.z), f3 = unpack_bf16x2(b.w);
+        r[8 * j + 0] = __float_as_uint(__uint_as_float(r[8 * j + 0]) + f0.x);
+        r[8 * j + 1] = __float_as_uint(__uint_as_float(r[8 * j + 1]) + f0.y);
+        r[8 * j + 2] = __float_as_uint(__uint_as_float(r[8 * j + 2]) + f1.x);
+        r[8 * j + 3] = __float_as_uint(__uint_as_float(r[8 * j + 3]) + f1.y);
+        r[8 * j + 4] = __float_as_uint(__uint_as_float(r[8 * j + 4]) + f2.x);
+        r[8 * j + 5] = __float_as_uint(__uint_as_float(r[8 * j + 5]) + f2.y);
+        r[8 * j + 6] = __float_as_uint(__uint_as_float(r[8 * j + 6]) + f3.x);
+        r[8 * j + 7] = __float_as_uint(__uint_as_float(r[8 * j + 7]) + f3.y);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (col0 + i < p.N) r[i] = __float_as_uint(__uint_as_float(r[i]) + __bfloat162float(p.bias[col0 + i]));
+    }
+  }
+  if (p.flags & GEMM_GELU) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(gelu_tanh(__uint_as_float(r[i])));
+  } else if (p.flags & GEMM_RELU) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(fmaxf(__uint_as_float(r[i]), 0.f));
+  }
+}
+__device__ __forceinline__ void add_bf16x8(uint32_t (&r)[32], int i, const uint4& a) {
+  const float2 f0 = unpack_bf16x2(a.x), f1 = unpack_bf16x2(a.y), f2 = unpack_bf16x2(a.z), f3 = unpack_bf16x2(a.w);
+  r[i + 0] = __float_as_uint(__uint_as_float(r[i + 0]) + f0.x);
+  r[i + 1] = __float_as_uint(__uint_as_float(r[i + 1]) + f0.y);
+  r[i + 2] = __float_as_uint(__uint_as_float(r[i + 2]) + f1.x);
+  r[i + 3] = __float_as_uint(__uint_as_float(r[i + 3]) + f1.y);
+  r[i + 4] = __float_as_uint(__uint_as_float(r[i + 4]) + f2.x);
+  r[i + 5] = __float_as_uint(__uint_as_float(r[i + 5]) + f2.y);
+  r[i + 6] = __float_as_uint(__uint_as_float(r[i + 6]) + f3.x);
+  r[i + 7] = __float_as_uint(__uint_as_float(r[i + 7]) + f3.y);
+}
+__device__ __forceinline__ uint4 pack_f32x8(const uint32_t (&r)[32], int i) {
+  uint4 o;
+  o.x = pack_bf16x2(__uint_as_float(r[i + 0]), __uint_as_float(r[i + 1]));
+  o.y = pack_bf16x2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+  o.z = pack_bf16x2(__uint_as_float(r[i + 4]), __uint_as_float(r[i + 5]));
+  o.w = pack_bf16x2(__uint_as_float(r[i + 6]), __uint_as_float(r[i + 7]));
+  return o;
 }
 
 
