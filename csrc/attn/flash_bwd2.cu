@@ -76,13 +76,16 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   uint8_t* sDS = sDO + QS * Cfg::TILE_BYTES;          // dS^T: [128 keys][128 queries], two 64-query blocks
   uint64_t* bars = reinterpret_cast<uint64_t*>(sDS + Cfg::DS_BYTES);
   uint64_t* kv_full = bars;             // 1
-  uint64_t* qdo_full = bars + 1;        // QS
-  uint64_t* qdo_empty = qdo_full + QS;  // QS
-  uint64_t* s_full = qdo_empty + QS;    // 1
+  uint64_t* q_full = bars + 1;          // QS
+  uint64_t* q_empty = q_full + QS;      // QS
+  uint64_t* do_full = q_empty + QS;     // QS
+  uint64_t* do_empty = do_full + QS;    // QS
+  uint64_t* s_full = do_empty + QS;     // 1
   uint64_t* dp_full = s_full + 1;       // 1
   uint64_t* pds_full = dp_full + 1;     // 1 (8 arrivals)
   uint64_t* dq_full = pds_full + 1;     // 1
   uint64_t* dq_empty = dq_full + 1;     // 1 (8 arrivals)
+  uint64_t* p_full = dq_empty;          // without the dQ part: P^T is in tensor memory
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dq_empty + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -116,8 +119,10 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     *abort_flag = 0;
     mbar_init(kv_full, 1);
     for (int i = 0; i < QS; ++i) {
-      mbar_init(&qdo_full[i], 1);
-      mbar_init(&qdo_empty[i], 1);
+      mbar_init(&q_full[i], 1);
+      mbar_init(&q_empty[i], 1);
+      mbar_init(&do_full[i], 1);
+      mbar_init(&do_empty[i], 1);
     }
     mbar_init(s_full, 1);
     mbar_init(dp_full, 1);
@@ -156,27 +161,45 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         const int head = kv_head * rep + it / per_head;
         const int q0 = (i_lo + it % per_head) * BM;
         if (!zb_in_bounds(q0 >= 0 && q0 < p.S && head < p.Hq && kv0 < p.S, p.status, 8)) break;
-        if (!mbar_wait(&qdo_empty[st], ph ^ 1, wctx, ST_TIMEOUT_EMPTY)) break;
-        tr(TB_TMA_STAGE_FREE);
-        mbar_expect_tx(&qdo_full[st], 2 * Cfg::TILE_BYTES + (DQ ? 0 : 1024));
+        // Q and dO have their own barriers: dO_i is free once dV_i is done, Q_i only after dK_i, more than half a step
+        // later, and the first S^T needs Q alone
+        auto load_q = [&]() -> bool {
+          if (!mbar_wait(&q_empty[st], ph ^ 1, wctx, ST_TIMEOUT_EMPTY)) return false;
+          tr(TB_TMA_STAGE_FREE);
+          mbar_expect_tx(&q_full[st], Cfg::TILE_BYTES + (DQ ? 0 : 1024));
 #pragma unroll
-        for (int b = 0; b < DB; ++b) {
-          tma_load_4d(sQ + st * Cfg::TILE_BYTES + b * BLK, &tmap_q, &qdo_full[st], b * 64, head, q0, batch);
-          tma_load_4d(sDO + st * Cfg::TILE_BYTES + b * BLK, &tmap_do, &qdo_full[st], b * 64, head, q0, batch);
-        }
-        if constexpr (!DQ) {
-          // lse (log2 units) and delta of the tile's 128 queries: 512 bytes each, next to the stage they belong to
-          // (rows of the statistics buffer are padded to a multiple of 128 entries, q0 is a multiple of 128)
-          const float* row = stats + (size_t(batch) * p.Hq + head) * 2 * size_t(s_pad) + q0;
-          bulk_load_1d(sDS + st * 1024, row, 512, &qdo_full[st]);
-          bulk_load_1d(sDS + st * 1024 + 512, row + s_pad, 512, &qdo_full[st]);
-        }
+          for (int b = 0; b < DB; ++b)
+            tma_load_4d(sQ + st * Cfg::TILE_BYTES + b * BLK, &tmap_q, &q_full[st], b * 64, head, q0, batch);
+          if constexpr (!DQ) {
+            // -lse (log2 units) and -delta of the tile's 128 queries: 512 bytes each, freed with Q_i, that is after
+            // every compute warp has formed dS_i (rows of the statistics buffer are padded to a multiple of 128
+            // entries, q0 is a multiple of 128)
+            const float* row = stats + (size_t(batch) * p.Hq + head) * 2 * size_t(s_pad) + q0;
+            bulk_load_1d(sDS + st * 1024, row, 512, &q_full[st]);
+            bulk_load_1d(sDS + st * 1024 + 512, row + s_pad, 512, &q_full[st]);
+          }
+          return true;
+        };
+        auto load_do = [&]() -> bool {
+          if (!mbar_wait(&do_empty[st], ph ^ 1, wctx, ST_TIMEOUT_EMPTY)) return false;
+          mbar_expect_tx(&do_full[st], Cfg::TILE_BYTES);
+#pragma unroll
+          for (int b = 0; b < DB; ++b)
+            tma_load_4d(sDO + st * Cfg::TILE_BYTES + b * BLK, &tmap_do, &do_full[st], b * 64, head, q0, batch);
+          return true;
+        };
+        if (it < QS ? !(load_q() && load_do()) : !(load_do() && load_q())) break;
         tr(TB_TMA_ISSUED);
       }
     }
   } else if (warp == 9) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0 && n_iters > 0) {
+    // The whole warp walks the loop, one elected lane issues (operands stay in uniform registers).  With that, P^T
+    // announced ahead of dS^T and fp32 P in registers the dK / dV kernel takes, for 4096 tokens, 32 heads, d = 128,
+    // 294 instead of 388 us, and for 2048 tokens, 32 / 8 heads, d = 64, 126 instead of 179 us (clocks per step of the
+    // first: 1460 exponentials, 630 dS^T, 1020 waiting for S^T and dP^T; the tensor pipe is busy for about 2260 of 3110).
+    if (n_iters > 0) {
+      const bool elected = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, false, false);  // K-major A and B
       constexpr uint32_t idesc_dkv = umma_idesc_bf16(128, D, false, true);   // A from TMEM, B = [q rows][d] (N-major)
       // D = 128: A = K (M = head dim, M-major), B = dS^T tile (N = queries, N-major); D = 64: A = dS^T tile, B = K
@@ -185,6 +208,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const uint32_t r_s = tmem_base, r_dp = tmem_base + Cfg::DP_COL;
       bool ok = mbar_wait(kv_full, 0, wctx, ST_TIMEOUT_FULL);
       auto issue_a = [&](uint32_t q_addr) {  // S^T = K Q^T
+        if (!elected) return;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t off = uint32_t(kk / 4) * BLK + uint32_t(kk % 4) * 32;
@@ -193,6 +217,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         umma_commit(s_full);
       };
       auto issue_b = [&](uint32_t do_addr) {  // dP^T = V dO^T
+        if (!elected) return;
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t off = uint32_t(kk / 4) * BLK + uint32_t(kk % 4) * 32;
@@ -200,51 +225,66 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         }
         umma_commit(dp_full);
       };
-      if (ok) ok = mbar_wait(&qdo_full[0], 0, wctx, ST_TIMEOUT_FULL);
+      if (ok) ok = mbar_wait(&q_full[0], 0, wctx, ST_TIMEOUT_FULL);
       if (ok) {
         tc_fence_after();
         issue_a(smem_u32(sQ));
+        ok = mbar_wait(&do_full[0], 0, wctx, ST_TIMEOUT_FULL);
+      }
+      if (ok) {
+        tc_fence_after();
         issue_b(smem_u32(sDO));
         tr(TB_MMA_B_ISSUED);
       }
       for (int it = 0; it < n_iters && ok; ++it) {
         const int st = it % QS;
         const uint32_t q_addr = smem_u32(sQ + st * Cfg::TILE_BYTES), do_addr = smem_u32(sDO + st * Cfg::TILE_BYTES);
-        if (!mbar_wait(pds_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_MISC)) break;
-        tr(TB_MMA_PDS_READY);
+        if (!mbar_wait(DQ ? pds_full : p_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_MISC)) break;
+        if (DQ) tr(TB_MMA_PDS_READY);
         tc_fence_after();
         // D: dV += P^T dO, E: dK += dS^T Q  (reduction over the 128 queries; bf16 A operands sit in the
         // first 32 columns of each 64-column half of R_S / R_dP)
+        if (elected) {
 #pragma unroll
-        for (int kk = 0; kk < BM / 16; ++kk) {
-          const uint32_t acol = uint32_t(kk / 4) * 64 + uint32_t(kk % 4) * 8;
-          umma_f16_ts(tmem_base + Cfg::DV_COL, r_s + acol, umma_desc_mnmajor(do_addr + kk * 2048, BLK), idesc_dkv,
-                      (it | kk) != 0 ? 1u : 0u);
+          for (int kk = 0; kk < BM / 16; ++kk) {
+            const uint32_t acol = uint32_t(kk / 4) * 64 + uint32_t(kk % 4) * 8;
+            umma_f16_ts(tmem_base + Cfg::DV_COL, r_s + acol, umma_desc_mnmajor(do_addr + kk * 2048, BLK), idesc_dkv,
+                        (it | kk) != 0 ? 1u : 0u);
+          }
+          umma_commit(&do_empty[st]);     // B_i and D_i are dO_i's readers
         }
         if constexpr (!DQ) {
-          // S^T of the next step right behind D (which was P^T's last reader), ahead of E: the next step's
-          // exponentials then start 8 products earlier, while E and B are still running
+          // D needs P^T only, and S^T of the next step goes right behind it (D was P^T's last reader): both run while
+          // the compute warps form dS^T, and the next step's exponentials run under E and B
           if (it + 1 < n_iters) {
             const int sn = (it + 1) % QS;
-            if (!mbar_wait(&qdo_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
+            if (!mbar_wait(&q_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
             tr(TB_MMA_QDO_READY);
             tc_fence_after();
             issue_a(smem_u32(sQ + sn * Cfg::TILE_BYTES));
             tr(TB_MMA_A_ISSUED);
           }
+          if (!mbar_wait(pds_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_MISC)) break;
+          tr(TB_MMA_PDS_READY);
+          tc_fence_after();
         }
+        if (elected) {
 #pragma unroll
-        for (int kk = 0; kk < BM / 16; ++kk) {
-          const uint32_t acol = uint32_t(kk / 4) * 64 + uint32_t(kk % 4) * 8;
-          umma_f16_ts(tmem_base + Cfg::DK_COL, r_dp + acol, umma_desc_mnmajor(q_addr + kk * 2048, BLK), idesc_dkv,
-                      (it | kk) != 0 ? 1u : 0u);
+          for (int kk = 0; kk < BM / 16; ++kk) {
+            const uint32_t acol = uint32_t(kk / 4) * 64 + uint32_t(kk % 4) * 8;
+            umma_f16_ts(tmem_base + Cfg::DK_COL, r_dp + acol, umma_desc_mnmajor(q_addr + kk * 2048, BLK), idesc_dkv,
+                        (it | kk) != 0 ? 1u : 0u);
+          }
+          umma_commit(&q_empty[st]);
         }
-        umma_commit(&qdo_empty[st]);
         if constexpr (!DQ) {
-          if (it + 1 == n_iters) umma_commit(dq_full);   // every dK / dV product is done: the write-out may start
+          if (it + 1 == n_iters && elected) umma_commit(dq_full);   // every dK / dV product is done: the write-out may start
           tr(TB_MMA_DEF_ISSUED);
           if (it + 1 < n_iters) {
-            issue_b(smem_u32(sDO + ((it + 1) % QS) * Cfg::TILE_BYTES));   // overwrites R_dP behind E, its last reader
+            const int sn = (it + 1) % QS;
+            if (!mbar_wait(&do_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
+            tc_fence_after();
+            issue_b(smem_u32(sDO + sn * Cfg::TILE_BYTES));   // overwrites R_dP behind E, its last reader
             tr(TB_MMA_B_ISSUED);
           }
           continue;
@@ -254,21 +294,24 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         // For D = 128 the product is formed transposed, dQ^T = K^T dS^T (same two shared-memory tiles with
         // the operand roles swapped): head-dim index on the TMEM lanes, so that the 32 lanes of a warp add
         // to 32 consecutive floats of one query row (one full 128-byte line per instruction) in G.
+        if (elected) {
 #pragma unroll
-        for (int kk = 0; kk < BN / 16; ++kk) {
-          if constexpr (D == 128)
-            umma_f16_ss(r_dp, umma_desc_mnmajor(k_addr + kk * 2048, BLK), umma_desc_mnmajor(ds_addr + kk * 2048, BLK),
-                        idesc_dq, kk != 0 ? 1u : 0u);
-          else
-            umma_f16_ss(r_dp, umma_desc_mnmajor(ds_addr + kk * 2048, BLK), umma_desc_mnmajor(k_addr + kk * 2048, BLK),
-                        idesc_dq, kk != 0 ? 1u : 0u);
+          for (int kk = 0; kk < BN / 16; ++kk) {
+            if constexpr (D == 128)
+              umma_f16_ss(r_dp, umma_desc_mnmajor(k_addr + kk * 2048, BLK), umma_desc_mnmajor(ds_addr + kk * 2048, BLK),
+                          idesc_dq, kk != 0 ? 1u : 0u);
+            else
+              umma_f16_ss(r_dp, umma_desc_mnmajor(ds_addr + kk * 2048, BLK), umma_desc_mnmajor(k_addr + kk * 2048, BLK),
+                          idesc_dq, kk != 0 ? 1u : 0u);
+          }
+          umma_commit(dq_full);
         }
-        umma_commit(dq_full);
         }
         tr(TB_MMA_DEF_ISSUED);
         if (it + 1 < n_iters) {
           const int sn = (it + 1) % QS;
-          if (!mbar_wait(&qdo_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
+          if (!mbar_wait(&q_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
+          if (!mbar_wait(&do_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
           tr(TB_MMA_QDO_READY);
           tc_fence_after();
           issue_a(smem_u32(sQ + sn * Cfg::TILE_BYTES));
@@ -298,14 +341,12 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const int q0 = (i_lo + it % per_head) * BM;
       const int qc0 = q0 + half * 64;            // first query column of this thread
       // statistics of the tile's queries: global rows indexed by the absolute query (one-kernel form), or the
-      // copy the producer placed in shared memory with the stage, indexed from the tile's first query
+      // copy the producer placed in shared memory with the stage
       const float* lse_q = stats + (size_t(batch) * p.Hq + head) * 2 * size_t(s_pad);
       const float* delta_q = lse_q + s_pad;
+      const uint32_t nlse_s = smem_u32(sDS + (it % QS) * 1024 + half * 256), ndelta_s = nlse_s + 512;
       if constexpr (!DQ) {
-        const int st = it % QS;
-        if (!__all_sync(0xffffffffu, mbar_wait(&qdo_full[st], uint32_t(it / QS) & 1, wctx, ST_TIMEOUT_FULL))) { ok = false; break; }
-        lse_q = reinterpret_cast<const float*>(sDS + st * 1024) - q0;
-        delta_q = reinterpret_cast<const float*>(sDS + st * 1024 + 512) - q0;
+        if (!__all_sync(0xffffffffu, mbar_wait(&q_full[it % QS], uint32_t(it / QS) & 1, wctx, ST_TIMEOUT_FULL))) { ok = false; break; }
       }
       const bool need_mask = (p.causal && kv0 + BN - 1 > q0) || (p.window > 0 && kv0 < q0 + BM - p.window) ||
                              (kv0 + BN > p.S) || (q0 + BM > p.S);
@@ -313,10 +354,84 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       if (!__all_sync(0xffffffffu, mbar_wait(s_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_TMEM_FULL))) { ok = false; break; }
       tr(TB_S_READY);
       tc_fence_after();
-      // lse_q (already in log2 units) and delta_q are the same for every lane: 16-byte loads from the
+      // queries of this half that this thread's key is seen by: columns [vis_lo, vis_lo + vis_n)
+      const int vis_lo = p.causal ? max(key - qc0, 0) : 0;
+      const int vis_hi = min((p.window > 0 ? min(key + p.window, p.S) : p.S) - qc0, 64);
+      const uint32_t vis_n = key_ok ? uint32_t(max(vis_hi - vis_lo, 0)) : 0u;
+      if constexpr (!DQ) {
+        // P stays in fp32 registers between its two uses; two-wide fp32 math; the softmax scale of dS is applied to
+        // dK once, when it is written out
+        float pr[64];
+        {
+          uint32_t rs0[32], rs1[32];
+          tmem_ld32(lane_addr + uint32_t(half * 64), rs0);
+          tmem_ld32(lane_addr + uint32_t(half * 64 + 32), rs1);
+          tmem_wait_ld();
+#pragma unroll
+          for (int k = 0; k < 64; k += 4) {
+            const float4 l = ld_shared_f4(nlse_s + k * 4);
+            const uint32_t* rs = k < 32 ? &rs0[k] : &rs1[k - 32];
+            float x0, x1, x2, x3;
+            ffma2(x0, x1, __uint_as_float(rs[0]), __uint_as_float(rs[1]), p.scale_log2, p.scale_log2, l.x, l.y);
+            ffma2(x2, x3, __uint_as_float(rs[2]), __uint_as_float(rs[3]), p.scale_log2, p.scale_log2, l.z, l.w);
+            pr[k] = exp2f(x0); pr[k + 1] = exp2f(x1); pr[k + 2] = exp2f(x2); pr[k + 3] = exp2f(x3);
+          }
+        }
+        if (need_mask) {
+#pragma unroll
+          for (int k = 0; k < 64; ++k) pr[k] = uint32_t(k - vis_lo) < vis_n ? pr[k] : 0.f;
+        }
+        {
+          uint32_t lo16[16], hi16[16];
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            lo16[k] = pack_bf16x2(pr[2 * k], pr[2 * k + 1]);
+            hi16[k] = pack_bf16x2(pr[32 + 2 * k], pr[33 + 2 * k]);
+          }
+          tmem_st16(lane_addr + uint32_t(half * 64), lo16);
+          tmem_st16(lane_addr + uint32_t(half * 64 + 16), hi16);
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+        tr(TB_P_DONE);
+        if (!__all_sync(0xffffffffu, mbar_wait(dp_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_TMEM_FULL))) { ok = false; break; }
+        tr(TB_DP_READY);
+        tc_fence_after();
+        {
+          uint32_t rd0[32], rd1[32];
+          tmem_ld32(lane_addr + uint32_t(Cfg::DP_COL + half * 64), rd0);
+          tmem_ld32(lane_addr + uint32_t(Cfg::DP_COL + half * 64 + 32), rd1);
+          tmem_wait_ld();
+          uint32_t ds0[16], ds1[16];
+#pragma unroll
+          for (int k = 0; k < 64; k += 4) {
+            const float4 d = ld_shared_f4(ndelta_s + k * 4);
+            const uint32_t* rd = k < 32 ? &rd0[k] : &rd1[k - 32];
+            uint32_t* ds = k < 32 ? &ds0[k >> 1] : &ds1[(k - 32) >> 1];
+            float x0, x1, x2, x3;
+            fadd2(x0, x1, __uint_as_float(rd[0]), __uint_as_float(rd[1]), d.x, d.y);
+            fadd2(x2, x3, __uint_as_float(rd[2]), __uint_as_float(rd[3]), d.z, d.w);
+            fmul2(x0, x1, x0, x1, pr[k], pr[k + 1]);
+            fmul2(x2, x3, x2, x3, pr[k + 2], pr[k + 3]);
+            ds[0] = pack_bf16x2(x0, x1);
+            ds[1] = pack_bf16x2(x2, x3);
+          }
+          // the other half's threads read their own 64 columns only, so the packed values may cover this half's first 32
+          tmem_st16(lane_addr + uint32_t(Cfg::DP_COL + half * 64), ds0);
+          tmem_st16(lane_addr + uint32_t(Cfg::DP_COL + half * 64 + 16), ds1);
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(pds_full);
+        tr(TB_DS_DONE);
+      } else {
+      // -lse_q (in log2 units) and -delta_q are the same for every lane: 16-byte loads from the
       // padded statistics rows
       auto load4 = [&](const float* base, int q, float (&v)[4]) {
-        const float4 a = DQ ? __ldg(reinterpret_cast<const float4*>(base + q)) : *reinterpret_cast<const float4*>(base + q);
+        const float4 a = __ldg(reinterpret_cast<const float4*>(base + q));
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
       };
       uint32_t pp[32];
@@ -325,7 +440,6 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         uint32_t rs[32];
         tmem_ld32(lane_addr + uint32_t(half * 64 + c * 32), rs);
         tmem_wait_ld();
-#pragma unroll
         // the mask test is hoisted out of the element loop: one branch per chunk, not one per element
         if (need_mask) {
 #pragma unroll
@@ -334,10 +448,8 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
             load4(lse_q, qc0 + c * 32 + k, l4);
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-              const int q = qc0 + c * 32 + k + u;
-              const float pe = exp2f(fmaf(__uint_as_float(rs[k + u]), p.scale_log2, -l4[u]));
-              const bool vis = key_ok && (q < p.S) && (!p.causal || key <= q) && (p.window <= 0 || q - key < p.window);
-              e[u] = vis ? pe : 0.f;
+              const float pe = exp2f(fmaf(__uint_as_float(rs[k + u]), p.scale_log2, l4[u]));
+              e[u] = uint32_t(c * 32 + k + u - vis_lo) < vis_n ? pe : 0.f;
             }
             pp[c * 16 + (k >> 1)] = pack_bf16x2(e[0], e[1]);
             pp[c * 16 + (k >> 1) + 1] = pack_bf16x2(e[2], e[3]);
@@ -348,7 +460,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
             float l4[4], e[4];
             load4(lse_q, qc0 + c * 32 + k, l4);
 #pragma unroll
-            for (int u = 0; u < 4; ++u) e[u] = exp2f(fmaf(__uint_as_float(rs[k + u]), p.scale_log2, -l4[u]));
+            for (int u = 0; u < 4; ++u) e[u] = exp2f(fmaf(__uint_as_float(rs[k + u]), p.scale_log2, l4[u]));
             pp[c * 16 + (k >> 1)] = pack_bf16x2(e[0], e[1]);
             pp[c * 16 + (k >> 1) + 1] = pack_bf16x2(e[2], e[3]);
           }
@@ -377,32 +489,29 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           float d4[4];
           load4(delta_q, qc0 + c * 32 + k, d4);
           const float2 pa = unpack_bf16x2(pp[c * 16 + (k >> 1)]), pb = unpack_bf16x2(pp[c * 16 + (k >> 1) + 1]);
-          const float s0 = pa.x * (__uint_as_float(rd[k]) - d4[0]) * p.scale;
-          const float s1 = pa.y * (__uint_as_float(rd[k + 1]) - d4[1]) * p.scale;
-          const float s2 = pb.x * (__uint_as_float(rd[k + 2]) - d4[2]) * p.scale;
-          const float s3 = pb.y * (__uint_as_float(rd[k + 3]) - d4[3]) * p.scale;
+          const float s0 = pa.x * (__uint_as_float(rd[k]) + d4[0]) * p.scale;
+          const float s1 = pa.y * (__uint_as_float(rd[k + 1]) + d4[1]) * p.scale;
+          const float s2 = pb.x * (__uint_as_float(rd[k + 2]) + d4[2]) * p.scale;
+          const float s3 = pb.y * (__uint_as_float(rd[k + 3]) + d4[3]) * p.scale;
           ds[k >> 1] = pack_bf16x2(s0, s1);
           ds[(k >> 1) + 1] = pack_bf16x2(s2, s3);
         }
         // the other half's threads read columns [64 h', 64 h' + 64) only, so writing the packed
         // values over this half's own first 32 columns cannot disturb them
         tmem_st16(lane_addr + uint32_t(Cfg::DP_COL + half * 64 + c * 16), ds);
-        if constexpr (DQ) {
 #pragma unroll
         for (int v4 = 0; v4 < 4; ++v4) {
           const int ch = c * 4 + v4;  // 16-byte chunk (8 queries) within the 128-byte row
           uint4 u = make_uint4(ds[v4 * 4 + 0], ds[v4 * 4 + 1], ds[v4 * 4 + 2], ds[v4 * 4 + 3]);
           *reinterpret_cast<uint4*>(ds_row + ((ch ^ (t & 7)) << 4)) = u;
         }
-        }
       }
       tmem_wait_st();
-      if constexpr (DQ) fence_proxy_async_smem();
+      fence_proxy_async_smem();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(pds_full);
       tr(TB_DS_DONE);
-      if constexpr (DQ) {
       // ---- G: dQ tile (lanes = query rows now) -> global fp32 accumulator ----
       if (!__all_sync(0xffffffffu, mbar_wait(dq_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_TMEM_FULL))) { ok = false; break; }
       tr(TB_DQ_READY);
@@ -455,6 +564,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll 1
     for (int which = 0; which < 2; ++which) {
       const uint32_t col0 = which == 0 ? Cfg::DK_COL : Cfg::DV_COL;
+      const float mul = !DQ && which == 0 ? p.scale : 1.f;   // the two-kernel form leaves dS unscaled
       __nv_bfloat16* dst = p.dqkv + (size_t(batch) * p.S + key) * width +
                            size_t(which == 0 ? (p.Hq + kv_head) : (p.Hq + p.Hkv + kv_head)) * D;
 #pragma unroll 1
@@ -468,6 +578,8 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           for (int k = 0; k < 32; ++k) r[k] = 0u;
         }
         if (ok && key_ok) {
+#pragma unroll
+          for (int k = 0; k < 32; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * mul);
 #pragma unroll
           for (int v4 = 0; v4 < 4; ++v4) {
             uint4 u;
@@ -494,7 +606,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   }
 }
 
-// stats[(b, h)][0][s] = lse * log2(e), stats[(b, h)][1][s] = sum_d dO * O; rows padded to s_pad
+// stats[(b, h)][0][s] = -lse * log2(e), stats[(b, h)][1][s] = -sum_d dO * O; rows padded to s_pad
 // entries that this kernel never writes (they must have been zeroed once). One warp per (token, head).
 __global__ void attn_bwd2_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                                        const float* __restrict__ lse, float* __restrict__ stats, int B, int S, int Hq,
@@ -518,8 +630,8 @@ __global__ void attn_bwd2_stats_kernel(const __nv_bfloat16* __restrict__ o, cons
   if (lane == 0) {
     const long b = tok / S, s = tok % S;
     float* row = stats + (b * Hq + h) * 2 * long(s_pad);
-    row[s] = lse[(b * Hq + h) * S + s] * 1.4426950408889634f;
-    row[s_pad + s] = acc;
+    row[s] = lse[(b * Hq + h) * S + s] * -1.4426950408889634f;
+    row[s_pad + s] = -acc;
   }
 }
 
