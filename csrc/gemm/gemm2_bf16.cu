@@ -1,4 +1,4 @@
-// bf16 GEMM on CTA pairs: tcgen05.mma.cta_group::2 with a 256 x 256 output tile per pair.
+// bf16 GEMM on CTA pairs: tcgen05.mma.cta_group::2 with a 256 x 256 (or 256 x 128) output tile per pair.
 //
 // Two CTAs of a cluster (2,1,1) share one tile: each holds 128 rows of A and of the fp32
 // accumulators (its own tensor memory) and loads HALF of the B tile (128 of the 256 rows);
@@ -85,22 +85,26 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
       : "memory");
 }
 
+// BN_: columns of a pair's tile, 256 or 128; each CTA loads half of them as rows of B.
+template <int BN_>
 struct Gemm2Cfg {
   static constexpr int BM = 256;   // per pair; 128 per CTA
-  static constexpr int BN = 256;   // per pair; each CTA loads 128 rows of B
+  static constexpr int BN = BN_;
   static constexpr int BK = 64;
   static constexpr int A_BYTES = 128 * BK * 2;
-  static constexpr int B_BYTES = 128 * BK * 2;
+  static constexpr int B_BYTES = BN / 2 * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int TMEM_COLS = 512;
+  static constexpr int TMEM_COLS = 2 * BN;
   static constexpr int EP_BYTES = 32 * 128;    // epilogue box: 32 rows x 128 bytes
   // Shared memory is split at launch: 6 operand stages and 2 epilogue boxes per epilogue warp, or 5 and 4.  The sixth
   // stage is worth 3 - 5 % of the main loop (4096 x 22016 x 4096: 486 -> 472 us), two more boxes shorten the epilogue
   // of a tile whose old C tile has to be read (load, add, store in flight at once).  The epilogue of a tile runs under
   // the main loop of the next one, so the boxes only count where that loop is short: K < 2048.
-  static constexpr int MAX_STAGES = 6, MAX_EP_BUFS = 4;
-  static constexpr int RING_BYTES = 6 * STAGE_BYTES + 4 * 2 * EP_BYTES;
-  static_assert(RING_BYTES == 5 * STAGE_BYTES + 4 * 4 * EP_BYTES, "both splits fill the same space");
+  // Tiles of 128 columns have stages of 24 KB instead of 32: 8 and 2, or 6 and 4.
+  static constexpr int MAX_STAGES = 8, MAX_EP_BUFS = 4;
+  static constexpr int STAGES_2 = BN == 256 ? 6 : 8, STAGES_4 = BN == 256 ? 5 : 6;   // with 2 / with 4 boxes
+  static constexpr int RING_BYTES = STAGES_2 * STAGE_BYTES + 4 * 2 * EP_BYTES;
+  static_assert(STAGES_4 * STAGE_BYTES + 4 * 4 * EP_BYTES <= RING_BYTES, "both splits fit the same space");
   static constexpr int SMEM_BYTES = RING_BYTES + 1024 + 512;
 };
 
@@ -117,7 +121,7 @@ struct Gemm2Extra {
   TileOrder order;
   int ep;          // EP_*
   int ep_load;     // EP_BF16: add the tensor behind tmap_x (old C or addend)
-  int a_3d, b_3d;  // MN-major operand fetched with one 3-D TMA box {64, BK, 2} instead of two 2-D boxes
+  int a_3d, b_3d;  // MN-major operand fetched with one 3-D TMA box {64, BK, 64-column blocks} instead of 2-D boxes
 };
 
 // SCATTER: the epilogue sends every output row to the staging slot of the rank that owns it in a
@@ -126,16 +130,16 @@ struct Gemm2Extra {
 // FUSED_AG (Params = GemmAgParams): four more warps per CTA pull the peers' parameter shards into the local
 // unsharded buffer while the tiles whose B rows are already present run; each CTA's producer waits for the
 // chunks that cover its own 128 rows of B.
-template <bool A_MN, bool B_MN, typename Params, int STAGES>
+template <bool A_MN, bool B_MN, typename Params, int BN, int EP_BUFS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(std::is_same<Params, GemmAgParams>::value ? 320 : 192, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_x, const Params p,
                   const Gemm2Extra ex) {
-  using Cfg = Gemm2Cfg;
+  using Cfg = Gemm2Cfg<BN>;
   constexpr bool SCATTER = std::is_same<Params, GemmScatterParams>::value;
   constexpr bool FUSED_AG = std::is_same<Params, GemmAgParams>::value;
-  constexpr int BK = Cfg::BK, MAXS = Cfg::MAX_STAGES, BN = Cfg::BN;
-  constexpr int EP_BUFS = STAGES == 6 ? 2 : 4;
+  constexpr int BK = Cfg::BK, MAXS = Cfg::MAX_STAGES, HALF_N = BN / 2;
+  constexpr int STAGES = EP_BUFS == 2 ? Cfg::STAGES_2 : Cfg::STAGES_4;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sE = smem + STAGES * Cfg::STAGE_BYTES;   // epilogue boxes, EP_BUFS per epilogue warp
@@ -193,14 +197,14 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         int tm, tn;
         tile_at(ex.order, tile, tm, tn);
         const int m0 = tm * Cfg::BM + int(cta) * 128;
-        const int n0 = tn * BN + int(cta) * 128;
+        const int n0 = tn * BN + int(cta) * HALF_N;
         // (the second CTA's half may start past the edge of a ragged tile: its loads then read the fill value)
-        if (!zb_in_bounds(m0 - int(cta) * 128 < p.M && n0 - int(cta) * 128 < p.N && tile >= 0, p.status, 1)) break;
+        if (!zb_in_bounds(m0 - int(cta) * 128 < p.M && n0 - int(cta) * HALF_N < p.N && tile >= 0, p.status, 1)) break;
         if constexpr (FUSED_AG) {
           if (p.gate_flags != nullptr && n0 < p.N) {
-            // rows [n0, n0 + 128) of B inside the flat buffer: wait for every chunk of a peer's shard they touch
+            // rows [n0, n0 + HALF_N) of B inside the flat buffer: wait for every chunk of a peer's shard they touch
             const long b0 = p.gate_base + long(n0) * p.gate_row_bytes;
-            const long b1 = p.gate_base + long(min(n0 + 128, p.N)) * p.gate_row_bytes - 1;
+            const long b1 = p.gate_base + long(min(n0 + HALF_N, p.N)) * p.gate_row_bytes - 1;
             const long i0 = (b0 / p.gate_shard_bytes) * p.gate_cps + (b0 % p.gate_shard_bytes) / p.gate_chunk_bytes;
             const long i1 = (b1 / p.gate_shard_bytes) * p.gate_cps + (b1 % p.gate_shard_bytes) / p.gate_chunk_bytes;
             for (long c = i0; c <= i1 && ok; ++c) {
@@ -230,8 +234,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             } else if (ex.b_3d) {
               tma_load_3d_pair(sb, &tmap_b, &full[stage], 0, kb * BK, n0 >> 6);
             } else {
-              tma_load_2d_pair(sb, &tmap_b, &full[stage], n0, kb * BK);
-              tma_load_2d_pair(sb + BK * 128, &tmap_b, &full[stage], n0 + 64, kb * BK);
+#pragma unroll
+              for (int j = 0; j < HALF_N / 64; ++j)
+                tma_load_2d_pair(sb + j * BK * 128, &tmap_b, &full[stage], n0 + j * 64, kb * BK);
             }
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -499,10 +504,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
 }
 
 // 3-D view of an MN-major operand stored [K rows, MN cols]: {64 within a block, K, MN/64 blocks}
-static int make_tmap_mn3d(CUtensorMap* out, const void* base, uint64_t krows, uint64_t mn, uint64_t ld) {
+static int make_tmap_mn3d(CUtensorMap* out, const void* base, uint64_t krows, uint64_t mn, uint64_t ld, uint32_t blocks) {
   uint64_t dims[3] = {64, krows, mn / 64};
   uint64_t strides[2] = {ld * 2, 128};
-  uint32_t box[3] = {64, 64, 2};
+  uint32_t box[3] = {64, 64, blocks};
   return make_tmap_nd_bf16(out, base, 3, dims, strides, box);
 }
 
@@ -513,26 +518,43 @@ static int make_tmap_mn3d(CUtensorMap* out, const void* base, uint64_t krows, ui
 // 8 - 10 tiles).  The all-gather kernel keeps rows of B ascending, the order in which its chunks arrive.
 // Weight gradient 22016 x 4096 x 4096 (fp32 bucket): 826 us with rows fastest, which read dY^T once per 256 columns,
 // 674 us so.
-template <typename Params>
+template <typename Params, int BN>
 static TileOrder gemm2_tile_order(int M, int N, int K) {
   constexpr long BAND_BYTES = 40l << 20;
   TileOrder o;
-  o.tiles_m = (M + Gemm2Cfg::BM - 1) / Gemm2Cfg::BM;
-  o.tiles_n = (N + Gemm2Cfg::BN - 1) / Gemm2Cfg::BN;
+  o.tiles_m = (M + Gemm2Cfg<BN>::BM - 1) / Gemm2Cfg<BN>::BM;
+  o.tiles_n = (N + BN - 1) / BN;
   o.n_fast = !std::is_same<Params, GemmAgParams>::value && o.tiles_n < o.tiles_m;
   const int nf = o.n_fast ? o.tiles_n : o.tiles_m;
   o.band = nf;
-  if (!std::is_same<Params, GemmAgParams>::value && (nf > 16 || long(nf) * 256 * K * 2 > BAND_BYTES)) {
+  if (!std::is_same<Params, GemmAgParams>::value && (nf > 16 || long(nf) * (o.n_fast ? BN : 256) * K * 2 > BAND_BYTES)) {
     const int bands = (nf + 9) / 10;
     o.band = (nf + bands - 1) / bands;
   }
   return o;
 }
 
-template <bool A_MN, bool B_MN, typename Params = GemmParams>
+// Width of a pair's tile.  A wave of 128-column tiles over the 74 pairs takes between 0.58 (K = 20480) and 0.67 (K = 2048)
+// of the time of a wave of 256-column tiles (A is read again for half as many columns, and the tile's fixed cost stays), so
+// the narrow tile wins where the wide one leaves many pairs without a tile or the last wave nearly empty.
+// Wide -> narrow, us: 1018 x 512 x 49152 225 -> 145, 3072 x 768 x 3072 25.4 -> 21.3, weight gradients 768 x 768 x 3072
+// 25.3 -> 20.5 and 3072 x 768 x 4616 34.8 -> 28.7 (fp32), 2048 x 2304 x 768 21.3 -> 17.3.  The line is drawn at 0.67:
+// 2048 x 5120 x 20480 (three waves against five) lost 5 %, 3072 x 2048 x 3000 (two against three) 4 %.
+static int gemm2_bn(int M, int N, int pairs) {
+  const long tm = (M + 255) / 256;
+  const long w256 = (tm * ((N + 255) / 256) + pairs - 1) / pairs, w128 = (tm * ((N + 127) / 128) + pairs - 1) / pairs;
+  return w128 * 134 < w256 * 200 ? 128 : 256;
+}
+
+template <bool A_MN, bool B_MN, typename Params = GemmParams, int BN = 256>
 static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, int ldb, int max_ctas,
                         cudaStream_t stream) {
-  using Cfg = Gemm2Cfg;
+  using Cfg = Gemm2Cfg<BN>;
+  int pairs = num_sms() / 2;
+  if (max_ctas > 0 && max_ctas / 2 < pairs) pairs = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
+  if constexpr (std::is_same<Params, GemmParams>::value && BN == 256) {
+    if (gemm2_bn(p.M, p.N, pairs) == 128) return launch_gemm2<A_MN, B_MN, Params, 128>(A, B, p, lda, ldb, max_ctas, stream);
+  }
   CUtensorMap ta, tb;
   Gemm2Extra ex = {};
   // TMA epilogue: 16-byte aligned rows, and at most one tensor to add to a bf16 output
@@ -551,28 +573,26 @@ static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, 
   }
   int rc;
   if (!A_MN) rc = make_tmap_2d_bf16(&ta, A, p.M, p.K, lda, 128, 64);
-  else if (p.M % 64 == 0) { rc = make_tmap_mn3d(&ta, A, p.K, p.M, lda); ex.a_3d = 1; }
+  else if (p.M % 64 == 0) { rc = make_tmap_mn3d(&ta, A, p.K, p.M, lda, 2); ex.a_3d = 1; }
   else rc = make_tmap_2d_bf16(&ta, A, p.K, p.M, lda, 64, 64);
   if (rc) return rc;
-  if (!B_MN) rc = make_tmap_2d_bf16(&tb, B, p.N, p.K, ldb, 128, 64);
-  else if (p.N % 64 == 0) { rc = make_tmap_mn3d(&tb, B, p.K, p.N, ldb); ex.b_3d = 1; }
+  if (!B_MN) rc = make_tmap_2d_bf16(&tb, B, p.N, p.K, ldb, BN / 2, 64);
+  else if (p.N % 64 == 0) { rc = make_tmap_mn3d(&tb, B, p.K, p.N, ldb, BN / 128); ex.b_3d = 1; }
   else rc = make_tmap_2d_bf16(&tb, B, p.K, p.N, ldb, 64, 64);
   if (rc) return rc;
-  // five stages and four boxes where the tile's epilogue is not hidden by a long main loop (comment at Gemm2Cfg)
+  // fewer stages and four boxes where the tile's epilogue is not hidden by a long main loop (comment at Gemm2Cfg)
   const bool short_k = std::is_same<Params, GemmParams>::value && ex.ep != EP_DIRECT && p.K < 2048;
-  auto kern = gemm2_bf16_kernel<A_MN, B_MN, Params, 6>;
+  auto kern = gemm2_bf16_kernel<A_MN, B_MN, Params, BN, 2>;
   if constexpr (std::is_same<Params, GemmParams>::value) {
-    if (short_k) kern = gemm2_bf16_kernel<A_MN, B_MN, Params, 5>;
+    if (short_k) kern = gemm2_bf16_kernel<A_MN, B_MN, Params, BN, 4>;
   }
   static bool attr_set[2] = {false, false};
   if (!attr_set[short_k]) {
     ZB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
     attr_set[short_k] = true;
   }
-  ex.order = gemm2_tile_order<Params>(p.M, p.N, p.K);
+  ex.order = gemm2_tile_order<Params, BN>(p.M, p.N, p.K);
   const int tiles = ex.order.tiles_m * ex.order.tiles_n;
-  int pairs = num_sms() / 2;
-  if (max_ctas > 0 && max_ctas / 2 < pairs) pairs = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
   if (tiles < pairs) pairs = tiles;
   kern<<<2 * pairs, std::is_same<Params, GemmAgParams>::value ? 320 : 192, Cfg::SMEM_BYTES, stream>>>(ta, tb, tc, tx, p, ex);
   ZB_CUDA_OK(cudaGetLastError());

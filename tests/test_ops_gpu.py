@@ -75,6 +75,32 @@ def test_gemm_pair_kernel(k, M, N, K, a_mn, b_mn):
     _close(acc, want + 1, atol=0.02 * math.sqrt(K), rtol=1e-2)
 
 
+@pytest.mark.parametrize("M,N,K", [(264, 264, 72), (1018, 1544, 520), (520, 1088, 1000),          # 256 x 128 tiles
+                                   (4104, 1032, 264), (2312, 1800, 2056)])                        # 256 x 256 tiles
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+def test_gemm_pair_kernel_tile_widths(k, M, N, K, a_mn, b_mn):
+    """Both tile widths of the pair kernel at ragged edges, bf16 and fp32 outputs, added to what is there.  Bounds: the
+    operands are bf16 (exact products), so fp32 sums of K terms of unit variance are off by at most K * 2^-24 * sqrt(K)
+    in the worst order; bf16 outputs add half an ulp, 2^-9 relative, doubled for the rounding of the comparison."""
+    if (a_mn and M % 8) or (b_mn and N % 8):
+        pytest.skip("MN-major operand needs a 16-byte aligned row stride")
+    a, b = _rand(M, K, seed=1), _rand(N, K, seed=2)
+    want = (a.cuda().double() @ b.cuda().double().t()).cpu()
+    ad = (a.t().contiguous() if a_mn else a).cuda()
+    bd = (b.t().contiguous() if b_mn else b).cuda()
+    old = _rand(M, N, seed=3).cuda()
+    for dtype in (torch.float32, torch.bfloat16):
+        out = old.to(dtype, copy=True)
+        k.gemm(ad, bd, out, a_mn=a_mn, b_mn=b_mn, kernel="2cta", accumulate=True)
+        plain = torch.full((M, N), 7.0, dtype=dtype, device="cuda")
+        k.gemm(ad, bd, plain, a_mn=a_mn, b_mn=b_mn, kernel="2cta")
+        k.check_status()
+        rtol = 0.0 if dtype == torch.float32 else 2.0 ** -8
+        atol = K * math.sqrt(K) * 2.0 ** -24 + 1e-5
+        _close(out, want + old.cpu().double(), atol=atol, rtol=rtol)
+        _close(plain, want, atol=atol, rtol=rtol)
+
+
 def test_gemm_epilogues(k):
     M, N, K = 300, 520, 192
     a, b = _rand(M, K, seed=3), _rand(N, K, seed=4)
