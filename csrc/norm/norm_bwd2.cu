@@ -152,10 +152,14 @@ norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
 
 // out[h] (+)= sum_p part[p, h] with a 32 x 8 thread block per 32 columns: thread (tx, ty) adds rows
 // ty, ty + 8, ...; the eight partial sums of a column are then added in order by the ty = 0 thread.
+// blockIdx.y selects one of two such sums (weight and bias gradient in one launch).
 template <typename OutT>
 __global__ void __launch_bounds__(256)
-colsum_accumulate2_kernel(const float* __restrict__ part, int P, int H, OutT* __restrict__ out, int accumulate) {
+colsum_accumulate2_kernel(const float* __restrict__ part0, const float* __restrict__ part1, int P, int H,
+                          OutT* __restrict__ out0, OutT* __restrict__ out1, int accumulate) {
   __shared__ float sm[8][33];
+  const float* __restrict__ part = blockIdx.y ? part1 : part0;
+  OutT* __restrict__ out = blockIdx.y ? out1 : out0;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int h = blockIdx.x * 32 + tx;
   float s = 0.f;
@@ -171,6 +175,20 @@ colsum_accumulate2_kernel(const float* __restrict__ part, int P, int H, OutT* __
     if (accumulate) t += float(out[h]);
     out[h] = OutT(t);
   }
+}
+
+// Finishes one or two column sums (out1 / part1 null: one).
+int colsum_finish(const float* part0, int P, int H, void* out0, const float* part1, void* out1, int grad_f32,
+                  int accumulate, cudaStream_t stream) {
+  const dim3 grid((H + 31) / 32, out1 != nullptr ? 2 : 1);
+  if (grad_f32)
+    colsum_accumulate2_kernel<float><<<grid, 256, 0, stream>>>(part0, part1, P, H, static_cast<float*>(out0),
+                                                               static_cast<float*>(out1), accumulate);
+  else
+    colsum_accumulate2_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(
+        part0, part1, P, H, static_cast<__nv_bfloat16*>(out0), static_cast<__nv_bfloat16*>(out1), accumulate);
+  ZB_CUDA_OK(cudaGetLastError());
+  return 0;
 }
 
 }  // namespace zb
@@ -195,15 +213,8 @@ extern "C" int zb_norm_bwd2(const void* dy, const void* x, const void* w, const 
     else norm_bwd2_kernel<false, NORM_MAXV><<<P, NORM_THREADS, 0, stream>>>(DY, X, W, stats, DR, DX, part_dw, nullptr, T, H);
   }
   ZB_CUDA_OK(cudaGetLastError());
-  const int nb = (H + 31) / 32;
-  if (dw != nullptr) {
-    if (grad_f32) colsum_accumulate2_kernel<float><<<nb, 256, 0, stream>>>(part_dw, P, H, static_cast<float*>(dw), accumulate);
-    else colsum_accumulate2_kernel<__nv_bfloat16><<<nb, 256, 0, stream>>>(part_dw, P, H, static_cast<__nv_bfloat16*>(dw), accumulate);
-  }
-  if (ln && db != nullptr) {
-    if (grad_f32) colsum_accumulate2_kernel<float><<<nb, 256, 0, stream>>>(part_db, P, H, static_cast<float*>(db), accumulate);
-    else colsum_accumulate2_kernel<__nv_bfloat16><<<nb, 256, 0, stream>>>(part_db, P, H, static_cast<__nv_bfloat16*>(db), accumulate);
-  }
-  ZB_CUDA_OK(cudaGetLastError());
+  const bool bias = ln && db != nullptr;
+  if (dw != nullptr) return colsum_finish(part_dw, P, H, dw, bias ? part_db : nullptr, bias ? db : nullptr, grad_f32, accumulate, stream);
+  if (bias) return colsum_finish(part_db, P, H, db, nullptr, nullptr, grad_f32, accumulate, stream);
   return 0;
 }

@@ -172,6 +172,19 @@ def test_colsum(k):
     _close(out, dy.float().sum(0), atol=1e-2, rtol=1e-3)
 
 
+@pytest.mark.parametrize("T", [1, 7, 9, 300, 4100])
+@pytest.mark.parametrize("N,width", [(8, 8), (264, 264), (260, 260), (512, 1536), (5120, 5120)])
+def test_colsum_sizes(k, T, N, width):
+    """Sizes at the edges of the split over CTAs and rows; 260 columns take the kernel for unaligned rows, 512 of 1536 a
+    strided matrix.  Bound: fp32 sums of T bf16 values of unit variance, any order; half an ulp of a bf16 result, doubled
+    for the rounding of the comparison."""
+    dy = _rand(T, width, seed=T + N).cuda()[:, :N]
+    for dtype, rtol in ((torch.float32, 0.0), (torch.bfloat16, 2.0 ** -8)):
+        out = torch.ones(N, dtype=dtype, device="cuda")
+        k.colsum_accumulate(dy, out)
+        _close(out, dy.double().sum(0) + 1, atol=T * math.sqrt(T) * 2.0 ** -24 + 2e-6, rtol=rtol)
+
+
 @pytest.mark.parametrize("d,hq,hkv", [(64, 4, 2), (128, 2, 2)])
 def test_rope(k, d, hq, hkv):
     B, S = 2, 96
