@@ -1,12 +1,15 @@
 // RMSNorm / LayerNorm backward, second version (same interface and scratch as zb_norm_bwd).
 // Differences from the first version (norm.cu):
-//   * the next row's x and dy (and its statistics) are requested before the current row is
-//     reduced, and the residual gradient of the current row before its reduction, so a CTA
-//     always has two rows of loads in flight instead of alternating load / reduce / store;
-//   * one __syncthreads per row: the (sum g*xhat, sum g) pair is reduced in one pass, every
-//     thread adds the eight warp partials itself, and the partial buffer alternates between rows;
+//   * a CTA works on RW rows at a time, a team of 256 / RW threads each with up to four 16-byte chunks per thread, so that
+//     narrow rows keep every thread busy;
+//   * x, dy and the residual gradient of the next one to three groups of rows are on their way into shared memory
+//     (cp.async) while a group is reduced.  A thread reads only the chunks it has requested itself, so the ring needs no
+//     barrier;
+//   * one barrier per row (none where a team is one warp): the (sum g*xhat, sum g) pair is reduced in one pass;
 //   * the column reduction of the per-CTA partial sums runs on H/32 CTAs of 32 x 8 threads (eight
 //     rows in flight per column) instead of H/256 CTAs walking all partial rows one after another.
+// Bound by memory latency: with one row per CTA and the next row requested into registers 4616 x 768 took 42 us, now 24;
+// 4096 x 4096 46 -> 38 us, 2048 x 5120 50 -> 34 us (operands not in L2; reduction of the partial sums included).
 // Sums are formed in a fixed order, so results are deterministic.
 #include "../common/host.h"
 #include "../common/ptx.cuh"
@@ -16,138 +19,190 @@ extern "C" int zb_norm_partial_rows(int T);
 
 namespace zb {
 
-template <bool LN, int MAXV>
-__global__ void __launch_bounds__(NORM_THREADS, MAXV <= 2 ? 2 : 1)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {   // all but the newest N groups of this thread have landed
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+template <int NV>   // 16-byte chunks per thread
+struct NormBwdCfg {
+  static constexpr int STAGES = NV == 4 ? 2 : NV == 3 ? 3 : 4;            // about 100 KB: two CTAs per SM
+  static constexpr int STAGE_BYTES = 3 * NV * NORM_THREADS * 16;          // x, dy, residual gradient
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES;
+};
+
+template <bool LN, int RW, int NV>
+__global__ void __launch_bounds__(NORM_THREADS, 2)
 norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                  const __nv_bfloat16* __restrict__ w, const float* __restrict__ stats,
                  const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                  float* __restrict__ part_dw, float* __restrict__ part_db, int T, int H) {
+  using Cfg = NormBwdCfg<NV>;
+  constexpr int TEAM = NORM_THREADS / RW, WARPS = TEAM / 32, NS = Cfg::STAGES;
+  extern __shared__ __align__(128) uint8_t ring[];
   __shared__ float2 red[2][NORM_THREADS / 32];
+  const int team = threadIdx.x / TEAM, tt = threadIdx.x % TEAM;
   const int nchunk = H >> 3;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float aw[MAXV][8], ab[LN ? MAXV : 1][8], wf[MAXV][8];
-  const uint4* wr = reinterpret_cast<const uint4*>(w);
+  const uint32_t slot0 = smem_u32(ring) + threadIdx.x * 16;
+  auto slot = [&](int stage, int tensor, int i) {
+    return slot0 + uint32_t(stage * Cfg::STAGE_BYTES + (tensor * NV + i) * (NORM_THREADS * 16));
+  };
+  float aw[NV][8], ab[LN ? NV : 1][8];
+  uint4 wraw[NV];
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const int c = threadIdx.x + i * NORM_THREADS;
+  for (int i = 0; i < NV; ++i) {
+    const int c = tt + i * TEAM;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { aw[i][j] = 0.f; wf[i][j] = 0.f; }
-    if (LN) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ab[i][j] = 0.f;
+    for (int j = 0; j < 8; ++j) {
+      aw[i][j] = 0.f;
+      if (LN) ab[i][j] = 0.f;
     }
-    if (c < nchunk) unpack8(wr[c], wf[i]);
+    wraw[i] = c < nchunk ? reinterpret_cast<const uint4*>(w)[c] : make_uint4(0u, 0u, 0u, 0u);
   }
-  uint4 cx[MAXV], cg[MAXV];
-  float cmean = 0.f, crstd = 0.f;
-  int row = blockIdx.x;
-  if (row < T) {
-    const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(row) * H);
-    const uint4* gr = reinterpret_cast<const uint4*>(dy + size_t(row) * H);
+  const int groups = (T + RW - 1) / RW;
+  auto request = [&](int g, int stage) {   // this thread's chunks of its team's row of group g
+    const int row = g * RW + team;
+    if (g < groups && row < T) {
+      const size_t base = size_t(row) * H;
 #pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nchunk) { cx[i] = xr[c]; cg[i] = gr[c]; }
-    }
-    cmean = stats[2 * row];
-    crstd = stats[2 * row + 1];
-  }
-  int buf = 0;
-  for (; row < T; row += gridDim.x, buf ^= 1) {
-    // requests that do not depend on this row's reduction: next row, this row's residual gradient
-    const int nrow = row + gridDim.x;
-    uint4 nx[MAXV], ng[MAXV], rres[MAXV];
-    float nmean = 0.f, nrstd = 0.f;
-    if (nrow < T) {
-      const uint4* xr = reinterpret_cast<const uint4*>(x + size_t(nrow) * H);
-      const uint4* gr = reinterpret_cast<const uint4*>(dy + size_t(nrow) * H);
-#pragma unroll
-      for (int i = 0; i < MAXV; ++i) {
-        const int c = threadIdx.x + i * NORM_THREADS;
-        if (c < nchunk) { nx[i] = xr[c]; ng[i] = gr[c]; }
-      }
-      nmean = stats[2 * nrow];
-      nrstd = stats[2 * nrow + 1];
-    }
-    if (dres != nullptr) {
-      const uint4* rr = reinterpret_cast<const uint4*>(dres + size_t(row) * H);
-#pragma unroll
-      for (int i = 0; i < MAXV; ++i) {
-        const int c = threadIdx.x + i * NORM_THREADS;
-        if (c < nchunk) rres[i] = rr[c];
+      for (int i = 0; i < NV; ++i) {
+        const int c = tt + i * TEAM;
+        if (c < nchunk) {
+          cp_async16(slot(stage, 0, i), x + base + c * 8);
+          cp_async16(slot(stage, 1, i), dy + base + c * 8);
+          if (dres != nullptr) cp_async16(slot(stage, 2, i), dres + base + c * 8);
+        }
       }
     }
-    float xh[MAXV][8], g[MAXV][8];
-    float s1 = 0.f, s2 = 0.f;
+    cp_async_commit();
+  };
 #pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nchunk) {
-        float xf[8], df[8];
-        unpack8(cx[i], xf);
-        unpack8(cg[i], df);
+  for (int s = 0; s < NS; ++s) request(blockIdx.x + s * gridDim.x, s);
+  float2 st = make_float2(0.f, 0.f);
+  {
+    const int row = blockIdx.x * RW + team;
+    if (row < T) st = *reinterpret_cast<const float2*>(stats + 2 * size_t(row));
+  }
+  int stage = 0, buf = 0;
+  for (int g = blockIdx.x; g < groups; g += gridDim.x, buf ^= 1) {
+    const int row = g * RW + team;
+    const float mean = st.x, rstd = st.y;
+    const long nrow = long(g + gridDim.x) * RW + team;
+    if (nrow < T) st = *reinterpret_cast<const float2*>(stats + 2 * nrow);
+    cp_async_wait<NS - 1>();
+    if (row < T) {   // the whole team
+      float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          xh[i][j] = (xf[j] - cmean) * crstd;
-          g[i][j] = df[j] * wf[i][j];
-          s1 += g[i][j] * xh[i][j];
-          aw[i][j] += df[j] * xh[i][j];
-          if (LN) {
-            s2 += g[i][j];
-            ab[i][j] += df[j];
+      for (int i = 0; i < NV; ++i) {
+        if (tt + i * TEAM < nchunk) {
+          float xf[8], df[8], wf[8];
+          unpack8(ld_shared_v4(slot(stage, 0, i)), xf);
+          unpack8(ld_shared_v4(slot(stage, 1, i)), df);
+          unpack8(wraw[i], wf);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float xh = (xf[j] - mean) * rstd, gg = df[j] * wf[j];
+            s1 += gg * xh;
+            aw[i][j] += df[j] * xh;
+            if (LN) {
+              s2 += gg;
+              ab[i][j] += df[j];
+            }
           }
         }
       }
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-      if (LN) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-    }
-    if (lane == 0) red[buf][warp] = make_float2(s1, s2);
-    __syncthreads();
-    float t1 = 0.f, t2 = 0.f;
+      for (int o = 16; o > 0; o >>= 1) {
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+        if (LN) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+      }
+      if constexpr (WARPS > 1) {
+        if ((threadIdx.x & 31) == 0) red[buf][threadIdx.x >> 5] = make_float2(s1, s2);
+        team_barrier<RW>(team);
+        s1 = 0.f;
+        s2 = 0.f;
 #pragma unroll
-    for (int k = 0; k < NORM_THREADS / 32; ++k) {
-      const float2 v = red[buf][k];
-      t1 += v.x;
-      t2 += v.y;
-    }
-    const float m1 = t1 / H, m2 = LN ? t2 / H : 0.f;
-    uint4* dxr = reinterpret_cast<uint4*>(dx + size_t(row) * H);
-#pragma unroll
-    for (int i = 0; i < MAXV; ++i) {
-      const int c = threadIdx.x + i * NORM_THREADS;
-      if (c < nchunk) {
-        float o[8], rf[8];
-        if (dres != nullptr) unpack8(rres[i], rf);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          o[j] = crstd * (g[i][j] - xh[i][j] * m1 - m2);
-          if (dres != nullptr) o[j] += rf[j];
+        for (int k = 0; k < WARPS; ++k) {
+          const float2 v = red[buf][team * WARPS + k];
+          s1 += v.x;
+          s2 += v.y;
         }
-        dxr[c] = pack8(o);
+      }
+      const float m1 = s1 / H, m2 = LN ? s2 / H : 0.f;
+      uint4* dxr = reinterpret_cast<uint4*>(dx + size_t(row) * H);
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int c = tt + i * TEAM;
+        if (c < nchunk) {
+          float xf[8], df[8], wf[8], rf[8], o[8];
+          unpack8(ld_shared_v4(slot(stage, 0, i)), xf);
+          unpack8(ld_shared_v4(slot(stage, 1, i)), df);
+          unpack8(wraw[i], wf);
+          if (dres != nullptr) unpack8(ld_shared_v4(slot(stage, 2, i)), rf);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float xh = (xf[j] - mean) * rstd;
+            o[j] = rstd * (df[j] * wf[j] - xh * m1 - m2);
+            if (dres != nullptr) o[j] += rf[j];
+          }
+          dxr[c] = pack8(o);
+        }
       }
     }
-#pragma unroll
-    for (int i = 0; i < MAXV; ++i) { cx[i] = nx[i]; cg[i] = ng[i]; }
-    cmean = nmean;
-    crstd = nrstd;
+    request(g + NS * gridDim.x, stage);   // behind the stores that used the last value read from this stage
+    stage = stage + 1 == NS ? 0 : stage + 1;
   }
+  // column sums of this CTA: teams in order, through shared memory (the ring: every copy into it has landed)
+  cp_async_wait<0>();
+  auto finish = [&](auto& acc, float* __restrict__ part) {
+    float* sm = reinterpret_cast<float*>(ring);
+    float* out = part + size_t(blockIdx.x) * H;
+    if (RW > 1) __syncthreads();
 #pragma unroll
-  for (int i = 0; i < MAXV; ++i) {
-    const int c = threadIdx.x + i * NORM_THREADS;
-    if (c < nchunk) {
-      float4* pw = reinterpret_cast<float4*>(part_dw + size_t(blockIdx.x) * H + c * 8);
-      pw[0] = make_float4(aw[i][0], aw[i][1], aw[i][2], aw[i][3]);
-      pw[1] = make_float4(aw[i][4], aw[i][5], aw[i][6], aw[i][7]);
-      if (LN && part_db != nullptr) {
-        float4* pb = reinterpret_cast<float4*>(part_db + size_t(blockIdx.x) * H + c * 8);
-        pb[0] = make_float4(ab[i][0], ab[i][1], ab[i][2], ab[i][3]);
-        pb[1] = make_float4(ab[i][4], ab[i][5], ab[i][6], ab[i][7]);
+    for (int i = 0; i < NV; ++i) {
+      const int c = tt + i * TEAM;
+      if (c < nchunk) {
+        float4* d = reinterpret_cast<float4*>((RW > 1 ? sm + team * H : out) + c * 8);
+        d[0] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        d[1] = make_float4(acc[i][4], acc[i][5], acc[i][6], acc[i][7]);
       }
     }
+    if (RW > 1) {
+      __syncthreads();
+      for (int c = threadIdx.x; c < H / 4; c += NORM_THREADS) {
+        float4 t = reinterpret_cast<const float4*>(sm)[c];
+#pragma unroll
+        for (int k = 1; k < RW; ++k) {
+          const float4 v = reinterpret_cast<const float4*>(sm + k * H)[c];
+          t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
+        }
+        reinterpret_cast<float4*>(out)[c] = t;
+      }
+    }
+  };
+  finish(aw, part_dw);
+  if constexpr (LN) {
+    if (part_db != nullptr) finish(ab, part_db);
   }
+}
+
+template <bool LN, int RW, int NV>
+static int launch_norm_bwd2(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w, const float* stats,
+                            const __nv_bfloat16* dres, __nv_bfloat16* dx, float* part_dw, float* part_db, int T, int H,
+                            int blocks, cudaStream_t stream) {
+  auto kern = norm_bwd2_kernel<LN, RW, NV>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    ZB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, NormBwdCfg<NV>::SMEM_BYTES));
+    attr_set = true;
+  }
+  kern<<<blocks, NORM_THREADS, NormBwdCfg<NV>::SMEM_BYTES, stream>>>(dy, x, w, stats, dres, dx, part_dw, part_db, T, H);
+  ZB_CUDA_OK(cudaGetLastError());
+  return 0;
 }
 
 // out[h] (+)= sum_p part[p, h] with a 32 x 8 thread block per 32 columns: thread (tx, ty) adds rows
@@ -199,20 +254,35 @@ extern "C" int zb_norm_bwd2(const void* dy, const void* x, const void* w, const 
   using namespace zb;
   if (H % 8 != 0 || H > NORM_THREADS * NORM_MAXV * 8) ZB_FAIL(-1, "norm: H=%d unsupported", H);
   if (T <= 0) return 0;
-  const int P = zb_norm_partial_rows(T);
   auto DY = static_cast<const __nv_bfloat16*>(dy);
   auto X = static_cast<const __nv_bfloat16*>(x);
   auto W = static_cast<const __nv_bfloat16*>(w);
   auto DR = static_cast<const __nv_bfloat16*>(dres);
   auto DX = static_cast<__nv_bfloat16*>(dx);
-  if (H <= NORM_THREADS * 2 * 8) {
-    if (ln) norm_bwd2_kernel<true, 2><<<P, NORM_THREADS, 0, stream>>>(DY, X, W, stats, DR, DX, part_dw, part_db, T, H);
-    else norm_bwd2_kernel<false, 2><<<P, NORM_THREADS, 0, stream>>>(DY, X, W, stats, DR, DX, part_dw, nullptr, T, H);
+  const int rw = norm_rows_per_cta(H), nv = (H / 8 + NORM_THREADS / rw - 1) / (NORM_THREADS / rw);
+  const int groups = (T + rw - 1) / rw, cap = zb_norm_partial_rows(T);   // two CTAs per SM, a row of partial sums each
+  const int P = groups < cap ? groups : cap;
+  int rc = 0;
+#define ZB_NORM_BWD(RW_, NV_)                                                                                        \
+  rc = ln ? launch_norm_bwd2<true, RW_, NV_>(DY, X, W, stats, DR, DX, part_dw, part_db, T, H, P, stream)              \
+          : launch_norm_bwd2<false, RW_, NV_>(DY, X, W, stats, DR, DX, part_dw, nullptr, T, H, P, stream)
+  if (rw == 8) {
+    if (nv == 1) ZB_NORM_BWD(8, 1);
+    else if (nv == 2) ZB_NORM_BWD(8, 2);
+    else if (nv == 3) ZB_NORM_BWD(8, 3);
+    else ZB_NORM_BWD(8, 4);
+  } else if (rw == 4) {
+    if (nv == 3) ZB_NORM_BWD(4, 3);
+    else ZB_NORM_BWD(4, 4);
+  } else if (rw == 2) {
+    if (nv == 3) ZB_NORM_BWD(2, 3);
+    else ZB_NORM_BWD(2, 4);
   } else {
-    if (ln) norm_bwd2_kernel<true, NORM_MAXV><<<P, NORM_THREADS, 0, stream>>>(DY, X, W, stats, DR, DX, part_dw, part_db, T, H);
-    else norm_bwd2_kernel<false, NORM_MAXV><<<P, NORM_THREADS, 0, stream>>>(DY, X, W, stats, DR, DX, part_dw, nullptr, T, H);
+    if (nv == 3) ZB_NORM_BWD(1, 3);
+    else ZB_NORM_BWD(1, 4);
   }
-  ZB_CUDA_OK(cudaGetLastError());
+#undef ZB_NORM_BWD
+  if (rc) return rc;
   const bool bias = ln && db != nullptr;
   if (dw != nullptr) return colsum_finish(part_dw, P, H, dw, bias ? part_db : nullptr, bias ? db : nullptr, grad_f32, accumulate, stream);
   if (bias) return colsum_finish(part_db, P, H, db, nullptr, nullptr, grad_f32, accumulate, stream);

@@ -165,6 +165,32 @@ def test_norm(k, T, H, ln, bwd_version):
             _close(db, br.grad + 1, atol=tol, rtol=2e-2)
 
 
+@pytest.mark.parametrize("H", [8, 264, 512, 768, 1024, 1032, 1536, 2056, 3072, 4104, 6144, 8192])
+@pytest.mark.parametrize("T", [1, 3, 2500])
+@pytest.mark.parametrize("ln", [False, True])
+def test_norm_row_widths(k, T, H, ln):
+    """Every split of a CTA into rows and chunks per thread, with and without the residual gradient, against fp64.  Bounds:
+    bf16 results to two ulp (2^-7) of values of a few units; weight gradients are fp32 sums of T products, each rounded
+    to 2^-22 relative at worst (statistics included), of values below 30."""
+    x, w, b = _rand(T, H, seed=1).cuda(), (_rand(H, seed=2) * 0.1 + 1).cuda(), _rand(H, seed=3, scale=0.1).cuda()
+    dy, dres = _rand(T, H, seed=4).cuda(), _rand(T, H, seed=5).cuda()
+    xr, wr, br = (t.double().requires_grad_(True) for t in (x, w, b))
+    if ln:
+        yr = torch.nn.functional.layer_norm(xr, (H,), wr, br, 1e-5)
+    else:
+        yr = xr * torch.rsqrt(xr.pow(2).mean(-1, keepdim=True) + 1e-5) * wr
+    yr.backward(dy.double())
+    y, stats = k.norm_fwd(x, w, b if ln else None, 1e-5, ln)
+    _close(y, yr.detach(), atol=1e-3, rtol=2.0 ** -7)
+    for res in (None, dres):
+        dw, db = torch.ones(H, device="cuda"), torch.ones(H, device="cuda")
+        dx = k.norm_bwd(dy, x, w, stats, res, dw, db if ln else None, ln)
+        _close(dx, xr.grad + (0 if res is None else res.double()), atol=4e-3, rtol=2.0 ** -7)
+        _close(dw, wr.grad + 1, atol=T * 30 * 2.0 ** -22 + 1e-4, rtol=1e-5)
+        if ln:
+            _close(db, br.grad + 1, atol=T * 30 * 2.0 ** -22 + 1e-5, rtol=1e-5)
+
+
 def test_colsum(k):
     dy = _rand(777, 520, seed=1)
     out = torch.zeros(520, dtype=torch.float32, device="cuda")
