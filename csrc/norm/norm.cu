@@ -23,8 +23,8 @@ __global__ void __launch_bounds__(NORM_THREADS)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                 const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
                 float* __restrict__ stats /* [T,2]: mean, rstd */, int T, int H, float eps) {
-  constexpr int TEAM = NORM_THREADS / RW;
-  __shared__ float red[2][NORM_THREADS / 32];
+  constexpr int TEAM = NORM_THREADS / RW, A = NORM_GROUPS<RW>;
+  __shared__ float red[2][RW * 8];
   const int team = threadIdx.x / TEAM, tt = threadIdx.x % TEAM;
   const int row = blockIdx.x * RW + team;
   if (row >= T) return;   // whole teams: their barriers are their own
@@ -36,26 +36,27 @@ norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
     const int c = tt + i * TEAM;
     raw[i] = c < nchunk ? xr[c] : make_uint4(0u, 0u, 0u, 0u);
   }
-  float s = 0.f, ss = 0.f;
+  float s[A] = {}, ss[A] = {};
 #pragma unroll
   for (int i = 0; i < NORM_MAXV; ++i) {
     float v[8];
     unpack8(raw[i], v);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { s += v[j]; ss += v[j] * v[j]; }
+    for (int j = 0; j < 8; ++j) { s[i % A] += v[j]; ss[i % A] += v[j] * v[j]; }
   }
   float mean = 0.f;
   if (LN) {
     mean = team_sum<RW>(s, red[0], team) / H;
     // two-pass variance from registers
-    ss = 0.f;
+#pragma unroll
+    for (int a = 0; a < A; ++a) ss[a] = 0.f;
 #pragma unroll
     for (int i = 0; i < NORM_MAXV; ++i) {
       if (tt + i * TEAM < nchunk) {
         float v[8];
         unpack8(raw[i], v);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) { const float d = v[j] - mean; ss += d * d; }
+        for (int j = 0; j < 8; ++j) { const float d = v[j] - mean; ss[i % A] += d * d; }
       }
     }
   }

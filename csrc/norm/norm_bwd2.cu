@@ -10,7 +10,7 @@
 //     rows in flight per column) instead of H/256 CTAs walking all partial rows one after another.
 // Bound by memory latency: with one row per CTA and the next row requested into registers 4616 x 768 took 42 us, now 24;
 // 4096 x 4096 46 -> 38 us, 2048 x 5120 50 -> 34 us (operands not in L2; reduction of the partial sums included).
-// Sums are formed in a fixed order, so results are deterministic.
+// Sums are formed in a fixed order, so results are deterministic; dx does not depend on the split into teams.
 #include "../common/host.h"
 #include "../common/ptx.cuh"
 #include "norm_common.cuh"
@@ -42,9 +42,9 @@ norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
                  const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                  float* __restrict__ part_dw, float* __restrict__ part_db, int T, int H) {
   using Cfg = NormBwdCfg<NV>;
-  constexpr int TEAM = NORM_THREADS / RW, WARPS = TEAM / 32, NS = Cfg::STAGES;
+  constexpr int TEAM = NORM_THREADS / RW, NS = Cfg::STAGES, A = NORM_GROUPS<RW>;
   extern __shared__ __align__(128) uint8_t ring[];
-  __shared__ float2 red[2][NORM_THREADS / 32];
+  __shared__ float2 red[2][RW * 8];
   const int team = threadIdx.x / TEAM, tt = threadIdx.x % TEAM;
   const int nchunk = H >> 3;
   const uint32_t slot0 = smem_u32(ring) + threadIdx.x * 16;
@@ -95,7 +95,7 @@ norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
     if (nrow < T) st = *reinterpret_cast<const float2*>(stats + 2 * nrow);
     cp_async_wait<NS - 1>();
     if (row < T) {   // the whole team
-      float s1 = 0.f, s2 = 0.f;
+      float2 s[A] = {};
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
         if (tt + i * TEAM < nchunk) {
@@ -105,32 +105,23 @@ norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
           unpack8(wraw[i], wf);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            const float xh = (xf[j] - mean) * rstd, gg = df[j] * wf[j];
-            s1 += gg * xh;
+            const float xh = (xf[j] - mean) * rstd, gg = __fmul_rn(df[j], wf[j]);
+            s[i % A].x += gg * xh;
             aw[i][j] += df[j] * xh;
             if (LN) {
-              s2 += gg;
+              s[i % A].y += gg;
               ab[i][j] += df[j];
             }
           }
         }
       }
+      float2 sums[8];
+      team_group_sums<RW>(s, red[buf], team, sums);
+      float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-        if (LN) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-      }
-      if constexpr (WARPS > 1) {
-        if ((threadIdx.x & 31) == 0) red[buf][threadIdx.x >> 5] = make_float2(s1, s2);
-        team_barrier<RW>(team);
-        s1 = 0.f;
-        s2 = 0.f;
-#pragma unroll
-        for (int k = 0; k < WARPS; ++k) {
-          const float2 v = red[buf][team * WARPS + k];
-          s1 += v.x;
-          s2 += v.y;
-        }
+      for (int k = 0; k < 8; ++k) {
+        s1 += sums[k].x;
+        s2 += sums[k].y;
       }
       const float m1 = s1 / H, m2 = LN ? s2 / H : 0.f;
       uint4* dxr = reinterpret_cast<uint4*>(dx + size_t(row) * H);
@@ -146,7 +137,7 @@ norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const float xh = (xf[j] - mean) * rstd;
-            o[j] = rstd * (df[j] * wf[j] - xh * m1 - m2);
+            o[j] = rstd * (__fmul_rn(df[j], wf[j]) - xh * m1 - m2);
             if (dres != nullptr) o[j] += rf[j];
           }
           dxr[c] = pack8(o);
