@@ -24,6 +24,7 @@
 #include "../common/host.h"
 #include "../common/ptx.cuh"
 #include "attn_bwd_common.h"
+#include <type_traits>
 
 namespace zb {
 
@@ -33,11 +34,12 @@ constexpr int BWD2_TRACE_EV = 256;
 template <int D>
 struct AttnBwd2Cfg {
   static constexpr int TILE_BYTES = 128 * D * 2;
-  static constexpr int QS = 2;                      // Q / dO stages
+  static constexpr int QS = D == 128 ? 2 : 4;       // Q / dO stages
   static constexpr int DS_BYTES = 128 * 128 * 2;
   static constexpr int SMEM_BYTES = 2 * TILE_BYTES + QS * 2 * TILE_BYTES + DS_BYTES + 1024 + 256;
   static constexpr int TMEM_COLS = 512;
   static constexpr int DP_COL = 128, DV_COL = 256, DK_COL = 256 + D;
+  static constexpr int S1_COL = 384;                // D = 64: second S^T buffer
 };
 
 enum : int {
@@ -56,9 +58,24 @@ __device__ __forceinline__ void red_add_f32(float* p, float a) {
   asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(a) : "memory");
 }
 
+__device__ __forceinline__ void cluster_barrier() {   // every thread of every CTA of the cluster
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+// fp32 at the same shared-memory offset in CTA `cta` of the cluster
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t cta) {
+  uint32_t ra;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(cta));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra));
+  return v;
+}
+
 // DQ = false: the key-tile half of the two-kernel backward (dK and dV only): no dS^T copy in shared memory,
 // no dQ product and no atomics; dQ then comes from flash_bwd_dq.cu.
-template <int D, bool TRACE, bool DQ>
+// CL > 1 (DQ = false): a cluster of CL CTAs shares a key tile, each taking its part of the query heads of the GQA group;
+// the fp32 sums are added up through distributed shared memory, in rank order, at the end.  One CTA per key tile leaves
+// 2048 tokens with 8 kv heads at 128 CTAs of 4 to 64 steps: the time is that of the longest.
+template <int D, bool TRACE, bool DQ, int CL>
 __global__ void __launch_bounds__(32 * BWD2_WARPS, 1)
 flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                   const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
@@ -66,6 +83,10 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
                   unsigned long long* trace, int trace_ctas) {
   using Cfg = AttnBwd2Cfg<D>;
   constexpr int BM = 128, BN = 128, QS = Cfg::QS, DB = D / 64;
+  // With d = 64 tensor memory has room for a second S^T (without the dQ part): the scores of the next step are then formed
+  // ahead of this step's P^T, and the compute warps go from one step's dS^T to the next step's exponentials without
+  // waiting for dV and S^T.  32 / 8 heads of 8192 tokens 795 -> 693 us, 2 x 4096 tokens 449 -> 407.
+  constexpr int NSB = (D == 64 && !DQ) ? 2 : 1;
   constexpr int BLK = 128 * 128;  // bytes of one [128 rows x 64 cols] bf16 block
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -80,8 +101,8 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   uint64_t* q_empty = q_full + QS;      // QS
   uint64_t* do_full = q_empty + QS;     // QS
   uint64_t* do_empty = do_full + QS;    // QS
-  uint64_t* s_full = do_empty + QS;     // 1
-  uint64_t* dp_full = s_full + 1;       // 1
+  uint64_t* s_full = do_empty + QS;     // NSB
+  uint64_t* dp_full = s_full + NSB;     // 1
   uint64_t* pds_full = dp_full + 1;     // 1 (8 arrivals)
   uint64_t* dq_full = pds_full + 1;     // 1
   uint64_t* dq_empty = dq_full + 1;     // 1 (8 arrivals)
@@ -92,9 +113,11 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // grid = (kv heads, key tiles, batch): x-fastest dispatch starts every head's heaviest key tile
   // (tile 0 sees all query tiles under a causal mask) before any light one
-  const int jt = blockIdx.y, kv_head = blockIdx.x, batch = blockIdx.z;
+  const int jt = blockIdx.y, kv_head = blockIdx.x / CL, batch = blockIdx.z;
+  const int cl_rank = blockIdx.x % CL;      // rank in the cluster
   const int kv0 = jt * BN;
-  const int rep = p.Hq / p.Hkv;
+  const int rep = p.Hq / p.Hkv / CL;        // query heads this CTA walks over
+  const int head0 = kv_head * (p.Hq / p.Hkv) + cl_rank * rep;
   const int n_qt = (p.S + BM - 1) / BM;
   const int i_lo = p.causal ? (kv0 / BM) : 0;
   int i_hi = n_qt;
@@ -124,7 +147,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       mbar_init(&do_full[i], 1);
       mbar_init(&do_empty[i], 1);
     }
-    mbar_init(s_full, 1);
+    for (int i = 0; i < NSB; ++i) mbar_init(&s_full[i], 1);
     mbar_init(dp_full, 1);
     mbar_init(pds_full, 8);
     mbar_init(dq_full, 1);
@@ -158,7 +181,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       for (int it = 0; it < n_iters; ++it) {
         const int st = it % QS;
         const uint32_t ph = uint32_t(it / QS) & 1;
-        const int head = kv_head * rep + it / per_head;
+        const int head = head0 + it / per_head;
         const int q0 = (i_lo + it % per_head) * BM;
         if (!zb_in_bounds(q0 >= 0 && q0 < p.S && head < p.Hq && kv0 < p.S, p.status, 8)) break;
         // Q and dO have their own barriers: dO_i is free once dV_i is done, Q_i only after dK_i, more than half a step
@@ -205,16 +228,18 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       // D = 128: A = K (M = head dim, M-major), B = dS^T tile (N = queries, N-major); D = 64: A = dS^T tile, B = K
       constexpr uint32_t idesc_dq = umma_idesc_bf16(128, D == 128 ? 128 : D, true, true);
       const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), ds_addr = smem_u32(sDS);
-      const uint32_t r_s = tmem_base, r_dp = tmem_base + Cfg::DP_COL;
+      const uint32_t r_dp = tmem_base + Cfg::DP_COL;
+      auto r_s = [&](int it) { return tmem_base + (NSB == 2 && (it & 1) ? uint32_t(Cfg::S1_COL) : 0u); };
       bool ok = mbar_wait(kv_full, 0, wctx, ST_TIMEOUT_FULL);
-      auto issue_a = [&](uint32_t q_addr) {  // S^T = K Q^T
+      auto issue_a = [&](int it) {  // S^T = K Q^T
         if (!elected) return;
+        const uint32_t q_addr = smem_u32(sQ + (it % QS) * Cfg::TILE_BYTES), d = r_s(it);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk) {
           const uint32_t off = uint32_t(kk / 4) * BLK + uint32_t(kk % 4) * 32;
-          umma_f16_ss(r_s, umma_desc_kmajor(k_addr + off), umma_desc_kmajor(q_addr + off), idesc_s, kk != 0 ? 1u : 0u);
+          umma_f16_ss(d, umma_desc_kmajor(k_addr + off), umma_desc_kmajor(q_addr + off), idesc_s, kk != 0 ? 1u : 0u);
         }
-        umma_commit(s_full);
+        umma_commit(&s_full[it % NSB]);
       };
       auto issue_b = [&](uint32_t do_addr) {  // dP^T = V dO^T
         if (!elected) return;
@@ -228,7 +253,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       if (ok) ok = mbar_wait(&q_full[0], 0, wctx, ST_TIMEOUT_FULL);
       if (ok) {
         tc_fence_after();
-        issue_a(smem_u32(sQ));
+        issue_a(0);
         ok = mbar_wait(&do_full[0], 0, wctx, ST_TIMEOUT_FULL);
       }
       if (ok) {
@@ -239,6 +264,14 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       for (int it = 0; it < n_iters && ok; ++it) {
         const int st = it % QS;
         const uint32_t q_addr = smem_u32(sQ + st * Cfg::TILE_BYTES), do_addr = smem_u32(sDO + st * Cfg::TILE_BYTES);
+        if (NSB == 2 && it + 1 < n_iters) {   // its buffer last held P^T of step it - 1, read by the D queued before this
+          const int sn = (it + 1) % QS;
+          if (!mbar_wait(&q_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
+          tr(TB_MMA_QDO_READY);
+          tc_fence_after();
+          issue_a(it + 1);
+          tr(TB_MMA_A_ISSUED);
+        }
         if (!mbar_wait(DQ ? pds_full : p_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_MISC)) break;
         if (DQ) tr(TB_MMA_PDS_READY);
         tc_fence_after();
@@ -248,7 +281,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
           for (int kk = 0; kk < BM / 16; ++kk) {
             const uint32_t acol = uint32_t(kk / 4) * 64 + uint32_t(kk % 4) * 8;
-            umma_f16_ts(tmem_base + Cfg::DV_COL, r_s + acol, umma_desc_mnmajor(do_addr + kk * 2048, BLK), idesc_dkv,
+            umma_f16_ts(tmem_base + Cfg::DV_COL, r_s(it) + acol, umma_desc_mnmajor(do_addr + kk * 2048, BLK), idesc_dkv,
                         (it | kk) != 0 ? 1u : 0u);
           }
           umma_commit(&do_empty[st]);     // B_i and D_i are dO_i's readers
@@ -256,12 +289,12 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         if constexpr (!DQ) {
           // D needs P^T only, and S^T of the next step goes right behind it (D was P^T's last reader): both run while
           // the compute warps form dS^T, and the next step's exponentials run under E and B
-          if (it + 1 < n_iters) {
+          if (NSB == 1 && it + 1 < n_iters) {
             const int sn = (it + 1) % QS;
             if (!mbar_wait(&q_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
             tr(TB_MMA_QDO_READY);
             tc_fence_after();
-            issue_a(smem_u32(sQ + sn * Cfg::TILE_BYTES));
+            issue_a(it + 1);
             tr(TB_MMA_A_ISSUED);
           }
           if (!mbar_wait(pds_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_MISC)) break;
@@ -314,7 +347,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           if (!mbar_wait(&do_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
           tr(TB_MMA_QDO_READY);
           tc_fence_after();
-          issue_a(smem_u32(sQ + sn * Cfg::TILE_BYTES));
+          issue_a(it + 1);
           tr(TB_MMA_A_ISSUED);
           if constexpr (DQ) {
             // dQ_it sits in R_dP until the compute warps have drained it
@@ -337,7 +370,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     uint8_t* ds_row = sDS + half * BLK + t * 128;  // this thread's 128-byte row of its 64-query block
     bool ok = true;
     for (int it = 0; it < n_iters; ++it) {
-      const int head = kv_head * rep + it / per_head;
+      const int head = head0 + it / per_head;
       const int q0 = (i_lo + it % per_head) * BM;
       const int qc0 = q0 + half * 64;            // first query column of this thread
       // statistics of the tile's queries: global rows indexed by the absolute query (one-kernel form), or the
@@ -351,7 +384,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const bool need_mask = (p.causal && kv0 + BN - 1 > q0) || (p.window > 0 && kv0 < q0 + BM - p.window) ||
                              (kv0 + BN > p.S) || (q0 + BM > p.S);
       // ---- C1: P^T = exp2(S^T c - lse_q), kept as packed bf16 pairs (queries 2i, 2i+1) ----
-      if (!__all_sync(0xffffffffu, mbar_wait(s_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_TMEM_FULL))) { ok = false; break; }
+      if (!__all_sync(0xffffffffu, mbar_wait(&s_full[it % NSB], uint32_t(it / NSB) & 1, wctx, ST_TIMEOUT_TMEM_FULL))) { ok = false; break; }
       tr(TB_S_READY);
       tc_fence_after();
       // queries of this half that this thread's key is seen by: columns [vis_lo, vis_lo + vis_n)
@@ -362,10 +395,11 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         // P stays in fp32 registers between its two uses; two-wide fp32 math; the softmax scale of dS is applied to
         // dK once, when it is written out
         float pr[64];
+        const uint32_t s_col = lane_addr + uint32_t(half * 64) + (NSB == 2 && (it & 1) ? uint32_t(Cfg::S1_COL) : 0u);
         {
           uint32_t rs0[32], rs1[32];
-          tmem_ld32(lane_addr + uint32_t(half * 64), rs0);
-          tmem_ld32(lane_addr + uint32_t(half * 64 + 32), rs1);
+          tmem_ld32(s_col, rs0);
+          tmem_ld32(s_col + 32u, rs1);
           tmem_wait_ld();
 #pragma unroll
           for (int k = 0; k < 64; k += 4) {
@@ -388,8 +422,8 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
             lo16[k] = pack_bf16x2(pr[2 * k], pr[2 * k + 1]);
             hi16[k] = pack_bf16x2(pr[32 + 2 * k], pr[33 + 2 * k]);
           }
-          tmem_st16(lane_addr + uint32_t(half * 64), lo16);
-          tmem_st16(lane_addr + uint32_t(half * 64 + 16), hi16);
+          tmem_st16(s_col, lo16);
+          tmem_st16(s_col + 16u, hi16);
         }
         tmem_wait_st();
         tc_fence_before();
@@ -561,16 +595,48 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     // the last dq_full arrival also covers every dK / dV MMA issued before it
     const int width = (p.Hq + 2 * p.Hkv) * D;
     ok = __all_sync(0xffffffffu, ok);
+    const uint32_t sums = smem_u32(sQ) + uint32_t(t) * 4;   // CL > 1: [which][column][key] fp32 over the Q / dO stages
+    if constexpr (CL > 1) {
+      // every copy into the stages has landed and every product that reads them is done (dq_full)
+#pragma unroll 1
+      for (int u = 0; u < 2 * (D / 64); ++u) {
+        const int which = u / (D / 64), c = half * (D / 64) + u % (D / 64);
+        uint32_t r[32];
+        if (n_iters > 0) {
+          tmem_ld32(lane_addr + (which == 0 ? Cfg::DK_COL : Cfg::DV_COL) + uint32_t(c * 32), r);
+          tmem_wait_ld();
+        } else {
+#pragma unroll
+          for (int k = 0; k < 32; ++k) r[k] = 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < 32; ++k)
+          asm volatile("st.shared.b32 [%0], %1;" ::"r"(sums + uint32_t((which * D + c * 32 + k) * 512)), "r"(r[k]) : "memory");
+      }
+      cluster_barrier();
+    }
 #pragma unroll 1
     for (int which = 0; which < 2; ++which) {
+      if (CL == 2 && which != cl_rank) continue;           // rank 0 writes dK, rank 1 dV
+      if (CL == 4 && which != (cl_rank >> 1)) continue;    // ranks 0 and 1: alternate column blocks of dK, 2 and 3: of dV
       const uint32_t col0 = which == 0 ? Cfg::DK_COL : Cfg::DV_COL;
       const float mul = !DQ && which == 0 ? p.scale : 1.f;   // the two-kernel form leaves dS unscaled
       __nv_bfloat16* dst = p.dqkv + (size_t(batch) * p.S + key) * width +
                            size_t(which == 0 ? (p.Hq + kv_head) : (p.Hq + p.Hkv + kv_head)) * D;
 #pragma unroll 1
       for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
+        if (CL == 4 && (c & 1) != (cl_rank & 1)) continue;
         uint32_t r[32];
-        if (n_iters > 0) {
+        if constexpr (CL > 1) {
+#pragma unroll
+          for (int k = 0; k < 32; ++k) {
+            const uint32_t a = sums + uint32_t((which * D + c * 32 + k) * 512);
+            float s = ld_cluster_f32(a, 0);
+#pragma unroll
+            for (int q = 1; q < CL; ++q) s += ld_cluster_f32(a, q);
+            r[k] = __float_as_uint(s);
+          }
+        } else if (n_iters > 0) {
           tmem_ld32(lane_addr + col0 + uint32_t(c * 32), r);
           tmem_wait_ld();
         } else {
@@ -595,6 +661,10 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   }
 
   __syncwarp();
+  if constexpr (CL > 1) {
+    if (warp >= 8) cluster_barrier();   // the compute warps' barrier in front of their write-out
+    cluster_barrier();                  // nobody leaves while its sums are read
+  }
   if (*abort_flag) {
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
   }
@@ -607,32 +677,66 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 }
 
 // stats[(b, h)][0][s] = -lse * log2(e), stats[(b, h)][1][s] = -sum_d dO * O; rows padded to s_pad
-// entries that this kernel never writes (they must have been zeroed once). One warp per (token, head).
-__global__ void attn_bwd2_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                       const float* __restrict__ lse, float* __restrict__ stats, int B, int S, int Hq,
-                                       int D, int s_pad) {
-  const long wid = (blockIdx.x * long(blockDim.x) + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const long total = long(B) * S * Hq;
-  if (wid >= total) return;
-  const int h = int(wid % Hq);
-  const long tok = wid / Hq;
-  const __nv_bfloat16* po = o + tok * (long(Hq) * D) + long(h) * D;
-  const __nv_bfloat16* pd = d_o + tok * (long(Hq) * D) + long(h) * D;
-  float acc = 0.f;
-  for (int c = lane * 2; c < D; c += 64) {
-    float2 a = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(po + c));
-    float2 b = unpack_bf16x2(*reinterpret_cast<const uint32_t*>(pd + c));
-    acc += a.x * b.x + a.y * b.y;
+// entries that this kernel never writes (they must have been zeroed once).  A CTA takes 64 tokens of one head: D / 8 lanes
+// read a token's row in 16-byte pieces, all rows of a thread in flight at once, and the 64 results leave as two row
+// segments. 32 heads of
+// 4096 tokens, d = 128 32 -> 12 us, 32 heads of 2048, d = 64 15 -> 4 us (one warp per token and head, four-byte loads).
+template <int D>
+__global__ void __launch_bounds__(256)
+attn_bwd2_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
+                       const float* __restrict__ lse, float* __restrict__ stats, int S, int Hq, int s_pad, int o_vec) {
+  constexpr int LANES = D / 8, GROUPS = 256 / LANES, N = 64 / GROUPS;   // lanes per token, tokens at a time, tokens per group
+  __shared__ float sm[64];
+  const int s0 = blockIdx.x * 64, h = blockIdx.y, b = blockIdx.z;
+  const int g = threadIdx.x / LANES, l = threadIdx.x % LANES;
+  uint4 x[N], y[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const int s = s0 + i * GROUPS + g;
+    x[i] = y[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (s < S) {
+      const size_t at = ((size_t(b) * S + s) * Hq + h) * D + l * 8;
+      y[i] = ld_nc_v4(d_o + at);
+      if (o_vec) {
+        x[i] = ld_nc_v4(o + at);
+      } else {
+        const uint32_t* p = reinterpret_cast<const uint32_t*>(o + at);
+        x[i] = make_uint4(p[0], p[1], p[2], p[3]);
+      }
+    }
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if (lane == 0) {
-    const long b = tok / S, s = tok % S;
-    float* row = stats + (b * Hq + h) * 2 * long(s_pad);
-    row[s] = lse[(b * Hq + h) * S + s] * -1.4426950408889634f;
-    row[s_pad + s] = -acc;
+  for (int i = 0; i < N; ++i) {
+    const uint32_t xs[4] = {x[i].x, x[i].y, x[i].z, x[i].w}, ys[4] = {y[i].x, y[i].y, y[i].z, y[i].w};
+    float acc = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 u = unpack_bf16x2(xs[k]), v = unpack_bf16x2(ys[k]);
+      acc += u.x * v.x + u.y * v.y;
+    }
+#pragma unroll
+    for (int off = LANES / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+    if (l == 0) sm[i * GROUPS + g] = acc;
   }
+  __syncthreads();
+  const int s = s0 + int(threadIdx.x);
+  if (threadIdx.x < 64 && s < S) {
+    const size_t bh = size_t(b) * Hq + h;
+    float* row = stats + bh * 2 * size_t(s_pad);
+    row[s] = lse[bh * S + s] * -1.4426950408889634f;
+    row[s_pad + s] = -sm[threadIdx.x];
+  }
+}
+
+static int launch_stats(const __nv_bfloat16* o, const __nv_bfloat16* d_o, const float* lse, float* stats, int B, int S, int Hq,
+                        int D, int s_pad, cudaStream_t stream) {
+  const dim3 grid((S + 63) / 64, Hq, B);
+  const int o_vec = (reinterpret_cast<uintptr_t>(o) & 15) == 0;   // (dO is fetched by TMA and aligned anyway)
+  if (reinterpret_cast<uintptr_t>(d_o) & 15) ZB_FAIL(-4, "attention: dO not 16-byte aligned");
+  if (D == 128) attn_bwd2_stats_kernel<128><<<grid, 256, 0, stream>>>(o, d_o, lse, stats, S, Hq, s_pad, o_vec);
+  else attn_bwd2_stats_kernel<64><<<grid, 256, 0, stream>>>(o, d_o, lse, stats, S, Hq, s_pad, o_vec);
+  ZB_CUDA_OK(cudaGetLastError());
+  return 0;
 }
 
 static int make_head_tmap_bwd2(CUtensorMap* out, const __nv_bfloat16* base, int B, int S, int heads, int D, int width) {
@@ -642,7 +746,7 @@ static int make_head_tmap_bwd2(CUtensorMap* out, const __nv_bfloat16* base, int 
   return make_tmap_nd_bf16(out, base, 4, dims, strides, box);
 }
 
-template <int D, bool TRACE, bool DQ = true>
+template <int D, bool TRACE, bool DQ = true, int CL = 1>
 static int launch_bwd2(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const AttnBwdParams& p, const float* stats,
                        int s_pad, unsigned long long* trace, int trace_ctas, cudaStream_t stream) {
   using Cfg = AttnBwd2Cfg<D>;
@@ -653,16 +757,43 @@ static int launch_bwd2(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const
   if ((rc = make_head_tmap_bwd2(&tk, qkv + size_t(p.Hq) * D, p.B, p.S, p.Hkv, D, width))) return rc;
   if ((rc = make_head_tmap_bwd2(&tv, qkv + size_t(p.Hq + p.Hkv) * D, p.B, p.S, p.Hkv, D, width))) return rc;
   if ((rc = make_head_tmap_bwd2(&tdo, d_o, p.B, p.S, p.Hq, D, p.Hq * D))) return rc;
-  auto kern = flash_bwd2_kernel<D, TRACE, DQ>;
+  auto kern = flash_bwd2_kernel<D, TRACE, DQ, CL>;
   static bool attr_set = false;
   if (!attr_set) {
     ZB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
     attr_set = true;
   }
-  dim3 grid(p.Hkv, (p.S + 127) / 128, p.B);
-  kern<<<grid, 32 * BWD2_WARPS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p, stats, s_pad, trace, trace_ctas);
-  ZB_CUDA_OK(cudaGetLastError());
+  dim3 grid(p.Hkv * CL, (p.S + 127) / 128, p.B);
+  if constexpr (CL > 1) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CL;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(32 * BWD2_WARPS);
+    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    ZB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, tdo, p, stats, s_pad, trace, trace_ctas));
+  } else {
+    kern<<<grid, 32 * BWD2_WARPS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p, stats, s_pad, trace, trace_ctas);
+    ZB_CUDA_OK(cudaGetLastError());
+  }
   return 0;
+}
+
+// CTAs per key tile of the dK / dV kernel.  Splitting pays where one CTA per tile leaves SMs idle or waiting for the
+// longest: 2048 tokens, 32 / 8 heads (128 CTAs) with d = 64 118 -> 81 us, with d = 128 159 -> 112; 512 tokens, d = 128
+// (32 CTAs) 52 -> 38 with two and 32 with four.  From two waves on the second prologue and the sum at the end cost more:
+// 4608 tokens, d = 128 (288 CTAs) 339 -> 357 us, 8 x 512, d = 64 (256 CTAs) 91 -> 95.
+static int bwd_cluster(int B, int S, int Hq, int Hkv) {
+  const int rep = Hq / Hkv;
+  const long ctas = long(Hkv) * ((S + 127) / 128) * B;
+  if (rep % 4 == 0 && 4 * ctas <= num_sms()) return 4;
+  return rep % 2 == 0 && ctas <= num_sms() ? 2 : 1;
 }
 
 int attn_bwd_dq(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const AttnBwdParams& p, const float* stats, int s_pad,
@@ -691,12 +822,7 @@ int zb_flash_bwd2(const void* d_o, const void* qkv, const void* o, const float* 
   auto O = static_cast<const __nv_bfloat16*>(o);
   auto QKV = static_cast<const __nv_bfloat16*>(qkv);
   const int s_pad = (S + 127) / 128 * 128;
-  {
-    const long warps = long(B) * S * Hq;
-    const long blocks = (warps * 32 + 255) / 256;
-    attn_bwd2_stats_kernel<<<(unsigned)blocks, 256, 0, stream>>>(O, DO, lse, stats, B, S, Hq, D, s_pad);
-    ZB_CUDA_OK(cudaGetLastError());
-  }
+  if (int rc_st = launch_stats(O, DO, lse, stats, B, S, Hq, D, s_pad, stream)) return rc_st;
   AttnBwdParams p;
   p.lse = lse; p.delta = nullptr; p.dq_acc = dq_acc;
   p.dqkv = static_cast<__nv_bfloat16*>(dqkv);
@@ -732,10 +858,7 @@ int zb_flash_bwd3(const void* d_o, const void* qkv, const void* o, const float* 
   auto QKV = static_cast<const __nv_bfloat16*>(qkv);
   const int s_pad = (S + 127) / 128 * 128;
   if (parts & 1) {
-    const long warps = long(B) * S * Hq;
-    const long blocks = (warps * 32 + 255) / 256;
-    attn_bwd2_stats_kernel<<<(unsigned)blocks, 256, 0, stream>>>(O, DO, lse, stats, B, S, Hq, D, s_pad);
-    ZB_CUDA_OK(cudaGetLastError());
+    if (int rc_st = launch_stats(O, DO, lse, stats, B, S, Hq, D, s_pad, stream)) return rc_st;
   }
   AttnBwdParams p;
   p.lse = lse; p.delta = nullptr; p.dq_acc = nullptr;
@@ -748,10 +871,16 @@ int zb_flash_bwd3(const void* d_o, const void* qkv, const void* o, const float* 
   int rc = 0;
   const bool trc = trace != nullptr && trace_ctas > 0;     // phase trace of the dK / dV kernel (as in zb_flash_bwd2)
   if (parts & 1) {
-    if (D == 128) rc = trc ? launch_bwd2<128, true, false>(QKV, DO, p, stats, s_pad, trace, trace_ctas, stream)
-                           : launch_bwd2<128, false, false>(QKV, DO, p, stats, s_pad, nullptr, 0, stream);
-    else rc = trc ? launch_bwd2<64, true, false>(QKV, DO, p, stats, s_pad, trace, trace_ctas, stream)
-                  : launch_bwd2<64, false, false>(QKV, DO, p, stats, s_pad, nullptr, 0, stream);
+    auto run = [&](auto d) {
+      constexpr int DD = decltype(d)::value;
+      if (trc) return launch_bwd2<DD, true, false>(QKV, DO, p, stats, s_pad, trace, trace_ctas, stream);
+      switch (bwd_cluster(B, S, Hq, Hkv)) {
+        case 4: return launch_bwd2<DD, false, false, 4>(QKV, DO, p, stats, s_pad, nullptr, 0, stream);
+        case 2: return launch_bwd2<DD, false, false, 2>(QKV, DO, p, stats, s_pad, nullptr, 0, stream);
+        default: return launch_bwd2<DD, false, false>(QKV, DO, p, stats, s_pad, nullptr, 0, stream);
+      }
+    };
+    rc = D == 128 ? run(std::integral_constant<int, 128>()) : run(std::integral_constant<int, 64>());
   }
   if (rc) return rc;
   return (parts & 2) ? attn_bwd_dq(QKV, DO, p, stats, s_pad, D, stream) : 0;

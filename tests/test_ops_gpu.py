@@ -387,6 +387,26 @@ def test_flash_bwd(k, B, S, Hq, Hkv, D, causal, window, version):
     _close(got, want, atol=4e-2, rtol=3e-2)
 
 
+@pytest.mark.parametrize("B,S,Hq,Hkv,causal,window", [(1, 130, 4, 1, True, 0), (1, 640, 8, 2, True, 0), (2, 600, 8, 2, True, 200),
+                                                      (1, 300, 4, 2, False, 0), (1, 2100, 6, 3, True, 0), (3, 1300, 8, 4, False, 0),
+                                                      (1, 1000, 12, 4, True, 0)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_flash_bwd_grouped_heads(k, B, S, Hq, Hkv, D, causal, window):
+    """Key tiles shared by clusters of one, two and four CTAs (by the number of tiles and the heads of a group), one to many
+    query tiles per head.  Bounds as in test_flash_bwd; a second call gives the same bits (sums in rank order)."""
+    qkv = _rand(B * S, (Hq + 2 * Hkv) * D, seed=21).cuda()
+    do = _rand(B * S, Hq * D, seed=22).cuda()
+    q = qkv.float().requires_grad_(True)
+    want_o = ref.attention(q, B, S, Hq, Hkv, D, causal, window)
+    (want,) = torch.autograd.grad(want_o, q, do.float())
+    out, lse = k.flash_fwd(qkv, B, S, Hq, Hkv, D, causal, window)
+    got = k.flash_bwd(do, qkv, out, lse, B, S, Hq, Hkv, D, causal, window)
+    again = k.flash_bwd(do, qkv, out, lse, B, S, Hq, Hkv, D, causal, window)
+    k.check_status()
+    _close(got, want, atol=4e-2, rtol=3e-2)
+    assert torch.equal(got, again)
+
+
 def test_attention_traces_run(k):
     """The in-kernel phase traces terminate, leave the status word clean and record plausible clocks."""
     from zorse_b200.profiler import attn_trace
