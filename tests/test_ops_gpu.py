@@ -241,6 +241,20 @@ def test_swiglu_and_act(k):
         _close(k.act_bwd(x.cuda(), dout.cuda(), kind), xr.grad, atol=3e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("B,C,H,W,p", [(1, 3, 32, 32, 16), (2, 3, 24, 40, 8), (3, 1, 10, 6, 2), (2, 3, 28, 42, 14),
+                                       (1, 3, 33, 35, 16)])
+def test_patches(k, B, C, H, W, p):
+    """Bit for bit the rows that unfolding the image gives, padded to a multiple of 8 columns; sizes with a rest, patches
+    whose rows are no multiple of 8, an image that is not contiguous or not 16-byte aligned."""
+    kdim = (C * p * p + 7) // 8 * 8
+    for img in (torch.randn(B, C, H, W), torch.randn(B, C, W, H).transpose(2, 3), torch.randn(B * C * H * W + 1)[1:].view(B, C, H, W)):
+        pt = torch.nn.functional.unfold(img[:, :, :H // p * p, :W // p * p], p, stride=p).transpose(1, 2).reshape(-1, C * p * p)
+        want = torch.nn.functional.pad(pt, (0, kdim - C * p * p)).to(torch.bfloat16)
+        dev = torch.empty(img.numel() + 1, device="cuda")[1:].view(B, C, H, W) if img.storage_offset() else None
+        got = k.patches(img.cuda() if dev is None else dev.copy_(img), p, kdim)
+        assert torch.equal(got.cpu(), want)
+
+
 def test_embedding(k):
     V, H, S, B = 1000, 512, 16, 3
     table, pos = _rand(V, H, seed=1), _rand(S + 2, H, seed=2)

@@ -310,8 +310,10 @@ class PatchEmbeddingLayer(Layer):
     def tokens_per_image(self):
         return self.n_patches + 1
 
-    def _patches(self, img):
+    def _patches(self, img, ops):
         B = img.shape[0]
+        if getattr(ops, "name", "") == "sm100" and img.is_cuda and self.p["proj_w"].dtype == torch.bfloat16:
+            return ops.patches(img.float(), self.patch, self.kdim)
         pt = torch.nn.functional.unfold(img.float(), self.patch, stride=self.patch).transpose(1, 2)
         pt = pt.reshape(B * self.n_patches, -1)
         if pt.shape[1] != self.kdim:
@@ -320,7 +322,7 @@ class PatchEmbeddingLayer(Layer):
 
     def forward(self, img, ctx, ops, saved=None):
         B = img.shape[0]
-        pt = self._patches(img)
+        pt = self._patches(img, ops)
         e = ops.linear_fwd(pt, self.p["proj_w"], self.p["proj_b"]).view(B, self.n_patches, self.H)
         x = torch.cat([self.p["cls"].expand(B, 1, self.H), e], dim=1) + self.p["pos"][None]
         if saved is not None:

@@ -201,6 +201,9 @@ class Sm100Ops:
     def act_bwd(self, x, dy, kind):
         return self.k.act_bwd(x, dy, _ACT_KINDS[kind])
 
+    def patches(self, img, patch, kdim):
+        return self.k.patches(img, patch, kdim)
+
     def embedding_fwd(self, ids, table, pos_table=None, S=1, pos_offset=0):
         return self.k.embedding_fwd(ids.reshape(-1), table, pos_table, S, pos_offset)
 

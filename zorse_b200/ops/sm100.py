@@ -247,6 +247,19 @@ def act_bwd(x, dy, kind: int):
     return dx
 
 
+def patches(img, patch: int, kdim: int):
+    """Non-overlapping patches of fp32 images [B, C, H, W] as bf16 rows [B * patches, kdim] (channel, row, column within
+    the patch; zeros behind C * patch^2)."""
+    if img.dtype != torch.float32 or not img.is_cuda:
+        raise TypeError(f"patches needs a CUDA fp32 tensor, got {img.dtype} on {img.device}")
+    img = img.contiguous()
+    B, C, H, W = img.shape
+    out = torch.empty(B * (H // patch) * (W // patch), kdim, dtype=torch.bfloat16, device=img.device)
+    _check(lib().zb_patches(_p(img), _p(out), c_int(B), c_int(C), c_int(H), c_int(W), c_int(patch), c_int(kdim),
+                            _stream()), "patches")
+    return out
+
+
 def embedding_fwd(ids, table, pos_table=None, S: int = 1, pos_offset: int = 0):
     T = ids.numel()
     V, H = table.shape
