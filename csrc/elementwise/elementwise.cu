@@ -6,6 +6,7 @@
 // (models/gpt_simple.py:119-134) and nn.Embedding (models/llama_simple.py:550-552).
 #include "../common/host.h"
 #include "../common/ptx.cuh"
+#include <type_traits>
 
 namespace zb {
 
@@ -174,7 +175,21 @@ template <>
 __device__ __forceinline__ void atomic_add2<__nv_bfloat16>(__nv_bfloat16* p, float a, float b) {
   atomicAdd(reinterpret_cast<__nv_bfloat162*>(p), __floats2bfloat162_rn(a, b));
 }
-template <typename GT>
+// Adds of 16 bytes each (p 16-byte aligned): one request to the L2 atomic units where two- and four-byte adds made eight
+// and four. 4096 x 4096 into fp32
+// 98 -> 40 us, into bf16 43 -> 23.
+__device__ __forceinline__ void red_add8(float* p, const uint4& u) {
+  float f[8];
+  unpack8e(u, f);
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(f[0]), "f"(f[1]), "f"(f[2]), "f"(f[3]) : "memory");
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + 4), "f"(f[4]), "f"(f[5]), "f"(f[6]), "f"(f[7]) : "memory");
+}
+__device__ __forceinline__ void red_add8(__nv_bfloat16* p, const uint4& u) {
+  asm volatile("red.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(u.x), "r"(u.y), "r"(u.z), "r"(u.w)
+               : "memory");
+}
+// VEC: both tables 16-byte aligned
+template <typename GT, bool VEC>
 __global__ void embedding_bwd_kernel(const long* __restrict__ ids, const __nv_bfloat16* __restrict__ dout,
                                      GT* __restrict__ dtable, GT* __restrict__ dpos, int T, int H, int V,
                                      int S, int pos_offset) {
@@ -184,9 +199,15 @@ __global__ void embedding_bwd_kernel(const long* __restrict__ ids, const __nv_bf
     const int t = int(i / cpr), c = int(i % cpr);
     long id = ids[t];
     id = id < 0 ? 0 : (id >= V ? V - 1 : id);
-    float a[8];
-    unpack8e(ld_nc_v4(dout + size_t(t) * H + c * 8), a);
+    const uint4 u = ld_nc_v4(dout + size_t(t) * H + c * 8);
     GT* dst = dtable + id * H + c * 8;
+    if constexpr (VEC) {
+      red_add8(dst, u);
+      if (dpos != nullptr) red_add8(dpos + size_t((t % S) + pos_offset) * H + c * 8, u);
+      continue;
+    }
+    float a[8];
+    unpack8e(u, a);
 #pragma unroll
     for (int j = 0; j < 8; j += 2) atomic_add2<GT>(dst + j, a[j], a[j + 1]);
     if (dpos != nullptr) {
@@ -328,14 +349,15 @@ int zb_embedding_bwd(const long* ids, const void* dout, void* dtable, void* dpos
   if (H % 8 != 0) ZB_FAIL(-1, "embedding: H=%d not a multiple of 8", H);
   if (T <= 0) return 0;
   const int g = grid_for(long(T) * (H / 8), 256);
-  if (grad_f32)
-    embedding_bwd_kernel<float><<<g, 256, 0, stream>>>(ids, static_cast<const __nv_bfloat16*>(dout),
-                                                       static_cast<float*>(dtable), static_cast<float*>(dpos), T,
-                                                       H, V, S, pos_offset);
-  else
-    embedding_bwd_kernel<__nv_bfloat16><<<g, 256, 0, stream>>>(
-        ids, static_cast<const __nv_bfloat16*>(dout), static_cast<__nv_bfloat16*>(dtable),
-        static_cast<__nv_bfloat16*>(dpos), T, H, V, S, pos_offset);
+  const bool vec = ((reinterpret_cast<uintptr_t>(dtable) | reinterpret_cast<uintptr_t>(dpos)) & 15) == 0;
+  auto D = static_cast<const __nv_bfloat16*>(dout);
+  auto launch = [&](auto* table, auto* pos) {
+    using GT = std::remove_pointer_t<decltype(table)>;
+    if (vec) embedding_bwd_kernel<GT, true><<<g, 256, 0, stream>>>(ids, D, table, pos, T, H, V, S, pos_offset);
+    else embedding_bwd_kernel<GT, false><<<g, 256, 0, stream>>>(ids, D, table, pos, T, H, V, S, pos_offset);
+  };
+  if (grad_f32) launch(static_cast<float*>(dtable), static_cast<float*>(dpos));
+  else launch(static_cast<__nv_bfloat16*>(dtable), static_cast<__nv_bfloat16*>(dpos));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -273,6 +273,20 @@ def test_embedding(k):
         _close(dp, wp, atol=5e-2, rtol=2e-2)
 
 
+@pytest.mark.parametrize("offset", [0, 2])     # gradient tables 16-byte aligned, or not
+@pytest.mark.parametrize("gdt", [torch.float32, torch.bfloat16])
+def test_embedding_bwd_alignment(k, offset, gdt):
+    """Both forms of the scatter-add; each id at most twice and small whole numbers, so every sum is exact."""
+    V, H, S, B = 40, 264, 10, 2
+    ids = torch.randperm(V, generator=torch.Generator().manual_seed(1))[:S].repeat(B)
+    dout = torch.randint(-8, 9, (B * S, H), generator=torch.Generator().manual_seed(2)).to(torch.bfloat16)
+    dt = torch.ones(V * H + offset, dtype=gdt, device="cuda")[offset:].view(V, H)
+    dp = torch.ones((S + 2) * H + offset, dtype=gdt, device="cuda")[offset:].view(S + 2, H)
+    k.embedding_bwd(ids.cuda(), dout.cuda(), dt, dp, S, 2)
+    assert torch.equal(dt.float().cpu(), torch.ones(V, H).index_add_(0, ids, dout.float()))
+    assert torch.equal(dp.float().cpu(), torch.ones(S + 2, H).index_add_(0, torch.arange(B * S) % S + 2, dout.float()))
+
+
 @pytest.mark.parametrize("T,V", [(9, 32000), (64, 50272), (4, 1001)])
 def test_cross_entropy(k, T, V):
     logits = _rand(T, V, seed=1, scale=2.0)
