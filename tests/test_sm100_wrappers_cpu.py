@@ -59,6 +59,25 @@ def lib(monkeypatch):
         assert nargs == protos[name], f"{name}: called with {nargs} arguments, the C function takes {protos[name]}"
 
 
+def test_signatures_match_the_sources():
+    """The argument types handed to ctypes are those of the C functions, one by one: pointers arrive as plain integers."""
+    import pathlib
+    import re
+
+    root = pathlib.Path(__file__).resolve().parent.parent / "csrc"
+    protos = {}
+    for f in root.rglob("*.cu"):
+        for m in re.finditer(r"\bint\s+(zb_\w+)\s*\(([^)]*)\)\s*\{", f.read_text()):
+            kinds = ""
+            for prm in m.group(2).split(","):
+                words = prm.replace("*", " * ").split()
+                kinds += "p" if "*" in words or "cudaStream_t" in words else {"int": "i", "long": "l", "float": "f"}[
+                    [w for w in words[:-1] if w != "const"][0]] if words and words[0] not in ("void", "double") else "?"
+            protos[m.group(1)] = kinds
+    for name, sig in k._SIGNATURES.items():
+        assert protos[name] == sig, name
+
+
 def bf(*shape):
     return torch.zeros(*shape, dtype=torch.bfloat16)
 

@@ -36,6 +36,22 @@ ACT_RELU = 1
 ACT_GELU_ERF = 2
 
 
+# Argument types of the entry points a training step calls all the time, in order (p pointer, i int, l long, f float):
+# with them ctypes converts plain Python numbers itself, which is cheaper than a c_int / c_void_p object per argument.
+_SIGNATURES = {
+    "zb_gemm2_bf16": "pppiiiiiiiippiiipp", "zb_gemm2_accpf_bf16": "pppiiiiiiiippiiipp",
+    "zb_gemm_bf16": "pppiiiiiiiippiiiipp",
+    "zb_norm_fwd": "pppppiifip", "zb_norm_fwd2": "pppppiifip",
+    "zb_norm_bwd": "ppppppppppiiiiip", "zb_norm_bwd2": "ppppppppppiiiiip",
+    "zb_colsum": "piiippiip", "zb_rope": "ppiiiiiip", "zb_swiglu_fwd": "pplip", "zb_swiglu_bwd": "ppplip",
+    "zb_act_fwd": "pplip", "zb_act_bwd": "ppplip", "zb_embedding_fwd": "ppppiiiiip", "zb_embedding_bwd": "ppppiiiiiip",
+    "zb_cross_entropy": "ppppiilflp", "zb_adam": "ppppplfffffifiip",
+    "zb_flash_fwd": "pppiiiiiiifipp", "zb_flash_fwd2": "pppiiiiiiifipp",
+    "zb_flash_fwd4": "pppiiiiiiifipipip", "zb_flash_bwd3": "ppppppiiiiiiifpipip",
+}
+_CTYPES = {"p": c_void_p, "i": c_int, "l": c_long, "f": c_float}
+
+
 class KernelError(RuntimeError):
     pass
 
@@ -60,6 +76,8 @@ def lib():
             _build.build()
         _lib = ctypes.CDLL(str(path))
         _lib.zb_last_error.restype = ctypes.c_char_p
+        for name, sig in _SIGNATURES.items():
+            getattr(_lib, name).argtypes = [_CTYPES[c] for c in sig]
         if "ZORSE_RS_ADAM_VARIANT" in os.environ:      # 0 / 1 select a peer-load kernel (1 is the library default)
             _lib.zb_set_rs_adam_variant(c_int(int(os.environ["ZORSE_RS_ADAM_VARIANT"])))
     return _lib
@@ -70,11 +88,17 @@ def launch_count() -> int:
 
 
 def _stream() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the raw handle: building a torch.cuda.Stream object for it costs a quarter of a launch's host time
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _p(t: Optional[torch.Tensor]) -> c_void_p:
     return c_void_p(0 if t is None else t.data_ptr())
+
+
+def _a(t: Optional[torch.Tensor]) -> int:
+    """Device address for an entry point listed in _SIGNATURES (a plain int: no other may take it)."""
+    return 0 if t is None else t.data_ptr()
 
 
 def status_word(device=None) -> torch.Tensor:
@@ -154,16 +178,16 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, a_mn: bool = Fa
     if kern in ("2cta", "2cta_accpf") and bn == 0 and M >= 256 and N >= 256:
         accpf = kern == "2cta_accpf" or (GEMM_ACC_PREFETCH and accumulate)
         fn = lib().zb_gemm2_accpf_bf16 if accpf else lib().zb_gemm2_bf16
-        rc = fn(_p(a), _p(b), _p(out), c_int(M), c_int(N), c_int(K), c_int(a.stride(0)),
-                                 c_int(b.stride(0)), c_int(out.stride(0)), c_int(int(a_mn)), c_int(int(b_mn)),
-                                 _p(bias), _p(addend), c_int(0 if addend is None else addend.stride(0)),
-                                 c_int(flags), c_int(max_ctas), _p(status_word(a.device)), _stream())
+        rc = fn(_a(a), _a(b), _a(out), M, N, K, a.stride(0),
+                                 b.stride(0), out.stride(0), int(a_mn), int(b_mn),
+                                 _a(bias), _a(addend), 0 if addend is None else addend.stride(0),
+                                 flags, max_ctas, _a(status_word(a.device)), _stream())
         _check(rc, "gemm2")
         return out
-    rc = lib().zb_gemm_bf16(_p(a), _p(b), _p(out), c_int(M), c_int(N), c_int(K), c_int(a.stride(0)),
-                            c_int(b.stride(0)), c_int(out.stride(0)), c_int(int(a_mn)), c_int(int(b_mn)),
-                            _p(bias), _p(addend), c_int(0 if addend is None else addend.stride(0)),
-                            c_int(flags), c_int(bn), c_int(max_ctas), _p(status_word(a.device)), _stream())
+    rc = lib().zb_gemm_bf16(_a(a), _a(b), _a(out), M, N, K, a.stride(0),
+                            b.stride(0), out.stride(0), int(a_mn), int(b_mn),
+                            _a(bias), _a(addend), 0 if addend is None else addend.stride(0),
+                            flags, bn, max_ctas, _a(status_word(a.device)), _stream())
     _check(rc, "gemm")
     return out
 
@@ -179,8 +203,8 @@ def norm_fwd(x, w, b, eps: float, layernorm: bool, version: Optional[int] = None
     y = torch.empty_like(x)
     stats = torch.empty(T, 2, dtype=torch.float32, device=x.device)
     fn = lib().zb_norm_fwd2 if (version or NORM_FWD_VERSION) == 2 else lib().zb_norm_fwd
-    _check(fn(_p(x), _p(w), _p(b), _p(y), _p(stats), c_int(T), c_int(H), c_float(eps),
-              c_int(int(layernorm)), _stream()), "norm_fwd")
+    _check(fn(_a(x), _a(w), _a(b), _a(y), _a(stats), T, H, eps,
+              int(layernorm), _stream()), "norm_fwd")
     return y, stats
 
 
@@ -197,9 +221,9 @@ def norm_bwd(dy, x, w, stats, dres, dw, db, layernorm: bool, accumulate: bool = 
     part_db = torch.empty(P, H, dtype=torch.float32, device=x.device) if (layernorm and db is not None) else None
     gf32 = int(dw.dtype == torch.float32)
     fn = lib().zb_norm_bwd2 if (version or NORM_BWD_VERSION) == 2 else lib().zb_norm_bwd
-    _check(fn(_p(dy), _p(x), _p(w), _p(stats), _p(dres), _p(dx), _p(part_dw), _p(part_db),
-                             _p(dw), _p(db), c_int(T), c_int(H), c_int(int(layernorm)), c_int(gf32),
-                             c_int(int(accumulate)), _stream()), "norm_bwd")
+    _check(fn(_a(dy), _a(x), _a(w), _a(stats), _a(dres), _a(dx), _a(part_dw), _a(part_db),
+                             _a(dw), _a(db), T, H, int(layernorm), gf32,
+                             int(accumulate), _stream()), "norm_bwd")
     return dx
 
 
@@ -207,8 +231,8 @@ def colsum_accumulate(dy, out, accumulate: bool = True):
     """out[n] (+)= sum_t dy[t, n] (bias gradients)."""
     T, N = dy.shape
     part = torch.empty(min(T, 64), N, dtype=torch.float32, device=dy.device)
-    _check(lib().zb_colsum(_p(dy), c_int(T), c_int(N), c_int(dy.stride(0)), _p(part), _p(out),
-                           c_int(int(out.dtype == torch.float32)), c_int(int(accumulate)), _stream()), "colsum")
+    _check(lib().zb_colsum(_a(dy), T, N, dy.stride(0), _a(part), _a(out),
+                           int(out.dtype == torch.float32), int(accumulate), _stream()), "colsum")
     return out
 
 
@@ -216,34 +240,34 @@ def colsum_accumulate(dy, out, accumulate: bool = True):
 def rope_(buf, cs, S: int, nheads: int, d: int, backward: bool = False):
     """In-place rotate-half RoPE on heads [0, nheads) of a packed [T, width] buffer."""
     T = buf.shape[0]
-    _check(lib().zb_rope(_p(buf), _p(cs), c_int(T), c_int(S), c_int(nheads), c_int(d), c_int(buf.stride(0)),
-                         c_int(int(backward)), _stream()), "rope")
+    _check(lib().zb_rope(_a(buf), _a(cs), T, S, nheads, d, buf.stride(0),
+                         int(backward), _stream()), "rope")
     return buf
 
 
 def swiglu_fwd(gu):
     T, F2 = gu.shape
     out = torch.empty(T, F2 // 2, dtype=gu.dtype, device=gu.device)
-    _check(lib().zb_swiglu_fwd(_p(gu), _p(out), c_long(T), c_int(F2 // 2), _stream()), "swiglu_fwd")
+    _check(lib().zb_swiglu_fwd(_a(gu), _a(out), T, F2 // 2, _stream()), "swiglu_fwd")
     return out
 
 
 def swiglu_bwd(gu, dout):
     dgu = torch.empty_like(gu)
     T, F2 = gu.shape
-    _check(lib().zb_swiglu_bwd(_p(gu), _p(dout), _p(dgu), c_long(T), c_int(F2 // 2), _stream()), "swiglu_bwd")
+    _check(lib().zb_swiglu_bwd(_a(gu), _a(dout), _a(dgu), T, F2 // 2, _stream()), "swiglu_bwd")
     return dgu
 
 
 def act_fwd(x, kind: int):
     y = torch.empty_like(x)
-    _check(lib().zb_act_fwd(_p(x), _p(y), c_long(x.numel()), c_int(kind), _stream()), "act_fwd")
+    _check(lib().zb_act_fwd(_a(x), _a(y), x.numel(), kind, _stream()), "act_fwd")
     return y
 
 
 def act_bwd(x, dy, kind: int):
     dx = torch.empty_like(x)
-    _check(lib().zb_act_bwd(_p(x), _p(dy), _p(dx), c_long(x.numel()), c_int(kind), _stream()), "act_bwd")
+    _check(lib().zb_act_bwd(_a(x), _a(dy), _a(dx), x.numel(), kind, _stream()), "act_bwd")
     return dx
 
 
@@ -264,16 +288,16 @@ def embedding_fwd(ids, table, pos_table=None, S: int = 1, pos_offset: int = 0):
     T = ids.numel()
     V, H = table.shape
     out = torch.empty(T, H, dtype=table.dtype, device=table.device)
-    _check(lib().zb_embedding_fwd(_p(ids), _p(table), _p(pos_table), _p(out), c_int(T), c_int(H), c_int(V),
-                                  c_int(S), c_int(pos_offset), _stream()), "embedding_fwd")
+    _check(lib().zb_embedding_fwd(_a(ids), _a(table), _a(pos_table), _a(out), T, H, V,
+                                  S, pos_offset, _stream()), "embedding_fwd")
     return out
 
 
 def embedding_bwd(ids, dout, dtable, dpos=None, S: int = 1, pos_offset: int = 0):
     T = ids.numel()
     V, H = dtable.shape
-    _check(lib().zb_embedding_bwd(_p(ids), _p(dout), _p(dtable), _p(dpos), c_int(T), c_int(H), c_int(V),
-                                  c_int(S), c_int(pos_offset), c_int(int(dtable.dtype == torch.float32)),
+    _check(lib().zb_embedding_bwd(_a(ids), _a(dout), _a(dtable), _a(dpos), T, H, V,
+                                  S, pos_offset, int(dtable.dtype == torch.float32),
                                   _stream()), "embedding_bwd")
 
 
@@ -283,8 +307,8 @@ def cross_entropy(logits, targets, grad_scale: float, dlogits=None, ignore_index
     (may alias logits) when given."""
     T, V = logits.shape
     loss_rows = torch.empty(T, dtype=torch.float32, device=logits.device)
-    _check(lib().zb_cross_entropy(_p(logits), _p(targets), _p(dlogits), _p(loss_rows), c_int(T), c_int(V),
-                                  c_long(logits.stride(0)), c_float(grad_scale), c_long(ignore_index),
+    _check(lib().zb_cross_entropy(_a(logits), _a(targets), _a(dlogits), _a(loss_rows), T, V,
+                                  logits.stride(0), grad_scale, ignore_index,
                                   _stream()), "cross_entropy")
     return loss_rows
 
@@ -292,9 +316,9 @@ def cross_entropy(logits, targets, grad_scale: float, dlogits=None, ignore_index
 # --------------------------------------------------------------------------- optimizer
 def adam_step(p, m, v, g, p16, *, lr, beta1, beta2, eps, weight_decay, step, grad_scale=1.0, zero_grad=False):
     n = p.numel()
-    _check(lib().zb_adam(_p(p), _p(m), _p(v), _p(g), _p(p16), c_long(n), c_float(lr), c_float(beta1),
-                         c_float(beta2), c_float(eps), c_float(weight_decay), c_int(step), c_float(grad_scale),
-                         c_int(int(g.dtype == torch.float32)), c_int(int(zero_grad)), _stream()), "adam")
+    _check(lib().zb_adam(_a(p), _a(m), _a(v), _a(g), _a(p16), n, lr, beta1,
+                         beta2, eps, weight_decay, step, grad_scale,
+                         int(g.dtype == torch.float32), int(zero_grad), _stream()), "adam")
 
 
 # --------------------------------------------------------------------------- attention
@@ -327,15 +351,15 @@ def flash_fwd(qkv, B: int, S: int, Hq: int, Hkv: int, D: int, causal: bool = Tru
     ver = version or ATTN_FWD_VERSION or _auto_fwd_version(B, S, Hq)
     if ver == 4:
         fl = ATTN_FWD4_FLAGS if flags is None else flags
-        _check(lib().zb_flash_fwd4(_p(qkv), _p(out), _p(lse), c_int(B), c_int(S), c_int(Hq), c_int(Hkv), c_int(D),
-                                   c_int(int(causal)), c_int(window), c_float(sc), c_int(out.stride(0)),
-                                   _p(status_word(qkv.device)), c_int(fl), _p(trace),
-                                   c_int(trace_ctas if trace is not None else 0), _stream()), "flash_fwd4")
+        _check(lib().zb_flash_fwd4(_a(qkv), _a(out), _a(lse), B, S, Hq, Hkv, D,
+                                   int(causal), window, sc, out.stride(0),
+                                   _a(status_word(qkv.device)), fl, _a(trace),
+                                   trace_ctas if trace is not None else 0, _stream()), "flash_fwd4")
         return out, lse
     fn = {1: lib().zb_flash_fwd, 2: lib().zb_flash_fwd2}[ver]
-    _check(fn(_p(qkv), _p(out), _p(lse), c_int(B), c_int(S), c_int(Hq), c_int(Hkv), c_int(D),
-                              c_int(int(causal)), c_int(window), c_float(sc), c_int(out.stride(0)),
-                              _p(status_word(qkv.device)), _stream()), "flash_fwd")
+    _check(fn(_a(qkv), _a(out), _a(lse), B, S, Hq, Hkv, D,
+                              int(causal), window, sc, out.stride(0),
+                              _a(status_word(qkv.device)), _stream()), "flash_fwd")
     return out, lse
 
 
@@ -369,10 +393,10 @@ def _flash_bwd3(do, qkv, o, lse, B, S, Hq, Hkv, D, causal, window, scale, parts:
     stats = _attn_scratch3[key]
     dqkv = torch.empty_like(qkv)
     sc = (1.0 / math.sqrt(D)) if scale is None else scale
-    _check(lib().zb_flash_bwd3(_p(do), _p(qkv), _p(o), _p(lse), _p(dqkv), _p(stats), c_int(B), c_int(S), c_int(Hq),
-                               c_int(Hkv), c_int(D), c_int(int(causal)), c_int(window), c_float(sc),
-                               _p(status_word(qkv.device)), c_int(parts), _p(trace),
-                               c_int(trace_ctas if trace is not None else 0), _stream()), "flash_bwd3")
+    _check(lib().zb_flash_bwd3(_a(do), _a(qkv), _a(o), _a(lse), _a(dqkv), _a(stats), B, S, Hq,
+                               Hkv, D, int(causal), window, sc,
+                               _a(status_word(qkv.device)), parts, _a(trace),
+                               trace_ctas if trace is not None else 0, _stream()), "flash_bwd3")
     global _launches
     _launches += 2  # statistics + the second main kernel
     return dqkv
