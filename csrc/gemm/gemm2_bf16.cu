@@ -14,6 +14,7 @@
 #include "../common/host.h"
 #include "../common/ptx.cuh"
 #include "gemm_common.cuh"
+#include <algorithm>
 #include <type_traits>
 
 namespace zb {
@@ -121,6 +122,10 @@ struct Gemm2Extra {
   TileOrder order;
   int ep;          // EP_*
   int ep_load;     // EP_BF16: add the tensor behind tmap_x (old C or addend)
+  // Split last wave: items [0, full) are whole tiles; the rest are tiles full, full + 1, ... in `splits` parts of their
+  // k-blocks each, whose fp32 sums go to the workspace behind tmap_w, one slot of 256 rows per part (gemm2_fixup_kernel
+  // adds them up).  Every pair gets at most one such part, as its last item.
+  int items, full, splits;
   int a_3d, b_3d;  // MN-major operand fetched with one 3-D TMA box {64, BK, 64-column blocks} instead of 2-D boxes
 };
 
@@ -133,8 +138,8 @@ struct Gemm2Extra {
 template <bool A_MN, bool B_MN, typename Params, int BN, int EP_BUFS>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(std::is_same<Params, GemmAgParams>::value ? 320 : 192, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                  const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_x, const Params p,
-                  const Gemm2Extra ex) {
+                  const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_x,
+                  const __grid_constant__ CUtensorMap tmap_w, const Params p, const Gemm2Extra ex) {
   using Cfg = Gemm2Cfg<BN>;
   constexpr bool SCATTER = std::is_same<Params, GemmScatterParams>::value;
   constexpr bool FUSED_AG = std::is_same<Params, GemmAgParams>::value;
@@ -156,8 +161,18 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   const uint32_t cta = cluster_ctarank();
   const bool leader = cta == 0;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  const int num_tiles = ex.order.tiles_m * ex.order.tiles_n;
+  const int num_items = ex.items;
   const int num_kb = (p.K + BK - 1) / BK;
+  auto tile_of = [&](int item) { return item < ex.full ? item : ex.full + (item - ex.full) / ex.splits; };
+  auto kb_range = [&](int item, int& kb0, int& kb1) {
+    kb0 = 0;
+    kb1 = num_kb;
+    if (item >= ex.full) {
+      const int part = (item - ex.full) % ex.splits;
+      kb0 = num_kb * part / ex.splits;
+      kb1 = num_kb * (part + 1) / ex.splits;
+    }
+  };
   WaitCtx wctx{abort_flag, p.status};
 
   if (threadIdx.x == 0) {
@@ -193,8 +208,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        int tm, tn;
+      for (int item = pair; item < num_items && ok; item += num_pairs) {
+        int tm, tn, kb0, kb1;
+        const int tile = tile_of(item);
+        kb_range(item, kb0, kb1);
         tile_at(ex.order, tile, tm, tn);
         const int m0 = tm * Cfg::BM + int(cta) * 128;
         const int n0 = tn * BN + int(cta) * HALF_N;
@@ -215,7 +232,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             asm volatile("fence.proxy.async.global;" ::: "memory");   // the gathered rows were written with plain stores
           }
         }
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, wctx, ST_TIMEOUT_EMPTY)) { ok = false; break; }
           uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
           uint8_t* sb = sa + Cfg::A_BYTES;
@@ -255,13 +272,15 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       uint32_t phase = 0;
       int local = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local) {
+      for (int item = pair; item < num_items && ok; item += num_pairs, ++local) {
+        int kb0, kb1;
+        kb_range(item, kb0, kb1);
         const int buf = local & 1;
         const uint32_t use = uint32_t(local >> 1);
         if (!mbar_wait(&tmem_empty[buf], (use & 1) ^ 1, wctx, ST_TIMEOUT_TMEM_EMPTY)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + uint32_t(buf * BN);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&full[stage], phase, wctx, ST_TIMEOUT_FULL)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE_BYTES);
@@ -271,7 +290,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             for (int kk = 0; kk < BK / 16; ++kk) {
               uint64_t da = A_MN ? umma_desc_mnmajor(sa + kk * 16 * 128, BK * 128) : umma_desc_kmajor(sa + kk * 32);
               uint64_t db = B_MN ? umma_desc_mnmajor(sb + kk * 16 * 128, BK * 128) : umma_desc_kmajor(sb + kk * 32);
-              umma_f16_ss_pair(d_tmem, da, db, idesc, (kb | kk) != 0 ? 1u : 0u);
+              umma_f16_ss_pair(d_tmem, da, db, idesc, kb > kb0 || kk != 0 ? 1u : 0u);
             }
             umma_commit_pair(&empty[stage]);
           }
@@ -290,23 +309,25 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     const int ahead = EP_BUFS == 4 ? 2 : 1;   // boxes of tmap_x requested ahead of the one being added
     uint32_t ep_count = 0;   // boxes this warp has stored: slot and barrier phase of the next one
     int local = 0;
-    for (int tile = pair; tile < num_tiles; tile += num_pairs, ++local) {
+    for (int item = pair; item < num_items; item += num_pairs, ++local) {
       int tm, tn;
-      tile_at(ex.order, tile, tm, tn);
+      tile_at(ex.order, tile_of(item), tm, tn);
+      const bool split = item >= ex.full;   // a part of a tile: plain fp32 sums to the workspace
       const int m0 = tm * Cfg::BM + int(cta) * 128;
       const int n0 = tn * BN;
       const int buf = local & 1;
       const uint32_t use = uint32_t(local >> 1);
       if (!SCATTER && ex.ep != EP_DIRECT) {
+        const bool f32 = split || ex.ep == EP_F32;
         const int row0 = m0 + q * 32;
-        const int wide = ex.ep == EP_F32 ? 32 : 64;                    // columns of a box
-        const int boxes = row0 < p.M ? min(BN / wide, (p.N - n0 + wide - 1) / wide) : 0;
+        const int wide = f32 ? 32 : 64;                    // columns of a box
+        const int boxes = split ? BN / 32 : row0 < p.M ? min(BN / wide, (p.N - n0 + wide - 1) / wide) : 0;
         auto load_box = [&](int c) {   // box c of this tile -> its ring slot (lane 0)
           const uint32_t k = ep_count + uint32_t(c);
           mbar_expect_tx(&my_full[k & slot_mask], Cfg::EP_BYTES);
           tma_load_2d(my_boxes + (k & slot_mask) * Cfg::EP_BYTES, &tmap_x, &my_full[k & slot_mask], n0 + c * 64, row0);
         };
-        if (ex.ep_load && lane == 0) {
+        if (ex.ep_load && !split && lane == 0) {
           bulk_wait_read<0>();   // stores of earlier boxes (issued a main loop ago) still hold the slots of boxes 0 and 1
           if (boxes > 0) load_box(0);
           if (boxes > 1) load_box(1);
@@ -329,13 +350,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           const uint32_t box = smem_u32(my_boxes + (k & slot_mask) * Cfg::EP_BYTES) + uint32_t(lane) * 128;
           const int col0 = n0 + c * wide;
           const uint32_t t_addr = tmem_base + (uint32_t(q * 32) << 16) + uint32_t(buf * BN + c * wide);
-          if (ex.ep == EP_F32) {
+          if (f32) {
             uint32_t r[32];
             tmem_ld32(t_addr, r);
             if (lane == 0) wait_slot();
             tmem_wait_ld();
             if (c == boxes - 1) release_tmem();
-            epilogue_bias_act(p, col0, r);
+            if (!split) epilogue_bias_act(p, col0, r);
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < 8; ++j)
@@ -379,7 +400,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           __syncwarp();
           if (lane == 0) {
             const void* src = my_boxes + (k & slot_mask) * Cfg::EP_BYTES;
-            if (zb_in_bounds(row0 >= 0 && row0 < p.M && col0 >= 0 && col0 < p.N, p.status, 2)) {
+            if (split) {
+              tma_store_2d(&tmap_w, src, c * 32, (item - ex.full) * Cfg::BM + int(cta) * 128 + q * 32);
+            } else if (zb_in_bounds(row0 >= 0 && row0 < p.M && col0 >= 0 && col0 < p.N, p.status, 2)) {
               if (ex.ep == EP_F32 && ecfg.accum) tma_reduce_add_2d(&tmap_c, src, col0, row0);
               else tma_store_2d(&tmap_c, src, col0, row0);
             }
@@ -534,31 +557,113 @@ static TileOrder gemm2_tile_order(int M, int N, int K) {
   return o;
 }
 
+// Adds up the parts of the split tiles, in their order, and finishes them like the epilogue: bias, activation, addend, old C.
+// One thread per 8 columns of a row; rows of C and of the addend are 16-byte aligned.
+template <int BN>
+__global__ void __launch_bounds__(256)
+gemm2_fixup_kernel(const float* __restrict__ ws, const GemmParams p, const TileOrder order, int first_tile, int splits) {
+  constexpr int CHUNKS = 256 * BN / 8;
+  const int w = blockIdx.x * 256 + threadIdx.x;
+  const int t = w / CHUNKS, e = w - t * CHUNKS;
+  const int rr = e / (BN / 8), cc = e % (BN / 8) * 8;
+  int tm, tn;
+  tile_at(order, first_tile + t, tm, tn);
+  const int row = tm * 256 + rr, col = tn * BN + cc;
+  if (row >= p.M || col >= p.N) return;
+  const float* src = ws + size_t(t) * splits * (256 * BN) + size_t(rr) * BN + cc;
+  float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int s = 0; s < splits; ++s, src += 256 * BN) {
+    const float4 a = reinterpret_cast<const float4*>(src)[0], b = reinterpret_cast<const float4*>(src)[1];
+    v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+    v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+  }
+  const int n = min(8, p.N - col);
+  const bool acc = (p.flags & GEMM_ACCUMULATE) != 0;
+  for (int j = 0; j < 8; ++j) {
+    if (p.bias != nullptr && j < n) v[j] += __bfloat162float(p.bias[col + j]);
+    if (p.flags & GEMM_GELU) v[j] = gelu_tanh(v[j]);
+    else if (p.flags & GEMM_RELU) v[j] = fmaxf(v[j], 0.f);
+  }
+  auto add8 = [&](const __nv_bfloat16* at) {
+    if (n == 8) {
+      const uint4 u = *reinterpret_cast<const uint4*>(at);
+      const float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
+      v[0] += a.x; v[1] += a.y; v[2] += b.x; v[3] += b.y; v[4] += c.x; v[5] += c.y; v[6] += d.x; v[7] += d.y;
+    } else {
+      for (int j = 0; j < n; ++j) v[j] += __bfloat162float(at[j]);
+    }
+  };
+  if (p.addend != nullptr) add8(p.addend + size_t(row) * p.ld_addend + col);
+  if (p.flags & GEMM_OUT_F32) {
+    float* c = static_cast<float*>(p.C) + size_t(row) * p.ldc + col;
+    for (int j = 0; j < n; ++j) c[j] = acc ? c[j] + v[j] : v[j];
+  } else {
+    __nv_bfloat16* c = static_cast<__nv_bfloat16*>(p.C) + size_t(row) * p.ldc + col;
+    if (acc) add8(c);
+    if (n == 8) {
+      uint4 o;
+      o.x = pack_bf16x2(v[0], v[1]); o.y = pack_bf16x2(v[2], v[3]);
+      o.z = pack_bf16x2(v[4], v[5]); o.w = pack_bf16x2(v[6], v[7]);
+      *reinterpret_cast<uint4*>(c) = o;
+    } else {
+      for (int j = 0; j < n; ++j) c[j] = __float2bfloat16(v[j]);
+    }
+  }
+}
+
 // Width of a pair's tile.  A wave of 128-column tiles over the 74 pairs takes between 0.58 (K = 20480) and 0.67 (K = 2048)
 // of the time of a wave of 256-column tiles (A is read again for half as many columns, and the tile's fixed cost stays), so
 // the narrow tile wins where the wide one leaves many pairs without a tile or the last wave nearly empty.
 // Wide -> narrow, us: 1018 x 512 x 49152 225 -> 145, 3072 x 768 x 3072 25.4 -> 21.3, weight gradients 768 x 768 x 3072
 // 25.3 -> 20.5 and 3072 x 768 x 4616 34.8 -> 28.7 (fp32), 2048 x 2304 x 768 21.3 -> 17.3.  The line is drawn at 0.67:
 // 2048 x 5120 x 20480 (three waves against five) lost 5 %, 3072 x 2048 x 3000 (two against three) 4 %.
-static int gemm2_bn(int M, int N, int pairs) {
-  const long tm = (M + 255) / 256;
-  const long w256 = (tm * ((N + 255) / 256) + pairs - 1) / pairs, w128 = (tm * ((N + 127) / 128) + pairs - 1) / pairs;
-  return w128 * 134 < w256 * 200 ? 128 : 256;
+//
+// Parts of a last wave: with a workspace the R tiles that are left behind the last full wave can be cut into
+// min(pairs / R, 16) parts of at least 8 k-blocks each.  That saves up to a wave and costs about 18 us (fp32 sums out and in
+// again, one more launch), the time of a 256-column wave at
+// K = 3000.  2048 x 5120 x 20480 (160 tiles, 12 left, six parts each) 331 -> 259 us, x 5120 87 -> 79; 4096 x 4096 x 22016 492 ->
+// 458; 3000 x 2048 x 8192 91 -> 75; 1018 x 512 x 49152 (all eight tiles in nine parts) 149 -> 56; weight gradient
+// 6144 x 4096 x 8192 280 -> 249.  Error against fp64 as before, in fp32 outputs a little smaller.
+struct Gemm2Plan {
+  int bn, splits;
+};
+static Gemm2Plan gemm2_plan(int M, int N, int K, int pairs, bool may_split) {
+  constexpr long SPLIT_COST = 3000 * 100;
+  Gemm2Plan best = {256, 1};
+  long best_cost = -1;
+  for (int bn = 256; bn >= 128; bn -= 128) {
+    const long unit = bn == 256 ? 100 : 67;   // cost of a wave per column of K
+    const long tiles = long((M + 255) / 256) * ((N + bn - 1) / bn), full = tiles / pairs, rest = tiles % pairs;
+    auto consider = [&](long cost, int splits) {
+      if (best_cost < 0 || cost < best_cost) {
+        best_cost = cost;
+        best = {bn, splits};
+      }
+    };
+    consider((full + (rest > 0)) * unit * K, 1);
+    if (may_split && rest > 0) {
+      const int parts = int(std::min(std::min(pairs / rest, 16l), long((K + 63) / 64 / 8)));
+      if (parts > 1) consider(full * unit * K + unit * K / parts + SPLIT_COST, parts);
+    }
+  }
+  return best;
 }
 
 template <bool A_MN, bool B_MN, typename Params = GemmParams, int BN = 256>
 static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, int ldb, int max_ctas,
-                        cudaStream_t stream) {
+                        cudaStream_t stream, float* ws = nullptr) {
   using Cfg = Gemm2Cfg<BN>;
   int pairs = num_sms() / 2;
   if (max_ctas > 0 && max_ctas / 2 < pairs) pairs = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
-  if constexpr (std::is_same<Params, GemmParams>::value && BN == 256) {
-    if (gemm2_bn(p.M, p.N, pairs) == 128) return launch_gemm2<A_MN, B_MN, Params, 128>(A, B, p, lda, ldb, max_ctas, stream);
+  Gemm2Plan plan = {BN, 1};
+  if constexpr (std::is_same<Params, GemmParams>::value) {
+    plan = gemm2_plan(p.M, p.N, p.K, pairs, ws != nullptr);
+    if (BN == 256 && plan.bn == 128) return launch_gemm2<A_MN, B_MN, Params, 128>(A, B, p, lda, ldb, max_ctas, stream, ws);
   }
   CUtensorMap ta, tb;
   Gemm2Extra ex = {};
   // TMA epilogue: 16-byte aligned rows, and at most one tensor to add to a bf16 output
-  CUtensorMap tc = {}, tx = {};
+  CUtensorMap tc = {}, tx = {}, tw = {};
   const bool f32 = (p.flags & GEMM_OUT_F32) != 0, acc = (p.flags & GEMM_ACCUMULATE) != 0, add = p.addend != nullptr;
   auto rows_ok = [](const void* base, long ld_bytes) { return (reinterpret_cast<uintptr_t>(base) & 15) == 0 && ld_bytes % 16 == 0; };
   if (std::is_same<Params, GemmParams>::value && rows_ok(p.C, long(p.ldc) * (f32 ? 4 : 2)) &&
@@ -593,18 +698,29 @@ static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, 
   }
   ex.order = gemm2_tile_order<Params, BN>(p.M, p.N, p.K);
   const int tiles = ex.order.tiles_m * ex.order.tiles_n;
-  if (tiles < pairs) pairs = tiles;
-  kern<<<2 * pairs, std::is_same<Params, GemmAgParams>::value ? 320 : 192, Cfg::SMEM_BYTES, stream>>>(ta, tb, tc, tx, p, ex);
+  ex.items = ex.full = tiles;
+  ex.splits = 1;
+  if (plan.splits > 1 && ex.ep != EP_DIRECT) {
+    ex.full = tiles / pairs * pairs;
+    ex.splits = plan.splits;
+    ex.items = ex.full + (tiles - ex.full) * ex.splits;
+    if ((rc = make_tmap_2d_out(&tw, ws, uint64_t(ex.items - ex.full) * 256, BN, BN, true, 32))) return rc;
+  }
+  if (ex.items < pairs) pairs = ex.items;
+  kern<<<2 * pairs, std::is_same<Params, GemmAgParams>::value ? 320 : 192, Cfg::SMEM_BYTES, stream>>>(ta, tb, tc, tx, tw, p, ex);
   ZB_CUDA_OK(cudaGetLastError());
+  if constexpr (std::is_same<Params, GemmParams>::value) {
+    if (ex.splits > 1) {
+      gemm2_fixup_kernel<BN><<<(tiles - ex.full) * (BN / 8), 256, 0, stream>>>(ws, p, ex.order, ex.full, ex.splits);
+      ZB_CUDA_OK(cudaGetLastError());
+    }
+  }
   return 0;
 }
 
-}  // namespace zb
-
-extern "C" int zb_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
-                             int a_mn_major, int b_mn_major, const void* bias, const void* addend, int ld_addend,
-                             int flags, int max_ctas, int* status, cudaStream_t stream) {
-  using namespace zb;
+static int gemm2_entry(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
+                       int a_mn_major, int b_mn_major, const void* bias, const void* addend, int ld_addend, int flags,
+                       int max_ctas, float* ws, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) ZB_FAIL(-1, "gemm2: empty problem %d x %d x %d", M, N, K);
   GemmParams p;
   p.C = C;
@@ -618,12 +734,39 @@ extern "C" int zb_gemm2_bf16(const void* A, const void* B, void* C, int M, int N
   p.gate_epoch = 0;
   p.gate_base = 0; p.gate_row_bytes = 0; p.gate_shard_bytes = 1;
   p.gate_chunk_bytes = 1; p.gate_cps = 1; p.gate_self = -1;
-  if (!a_mn_major && !b_mn_major) return launch_gemm2<false, false>(A, B, p, lda, ldb, max_ctas, stream);
-  if (!a_mn_major && b_mn_major) return launch_gemm2<false, true>(A, B, p, lda, ldb, max_ctas, stream);
-  if (a_mn_major && b_mn_major) return launch_gemm2<true, true>(A, B, p, lda, ldb, max_ctas, stream);
-  return launch_gemm2<true, false>(A, B, p, lda, ldb, max_ctas, stream);
+  if (!a_mn_major && !b_mn_major) return launch_gemm2<false, false>(A, B, p, lda, ldb, max_ctas, stream, ws);
+  if (!a_mn_major && b_mn_major) return launch_gemm2<false, true>(A, B, p, lda, ldb, max_ctas, stream, ws);
+  if (a_mn_major && b_mn_major) return launch_gemm2<true, true>(A, B, p, lda, ldb, max_ctas, stream, ws);
+  return launch_gemm2<true, false>(A, B, p, lda, ldb, max_ctas, stream, ws);
 }
 
+}  // namespace zb
+
+// Bytes of fp32 workspace (16-byte aligned) with which zb_gemm2_split_bf16 would cut the last wave of this product into
+// parts; 0: it would not.
+extern "C" int zb_gemm2_workspace(int M, int N, int K) {
+  using namespace zb;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  const int pairs = num_sms() / 2;
+  const Gemm2Plan plan = gemm2_plan(M, N, K, pairs, true);
+  if (plan.splits <= 1) return 0;
+  const long tiles = long((M + 255) / 256) * ((N + plan.bn - 1) / plan.bn);
+  return int(tiles % pairs * plan.splits * 256 * plan.bn * 4);   // at most one slot per pair
+}
+
+extern "C" int zb_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
+                             int a_mn_major, int b_mn_major, const void* bias, const void* addend, int ld_addend,
+                             int flags, int max_ctas, int* status, cudaStream_t stream) {
+  return zb::gemm2_entry(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, bias, addend, ld_addend, flags, max_ctas,
+                         nullptr, status, stream);
+}
+// zb_gemm2_bf16 on the whole GPU with a workspace of zb_gemm2_workspace(M, N, K) bytes.
+extern "C" int zb_gemm2_split_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
+                                   int a_mn_major, int b_mn_major, const void* bias, const void* addend, int ld_addend,
+                                   int flags, void* workspace, int* status, cudaStream_t stream) {
+  return zb::gemm2_entry(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, bias, addend, ld_addend, flags, 0,
+                         static_cast<float*>(workspace), status, stream);
+}
 // C = A @ B^T (b_mn_major: A @ B) with the output rows scattered for a row-wise reduce-scatter over
 // R ranks: rows [q * M / R, (q + 1) * M / R) go to dst_ptrs[q] (this rank's bf16 staging slot in rank
 // q's memory, [M / R, N] with row stride ldc); when the grid is done `epoch` is stored to

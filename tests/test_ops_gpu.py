@@ -101,6 +101,39 @@ def test_gemm_pair_kernel_tile_widths(k, M, N, K, a_mn, b_mn):
         _close(plain, want, atol=atol, rtol=rtol)
 
 
+@pytest.mark.parametrize("M,N,K", [(300, 520, 8200), (264, 264, 8200), (256, 504, 20008), (1018, 504, 12296), (2500, 2040, 4104), (2560, 2048, 4096),
+                                   (4096, 1288, 6152)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+def test_gemm_split_last_wave(k, M, N, K, a_mn, b_mn):
+    """Products whose last tiles are cut along K (all of them, or those behind one to two full waves), ragged in every
+    direction, through every epilogue.  Bounds as in test_gemm_pair_kernel_tile_widths."""
+    if (a_mn and M % 8) or (b_mn and N % 8):
+        pytest.skip("MN-major operand needs a 16-byte aligned row stride")
+    assert k._gemm2_workspace(M, N, K) > 0
+    a, b = _rand(M, K, seed=1).cuda(), _rand(N, K, seed=2).cuda()
+    want = a.double() @ b.double().t()
+    ad, bd = (a.t().contiguous() if a_mn else a), (b.t().contiguous() if b_mn else b)
+    old, bias = _rand(M, N, seed=3).cuda(), _rand(N, seed=4).cuda()
+    atol = K * math.sqrt(K) * 2.0 ** -24 + 1e-5
+    for dtype, rtol in ((torch.float32, 0.0), (torch.bfloat16, 2.0 ** -8)):
+        acc = old.to(dtype, copy=True)
+        k.gemm(ad, bd, acc, a_mn=a_mn, b_mn=b_mn, kernel="2cta", accumulate=True)
+        out = torch.full((M, N), 7.0, dtype=dtype, device="cuda")
+        k.gemm(ad, bd, out, a_mn=a_mn, b_mn=b_mn, kernel="2cta")
+        again = torch.full((M, N), 5.0, dtype=dtype, device="cuda")
+        k.gemm(ad, bd, again, a_mn=a_mn, b_mn=b_mn, kernel="2cta")
+        k.check_status()
+        _close(acc, want + old.double(), atol=atol, rtol=rtol)
+        _close(out, want, atol=atol, rtol=rtol)
+        assert torch.equal(out, again)
+    out = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    k.gemm(ad, bd, out, a_mn=a_mn, b_mn=b_mn, kernel="2cta", bias=bias, addend=old)
+    _close(out, want + bias.double() + old.double(), atol=atol, rtol=2.0 ** -8)
+    k.gemm(ad, bd, out, a_mn=a_mn, b_mn=b_mn, kernel="2cta", bias=bias, act="relu")
+    _close(out, (want + bias.double()).clamp(min=0), atol=atol, rtol=2.0 ** -8)
+    k.check_status()
+
+
 def test_gemm_epilogues(k):
     M, N, K = 300, 520, 192
     a, b = _rand(M, K, seed=3), _rand(N, K, seed=4)

@@ -9,6 +9,7 @@ the import of the library raises.  Tensors are passed as raw device pointers.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 import os
 from ctypes import c_float, c_int, c_long, c_void_p
@@ -40,7 +41,7 @@ ACT_GELU_ERF = 2
 # with them ctypes converts plain Python numbers itself, which is cheaper than a c_int / c_void_p object per argument.
 _SIGNATURES = {
     "zb_gemm2_bf16": "pppiiiiiiiippiiipp", "zb_gemm2_accpf_bf16": "pppiiiiiiiippiiipp",
-    "zb_gemm_bf16": "pppiiiiiiiippiiiipp",
+    "zb_gemm2_split_bf16": "pppiiiiiiiippiippp", "zb_gemm_bf16": "pppiiiiiiiippiiiipp",
     "zb_norm_fwd": "pppppiifip", "zb_norm_fwd2": "pppppiifip",
     "zb_norm_bwd": "ppppppppppiiiiip", "zb_norm_bwd2": "ppppppppppiiiiip",
     "zb_colsum": "piiippiip", "zb_rope": "ppiiiiiip", "zb_swiglu_fwd": "pplip", "zb_swiglu_bwd": "ppplip",
@@ -147,6 +148,12 @@ def _bf16(t: torch.Tensor, name: str) -> None:
 
 
 # --------------------------------------------------------------------------- GEMM
+@functools.lru_cache(maxsize=4096)
+def _gemm2_workspace(M: int, N: int, K: int) -> int:
+    """Bytes of workspace the pair kernel wants for this product (a function of the sizes), 0 for none."""
+    return lib().zb_gemm2_workspace(c_int(M), c_int(N), c_int(K))
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
          bias: Optional[torch.Tensor] = None, addend: Optional[torch.Tensor] = None, accumulate: bool = False,
          act: Optional[str] = None, bn: int = 0, max_ctas: int = 0, kernel: Optional[str] = None) -> torch.Tensor:
@@ -177,6 +184,17 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, a_mn: bool = Fa
     kern = kernel or GEMM_KERNEL
     if kern in ("2cta", "2cta_accpf") and bn == 0 and M >= 256 and N >= 256:
         accpf = kern == "2cta_accpf" or (GEMM_ACC_PREFETCH and accumulate)
+        # a long reduction whose last wave of tiles would leave most of the GPU idle is cut up there (below this length
+        # it never is: see the kernel's plan)
+        ws_bytes = _gemm2_workspace(M, N, K) if K > 3000 and max_ctas == 0 and not accpf else 0
+        if ws_bytes:
+            ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device)
+            rc = lib().zb_gemm2_split_bf16(_a(a), _a(b), _a(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+                                           int(a_mn), int(b_mn), _a(bias), _a(addend),
+                                           0 if addend is None else addend.stride(0), flags, _a(ws),
+                                           _a(status_word(a.device)), _stream())
+            _check(rc, "gemm2_split")
+            return out
         fn = lib().zb_gemm2_accpf_bf16 if accpf else lib().zb_gemm2_bf16
         rc = fn(_a(a), _a(b), _a(out), M, N, K, a.stride(0),
                                  b.stride(0), out.stride(0), int(a_mn), int(b_mn),
