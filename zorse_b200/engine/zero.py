@@ -184,6 +184,8 @@ class ZeroUnit:
         self.update_event = None
         # ---- offload ----------------------------------------------------------------
         self.host_master = self.host_p = None
+        self.master_dev = self.master_event = None   # device copy of a parked master on its way to the optimizer
+        self.below: Optional["ZeroUnit"] = None       # the unit whose backward comes next
         if cfg.offload_params:
             self._offload_init()
         if self.R == 1 and not cfg.offload_params:
@@ -215,6 +217,20 @@ class ZeroUnit:
         else:
             self.p_shard = self.host_p.clone()
         self.counters.h2d_bytes += self.host_p.numel() * self.host_p.element_size()
+
+    def _fetch_master(self):
+        """Starts the H2D copy of the parked fp32 master for an optimizer inside the backward pass, ahead of the gradient
+        reduction that will wait for it.  It leaves the copy stream's queue as soon as last step's write-back is done, so
+        it runs under the backward pass, and the write-backs have the communication stream to themselves."""
+        if not self.cuda or self.host_master is None or self.master_dev is not None or not self.cfg.optimizer_in_backward:
+            return
+        copy = self.streams.copy
+        if self.update_event is not None:
+            copy.wait_event(self.update_event)
+        with phase("offload.h2d_master"), torch.cuda.stream(copy):
+            self.master_dev = self.host_master.to(self.device, non_blocking=True)
+            self.master_event = torch.cuda.Event()
+            self.master_event.record(copy)
 
     # ------------------------------------------------------------------ parameters
     def prefetch(self):
@@ -306,7 +322,13 @@ class ZeroUnit:
         self.step_count += 1
         offl = self.host_master is not None
         if offl:
-            master = self.host_master.to(self.device, non_blocking=True)
+            master, self.master_dev = self.master_dev, None
+            if master is None:
+                master = self.host_master.to(self.device, non_blocking=True)
+            else:
+                cur = torch.cuda.current_stream()
+                cur.wait_event(self.master_event)
+                master.record_stream(cur)
             p16 = torch.empty(self.shard_n, dtype=self.cfg.compute_dtype, device=self.device)
             self.counters.h2d_bytes += self.host_master.numel() * 4
         else:
@@ -326,6 +348,9 @@ class ZeroUnit:
         g_full = self.grad
         self.grad = None
         self.layer.bind(self.full, None)
+        self._fetch_master()
+        if self.below is not None:
+            self.below._fetch_master()
         gscale = 1.0 / self.R if self.cfg.grad_divide_by_group else 1.0
         if self.rep_group.size > 1 and self.cfg.grad_divide_by_group:
             gscale /= self.rep_group.size
@@ -402,6 +427,7 @@ class ZeroUnit:
 
     def finish_step(self) -> None:
         """End of step: ZeRO-2 units drop their now stale unsharded parameters."""
+        self.master_dev = None
         if self.R > 1 or self.host_p is not None:
             self.full = None
             self.full_event = None
@@ -423,6 +449,7 @@ class ZeroUnit:
         return {"master": mine, "m": self.m, "v": self.v}
 
     def load_state(self, master: torch.Tensor, m: torch.Tensor, v: torch.Tensor, step: int) -> None:
+        self.master_dev = None
         if self.host_master is not None:
             self.host_master.copy_(master)
             self.host_p.copy_(master.to(self.cfg.compute_dtype))
@@ -457,6 +484,8 @@ class StageEngine:
                           streams=self.streams, zero_level=zero_level, counters=self.counters, meta_init=meta_init,
                           shard_ratios=shard_ratios, **kw)
                       for ly, gid in zip(layers, gids)]
+        for lower, upper in zip(self.units, self.units[1:]):
+            upper.below = lower
 
     def __len__(self):
         return len(self.units)
