@@ -6,7 +6,7 @@
 //     (cp.async) while a group is reduced.  A thread reads only the chunks it has requested itself, so the ring needs no
 //     barrier;
 //   * one barrier per row (none where a team is one warp): the (sum g*xhat, sum g) pair is reduced in one pass;
-//   * the column reduction of the per-CTA partial sums runs on H/32 CTAs of 32 x 8 threads (eight
+//   * the column reduction of the per-CTA partial sums runs on H/32 CTAs of 32 x 32 threads (32
 //     rows in flight per column) instead of H/256 CTAs walking all partial rows one after another.
 // Bound by memory latency: with one row per CTA and the next row requested into registers 4616 x 768 took 42 us, now 24;
 // 4096 x 4096 46 -> 38 us, 2048 x 5120 50 -> 34 us (operands not in L2; reduction of the partial sums included).
@@ -196,30 +196,32 @@ static int launch_norm_bwd2(const __nv_bfloat16* dy, const __nv_bfloat16* x, con
   return 0;
 }
 
-// out[h] (+)= sum_p part[p, h] with a 32 x 8 thread block per 32 columns: thread (tx, ty) adds rows
-// ty, ty + 8, ...; the eight partial sums of a column are then added in order by the ty = 0 thread.
+// out[h] (+)= sum_p part[p, h] with a 32 x 32 thread block per 32 columns: thread (tx, ty) adds rows
+// ty, ty + 32, ...; the partial sums of a column are then added by a warp, lane by lane.
 // blockIdx.y selects one of two such sums (weight and bias gradient in one launch).
 template <typename OutT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(1024)
 colsum_accumulate2_kernel(const float* __restrict__ part0, const float* __restrict__ part1, int P, int H,
                           OutT* __restrict__ out0, OutT* __restrict__ out1, int accumulate) {
-  __shared__ float sm[8][33];
+  __shared__ float sm[32][33];
   const float* __restrict__ part = blockIdx.y ? part1 : part0;
   OutT* __restrict__ out = blockIdx.y ? out1 : out0;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int h = blockIdx.x * 32 + tx;
   float s = 0.f;
   if (h < H) {
-    for (int p = ty; p < P; p += 8) s += part[size_t(p) * H + h];
+#pragma unroll 4
+    for (int p = ty; p < P; p += 32) s += part[size_t(p) * H + h];
   }
   sm[ty][tx] = s;
   __syncthreads();
-  if (ty == 0 && h < H) {
-    float t = 0.f;
+  float t = sm[tx][ty];   // column ty, rows tx, tx + 32, ...
 #pragma unroll
-    for (int k = 0; k < 8; ++k) t += sm[k][tx];
-    if (accumulate) t += float(out[h]);
-    out[h] = OutT(t);
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  const int c = blockIdx.x * 32 + ty;
+  if (tx == 0 && c < H) {
+    if (accumulate) t += float(out[c]);
+    out[c] = OutT(t);
   }
 }
 
@@ -228,10 +230,10 @@ int colsum_finish(const float* part0, int P, int H, void* out0, const float* par
                   int accumulate, cudaStream_t stream) {
   const dim3 grid((H + 31) / 32, out1 != nullptr ? 2 : 1);
   if (grad_f32)
-    colsum_accumulate2_kernel<float><<<grid, 256, 0, stream>>>(part0, part1, P, H, static_cast<float*>(out0),
+    colsum_accumulate2_kernel<float><<<grid, 1024, 0, stream>>>(part0, part1, P, H, static_cast<float*>(out0),
                                                                static_cast<float*>(out1), accumulate);
   else
-    colsum_accumulate2_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>(
+    colsum_accumulate2_kernel<__nv_bfloat16><<<grid, 1024, 0, stream>>>(
         part0, part1, P, H, static_cast<__nv_bfloat16*>(out0), static_cast<__nv_bfloat16*>(out1), accumulate);
   ZB_CUDA_OK(cudaGetLastError());
   return 0;

@@ -104,7 +104,10 @@ def _a(t: Optional[torch.Tensor]) -> int:
 
 def status_word(device=None) -> torch.Tensor:
     """Device int32 that kernels write a non-zero code to when a bounded wait runs out."""
-    dev = torch.cuda.current_device() if device is None else torch.device(device).index
+    if isinstance(device, torch.device):
+        dev = device.index
+    else:
+        dev = torch.cuda.current_device() if device is None else torch.device(device).index
     if dev not in _status:
         _status[dev] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{dev}")
     return _status[dev]
@@ -165,15 +168,18 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, a_mn: bool = Fa
     tile ahead of the accumulators) or None = GEMM_KERNEL default ("2cta" for M, N >= 256).
     """
     _bf16(a, "a"); _bf16(b, "b")
+    # shapes, strides and types are read once each: this function runs for every product of a step
     M, N = out.shape
-    K = a.shape[0] if a_mn else a.shape[1]
-    assert (a.shape[1] if a_mn else a.shape[0]) == M, (a.shape, out.shape, a_mn)
-    assert (b.shape == (K, N)) if b_mn else (b.shape == (N, K)), (b.shape, (N, K), b_mn)
-    assert a.stride(-1) == 1 and b.stride(-1) == 1 and out.stride(-1) == 1
-    flags = 0
-    if out.dtype == torch.float32:
+    (rows_a, cols_a), (rows_b, cols_b) = a.shape, b.shape
+    K = rows_a if a_mn else cols_a
+    assert (cols_a if a_mn else rows_a) == M, (a.shape, out.shape, a_mn)
+    assert (rows_b == K and cols_b == N) if b_mn else (rows_b == N and cols_b == K), (b.shape, (N, K), b_mn)
+    (lda, step_a), (ldb, step_b), (ldc, step_c) = a.stride(), b.stride(), out.stride()
+    assert step_a == 1 and step_b == 1 and step_c == 1
+    flags, dtype = 0, out.dtype
+    if dtype == torch.float32:
         flags |= GEMM_OUT_F32
-    elif out.dtype != torch.bfloat16:
+    elif dtype != torch.bfloat16:
         raise TypeError("gemm output must be bf16 or fp32")
     if accumulate:
         flags |= GEMM_ACCUMULATE
@@ -189,21 +195,19 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, a_mn: bool = Fa
         ws_bytes = _gemm2_workspace(M, N, K) if K > 3000 and max_ctas == 0 and not accpf else 0
         if ws_bytes:
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device)
-            rc = lib().zb_gemm2_split_bf16(_a(a), _a(b), _a(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+            rc = lib().zb_gemm2_split_bf16(_a(a), _a(b), _a(out), M, N, K, lda, ldb, ldc,
                                            int(a_mn), int(b_mn), _a(bias), _a(addend),
                                            0 if addend is None else addend.stride(0), flags, _a(ws),
                                            _a(status_word(a.device)), _stream())
             _check(rc, "gemm2_split")
             return out
         fn = lib().zb_gemm2_accpf_bf16 if accpf else lib().zb_gemm2_bf16
-        rc = fn(_a(a), _a(b), _a(out), M, N, K, a.stride(0),
-                                 b.stride(0), out.stride(0), int(a_mn), int(b_mn),
+        rc = fn(_a(a), _a(b), _a(out), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn),
                                  _a(bias), _a(addend), 0 if addend is None else addend.stride(0),
                                  flags, max_ctas, _a(status_word(a.device)), _stream())
         _check(rc, "gemm2")
         return out
-    rc = lib().zb_gemm_bf16(_a(a), _a(b), _a(out), M, N, K, a.stride(0),
-                            b.stride(0), out.stride(0), int(a_mn), int(b_mn),
+    rc = lib().zb_gemm_bf16(_a(a), _a(b), _a(out), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn),
                             _a(bias), _a(addend), 0 if addend is None else addend.stride(0),
                             flags, bn, max_ctas, _a(status_word(a.device)), _stream())
     _check(rc, "gemm")
