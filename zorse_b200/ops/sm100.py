@@ -344,16 +344,19 @@ def adam_step(p, m, v, g, p16, *, lr, beta1, beta2, eps, weight_decay, step, gra
 
 
 # --------------------------------------------------------------------------- attention
-# 0 = by problem size: version 4 (two query tiles per CTA, 256 query rows) when that still gives every SM a
-# CTA, version 1 (one 128-row tile per CTA) for smaller problems; 1 / 2 / 4 force a version.
+# 0 = by problem size: version 4 (two query tiles per CTA, 256 query rows), or version 1 (one 128-row tile per CTA) for
+# small problems; 1 / 2 / 4 force a version.
 ATTN_FWD_VERSION = int(os.environ.get("ZORSE_ATTN_FWD", "0"))
 
 
 ATTN_FWD4_FLAGS = int(os.environ.get("ZORSE_ATTN_FWD4_FLAGS", "1"))
 
 
-def _auto_fwd_version(B: int, S: int, Hq: int) -> int:
-    return 4 if B * Hq * ((S + 255) // 256) >= 148 else 1
+def _auto_fwd_version(B: int, S: int, Hq: int, D: int = 64) -> int:
+    # d = 128: one CTA for two query tiles beats two CTAs long before that fills the GPU (32 heads of 1000 tokens, 128 CTAs:
+    # 38 -> 23 us; 32 heads of 512, 64 CTAs: 16.2 -> 15.2).  d = 64 stays at one CTA per SM: the two versions differ in the
+    # last bit, which steps of the narrow twelve-layer models amplify, for 10 us of 44 (12 heads of 2048 tokens).
+    return 4 if B * Hq * ((S + 255) // 256) >= (64 if D == 128 else 148) else 1
 
 
 def flash_fwd(qkv, B: int, S: int, Hq: int, Hkv: int, D: int, causal: bool = True, window: int = 0,
@@ -361,7 +364,7 @@ def flash_fwd(qkv, B: int, S: int, Hq: int, Hkv: int, D: int, causal: bool = Tru
               trace: Optional[torch.Tensor] = None, trace_ctas: int = 0):
     """qkv: packed [B*S, (Hq+2Hkv)*D]. Returns (out [B*S, Hq*D], lse [B, Hq, S]).
     version 1: one query tile per CTA, S double-buffered in TMEM, P staged through shared memory (default
-    for problems with fewer than 148 pairs of query tiles); version 2: two query tiles per CTA, P kept in
+    for small problems); version 2: two query tiles per CTA, P kept in
     TMEM; version 4 (default otherwise, 143 against 257 us on 32 heads of 4096 tokens, d = 128): two
     query tiles, one MMA issuer, score rows in registers (`flags` 1: two-wide
     fp32 math, 2: also a quarter of the exponentials as a polynomial on the fma pipe; `trace`: zeroed int64 buffer from `flash_fwd4_trace_buffer` for a phase timeline)."""
@@ -370,7 +373,7 @@ def flash_fwd(qkv, B: int, S: int, Hq: int, Hkv: int, D: int, causal: bool = Tru
     out = torch.empty(B * S, Hq * D, dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty(B, Hq, S, dtype=torch.float32, device=qkv.device)
     sc = (1.0 / math.sqrt(D)) if scale is None else scale
-    ver = version or ATTN_FWD_VERSION or _auto_fwd_version(B, S, Hq)
+    ver = version or ATTN_FWD_VERSION or _auto_fwd_version(B, S, Hq, D)
     if ver == 4:
         fl = ATTN_FWD4_FLAGS if flags is None else flags
         _check(lib().zb_flash_fwd4(_a(qkv), _a(out), _a(lse), B, S, Hq, Hkv, D,
