@@ -162,6 +162,10 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if constexpr (!DQ) {
+    chain_trigger();
+    chain_wait();
+  }
 
   if (warp == 8) {
     // ------------------------------ TMA producer ------------------------------
@@ -685,6 +689,7 @@ template <int D>
 __global__ void __launch_bounds__(256)
 attn_bwd2_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                        const float* __restrict__ lse, float* __restrict__ stats, int S, int Hq, int s_pad, int o_vec) {
+  chain_trigger();
   constexpr int LANES = D / 8, GROUPS = 256 / LANES, N = 64 / GROUPS;   // lanes per token, tokens at a time, tokens per group
   __shared__ float sm[64];
   const int s0 = blockIdx.x * 64, h = blockIdx.y, b = blockIdx.z;
@@ -764,20 +769,9 @@ static int launch_bwd2(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const
     attr_set = true;
   }
   dim3 grid(p.Hkv * CL, (p.S + 127) / 128, p.B);
-  if constexpr (CL > 1) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = CL;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(32 * BWD2_WARPS);
-    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-    cfg.stream = stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    ZB_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, tq, tk, tv, tdo, p, stats, s_pad, trace, trace_ctas));
+  if constexpr (!DQ) {
+    ZB_CUDA_OK(launch_chained(kern, grid, 32 * BWD2_WARPS, Cfg::SMEM_BYTES, stream, CL > 1 ? CL : 0, tq, tk, tv, tdo, p, stats,
+                              s_pad, trace, trace_ctas));
   } else {
     kern<<<grid, 32 * BWD2_WARPS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p, stats, s_pad, trace, trace_ctas);
     ZB_CUDA_OK(cudaGetLastError());

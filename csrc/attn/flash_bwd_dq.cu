@@ -44,7 +44,7 @@ template <int D>
 __global__ void __launch_bounds__(320, 1)
 flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
-                    const AttnBwdParams p, const float* __restrict__ stats, int s_pad) {
+                    const AttnBwdParams p, const float* stats, int s_pad) {
   using Cfg = AttnDqCfg<D>;
   constexpr int BM = 128, BN = 128, NK = Cfg::NK, NV = Cfg::NV, DB = D / 64;
   constexpr int BLK = 128 * 128;  // bytes of one [128 rows x 64 cols] bf16 block
@@ -108,6 +108,8 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_trigger();
+  chain_wait();
 
   if (warp == 8) {
     // ------------------------------ TMA producer ------------------------------
@@ -354,8 +356,7 @@ static int launch_dq(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const A
     attr_set = true;
   }
   dim3 grid(p.Hq, (p.S + 127) / 128, p.B);
-  kern<<<grid, 320, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p, stats, s_pad);
-  ZB_CUDA_OK(cudaGetLastError());
+  ZB_CUDA_OK(launch_chained(kern, grid, 320, Cfg::SMEM_BYTES, stream, 0, tq, tk, tv, tdo, p, stats, s_pad));
   return 0;
 }
 

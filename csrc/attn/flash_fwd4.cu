@@ -161,6 +161,8 @@ flash_fwd4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_trigger();
+  chain_wait();
 
   if (warp >= 8) {
     setmaxnreg_dec<FWD4_OTHER_REGS>();
@@ -506,8 +508,7 @@ static int launch_fwd4(const __nv_bfloat16* qkv, int width, const AttnFwd4Params
     attr_set = true;
   }
   dim3 grid(p.Hq, (p.S + 255) / 256, p.B);
-  kern<<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, p);
-  ZB_CUDA_OK(cudaGetLastError());
+  ZB_CUDA_OK(launch_chained(kern, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, 0, tq, tk, tv, p));
   return 0;
 }
 

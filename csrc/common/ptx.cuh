@@ -46,6 +46,13 @@ __device__ __forceinline__ bool zb_in_bounds(bool cond, int* status, int site) {
   return true;
 }
 
+// Overlap of a kernel's start with the end of the one before it in the stream.  chain_trigger: the next kernel may be
+// launched once every CTA of this one has got here (it only lets it take up idle resources early).  chain_wait: returns
+// when the kernel before this one has finished and its writes are visible; every thread of a kernel launched with
+// launch_chained calls it before it touches global memory.  Kernels that wait for other processes do neither.
+__device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 #ifndef ZB_WAIT_NS
 #define ZB_WAIT_NS 2000000000ull  // 2 s per wait
 #endif

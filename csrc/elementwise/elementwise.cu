@@ -27,6 +27,7 @@ __device__ __forceinline__ uint4 pack8e(const float* f) {
 // position of token t = (t % S). sign = +1 forward, -1 backward (transpose rotation).
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ buf, const float* __restrict__ cs, int T,
                             int S, int nheads, int d, int row_stride, float sign) {
+  chain_trigger();
   const int half = d >> 1;
   const int cpr = half >> 3;  // 16-byte chunks per half head
   const long total = long(T) * nheads * cpr;
@@ -61,6 +62,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ buf, const float* __rest
 // gu: [T, 2F] (gate | up), out: [T, F] = silu(gate) * up
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                                   long T, int F) {
+  chain_trigger();
   const int cpr = F >> 3;
   const long total = T * cpr;
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
@@ -78,6 +80,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
 // dgu: [T, 2F]: dgate = dout * up * silu'(gate), dup = dout * silu(gate)
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dout,
                                   __nv_bfloat16* __restrict__ dgu, long T, int F) {
+  chain_trigger();
   const int cpr = F >> 3;
   const long total = T * cpr;
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
@@ -120,6 +123,7 @@ __device__ __forceinline__ float act_bwd(float x, int kind) {
   return 0.5f * (1.f + th) + 0.5f * x * (1.f - th * th) * k0 * (1.f + 3.f * k1 * x * x);
 }
 __global__ void act_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long n8, int kind) {
+  chain_trigger();
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < n8; i += long(gridDim.x) * blockDim.x) {
     float a[8], o[8];
     unpack8e(ld_nc_v4(x + i * 8), a);
@@ -130,6 +134,7 @@ __global__ void act_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat1
 }
 __global__ void act_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
                                __nv_bfloat16* __restrict__ dx, long n8, int kind) {
+  chain_trigger();
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < n8; i += long(gridDim.x) * blockDim.x) {
     float a[8], d[8], o[8];
     unpack8e(ld_nc_v4(x + i * 8), a);
@@ -145,6 +150,7 @@ __global__ void act_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
 __global__ void embedding_fwd_kernel(const long* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
                                      const __nv_bfloat16* __restrict__ pos_table, __nv_bfloat16* __restrict__ out,
                                      int T, int H, int V, int S, int pos_offset) {
+  chain_trigger();
   const int cpr = H >> 3;
   const long total = long(T) * cpr;
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
@@ -225,6 +231,7 @@ __global__ void embedding_bwd_kernel(const long* __restrict__ ids, const __nv_bf
 // 712 us with torch unfold, transpose and conversion, 19 us so.
 __global__ void patches_kernel(const float* __restrict__ img, __nv_bfloat16* __restrict__ out, int C, int Hi, int Wi, int p,
                                int kdim, long total) {
+  chain_trigger();
   const int cpr = kdim >> 3, nx = Wi / p, ny = Hi / p, pp = p * p;
   for (long w = blockIdx.x * long(blockDim.x) + threadIdx.x; w < total; w += long(gridDim.x) * blockDim.x) {
     const int k0 = int(w % cpr) * 8;
@@ -244,6 +251,7 @@ __global__ void patches_kernel(const float* __restrict__ img, __nv_bfloat16* __r
 // p a multiple of 8, Wi of 4, no padding: two 16-byte loads per thread
 __global__ void patches8_kernel(const float* __restrict__ img, __nv_bfloat16* __restrict__ out, int C, int Hi, int Wi, int p,
                                 long total) {
+  chain_trigger();
   const int pp = p * p, cpr = C * pp >> 3, nx = Wi / p, ny = Hi / p;
   for (long w = blockIdx.x * long(blockDim.x) + threadIdx.x; w < total; w += long(gridDim.x) * blockDim.x) {
     const int k = int(w % cpr) * 8;

@@ -196,6 +196,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   cluster_sync_all();  // barriers of both CTAs are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if constexpr (!SCATTER && !FUSED_AG) {
+    chain_trigger();
+    chain_wait();
+  }
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
@@ -562,6 +566,7 @@ static TileOrder gemm2_tile_order(int M, int N, int K) {
 template <int BN>
 __global__ void __launch_bounds__(256)
 gemm2_fixup_kernel(const float* __restrict__ ws, const GemmParams p, const TileOrder order, int first_tile, int splits) {
+  chain_trigger();
   constexpr int CHUNKS = 256 * BN / 8;
   const int w = blockIdx.x * 256 + threadIdx.x;
   const int t = w / CHUNKS, e = w - t * CHUNKS;
@@ -707,8 +712,12 @@ static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, 
     if ((rc = make_tmap_2d_out(&tw, ws, uint64_t(ex.items - ex.full) * 256, BN, BN, true, 32))) return rc;
   }
   if (ex.items < pairs) pairs = ex.items;
-  kern<<<2 * pairs, std::is_same<Params, GemmAgParams>::value ? 320 : 192, Cfg::SMEM_BYTES, stream>>>(ta, tb, tc, tx, tw, p, ex);
-  ZB_CUDA_OK(cudaGetLastError());
+  if constexpr (std::is_same<Params, GemmParams>::value) {
+    ZB_CUDA_OK(launch_chained(kern, dim3(2 * pairs), 192, Cfg::SMEM_BYTES, stream, 0, ta, tb, tc, tx, tw, p, ex));
+  } else {
+    kern<<<2 * pairs, std::is_same<Params, GemmAgParams>::value ? 320 : 192, Cfg::SMEM_BYTES, stream>>>(ta, tb, tc, tx, tw, p, ex);
+    ZB_CUDA_OK(cudaGetLastError());
+  }
   if constexpr (std::is_same<Params, GemmParams>::value) {
     if (ex.splits > 1) {
       gemm2_fixup_kernel<BN><<<(tiles - ex.full) * (BN / 8), 256, 0, stream>>>(ws, p, ex.order, ex.full, ex.splits);

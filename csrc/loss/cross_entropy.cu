@@ -20,6 +20,7 @@ __global__ void __launch_bounds__(CE_THREADS)
 ce_fwd_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const long* __restrict__ targets,
                   __nv_bfloat16* __restrict__ dlogits, float* __restrict__ loss_rows, int T, int V,
                   long ld, float grad_scale, long ignore_index) {
+  chain_trigger();
   __shared__ float red_m[CE_THREADS / 32], red_s[CE_THREADS / 32];
   __shared__ float bc[2];
   const int row = blockIdx.x;

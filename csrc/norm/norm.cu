@@ -23,6 +23,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                 const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
                 float* __restrict__ stats /* [T,2]: mean, rstd */, int T, int H, float eps) {
+  chain_trigger();
   constexpr int TEAM = NORM_THREADS / RW, A = NORM_GROUPS<RW>;
   __shared__ float red[2][RW * 8];
   const int team = threadIdx.x / TEAM, tt = threadIdx.x % TEAM;
@@ -186,6 +187,7 @@ __global__ void colsum_accumulate_kernel(const float* __restrict__ part, int P, 
 // sums were bound by the latency of two-byte loads: 2048 x 20480 91 -> 30 us, 4616 x 3072 48 -> 17 us, finish included.
 __global__ void __launch_bounds__(256)
 colsum_partial8_kernel(const __nv_bfloat16* __restrict__ dy, int T, int N, int ld, float* __restrict__ part) {
+  chain_trigger();
   __shared__ float sm[8][256 + 8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = blockIdx.x * 256 + lane * 8;
@@ -227,6 +229,7 @@ colsum_partial8_kernel(const __nv_bfloat16* __restrict__ dy, int T, int N, int l
 template <typename OutT>
 __global__ void __launch_bounds__(1024)
 colsum_one_kernel(const __nv_bfloat16* __restrict__ dy, int T, int N, int ld, OutT* __restrict__ out, int accumulate) {
+  chain_trigger();
   __shared__ float sm[32][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + (lane & 3) * 8;
@@ -274,6 +277,7 @@ colsum_one_kernel(const __nv_bfloat16* __restrict__ dy, int T, int N, int ld, Ou
 __global__ void __launch_bounds__(256)
 colsum_partial_kernel(const __nv_bfloat16* __restrict__ dy, int T, int N, int ld,
                       float* __restrict__ part) {
+  chain_trigger();
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= N) return;
   float s = 0.f;

@@ -41,6 +41,7 @@ norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
                  const __nv_bfloat16* __restrict__ w, const float* __restrict__ stats,
                  const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                  float* __restrict__ part_dw, float* __restrict__ part_db, int T, int H) {
+  chain_trigger();
   using Cfg = NormBwdCfg<NV>;
   constexpr int TEAM = NORM_THREADS / RW, NS = Cfg::STAGES, A = NORM_GROUPS<RW>;
   extern __shared__ __align__(128) uint8_t ring[];
@@ -203,6 +204,7 @@ template <typename OutT>
 __global__ void __launch_bounds__(1024)
 colsum_accumulate2_kernel(const float* __restrict__ part0, const float* __restrict__ part1, int P, int H,
                           OutT* __restrict__ out0, OutT* __restrict__ out1, int accumulate) {
+  chain_trigger();
   __shared__ float sm[32][33];
   const float* __restrict__ part = blockIdx.y ? part1 : part0;
   OutT* __restrict__ out = blockIdx.y ? out1 : out0;
