@@ -106,8 +106,8 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   uint64_t* pds_full = dp_full + 1;     // 1 (8 arrivals)
   uint64_t* dq_full = pds_full + 1;     // 1
   uint64_t* dq_empty = dq_full + 1;     // 1 (8 arrivals)
-  uint64_t* p_full = dq_empty;          // without the dQ part: P^T is in tensor memory
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dq_empty + 1);
+  uint64_t* p_full = dq_empty;          // without the dQ part: P^T is in tensor memory, one barrier per score buffer
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(dq_empty + NSB);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -151,7 +151,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     mbar_init(dp_full, 1);
     mbar_init(pds_full, 8);
     mbar_init(dq_full, 1);
-    mbar_init(dq_empty, 8);
+    for (int i = 0; i < NSB; ++i) mbar_init(&dq_empty[i], 8);
     mbar_fence_init();
   }
   if (warp == 9) {
@@ -276,7 +276,10 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           issue_a(it + 1);
           tr(TB_MMA_A_ISSUED);
         }
-        if (!mbar_wait(DQ ? pds_full : p_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_MISC)) break;
+        // With two score buffers the compute warps may announce P^T of step it + 1 before this wait has seen that of step
+        // it (their next scores are there already), so each buffer has a barrier of its own: the next phase of this one
+        // needs S^T of step it + 2, which is only issued behind this wait.
+        if (!mbar_wait(DQ ? pds_full : &p_full[it % NSB], uint32_t(DQ ? it : it / NSB) & 1, wctx, ST_TIMEOUT_MISC)) break;
         if (DQ) tr(TB_MMA_PDS_READY);
         tc_fence_after();
         // D: dV += P^T dO, E: dK += dS^T Q  (reduction over the 128 queries; bf16 A operands sit in the
@@ -432,7 +435,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_full);
+        if (lane == 0) mbar_arrive(&p_full[it % NSB]);
         tr(TB_P_DONE);
         if (!__all_sync(0xffffffffu, mbar_wait(dp_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_TMEM_FULL))) { ok = false; break; }
         tr(TB_DP_READY);

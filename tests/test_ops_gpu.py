@@ -468,6 +468,39 @@ def test_flash_bwd_grouped_heads(k, B, S, Hq, Hkv, D, causal, window):
     assert torch.equal(got, again)
 
 
+@pytest.mark.parametrize("B,S,Hq,Hkv", [(1, 640, 8, 2), (1, 2048, 32, 8), (1, 2560, 16, 8), (2, 1000, 12, 12)])
+def test_flash_bwd_narrow_heads_beside_a_busy_stream(k, B, S, Hq, Hkv):
+    """200 backward passes at head size 64 (clusters of four, two and one CTA per key tile, grouped and single heads) while
+    an optimizer saturates memory on another stream: the issuer and the compute warps run against each other at other
+    speeds than on an idle GPU.  Every pass gives the bits of the first, and no wait runs out."""
+    D = 64
+    qkv = _rand(B * S, (Hq + 2 * Hkv) * D, seed=31).cuda()
+    do = _rand(B * S, Hq * D, seed=32).cuda()
+    out, lse = k.flash_fwd(qkv, B, S, Hq, Hkv, D, True, 0)
+    q = qkv.float().requires_grad_(True)
+    (want,) = torch.autograd.grad(ref.attention(q, B, S, Hq, Hkv, D, True, 0), q, do.float())
+    n = 1 << 25
+    p, m, v = (torch.zeros(n, device="cuda") for _ in range(3))
+    g, p16 = torch.ones(n, device="cuda"), torch.empty(n, dtype=torch.bfloat16, device="cuda")
+    k.status_word()
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    first, bad = None, torch.zeros((), dtype=torch.int64, device="cuda")
+    for i in range(200):
+        if i % 2 == 0:      # about one update per two backward passes keeps the other stream busy throughout
+            with torch.cuda.stream(side):
+                k.adam_step(p, m, v, g, p16, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0, step=i + 1)
+        got = k.flash_bwd(do, qkv, out, lse, B, S, Hq, Hkv, D, True, 0)
+        if first is None:
+            first = got
+        else:
+            bad += (got.view(torch.int16) != first.view(torch.int16)).any()
+    torch.cuda.synchronize()
+    k.check_status()
+    assert int(bad) == 0
+    _close(first, want, atol=4e-2, rtol=3e-2)
+
+
 def test_attention_traces_run(k):
     """The in-kernel phase traces terminate, leave the status word clean and record plausible clocks."""
     from zorse_b200.profiler import attn_trace
