@@ -234,31 +234,35 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), ds_addr = smem_u32(sDS);
       const uint32_t r_dp = tmem_base + Cfg::DP_COL;
       auto r_s = [&](int it) { return tmem_base + (NSB == 2 && (it & 1) ? uint32_t(Cfg::S1_COL) : 0u); };
-      bool ok = mbar_wait(kv_full, 0, wctx, ST_TIMEOUT_FULL);
+      bool ok = mbar_wait_warp(kv_full, 0, wctx, ST_TIMEOUT_FULL);
       auto issue_a = [&](int it) {  // S^T = K Q^T
-        if (!elected) return;
-        const uint32_t q_addr = smem_u32(sQ + (it % QS) * Cfg::TILE_BYTES), d = r_s(it);
+        if (elected) {
+          const uint32_t q_addr = smem_u32(sQ + (it % QS) * Cfg::TILE_BYTES), d = r_s(it);
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = uint32_t(kk / 4) * BLK + uint32_t(kk % 4) * 32;
-          umma_f16_ss(d, umma_desc_kmajor(k_addr + off), umma_desc_kmajor(q_addr + off), idesc_s, kk != 0 ? 1u : 0u);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t off = uint32_t(kk / 4) * BLK + uint32_t(kk % 4) * 32;
+            umma_f16_ss(d, umma_desc_kmajor(k_addr + off), umma_desc_kmajor(q_addr + off), idesc_s, kk != 0 ? 1u : 0u);
+          }
+          umma_commit(&s_full[it % NSB]);
         }
-        umma_commit(&s_full[it % NSB]);
+        __syncwarp();
       };
       auto issue_b = [&](uint32_t do_addr) {  // dP^T = V dO^T
-        if (!elected) return;
+        if (elected) {
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = uint32_t(kk / 4) * BLK + uint32_t(kk % 4) * 32;
-          umma_f16_ss(r_dp, umma_desc_kmajor(v_addr + off), umma_desc_kmajor(do_addr + off), idesc_s, kk != 0 ? 1u : 0u);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t off = uint32_t(kk / 4) * BLK + uint32_t(kk % 4) * 32;
+            umma_f16_ss(r_dp, umma_desc_kmajor(v_addr + off), umma_desc_kmajor(do_addr + off), idesc_s, kk != 0 ? 1u : 0u);
+          }
+          umma_commit(dp_full);
         }
-        umma_commit(dp_full);
+        __syncwarp();
       };
-      if (ok) ok = mbar_wait(&q_full[0], 0, wctx, ST_TIMEOUT_FULL);
+      if (ok) ok = mbar_wait_warp(&q_full[0], 0, wctx, ST_TIMEOUT_FULL);
       if (ok) {
         tc_fence_after();
         issue_a(0);
-        ok = mbar_wait(&do_full[0], 0, wctx, ST_TIMEOUT_FULL);
+        ok = mbar_wait_warp(&do_full[0], 0, wctx, ST_TIMEOUT_FULL);
       }
       if (ok) {
         tc_fence_after();
@@ -270,7 +274,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         const uint32_t q_addr = smem_u32(sQ + st * Cfg::TILE_BYTES), do_addr = smem_u32(sDO + st * Cfg::TILE_BYTES);
         if (NSB == 2 && it + 1 < n_iters) {   // its buffer last held P^T of step it - 1, read by the D queued before this
           const int sn = (it + 1) % QS;
-          if (!mbar_wait(&q_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
+          if (!mbar_wait_warp(&q_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
           tr(TB_MMA_QDO_READY);
           tc_fence_after();
           issue_a(it + 1);
@@ -279,7 +283,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         // With two score buffers the compute warps may announce P^T of step it + 1 before this wait has seen that of step
         // it (their next scores are there already), so each buffer has a barrier of its own: the next phase of this one
         // needs S^T of step it + 2, which is only issued behind this wait.
-        if (!mbar_wait(DQ ? pds_full : &p_full[it % NSB], uint32_t(DQ ? it : it / NSB) & 1, wctx, ST_TIMEOUT_MISC)) break;
+        if (!mbar_wait_warp(DQ ? pds_full : &p_full[it % NSB], uint32_t(DQ ? it : it / NSB) & 1, wctx, ST_TIMEOUT_MISC)) break;
         if (DQ) tr(TB_MMA_PDS_READY);
         tc_fence_after();
         // D: dV += P^T dO, E: dK += dS^T Q  (reduction over the 128 queries; bf16 A operands sit in the
@@ -293,18 +297,19 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           }
           umma_commit(&do_empty[st]);     // B_i and D_i are dO_i's readers
         }
+        __syncwarp();
         if constexpr (!DQ) {
           // D needs P^T only, and S^T of the next step goes right behind it (D was P^T's last reader): both run while
           // the compute warps form dS^T, and the next step's exponentials run under E and B
           if (NSB == 1 && it + 1 < n_iters) {
             const int sn = (it + 1) % QS;
-            if (!mbar_wait(&q_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
+            if (!mbar_wait_warp(&q_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
             tr(TB_MMA_QDO_READY);
             tc_fence_after();
             issue_a(it + 1);
             tr(TB_MMA_A_ISSUED);
           }
-          if (!mbar_wait(pds_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_MISC)) break;
+          if (!mbar_wait_warp(pds_full, uint32_t(it) & 1, wctx, ST_TIMEOUT_MISC)) break;
           tr(TB_MMA_PDS_READY);
           tc_fence_after();
         }
@@ -317,12 +322,14 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           }
           umma_commit(&q_empty[st]);
         }
+        __syncwarp();
         if constexpr (!DQ) {
           if (it + 1 == n_iters && elected) umma_commit(dq_full);   // every dK / dV product is done: the write-out may start
+          __syncwarp();
           tr(TB_MMA_DEF_ISSUED);
           if (it + 1 < n_iters) {
             const int sn = (it + 1) % QS;
-            if (!mbar_wait(&do_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
+            if (!mbar_wait_warp(&do_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
             tc_fence_after();
             issue_b(smem_u32(sDO + sn * Cfg::TILE_BYTES));   // overwrites R_dP behind E, its last reader
             tr(TB_MMA_B_ISSUED);
@@ -346,19 +353,20 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           }
           umma_commit(dq_full);
         }
+        __syncwarp();
         }
         tr(TB_MMA_DEF_ISSUED);
         if (it + 1 < n_iters) {
           const int sn = (it + 1) % QS;
-          if (!mbar_wait(&q_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
-          if (!mbar_wait(&do_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
+          if (!mbar_wait_warp(&q_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
+          if (!mbar_wait_warp(&do_full[sn], uint32_t((it + 1) / QS) & 1, wctx, ST_TIMEOUT_FULL)) break;
           tr(TB_MMA_QDO_READY);
           tc_fence_after();
           issue_a(it + 1);
           tr(TB_MMA_A_ISSUED);
           if constexpr (DQ) {
             // dQ_it sits in R_dP until the compute warps have drained it
-            if (!mbar_wait(dq_empty, uint32_t(it) & 1, wctx, ST_TIMEOUT_TMEM_EMPTY)) break;
+            if (!mbar_wait_warp(dq_empty, uint32_t(it) & 1, wctx, ST_TIMEOUT_TMEM_EMPTY)) break;
             tr(TB_MMA_DQ_EMPTY);
             tc_fence_after();
           }

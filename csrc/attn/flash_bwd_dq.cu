@@ -152,31 +152,35 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       auto k_of = [&](int i) { return smem_u32(sK + (i % NK) * Cfg::TILE_BYTES); };
       auto v_of = [&](int i) { return smem_u32(sV + (i % NV) * Cfg::TILE_BYTES); };
       auto issue_s = [&](int i) {    // S_i = Q K_i^T into S[i & 1]
-        if (!elected) return;
-        const uint32_t k_addr = k_of(i);
+        if (elected) {
+          const uint32_t k_addr = k_of(i);
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = uint32_t(kk / 4) * BLK + uint32_t(kk % 4) * 32;
-          umma_f16_ss(tmem_base + uint32_t((i & 1) * 128), umma_desc_kmajor(q_addr + off), umma_desc_kmajor(k_addr + off),
-                      idesc_s, kk != 0 ? 1u : 0u);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t off = uint32_t(kk / 4) * BLK + uint32_t(kk % 4) * 32;
+            umma_f16_ss(tmem_base + uint32_t((i & 1) * 128), umma_desc_kmajor(q_addr + off), umma_desc_kmajor(k_addr + off),
+                        idesc_s, kk != 0 ? 1u : 0u);
+          }
+          umma_commit(&s_full[i & 1]);
         }
-        umma_commit(&s_full[i & 1]);
+        __syncwarp();
       };
       auto issue_dp = [&](int i) {   // dP_i = dO V_i^T
-        if (!elected) return;
-        const uint32_t v_addr = v_of(i);
+        if (elected) {
+          const uint32_t v_addr = v_of(i);
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint32_t off = uint32_t(kk / 4) * BLK + uint32_t(kk % 4) * 32;
-          umma_f16_ss(tmem_base + Cfg::DP_COL, umma_desc_kmajor(do_addr + off), umma_desc_kmajor(v_addr + off), idesc_s,
-                      kk != 0 ? 1u : 0u);
+          for (int kk = 0; kk < D / 16; ++kk) {
+            const uint32_t off = uint32_t(kk / 4) * BLK + uint32_t(kk % 4) * 32;
+            umma_f16_ss(tmem_base + Cfg::DP_COL, umma_desc_kmajor(do_addr + off), umma_desc_kmajor(v_addr + off), idesc_s,
+                        kk != 0 ? 1u : 0u);
+          }
+          umma_commit(dp_full);
+          umma_commit(&v_empty[i % NV]);     // dP_i is V_i's only reader
         }
-        umma_commit(dp_full);
-        umma_commit(&v_empty[i % NV]);     // dP_i is V_i's only reader
+        __syncwarp();
       };
-      bool ok = mbar_wait(qdo_full, 0, wctx, ST_TIMEOUT_FULL);
-      if (ok) ok = mbar_wait(&k_full[0], 0, wctx, ST_TIMEOUT_FULL);
-      if (ok) ok = mbar_wait(&v_full[0], 0, wctx, ST_TIMEOUT_FULL);
+      bool ok = mbar_wait_warp(qdo_full, 0, wctx, ST_TIMEOUT_FULL);
+      if (ok) ok = mbar_wait_warp(&k_full[0], 0, wctx, ST_TIMEOUT_FULL);
+      if (ok) ok = mbar_wait_warp(&v_full[0], 0, wctx, ST_TIMEOUT_FULL);
       if (ok) {
         tc_fence_after();
         issue_s(0);
@@ -184,11 +188,11 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       }
       for (int i = 0; i < n && ok; ++i) {
         if (i + 1 < n) {
-          if (!mbar_wait(&k_full[(i + 1) % NK], uint32_t((i + 1) / NK) & 1, wctx, ST_TIMEOUT_FULL)) break;
+          if (!mbar_wait_warp(&k_full[(i + 1) % NK], uint32_t((i + 1) / NK) & 1, wctx, ST_TIMEOUT_FULL)) break;
           tc_fence_after();
           issue_s(i + 1);            // its buffer last held dS_{i-1}, consumed by the dQ product queued before this
         }
-        if (!mbar_wait(ds_ready, uint32_t(i) & 1, wctx, ST_TIMEOUT_MISC)) break;
+        if (!mbar_wait_warp(ds_ready, uint32_t(i) & 1, wctx, ST_TIMEOUT_MISC)) break;
         tc_fence_after();
         // dQ += dS_i K_i (reduction over the 128 keys; the bf16 A operand sits in the first 32 columns of each
         // 64-column half of S[i & 1])
@@ -203,12 +207,14 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           }
           umma_commit(&k_empty[i % NK]);     // S_i (queued earlier) and dQ_i are K_i's readers
         }
+        __syncwarp();
         if (i + 1 < n) {
-          if (!mbar_wait(&v_full[(i + 1) % NV], uint32_t((i + 1) / NV) & 1, wctx, ST_TIMEOUT_FULL)) break;
+          if (!mbar_wait_warp(&v_full[(i + 1) % NV], uint32_t((i + 1) / NV) & 1, wctx, ST_TIMEOUT_FULL)) break;
           tc_fence_after();
           issue_dp(i + 1);                 // the compute warps had dP_i in registers before they announced dS_i
-        } else if (elected) {
-          umma_commit(dq_done);
+        } else {
+          if (elected) umma_commit(dq_done);
+          __syncwarp();
         }
       }
     }

@@ -212,7 +212,7 @@ flash_fwd4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         auto chain_has = [&](int c, int j) { return hi[c] > lo[c] && j >= lo[c] && j < hi[c]; };
         auto issue_qk = [&](int c, int slot) -> bool {
           if (used[c] == 0) {
-            if (!mbar_wait(&q_full[c], 0, wctx, ST_TIMEOUT_FULL)) return false;
+            if (!mbar_wait_warp(&q_full[c], 0, wctx, ST_TIMEOUT_FULL)) return false;
             tc_fence_after();
           }
           const uint32_t q_addr = smem_u32(sQ + c * Cfg::TILE_BYTES), k_addr = smem_u32(sR + slot * Cfg::TILE_BYTES);
@@ -225,18 +225,20 @@ flash_fwd4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
             }
             umma_commit(&s_full[c]);
           }
+          __syncwarp();
           ++used[c];
           return true;
         };
         // prologue: S_c = Q_c K_{j_lo}^T for the chains that use the first tile
         if (n_tiles > 0) {
-          ok = mbar_wait(&r_full[0], 0, wctx, ST_TIMEOUT_FULL);
+          ok = mbar_wait_warp(&r_full[0], 0, wctx, ST_TIMEOUT_FULL);
           tr(TR_MMA_K_READY);
           tc_fence_after();
 #pragma unroll
           for (int c = 0; c < 2; ++c)
             if (ok && chain_has(c, j_lo)) ok = issue_qk(c, 0);
           if (ok && elected) umma_commit(&r_empty[0]);
+          __syncwarp();
           tr(TR_MMA_QK_ISSUED);
         }
         for (int i = 0; i < n_tiles && ok; ++i) {
@@ -244,7 +246,7 @@ flash_fwd4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           const int tv = 2 * i + 1, tk = 2 * i + 2;  // ring entries of V_j and K_{j+1}
           const int vslot = tv % NSLOT, kslot = tk % NSLOT;
           const bool more = i + 1 < n_tiles;
-          if (!mbar_wait(&r_full[vslot], uint32_t(tv / NSLOT) & 1, wctx, ST_TIMEOUT_FULL)) { ok = false; break; }
+          if (!mbar_wait_warp(&r_full[vslot], uint32_t(tv / NSLOT) & 1, wctx, ST_TIMEOUT_FULL)) { ok = false; break; }
           tr(TR_MMA_V_READY);
           bool k_ready = false;
           const uint32_t v_addr = smem_u32(sR + vslot * Cfg::TILE_BYTES);
@@ -257,7 +259,7 @@ flash_fwd4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
               const uint32_t par = uint32_t(pv_done[c]) & 1;
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
-                if (!mbar_wait(&p_half[2 * c + h], par, wctx, ST_TIMEOUT_MISC)) { ok = false; break; }
+                if (!mbar_wait_warp(&p_half[2 * c + h], par, wctx, ST_TIMEOUT_MISC)) { ok = false; break; }
                 tr(h == 0 ? TR_MMA_P0_READY : TR_MMA_P1_READY);
                 tc_fence_after();
                 if (elected) {
@@ -268,15 +270,17 @@ flash_fwd4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
                                 (pv_done[c] | kk) != 0 ? 1u : 0u);
                   }
                 }
+                __syncwarp();
               }
               if (!ok) break;
               ++pv_done[c];
               if (j == hi[c] - 1 && elected) umma_commit(&o_done[c]);
+              __syncwarp();
               tr(TR_MMA_PV_ISSUED);
             }
             if (more && chain_has(c, j + 1)) {
               if (!k_ready) {
-                if (!mbar_wait(&r_full[kslot], uint32_t(tk / NSLOT) & 1, wctx, ST_TIMEOUT_FULL)) { ok = false; break; }
+                if (!mbar_wait_warp(&r_full[kslot], uint32_t(tk / NSLOT) & 1, wctx, ST_TIMEOUT_FULL)) { ok = false; break; }
                 tr(TR_MMA_K_READY);
                 tc_fence_after();
                 k_ready = true;
@@ -287,12 +291,14 @@ flash_fwd4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           }
           if (!ok) break;
           if (elected) umma_commit(&r_empty[vslot]);
+          __syncwarp();
           if (more) {
             if (!k_ready) {
               // no chain uses K_{j+1} (cannot happen for a key tile inside the union, kept for safety)
-              if (!mbar_wait(&r_full[kslot], uint32_t(tk / NSLOT) & 1, wctx, ST_TIMEOUT_FULL)) { ok = false; break; }
+              if (!mbar_wait_warp(&r_full[kslot], uint32_t(tk / NSLOT) & 1, wctx, ST_TIMEOUT_FULL)) { ok = false; break; }
             }
             if (elected) umma_commit(&r_empty[kslot]);
+            __syncwarp();
           }
         }
       }

@@ -132,6 +132,13 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   }
 }
 
+// mbar_wait of a whole warp: every lane gets the same answer, and none goes on before all have it.  For the loops a warp
+// walks together while one elected lane issues: nothing else there brings the lanes together again, and a lane that lagged
+// by two phases of a barrier would wait for one that is past.  Such a loop also puts a __syncwarp() behind each issue.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, const WaitCtx& w, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, w, code));
+}
+
 // ---------------------------------------------------------------------------
 // proxies / fences
 // ---------------------------------------------------------------------------

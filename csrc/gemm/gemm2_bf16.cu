@@ -232,12 +232,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
               if (int(c / p.gate_cps) == p.gate_self) continue;
               ok = flag_wait_ge(p.gate_flags + c, p.gate_epoch, ZB_WAIT_NS, p.status, ST_TIMEOUT_FLAG);
             }
+            ok = __all_sync(0xffffffffu, ok);
             if (!ok) { *abort_flag = 1; break; }
             asm volatile("fence.proxy.async.global;" ::: "memory");   // the gathered rows were written with plain stores
           }
         }
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, wctx, ST_TIMEOUT_EMPTY)) { ok = false; break; }
+          if (!mbar_wait_warp(&empty[stage], phase ^ 1, wctx, ST_TIMEOUT_EMPTY)) { ok = false; break; }
           uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
           uint8_t* sb = sa + Cfg::A_BYTES;
           if (elected) {
@@ -260,6 +261,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 tma_load_2d_pair(sb + j * BK * 128, &tmap_b, &full[stage], n0 + j * 64, kb * BK);
             }
           }
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -281,11 +283,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         kb_range(item, kb0, kb1);
         const int buf = local & 1;
         const uint32_t use = uint32_t(local >> 1);
-        if (!mbar_wait(&tmem_empty[buf], (use & 1) ^ 1, wctx, ST_TIMEOUT_TMEM_EMPTY)) break;
+        if (!mbar_wait_warp(&tmem_empty[buf], (use & 1) ^ 1, wctx, ST_TIMEOUT_TMEM_EMPTY)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + uint32_t(buf * BN);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full[stage], phase, wctx, ST_TIMEOUT_FULL)) { ok = false; break; }
+          if (!mbar_wait_warp(&full[stage], phase, wctx, ST_TIMEOUT_FULL)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE_BYTES);
           const uint32_t sb = sa + Cfg::A_BYTES;
@@ -298,9 +300,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             }
             umma_commit_pair(&empty[stage]);
           }
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (ok && elected) umma_commit_pair(&tmem_full[buf]);
+        __syncwarp();
       }
     }
   } else if (warp < 6) {

@@ -78,6 +78,31 @@ def test_signatures_match_the_sources():
         assert protos[name] == sig, name
 
 
+def test_loops_walked_by_a_whole_warp_keep_its_lanes_together():
+    """Where one elected lane issues for a warp that walks the loop together, every wait is the warp's (one answer for all
+    lanes) and every issue is followed by a __syncwarp: a lane left behind could wait for a phase that is past."""
+    import pathlib
+    import re
+
+    root = pathlib.Path(__file__).resolve().parent.parent / "csrc"
+    loops = 0
+    for f in root.rglob("*.cu"):
+        for part in f.read_text().split("const bool elected = elect_one();")[1:]:
+            loops += 1
+            body = part[:re.search(r"// -{20,}", part).start()]
+            assert not re.search(r"\bmbar_wait\(", body), f.name
+            for m in re.finditer(r"if \([^()\n]*\belected\) (\{|[^\n{]*\n)", body):
+                end = m.end()
+                if m.group(1) == "{":
+                    depth = 1
+                    while depth:
+                        depth += {"{": 1, "}": -1}.get(body[end], 0)
+                        end += 1
+                rest = re.sub(r"//[^\n]*", "", body[end:]).split()
+                assert rest[0] == "__syncwarp();" or "prefetch_desc" in body[m.end():end], (f.name, body[m.start():end])
+    assert loops == 5
+
+
 def bf(*shape):
     return torch.zeros(*shape, dtype=torch.bfloat16)
 
