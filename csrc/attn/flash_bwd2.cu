@@ -61,13 +61,15 @@ __device__ __forceinline__ void red_add_f32(float* p, float a) {
 __device__ __forceinline__ void cluster_barrier() {   // every thread of every CTA of the cluster
   asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
-// fp32 at the same shared-memory offset in CTA `cta` of the cluster
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t cta) {
-  uint32_t ra;
-  float v;
+// the word at the same shared-memory offset in CTA `cta` of the cluster
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t addr, uint32_t cta) {
+  uint32_t ra, v;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(cta));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(ra) : "memory");
   return v;
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t cta) {
+  return __uint_as_float(ld_cluster_u32(addr, cta));
 }
 
 // DQ = false: the key-tile half of the two-kernel backward (dK and dV only): no dS^T copy in shared memory,
@@ -629,6 +631,11 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           asm volatile("st.shared.b32 [%0], %1;" ::"r"(sums + uint32_t((which * D + c * 32 + k) * 512)), "r"(r[k]) : "memory");
       }
       cluster_barrier();
+      // A rank that gave up holds incomplete sums.  Every warp of it has been through this barrier (a wait that runs out
+      // raises the CTA's abort word first), so all ranks see the same words here and none of them stores.
+      const uint32_t abort_addr = smem_u32(const_cast<int*>(abort_flag));
+#pragma unroll
+      for (int q = 0; q < CL; ++q) ok = ok && ld_cluster_u32(abort_addr, q) == 0;
     }
 #pragma unroll 1
     for (int which = 0; which < 2; ++which) {
