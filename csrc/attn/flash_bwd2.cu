@@ -81,7 +81,7 @@ template <int D, bool TRACE, bool DQ, int CL>
 __global__ void __launch_bounds__(32 * BWD2_WARPS, 1)
 flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                   const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
-                  const AttnBwdParams p, const float* __restrict__ stats, int s_pad,
+                  const AttnBwdParams p, const float* stats, int s_pad,
                   unsigned long long* trace, int trace_ctas) {
   using Cfg = AttnBwd2Cfg<D>;
   constexpr int BM = 128, BN = 128, QS = Cfg::QS, DB = D / 64;

@@ -100,10 +100,11 @@ __host__ __device__ __forceinline__ void tile_at(const TileOrder& o, int tile, i
 __device__ __forceinline__ void epilogue_bias_act(const GemmParams& p, int col0, uint32_t (&r)[32]) {
   if (p.bias != nullptr) {
     if (col0 + 32 <= p.N && (reinterpret_cast<uintptr_t>(p.bias + col0) & 15) == 0) {
+      // plain loads: the kernel may have begun while the one before it was still writing the bias
       const uint4* bp = reinterpret_cast<const uint4*>(p.bias + col0);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const uint4 b = __ldg(bp + j);
+        const uint4 b = bp[j];
         const float2 f0 = unpack_bf16x2(b.x), f1 = unpack_bf16x2(b.y), f2 = unpack_bf16x2(b.z), f3 = unpack_bf16x2(b.w);
         r[8 * j + 0] = __float_as_uint(__uint_as_float(r[8 * j + 0]) + f0.x);
         r[8 * j + 1] = __float_as_uint(__uint_as_float(r[8 * j + 1]) + f0.y);

@@ -134,6 +134,24 @@ def test_gemm_split_last_wave(k, M, N, K, a_mn, b_mn):
     k.check_status()
 
 
+def test_gemm_reads_a_bias_written_by_the_kernel_before(k):
+    """The pair kernel starts under the tail of its predecessor; here that one writes the bias (other values each time, into
+    the same place, from a kernel that lets its successor start at once).  fp32 outputs of exact small whole numbers."""
+    M, N, K = 512, 2048, 256
+    a = torch.ones(M, K, dtype=torch.bfloat16, device="cuda")
+    b = torch.ones(N, K, dtype=torch.bfloat16, device="cuda")
+    bias = torch.zeros(N, dtype=torch.bfloat16, device="cuda")
+    dy = torch.ones(4096, N, dtype=torch.bfloat16, device="cuda") / 4096
+    out = torch.empty(M, N, dtype=torch.float32, device="cuda")
+    bad = torch.zeros((), dtype=torch.int64, device="cuda")
+    for i in range(50):
+        k.colsum_accumulate(dy, bias)                       # bias += 1
+        k.gemm(a, b, out, bias=bias, kernel="2cta")
+        bad += (out != K + i + 1).any()
+    k.check_status()
+    assert int(bad) == 0
+
+
 def test_gemm_epilogues(k):
     M, N, K = 300, 520, 192
     a, b = _rand(M, K, seed=3), _rand(N, K, seed=4)

@@ -103,6 +103,22 @@ def test_loops_walked_by_a_whole_warp_keep_its_lanes_together():
     assert loops == 5
 
 
+def test_kernels_that_start_early_use_coherent_loads():
+    """A kernel launched with launch_chained begins while its predecessor may still write, and a non-coherent load needs
+    memory that nobody writes during the kernel.  (flash_bwd2.cu keeps one in the form that is launched plainly.)"""
+    import pathlib
+    import re
+
+    root = pathlib.Path(__file__).resolve().parent.parent / "csrc"
+    chained = {f.name for f in root.rglob("*.cu") if "launch_chained(" in f.read_text()}
+    assert chained == {"gemm2_bf16.cu", "flash_fwd4.cu", "flash_bwd_dq.cu", "flash_bwd2.cu"}
+    for name in ("gemm/gemm2_bf16.cu", "gemm/gemm_common.cuh", "attn/flash_fwd4.cu", "attn/flash_bwd_dq.cu"):
+        assert not re.search(r"__ldg|ld_nc|ld\.global\.nc", (root / name).read_text()), name
+    main = (root / "attn" / "flash_bwd2.cu").read_text().split("attn_bwd2_stats_kernel")[0]
+    plain = main[main.index("// -lse_q (in log2 units) and -delta_q are the same for every lane"):]   # DQ = true only
+    assert not re.search(r"__ldg|ld_nc|__restrict__", main[:len(main) - len(plain)])
+
+
 def bf(*shape):
     return torch.zeros(*shape, dtype=torch.bfloat16)
 
