@@ -22,10 +22,14 @@ ce_fwd_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const long* __restri
                   long ld, float grad_scale, long ignore_index) {
   chain_trigger();
   __shared__ float red_m[CE_THREADS / 32], red_s[CE_THREADS / 32];
-  __shared__ float bc[2];
+  __shared__ float bc[3];
   const int row = blockIdx.x;
   const __nv_bfloat16* x = logits + row * ld;
   const bool vec = (V % 8 == 0) && (ld % 8 == 0);
+  const long tgt = targets[row];
+  const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= V;
+  // The target's logit is read ahead of the last barrier: behind it other threads may have written the gradient over it.
+  if (threadIdx.x == 0) bc[2] = ignored ? 0.f : __bfloat162float(x[tgt]);
   float m = -INFINITY, s = 0.f;
   if (vec) {
     const uint4* xv = reinterpret_cast<const uint4*>(x);
@@ -71,13 +75,7 @@ ce_fwd_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const long* __restri
   __syncthreads();
   m = bc[0];
   s = bc[1];
-  const long tgt = targets[row];
-  const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= V;
-  if (threadIdx.x == 0) {
-    float l = 0.f;
-    if (!ignored) l = (m + __logf(s)) - __bfloat162float(x[tgt]);
-    loss_rows[row] = l;
-  }
+  if (threadIdx.x == 0) loss_rows[row] = ignored ? 0.f : (m + __logf(s)) - bc[2];
   if (dlogits == nullptr) return;
   const float inv = ignored ? 0.f : grad_scale / s;
   const float gs = ignored ? 0.f : grad_scale;

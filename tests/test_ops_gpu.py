@@ -338,6 +338,22 @@ def test_embedding_bwd_alignment(k, offset, gdt):
     assert torch.equal(dp.float().cpu(), torch.ones(S + 2, H).index_add_(0, torch.arange(B * S) % S + 2, dout.float()))
 
 
+@pytest.mark.parametrize("V", [4104, 32000, 1001])
+def test_cross_entropy_in_place_gives_the_loss_of_the_logits(k, V):
+    """The gradient is written over the logits by all threads of a row while one of them forms the loss.  Targets in the
+    columns that are written first; the loss is that of separate buffers bit for bit, and so is the gradient."""
+    T = 4096
+    logits = (torch.randn(T, V, device="cuda", generator=torch.Generator("cuda").manual_seed(V)) * 2).to(torch.bfloat16)
+    targets = (torch.arange(T, device="cuda") * 8) % min(V, 4096)
+    targets[5] = -100
+    grad = torch.empty_like(logits)
+    want = k.cross_entropy(logits, targets, 0.5, grad)
+    for _ in range(10):
+        x = logits.clone()
+        got = k.cross_entropy(x, targets, 0.5, x)
+        assert torch.equal(got, want) and torch.equal(x, grad)
+
+
 @pytest.mark.parametrize("T,V", [(9, 32000), (64, 50272), (4, 1001)])
 def test_cross_entropy(k, T, V):
     logits = _rand(T, V, seed=1, scale=2.0)
