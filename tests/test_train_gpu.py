@@ -105,6 +105,30 @@ def test_activation_offload_to_pinned_host_matches_the_resident_stash():
     assert losses[True] == pytest.approx(losses[False], rel=2e-3, abs=2e-3), losses
 
 
+def test_a_kernel_that_gave_up_ends_the_step_it_was_part_of(monkeypatch):
+    """train_step_from_host reads the kernels' status word with the loss.  The word is set from the host here, as a kernel
+    does whose wait ran out; a rank that has no loss to wait for raises at its next call."""
+    from zorse_b200.ops.sm100 import KernelError
+    from zorse_b200.trainer import Trainer, TrainerOptions
+
+    tr = Trainer(_cfg(), TrainerOptions(schedule="1f1b", ops="sm100"))
+    batch = tr.synthetic_batch()
+    first = tr.train_step_from_host(batch)
+    word = tr.ops.k.status_word(tr.device)
+    word.fill_(3)
+    with pytest.raises(KernelError, match="accumulator never completed"):
+        tr.train_step_from_host(batch)
+    assert tr.train_step_from_host(batch) < first            # reported once, and the trainer goes on
+    monkeypatch.setattr(tr, "train_step", lambda inputs, targets: None)
+    word.fill_(7)
+    assert tr.train_step_from_host(batch) is None
+    torch.cuda.synchronize()
+    with pytest.raises(KernelError, match="wait ran out"):
+        tr.train_step_from_host(batch)
+    assert tr.train_step_from_host(batch) is None
+    tr.check_kernels()
+
+
 def test_smoke_entry():
     import __graft_entry__ as g
 

@@ -125,10 +125,13 @@ _BOUNDS_SITES = {1: "GEMM tile origin", 2: "GEMM epilogue row / column", 3: "all
 
 def check_status(device=None) -> None:
     """Synchronising read of the status word; raises KernelError if a kernel gave up."""
-    s = status_word(device)
-    v = int(s.item())
+    raise_status(int(status_word(device).item()), device)
+
+
+def raise_status(v: int, device=None) -> None:
+    """Raises KernelError if `v`, a value read from the device's status word, says that a kernel gave up (the word is cleared)."""
     if v != 0:
-        s.zero_()
+        status_word(device).zero_()
         code = v & 0xf
         if code == 8:
             site = (v >> 4) & 0xf

@@ -125,6 +125,8 @@ class Trainer:
                                        defer_tail_wgrad=opt.defer_tail_wgrad or cfg.defer_tail_wgrad or 0,
                                        prepost_recv=opt.prepost_recv)
         self.step_idx = 0
+        self._status_host = (torch.zeros(1, dtype=torch.int32).pin_memory()
+                             if self.ops.name == "sm100" and self.device.type == "cuda" else None)
 
     # ------------------------------------------------------------------ data
     def synthetic_batch(self, seed: Optional[int] = None, pin: bool = True) -> dict:
@@ -181,10 +183,27 @@ class Trainer:
         return loss
 
     def train_step_from_host(self, batch: dict) -> Optional[float]:
-        """Host-to-device copy of this step's inputs, one step, device-to-host read of the loss."""
+        """Host-to-device copy of this step's inputs, one step, device-to-host read of the loss.  Raises KernelError if a
+        kernel of the step gave up, so that its results are not trained on; a rank without the last stage, which waits for
+        nothing here, raises at its next call."""
+        self._raise_kernel_status()
         inputs, targets, _ = self.to_device(batch)
         loss = self.train_step(inputs, targets)
-        return None if loss is None else float(loss.item())
+        if self._status_host is not None:     # rides ahead of the loss on the same stream: one wait for both
+            self._status_host.copy_(self.ops.k.status_word(self.device), non_blocking=True)
+        if loss is None:
+            return None
+        value = float(loss.item())
+        self._raise_kernel_status()
+        return value
+
+    def _raise_kernel_status(self) -> None:
+        """Looks at the last copy of the kernels' status word (no wait: a copy still on its way is seen by the next look)."""
+        if self._status_host is not None:
+            v = int(self._status_host)
+            if v != 0:
+                self._status_host.zero_()
+                self.ops.k.raise_status(v, self.device)
 
     def global_loss(self, loss) -> float:
         """Sum of the last-stage ranks' loss shares (= mean loss of the global batch)."""
