@@ -85,6 +85,55 @@ def test_parameter_offload_trains_like_the_resident_run(schedule):
     assert losses[True] == pytest.approx(losses[False], rel=2e-3, abs=2e-3), losses
 
 
+@pytest.mark.parametrize("schedule", ["layer_major", "zero2", "1f1b"])
+def test_masters_on_their_way_to_the_optimizer_take_few_buffers(schedule, monkeypatch):
+    """Parked fp32 masters travel to the GPU ahead of the optimizer.  With the communication stream held up, so that the host
+    runs a whole backward pass ahead of it, a step needs at most two more units' masters of device memory than one that
+    fetches none ahead (three buffers against the one of its optimizer); a unit that was updated already is not fetched again; every copy is counted once."""
+    from zorse_b200.engine.zero import ZeroUnit
+    from zorse_b200.trainer import Trainer, TrainerOptions
+
+    def peak(ahead):
+        with monkeypatch.context() as m:
+            if not ahead:
+                m.setattr(ZeroUnit, "_fetch_master", lambda self: None)
+            torch.cuda.synchronize()
+            torch.cuda.empty_cache()
+            before = torch.cuda.memory_stats()["active_bytes.all.current"]
+            tr = Trainer(_cfg(model="opt_125m", gbs=1, mbs=1, seq=128, layers=(0, 12)),
+                         TrainerOptions(schedule=schedule, ops="sm100", optimizer_in_backward=True, offload_model_params=True))
+            batch = tr.synthetic_batch()
+            units = tr.stages[0].engine.units
+            counters = tr.stages[0].engine.counters
+            masters = sum(u.host_master.numel() * 4 for u in units)
+            got, losses = [], []
+            for _ in range(3):
+                h2d, d2h = counters.h2d_bytes, counters.d2h_bytes
+                torch.cuda.synchronize()
+                torch.cuda.reset_peak_memory_stats()
+                with torch.cuda.stream(tr.streams.comm):
+                    torch.cuda._sleep(200_000_000)       # about 0.1 s
+                losses.append(tr.train_step_from_host(batch))
+                got.append(torch.cuda.memory_stats()["active_bytes.all.peak"] - before)
+                assert (counters.h2d_bytes - h2d - masters) % 2 == 0
+                bf16 = (counters.h2d_bytes - h2d - masters) / (masters / 2)
+                assert 1 <= bf16 <= 2, "bf16 copies in: one per pass at most, masters once"
+                assert counters.d2h_bytes - d2h == masters + masters // 2
+            tr.check_kernels()
+            if ahead:
+                lower, upper = units[3], units[4]
+                lower.step_count += 1                     # as after its update in this step
+                upper.grad_views()
+                upper.reduce_grads()
+                torch.cuda.synchronize()
+                assert lower.master_slot is None and units[3].below.master_slot is None
+            return max(got), max(u.shard_n for u in units) * 4, losses
+
+    (without, _, want), (with_, unit, losses) = peak(False), peak(True)
+    assert with_ - without <= 2 * unit + (1 << 20), (with_, without, unit)
+    assert losses == pytest.approx(want, rel=1e-3)
+
+
 def test_activation_offload_to_pinned_host_matches_the_resident_stash():
     """Layer inputs parked in pinned host buffers between forward and backward (copy stream both ways)
     against the same recomputing schedule with the stash kept on the device."""

@@ -26,6 +26,7 @@ never on the whole stream (patch.py:873-879).  On CPU (gloo) everything is synch
 """
 from __future__ import annotations
 
+from collections import deque
 from dataclasses import dataclass, field
 from typing import Optional
 
@@ -133,6 +134,40 @@ class Streams:
         return out if by_kind else sum(out.values())
 
 
+class MasterLanding:
+    """Device buffers in which parked fp32 masters land on their way to an optimizer inside the backward pass: three, of the
+    largest unit's size, kept for the life of the stage.  A buffer is taken when a copy into it is issued and given back
+    with the event behind its last use, which the next copy into it waits for.  (A block per fetch from the caching
+    allocator crosses streams and cannot be handed out again before the GPU has passed that point, while the host runs a
+    whole backward pass ahead: every master became resident.)  With two buffers the copy stream, which also brings the bf16
+    shards, waits for a write-back too often: OPT 125M step 41.1 ms against 39.7; a stream of their own lets the masters
+    take link bandwidth from the shards: 42.7; no copy ahead of the optimizer: 44.1."""
+    BUFFERS = 3
+
+    def __init__(self, device: torch.device, streams: Streams, n: int):
+        self.stream = streams.copy
+        self.stream.wait_stream(torch.cuda.current_stream(device))   # the blocks may have been in use there
+        self.bufs = [torch.empty(n, dtype=torch.float32, device=device) for _ in range(self.BUFFERS)]
+        for b in self.bufs:          # not handed out again before both streams have passed, when the stage goes
+            b.record_stream(self.stream)
+            b.record_stream(streams.comm)
+        self.used: list = [None] * self.BUFFERS
+        self.idle = deque(range(self.BUFFERS))
+
+    def take(self) -> Optional[int]:
+        """A buffer, ready for work queued on `stream` from now on; None while all are waited for."""
+        if not self.idle:
+            return None
+        slot = self.idle.popleft()
+        if self.used[slot] is not None:
+            self.stream.wait_event(self.used[slot])
+        return slot
+
+    def give(self, slot: int, event) -> None:
+        self.used[slot] = event
+        self.idle.append(slot)
+
+
 @dataclass
 class Counters:
     all_gathers: int = 0
@@ -184,7 +219,8 @@ class ZeroUnit:
         self.update_event = None
         # ---- offload ----------------------------------------------------------------
         self.host_master = self.host_p = None
-        self.master_dev = self.master_event = None   # device copy of a parked master on its way to the optimizer
+        self.landing: Optional[MasterLanding] = None  # where parked masters land (shared by the stage's units)
+        self.master_slot = self.master_event = None   # buffer of `landing` that holds this unit's, and when it is there
         self.below: Optional["ZeroUnit"] = None       # the unit whose backward comes next
         if cfg.offload_params:
             self._offload_init()
@@ -220,17 +256,29 @@ class ZeroUnit:
 
     def _fetch_master(self):
         """Starts the H2D copy of the parked fp32 master for an optimizer inside the backward pass, ahead of the gradient
-        reduction that will wait for it.  It leaves the copy stream's queue as soon as last step's write-back is done, so
-        it runs under the backward pass, and the write-backs have the communication stream to themselves."""
-        if not self.cuda or self.host_master is None or self.master_dev is not None or not self.cfg.optimizer_in_backward:
+        reduction that will wait for it.  It starts as soon as last step's write-back is done and a landing buffer is free,
+        so it runs under the backward pass, and the write-backs have the communication stream to themselves.  Without a free
+        buffer the optimizer copies the master itself, in line."""
+        if self.landing is None or self.master_slot is not None:
             return
-        copy = self.streams.copy
+        slot = self.landing.take()
+        if slot is None:
+            return
+        stream = self.landing.stream
         if self.update_event is not None:
-            copy.wait_event(self.update_event)
-        with phase("offload.h2d_master"), torch.cuda.stream(copy):
-            self.master_dev = self.host_master.to(self.device, non_blocking=True)
+            stream.wait_event(self.update_event)
+        with phase("offload.h2d_master"), torch.cuda.stream(stream):
+            self.landing.bufs[slot][:self.shard_n].copy_(self.host_master, non_blocking=True)
             self.master_event = torch.cuda.Event()
-            self.master_event.record(copy)
+            self.master_event.record(stream)
+        self.master_slot = slot
+        self.counters.h2d_bytes += self.host_master.numel() * 4
+
+    def _drop_master(self):
+        """Gives back the landing buffer of a master that no optimizer has taken."""
+        if self.master_slot is not None:
+            self.landing.give(self.master_slot, self.master_event)
+            self.master_slot = None
 
     # ------------------------------------------------------------------ parameters
     def prefetch(self):
@@ -322,15 +370,14 @@ class ZeroUnit:
         self.step_count += 1
         offl = self.host_master is not None
         if offl:
-            master, self.master_dev = self.master_dev, None
-            if master is None:
+            slot, self.master_slot = self.master_slot, None
+            if slot is None:
                 master = self.host_master.to(self.device, non_blocking=True)
+                self.counters.h2d_bytes += self.host_master.numel() * 4
             else:
-                cur = torch.cuda.current_stream()
-                cur.wait_event(self.master_event)
-                master.record_stream(cur)
+                torch.cuda.current_stream().wait_event(self.master_event)
+                master = self.landing.bufs[slot][:self.shard_n]
             p16 = torch.empty(self.shard_n, dtype=self.cfg.compute_dtype, device=self.device)
-            self.counters.h2d_bytes += self.host_master.numel() * 4
         else:
             master, p16 = self.master, self.p_shard
         self.ops.adam_step(master, self.m, self.v, g, p16, lr=cfg.lr, beta1=cfg.beta1, beta2=cfg.beta2, eps=cfg.eps,
@@ -338,6 +385,10 @@ class ZeroUnit:
         self.counters.adam_steps += 1
         if offl:
             self.host_master.copy_(master, non_blocking=True)
+            if slot is not None:
+                ev = torch.cuda.Event()
+                ev.record(torch.cuda.current_stream())
+                self.landing.give(slot, ev)
             self.host_p.copy_(p16, non_blocking=True)
             self.counters.d2h_bytes += self.host_master.numel() * 4 + self.host_p.numel() * self.host_p.element_size()
 
@@ -349,7 +400,7 @@ class ZeroUnit:
         self.grad = None
         self.layer.bind(self.full, None)
         self._fetch_master()
-        if self.below is not None:
+        if self.below is not None and self.below.step_count == self.step_count:   # not updated in this step already
             self.below._fetch_master()
         gscale = 1.0 / self.R if self.cfg.grad_divide_by_group else 1.0
         if self.rep_group.size > 1 and self.cfg.grad_divide_by_group:
@@ -427,7 +478,7 @@ class ZeroUnit:
 
     def finish_step(self) -> None:
         """End of step: ZeRO-2 units drop their now stale unsharded parameters."""
-        self.master_dev = None
+        self._drop_master()
         if self.R > 1 or self.host_p is not None:
             self.full = None
             self.full_event = None
@@ -449,7 +500,7 @@ class ZeroUnit:
         return {"master": mine, "m": self.m, "v": self.v}
 
     def load_state(self, master: torch.Tensor, m: torch.Tensor, v: torch.Tensor, step: int) -> None:
-        self.master_dev = None
+        self._drop_master()
         if self.host_master is not None:
             self.host_master.copy_(master)
             self.host_p.copy_(master.to(self.cfg.compute_dtype))
@@ -486,6 +537,10 @@ class StageEngine:
                       for ly, gid in zip(layers, gids)]
         for lower, upper in zip(self.units, self.units[1:]):
             upper.below = lower
+        if device.type == "cuda" and cfg.offload_params and cfg.optimizer_in_backward and self.units:
+            landing = MasterLanding(device, self.streams, max(u.shard_n for u in self.units))
+            for u in self.units:
+                u.landing = landing
 
     def __len__(self):
         return len(self.units)
