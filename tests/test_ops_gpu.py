@@ -134,6 +134,26 @@ def test_gemm_split_last_wave(k, M, N, K, a_mn, b_mn):
     k.check_status()
 
 
+@pytest.mark.parametrize("M,N,K", [(512, 768, 256), (300, 520, 4104), (2500, 2040, 4104)])
+def test_gemm_addend_forms(k, M, N, K):
+    """Every form of addend the pair kernel accepts, with and without a split last wave: own rows, a row stride of its own,
+    one row for all (stride 0), rows that are not 16-byte aligned, and the output itself.  Bounds as in
+    test_gemm_pair_kernel_tile_widths."""
+    a, b = _rand(M, K, seed=1).cuda(), _rand(N, K, seed=2).cuda()
+    want = a.double() @ b.double().t()
+    wide = _rand(M, N + 24, seed=3).cuda()
+    atol = K * math.sqrt(K) * 2.0 ** -24 + 1e-5
+    for add in (wide[:, :N].contiguous(), wide[:, 8:8 + N], wide[:1, :N].expand(M, N), wide[:, 3:3 + N]):
+        for dtype, rtol in ((torch.float32, 0.0), (torch.bfloat16, 2.0 ** -8)):
+            out = torch.full((M, N), 7.0, dtype=dtype, device="cuda")
+            k.gemm(a, b, out, addend=add, kernel="2cta")
+            _close(out, want + add.double(), atol=atol, rtol=rtol)
+    out = wide[:, :N].contiguous()
+    k.gemm(a, b, out, addend=out, kernel="2cta")
+    _close(out, want + wide[:, :N].double(), atol=atol, rtol=2.0 ** -8)
+    k.check_status()
+
+
 def test_gemm_reads_a_bias_written_by_the_kernel_before(k):
     """The pair kernel starts under the tail of its predecessor; here that one writes the bias (other values each time, into
     the same place, from a kernel that lets its successor start at once).  fp32 outputs of exact small whole numbers."""
