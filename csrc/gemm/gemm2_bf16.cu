@@ -658,17 +658,19 @@ static Gemm2Plan gemm2_plan(int M, int N, int K, int pairs, bool may_split) {
   return best;
 }
 
+// Bytes of the fp32 sums of a plan's split tiles (at most one slot per pair).
+static long gemm2_ws_bytes(const Gemm2Plan& plan, int M, int N, int pairs) {
+  if (plan.splits <= 1) return 0;
+  const long tiles = long((M + 255) / 256) * ((N + plan.bn - 1) / plan.bn);
+  return tiles % pairs * plan.splits * 256 * plan.bn * 4;
+}
+
 template <bool A_MN, bool B_MN, typename Params = GemmParams, int BN = 256>
 static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, int ldb, int max_ctas,
-                        cudaStream_t stream, float* ws = nullptr) {
+                        cudaStream_t stream, float* ws = nullptr, long ws_bytes = 0) {
   using Cfg = Gemm2Cfg<BN>;
   int pairs = num_sms() / 2;
   if (max_ctas > 0 && max_ctas / 2 < pairs) pairs = max_ctas / 2 > 0 ? max_ctas / 2 : 1;
-  Gemm2Plan plan = {BN, 1};
-  if constexpr (std::is_same<Params, GemmParams>::value) {
-    plan = gemm2_plan(p.M, p.N, p.K, pairs, ws != nullptr);
-    if (BN == 256 && plan.bn == 128) return launch_gemm2<A_MN, B_MN, Params, 128>(A, B, p, lda, ldb, max_ctas, stream, ws);
-  }
   CUtensorMap ta, tb;
   Gemm2Extra ex = {};
   // TMA epilogue: 16-byte aligned rows that do not overlap (a broadcast addend has a row stride of 0, which no tensor map
@@ -682,6 +684,16 @@ static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, 
       !(f32 ? add : (add && acc)) && (!add || rows_ok(p.addend, p.ld_addend, 2))) {
     ex.ep = f32 ? EP_F32 : EP_BF16;
     ex.ep_load = !f32 && (acc || add);
+  }
+  Gemm2Plan plan = {BN, 1};
+  if constexpr (std::is_same<Params, GemmParams>::value) {
+    // Parts need the boxes of the TMA epilogue and room for the sums of the plan this device gives; whole tiles otherwise.
+    plan = gemm2_plan(p.M, p.N, p.K, pairs, ws != nullptr && ex.ep != EP_DIRECT);
+    if (gemm2_ws_bytes(plan, p.M, p.N, pairs) > ws_bytes) plan = gemm2_plan(p.M, p.N, p.K, pairs, false);
+    if (BN == 256 && plan.bn == 128)
+      return launch_gemm2<A_MN, B_MN, Params, 128>(A, B, p, lda, ldb, max_ctas, stream, ws, ws_bytes);
+  }
+  if (ex.ep != EP_DIRECT) {
     int rc_ep = make_tmap_2d_out(&tc, p.C, p.M, p.N, p.ldc, f32, 32);
     if (rc_ep) return rc_ep;
     if (add) rc_ep = make_tmap_2d_out(&tx, p.addend, p.M, p.N, p.ld_addend, false, 32);
@@ -712,7 +724,7 @@ static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, 
   const int tiles = ex.order.tiles_m * ex.order.tiles_n;
   ex.items = ex.full = tiles;
   ex.splits = 1;
-  if (plan.splits > 1 && ex.ep != EP_DIRECT) {
+  if (plan.splits > 1) {
     ex.full = tiles / pairs * pairs;
     ex.splits = plan.splits;
     ex.items = ex.full + (tiles - ex.full) * ex.splits;
@@ -736,7 +748,7 @@ static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, 
 
 static int gemm2_entry(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                        int a_mn_major, int b_mn_major, const void* bias, const void* addend, int ld_addend, int flags,
-                       int max_ctas, float* ws, int* status, cudaStream_t stream) {
+                       int max_ctas, float* ws, long ws_bytes, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) ZB_FAIL(-1, "gemm2: empty problem %d x %d x %d", M, N, K);
   GemmParams p;
   p.C = C;
@@ -750,10 +762,10 @@ static int gemm2_entry(const void* A, const void* B, void* C, int M, int N, int 
   p.gate_epoch = 0;
   p.gate_base = 0; p.gate_row_bytes = 0; p.gate_shard_bytes = 1;
   p.gate_chunk_bytes = 1; p.gate_cps = 1; p.gate_self = -1;
-  if (!a_mn_major && !b_mn_major) return launch_gemm2<false, false>(A, B, p, lda, ldb, max_ctas, stream, ws);
-  if (!a_mn_major && b_mn_major) return launch_gemm2<false, true>(A, B, p, lda, ldb, max_ctas, stream, ws);
-  if (a_mn_major && b_mn_major) return launch_gemm2<true, true>(A, B, p, lda, ldb, max_ctas, stream, ws);
-  return launch_gemm2<true, false>(A, B, p, lda, ldb, max_ctas, stream, ws);
+  if (!a_mn_major && !b_mn_major) return launch_gemm2<false, false>(A, B, p, lda, ldb, max_ctas, stream, ws, ws_bytes);
+  if (!a_mn_major && b_mn_major) return launch_gemm2<false, true>(A, B, p, lda, ldb, max_ctas, stream, ws, ws_bytes);
+  if (a_mn_major && b_mn_major) return launch_gemm2<true, true>(A, B, p, lda, ldb, max_ctas, stream, ws, ws_bytes);
+  return launch_gemm2<true, false>(A, B, p, lda, ldb, max_ctas, stream, ws, ws_bytes);
 }
 
 }  // namespace zb
@@ -764,24 +776,22 @@ extern "C" int zb_gemm2_workspace(int M, int N, int K) {
   using namespace zb;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const int pairs = num_sms() / 2;
-  const Gemm2Plan plan = gemm2_plan(M, N, K, pairs, true);
-  if (plan.splits <= 1) return 0;
-  const long tiles = long((M + 255) / 256) * ((N + plan.bn - 1) / plan.bn);
-  return int(tiles % pairs * plan.splits * 256 * plan.bn * 4);   // at most one slot per pair
+  return int(gemm2_ws_bytes(gemm2_plan(M, N, K, pairs, true), M, N, pairs));
 }
 
 extern "C" int zb_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                              int a_mn_major, int b_mn_major, const void* bias, const void* addend, int ld_addend,
                              int flags, int max_ctas, int* status, cudaStream_t stream) {
   return zb::gemm2_entry(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, bias, addend, ld_addend, flags, max_ctas,
-                         nullptr, status, stream);
+                         nullptr, 0, status, stream);
 }
-// zb_gemm2_bf16 on the whole GPU with a workspace of zb_gemm2_workspace(M, N, K) bytes.
+// zb_gemm2_bf16 on the whole GPU with a workspace of `workspace_bytes`; one of fewer than the bytes zb_gemm2_workspace(M, N, K)
+// gives on this device is not used.
 extern "C" int zb_gemm2_split_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                                    int a_mn_major, int b_mn_major, const void* bias, const void* addend, int ld_addend,
-                                   int flags, void* workspace, int* status, cudaStream_t stream) {
+                                   int flags, void* workspace, long workspace_bytes, int* status, cudaStream_t stream) {
   return zb::gemm2_entry(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, bias, addend, ld_addend, flags, 0,
-                         static_cast<float*>(workspace), status, stream);
+                         static_cast<float*>(workspace), workspace_bytes, status, stream);
 }
 // C = A @ B^T (b_mn_major: A @ B) with the output rows scattered for a row-wise reduce-scatter over
 // R ranks: rows [q * M / R, (q + 1) * M / R) go to dst_ptrs[q] (this rank's bf16 staging slot in rank

@@ -109,7 +109,7 @@ def test_gemm_split_last_wave(k, M, N, K, a_mn, b_mn):
     direction, through every epilogue.  Bounds as in test_gemm_pair_kernel_tile_widths."""
     if (a_mn and M % 8) or (b_mn and N % 8):
         pytest.skip("MN-major operand needs a 16-byte aligned row stride")
-    assert k._gemm2_workspace(M, N, K) > 0
+    assert k._gemm2_workspace(M, N, K, 0) > 0
     a, b = _rand(M, K, seed=1).cuda(), _rand(N, K, seed=2).cuda()
     want = a.double() @ b.double().t()
     ad, bd = (a.t().contiguous() if a_mn else a), (b.t().contiguous() if b_mn else b)
@@ -132,6 +132,25 @@ def test_gemm_split_last_wave(k, M, N, K, a_mn, b_mn):
     k.gemm(ad, bd, out, a_mn=a_mn, b_mn=b_mn, kernel="2cta", bias=bias, act="relu")
     _close(out, (want + bias.double()).clamp(min=0), atol=atol, rtol=2.0 ** -8)
     k.check_status()
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 520, 8200), (2500, 2040, 4104)])
+@pytest.mark.parametrize("room", [-16, -4, 0])
+def test_gemm_split_stays_inside_its_workspace(k, M, N, K, room):
+    """A workspace smaller than the plan needs is left alone (the product runs in whole tiles); one of the right size is
+    not written past its end.  Guard bytes on both sides."""
+    need = k._gemm2_workspace(M, N, K, 0)
+    assert need > 0
+    a, b = _rand(M, K, seed=1).cuda(), _rand(N, K, seed=2).cuda()
+    out = torch.full((M, N), 7.0, device="cuda")
+    buf = torch.full((need + 8192,), 0x5a, dtype=torch.uint8, device="cuda")
+    rc = k.lib().zb_gemm2_split_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, K, K, N, 0, 0, 0, 0, 0, k.GEMM_OUT_F32,
+                                     buf.data_ptr() + 4096, need + room, k.status_word().data_ptr(), k._stream())
+    k._check(rc, "gemm2_split")
+    k.check_status()
+    _close(out, a.double() @ b.double().t(), atol=K * math.sqrt(K) * 2.0 ** -24 + 1e-5, rtol=0.0)
+    assert bool((buf[:4096] == 0x5a).all()) and bool((buf[4096 + need:] == 0x5a).all())
+    assert bool((buf == 0x5a).all()) == (room < 0)
 
 
 @pytest.mark.parametrize("M,N,K", [(512, 768, 256), (300, 520, 4104), (2500, 2040, 4104)])

@@ -103,6 +103,19 @@ def test_loops_walked_by_a_whole_warp_keep_its_lanes_together():
     assert loops == 5
 
 
+def test_gemm_workspace_sizes_are_kept_per_device(monkeypatch):
+    """The size follows from the SM count of the device, so two devices of one process have entries of their own."""
+    import types
+
+    answers = iter([4096, 8192])
+    monkeypatch.setattr(k, "_lib", types.SimpleNamespace(zb_gemm2_workspace=lambda m, n, kk: next(answers)))
+    k._gemm2_workspace.cache_clear()
+    try:
+        assert [k._gemm2_workspace(304, 264, 8192, d) for d in (0, 1, 0, 1)] == [4096, 8192, 4096, 8192]
+    finally:
+        k._gemm2_workspace.cache_clear()
+
+
 def test_kernels_that_start_early_use_coherent_loads():
     """A kernel launched with launch_chained begins while its predecessor may still write, and a non-coherent load needs
     memory that nobody writes during the kernel.  (flash_bwd2.cu keeps one in the form that is launched plainly.)"""

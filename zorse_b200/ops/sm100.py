@@ -41,7 +41,7 @@ ACT_GELU_ERF = 2
 # with them ctypes converts plain Python numbers itself, which is cheaper than a c_int / c_void_p object per argument.
 _SIGNATURES = {
     "zb_gemm2_bf16": "pppiiiiiiiippiiipp", "zb_gemm2_accpf_bf16": "pppiiiiiiiippiiipp",
-    "zb_gemm2_split_bf16": "pppiiiiiiiippiippp", "zb_gemm_bf16": "pppiiiiiiiippiiiipp",
+    "zb_gemm2_split_bf16": "pppiiiiiiiippiiplpp", "zb_gemm_bf16": "pppiiiiiiiippiiiipp",
     "zb_norm_fwd": "pppppiifip", "zb_norm_fwd2": "pppppiifip",
     "zb_norm_bwd": "ppppppppppiiiiip", "zb_norm_bwd2": "ppppppppppiiiiip",
     "zb_colsum": "piiippiip", "zb_rope": "ppiiiiiip", "zb_swiglu_fwd": "pplip", "zb_swiglu_bwd": "ppplip",
@@ -155,8 +155,9 @@ def _bf16(t: torch.Tensor, name: str) -> None:
 
 # --------------------------------------------------------------------------- GEMM
 @functools.lru_cache(maxsize=4096)
-def _gemm2_workspace(M: int, N: int, K: int) -> int:
-    """Bytes of workspace the pair kernel wants for this product (a function of the sizes), 0 for none."""
+def _gemm2_workspace(M: int, N: int, K: int, device: int) -> int:
+    """Bytes of workspace the pair kernel wants for this product (a function of the sizes and of the number of SMs of the
+    current device, whose index is `device`, as the operands' is), 0 for none."""
     return lib().zb_gemm2_workspace(c_int(M), c_int(N), c_int(K))
 
 
@@ -195,12 +196,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, a_mn: bool = Fa
         accpf = kern == "2cta_accpf" or (GEMM_ACC_PREFETCH and accumulate)
         # a long reduction whose last wave of tiles would leave most of the GPU idle is cut up there (below this length
         # it never is: see the kernel's plan)
-        ws_bytes = _gemm2_workspace(M, N, K) if K > 3000 and max_ctas == 0 and not accpf else 0
+        ws_bytes = _gemm2_workspace(M, N, K, a.device.index) if K > 3000 and max_ctas == 0 and not accpf else 0
         if ws_bytes:
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device)
             rc = lib().zb_gemm2_split_bf16(_a(a), _a(b), _a(out), M, N, K, lda, ldb, ldc,
                                            int(a_mn), int(b_mn), _a(bias), _a(addend),
-                                           0 if addend is None else addend.stride(0), flags, _a(ws),
+                                           0 if addend is None else addend.stride(0), flags, _a(ws), ws_bytes,
                                            _a(status_word(a.device)), _stream())
             _check(rc, "gemm2_split")
             return out
