@@ -541,6 +541,23 @@ def test_flash_bwd_grouped_heads(k, B, S, Hq, Hkv, D, causal, window):
     assert torch.equal(got, again)
 
 
+@pytest.mark.parametrize("window", [300, 301, 4096, 2 ** 31 - 1, 2 ** 40])
+@pytest.mark.parametrize("D", [64, 128])
+def test_flash_window_no_shorter_than_the_sequence(k, D, window):
+    """Such a window hides no key: outputs and gradients have the bits of the call without one, in every version."""
+    B, S, Hq, Hkv = 1, 300, 4, 2
+    qkv, do = _rand(B * S, (Hq + 2 * Hkv) * D, seed=41).cuda(), _rand(B * S, Hq * D, seed=42).cuda()
+    for fwd, bwd in ((1, 2), (2, 3), (4, 3)):
+        want, lse = k.flash_fwd(qkv, B, S, Hq, Hkv, D, True, 0, version=fwd)
+        got, lse2 = k.flash_fwd(qkv, B, S, Hq, Hkv, D, True, window, version=fwd)
+        assert torch.equal(got, want) and torch.equal(lse, lse2)
+        g0 = k.flash_bwd(do, qkv, want, lse, B, S, Hq, Hkv, D, True, 0, version=bwd)
+        g1 = k.flash_bwd(do, qkv, want, lse, B, S, Hq, Hkv, D, True, window, version=bwd)
+        kv = slice(Hq * D, None) if bwd == 2 else slice(None)     # version 2 adds dQ with atomics
+        assert torch.equal(g0[:, kv], g1[:, kv])
+    k.check_status()
+
+
 @pytest.mark.parametrize("B,S,Hq,Hkv", [(1, 640, 8, 2), (1, 2048, 32, 8), (1, 2560, 16, 8), (2, 1000, 12, 12)])
 def test_flash_bwd_narrow_heads_beside_a_busy_stream(k, B, S, Hq, Hkv):
     """200 backward passes at head size 64 (clusters of four, two and one CTA per key tile, grouped and single heads) while

@@ -348,6 +348,12 @@ def adam_step(p, m, v, g, p16, *, lr, beta1, beta2, eps, weight_decay, step, gra
 
 
 # --------------------------------------------------------------------------- attention
+def _window(window: int, S: int) -> int:
+    """0 (none) for a window no shorter than the sequence: every earlier key is visible, and the kernels' 32-bit tile bounds
+    (key + window and the like) stay far from their limit."""
+    return 0 if window >= S else window
+
+
 # 0 = by problem size: version 4 (two query tiles per CTA, 256 query rows), or version 1 (one 128-row tile per CTA) for
 # small problems; 1 / 2 / 4 force a version.
 ATTN_FWD_VERSION = int(os.environ.get("ZORSE_ATTN_FWD", "0"))
@@ -377,6 +383,7 @@ def flash_fwd(qkv, B: int, S: int, Hq: int, Hkv: int, D: int, causal: bool = Tru
     out = torch.empty(B * S, Hq * D, dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty(B, Hq, S, dtype=torch.float32, device=qkv.device)
     sc = (1.0 / math.sqrt(D)) if scale is None else scale
+    window = _window(window, S)
     ver = version or ATTN_FWD_VERSION or _auto_fwd_version(B, S, Hq, D)
     if ver == 4:
         fl = ATTN_FWD4_FLAGS if flags is None else flags
@@ -465,6 +472,7 @@ def flash_bwd(do, qkv, o, lse, B: int, S: int, Hq: int, Hkv: int, D: int, causal
     key tile and dQ per query tile (scores are formed twice; no fp32 dQ accumulator)."""
     _bf16(do, "do"); _bf16(qkv, "qkv")
     assert do.is_contiguous() and qkv.is_contiguous() and o.is_contiguous()
+    window = _window(window, S)
     ver = version or ATTN_BWD_VERSION or 3
     if ver == 3:
         return _flash_bwd3(do, qkv, o, lse, B, S, Hq, Hkv, D, causal, window, scale, trace=trace, trace_ctas=trace_ctas)
