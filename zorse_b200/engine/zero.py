@@ -141,16 +141,19 @@ class MasterLanding:
     allocator crosses streams and cannot be handed out again before the GPU has passed that point, while the host runs a
     whole backward pass ahead: every master became resident.)  With two buffers the copy stream, which also brings the bf16
     shards, waits for a write-back too often: OPT 125M step 41.1 ms against 39.7; a stream of their own lets the masters
-    take link bandwidth from the shards: 42.7; no copy ahead of the optimizer: 44.1."""
+    take link bandwidth from the shards: 42.7; no copy ahead of the optimizer: 44.1.
+    `p16` takes the bf16 image of an update on its way to the host; only the communication stream touches it.  Nothing is
+    then left for the first step of a stage to allocate there (two allocations while the GPU is busy, 1 to 60 ms each)."""
     BUFFERS = 3
 
-    def __init__(self, device: torch.device, streams: Streams, n: int):
+    def __init__(self, device: torch.device, streams: Streams, n: int, compute_dtype: torch.dtype):
         self.stream = streams.copy
-        self.stream.wait_stream(torch.cuda.current_stream(device))   # the blocks may have been in use there
         self.bufs = [torch.empty(n, dtype=torch.float32, device=device) for _ in range(self.BUFFERS)]
-        for b in self.bufs:          # not handed out again before both streams have passed, when the stage goes
-            b.record_stream(self.stream)
-            b.record_stream(streams.comm)
+        self.p16 = torch.empty(n, dtype=compute_dtype, device=device)
+        for s in (streams.copy, streams.comm):
+            s.wait_stream(torch.cuda.current_stream(device))   # the blocks may have been in use there
+            for b in (*self.bufs, self.p16):                   # nor are they handed out before `s` has passed, in the end
+                b.record_stream(s)
         self.used: list = [None] * self.BUFFERS
         self.idle = deque(range(self.BUFFERS))
 
@@ -377,7 +380,8 @@ class ZeroUnit:
             else:
                 torch.cuda.current_stream().wait_event(self.master_event)
                 master = self.landing.bufs[slot][:self.shard_n]
-            p16 = torch.empty(self.shard_n, dtype=self.cfg.compute_dtype, device=self.device)
+            p16 = (self.landing.p16[:self.shard_n] if self.landing is not None else
+                   torch.empty(self.shard_n, dtype=self.cfg.compute_dtype, device=self.device))
         else:
             master, p16 = self.master, self.p_shard
         self.ops.adam_step(master, self.m, self.v, g, p16, lr=cfg.lr, beta1=cfg.beta1, beta2=cfg.beta2, eps=cfg.eps,
@@ -538,7 +542,7 @@ class StageEngine:
         for lower, upper in zip(self.units, self.units[1:]):
             upper.below = lower
         if device.type == "cuda" and cfg.offload_params and cfg.optimizer_in_backward and self.units:
-            landing = MasterLanding(device, self.streams, max(u.shard_n for u in self.units))
+            landing = MasterLanding(device, self.streams, max(u.shard_n for u in self.units), cfg.compute_dtype)
             for u in self.units:
                 u.landing = landing
 
