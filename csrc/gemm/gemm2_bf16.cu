@@ -826,15 +826,6 @@ extern "C" int zb_gemm2_rs_bf16(const void* A, const void* B, int M, int N, int 
   return launch_gemm2<false, false, GemmScatterParams>(A, B, p, lda, ldb, max_ctas, stream);
 }
 
-// Another name of zb_gemm2_bf16: its epilogue requests the old C tile of a bf16 accumulation ahead of the accumulators.
-extern "C" int zb_gemm2_accpf_bf16(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb,
-                                   int ldc, int a_mn_major, int b_mn_major, const void* bias, const void* addend,
-                                   int ld_addend, int flags, int max_ctas, int* status, cudaStream_t stream) {
-  return zb_gemm2_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, bias, addend, ld_addend, flags, max_ctas,
-                       status, stream);
-}
-
-
 // All-gather fused with the GEMM that first consumes the gathered weights, on the 2-CTA core
 // (same contract as zb_ag_gemm_bf16 in gemm_bf16.cu): C[M,N] = A[M,K] * B[N,K]^T (+bias)(+addend),
 // B = a [N,K] weight inside the unit's flat unsharded buffer `full` at byte offset b_offset_bytes.

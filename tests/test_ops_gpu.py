@@ -224,9 +224,6 @@ def test_gemm_large_vs_fp32(k):
     _close(out, want, atol=0.15, rtol=1e-2)
 
 
-CANDIDATES = os.environ.get("ZORSE_TEST_CANDIDATES") == "1"   # kernel versions not yet validated on hardware
-
-
 @pytest.mark.parametrize("bwd_version", [1, 2])
 @pytest.mark.parametrize("T,H", [(5, 512), (300, 4096), (64, 2048), (33, 5120), (1000, 4096)])
 @pytest.mark.parametrize("ln", [False, True])
@@ -620,20 +617,23 @@ def test_a_wait_that_runs_out_reports_and_leaves_the_context_usable(k):
     assert float(x.sum().item()) == 28.0
 
 
-@pytest.mark.skipif(not CANDIDATES, reason="ZORSE_TEST_CANDIDATES=1: first run on hardware pending")
-@pytest.mark.parametrize("M,N,K,a_mn,b_mn", [(512, 768, 1024, True, True), (300, 520, 256, True, True),
-                                              (512, 512, 512, False, False), (256, 1000, 384, False, True)])
+@pytest.mark.parametrize("M,N,K,a_mn,b_mn", [(512, 768, 1024, True, True), (304, 520, 256, True, True),
+                                              (512, 512, 512, False, False), (256, 1000, 384, False, True),
+                                              (300, 1030, 2056, False, False)])
 def test_accumulate_prefetch_gemm_matches_the_default(k, M, N, K, a_mn, b_mn):
-    """The accumulating GEMM that reads the old C tile ahead of the accumulators must give the default kernel's
-    result bit for bit (same arithmetic, same order), ragged edges included, twice in a row."""
+    """The epilogue that requests the old C tile ahead of the accumulators by TMA gives the bits of the one that reads it
+    from global memory, which rows that are not 16-byte aligned take (same arithmetic, same order), ragged edges included,
+    twice in a row."""
     g = torch.Generator(device="cuda").manual_seed(M + N)
     a = torch.randn((K, M) if a_mn else (M, K), device="cuda", generator=g).to(torch.bfloat16)
     b = torch.randn((K, N) if b_mn else (N, K), device="cuda", generator=g).to(torch.bfloat16)
     c0 = torch.randn(M, N, device="cuda", generator=g).to(torch.bfloat16)
-    want, got = c0.clone(), c0.clone()
+    got = torch.empty(M, (N + 7) // 8 * 8, dtype=torch.bfloat16, device="cuda")[:, :N].copy_(c0)
+    want = torch.empty(M, N + 9 + N % 2, dtype=torch.bfloat16, device="cuda")[:, 3:3 + N].copy_(c0)
+    assert want.stride(0) % 2 == 1 and got.stride(0) % 8 == 0
     for _ in range(2):
         k.gemm(a, b, want, a_mn=a_mn, b_mn=b_mn, accumulate=True, kernel="2cta")
-        k.gemm(a, b, got, a_mn=a_mn, b_mn=b_mn, accumulate=True, kernel="2cta_accpf")
+        k.gemm(a, b, got, a_mn=a_mn, b_mn=b_mn, accumulate=True, kernel="2cta")
     k.check_status()
     assert torch.equal(got, want)
 

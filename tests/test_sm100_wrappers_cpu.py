@@ -146,11 +146,12 @@ def test_gemm_dispatch(lib, monkeypatch):
     k.gemm(a, w, out, accumulate=True, kernel="2cta_accpf")
     k.gemm(a[:100], w, out[:100])                        # below the 2-CTA tile: single-CTA kernel
     k.gemm(a, w, out, kernel="1cta", act="gelu", bias=bf(384), addend=bf(512, 384))
-    monkeypatch.setattr(k, "GEMM_ACC_PREFETCH", True)
-    k.gemm(a, w, out, accumulate=True)
-    k.gemm(a, w, out)
-    assert names(lib) == ["zb_gemm2_bf16", "zb_gemm2_accpf_bf16", "zb_gemm_bf16", "zb_gemm_bf16",
-                          "zb_gemm2_accpf_bf16", "zb_gemm2_bf16"]
+    monkeypatch.setattr(k, "_gemm2_workspace", lambda M, N, K, device: 4096)     # a last wave that is worth cutting
+    long_k = bf(512, 4096), bf(384, 4096)
+    for kernel in (None, "2cta", "2cta_accpf"):                                  # names of one kernel, one dispatch
+        k.gemm(*long_k, out, accumulate=True, kernel=kernel)
+    assert names(lib) == ["zb_gemm2_bf16", "zb_gemm2_bf16", "zb_gemm_bf16", "zb_gemm_bf16",
+                          "zb_gemm2_split_bf16", "zb_gemm2_split_bf16", "zb_gemm2_split_bf16"]
     with pytest.raises(TypeError):
         k.gemm(a, w, torch.zeros(512, 384, dtype=torch.float16))
 
@@ -274,7 +275,6 @@ def test_candidate_report_cases_run_end_to_end_on_the_stand_in_library(lib, monk
     monkeypatch.setattr(C, "ATTN_SHAPES", {"7b": (1, 256, 4, 4, 128, 0), "gqa64": (2, 128, 4, 2, 64, 0),
                                            "ragged_window": (1, 200, 4, 2, 128, 64)})
     monkeypatch.setattr(C, "NORM_SHAPES", {"7b": (64, 256), "gqa64": (64, 128), "ragged_window": (50, 320)})
-    monkeypatch.setattr(C, "WGRAD_SHAPES", {"7b_qkv": (256, 512, 256), "7b_gate_up": (256, 768, 256), "ragged": (100, 300, 264)})
     for case in C.CASES:
         r = C.run_case(case, dev="cpu", flush_floats=16)
         assert r["case"] == case and "max_diff" in r and "tolerance" in r and "agrees" in r, r
@@ -307,7 +307,6 @@ def test_a_whole_step_with_every_candidate_version_selected(lib, monkeypatch):
     monkeypatch.setattr(k, "ATTN_BWD_VERSION", 2)
     monkeypatch.setattr(k, "NORM_FWD_VERSION", 2)
     monkeypatch.setattr(k, "NORM_BWD_VERSION", 2)
-    monkeypatch.setattr(k, "GEMM_ACC_PREFETCH", True)
     cfg = parse_pipeline_dict({"model_name": "tiny_llama", "global_batch_size": 4, "microbatch_size": 2,
                                "sequence_length": 256, "vocab_size": 512, "autocast_dtype": "bfloat16",
                                "reduce_dtype": "bfloat16",
@@ -316,7 +315,7 @@ def test_a_whole_step_with_every_candidate_version_selected(lib, monkeypatch):
     tr = Trainer(cfg, TrainerOptions(schedule="1f1b", ops="sm100", activation_recompute=False))
     tr.train_step_from_host(tr.synthetic_batch())
     made = {n for n, _ in lib.calls}
-    assert {"zb_flash_fwd4", "zb_flash_bwd2", "zb_norm_fwd2", "zb_norm_bwd2", "zb_gemm2_accpf_bf16"} <= made, sorted(made)
+    assert {"zb_flash_fwd4", "zb_flash_bwd2", "zb_norm_fwd2", "zb_norm_bwd2", "zb_gemm2_bf16"} <= made, sorted(made)
     assert not ({"zb_flash_fwd", "zb_flash_bwd", "zb_norm_fwd", "zb_norm_bwd"} & made), sorted(made)
 
 
@@ -338,7 +337,7 @@ def test_kernel_bench_with_candidate_rows_runs_end_to_end(lib, monkeypatch, tmp_
 
     rows = json.loads(out.read_text())["rows"]
     ops_seen = {r["op"] for r in rows}
-    assert {"gemm wgrad+= 2cta_accpf", "flash fwd v4 mode2", "flash bwd v2", "rmsnorm fwd v2", "rmsnorm bwd v2",
+    assert {"gemm wgrad+= 2cta", "flash fwd v4 mode2", "flash bwd v2", "rmsnorm fwd v2", "rmsnorm bwd v2",
             "gemm fwd 2cta", "flash fwd", "adam (bf16 grad)"} <= ops_seen, sorted(ops_seen)
     assert capsys.readouterr().out.count("\n") == len(rows)
 

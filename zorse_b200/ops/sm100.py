@@ -29,8 +29,6 @@ GEMM_GELU = 4
 GEMM_RELU = 8
 
 GEMM_KERNEL = os.environ.get("ZORSE_GEMM", "2cta")
-# candidate: accumulating GEMMs (weight gradients) request the old C tile before the tile's accumulators are ready
-GEMM_ACC_PREFETCH = os.environ.get("ZORSE_GEMM_ACC_PREFETCH", "0") == "1"
 
 ACT_GELU_TANH = 0
 ACT_RELU = 1
@@ -40,7 +38,7 @@ ACT_GELU_ERF = 2
 # Argument types of the entry points a training step calls all the time, in order (p pointer, i int, l long, f float):
 # with them ctypes converts plain Python numbers itself, which is cheaper than a c_int / c_void_p object per argument.
 _SIGNATURES = {
-    "zb_gemm2_bf16": "pppiiiiiiiippiiipp", "zb_gemm2_accpf_bf16": "pppiiiiiiiippiiipp",
+    "zb_gemm2_bf16": "pppiiiiiiiippiiipp",
     "zb_gemm2_split_bf16": "pppiiiiiiiippiiplpp", "zb_gemm_bf16": "pppiiiiiiiippiiiipp",
     "zb_norm_fwd": "pppppiifip", "zb_norm_fwd2": "pppppiifip",
     "zb_norm_bwd": "ppppppppppiiiiip", "zb_norm_bwd2": "ppppppppppiiiiip",
@@ -168,8 +166,8 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, a_mn: bool = Fa
 
     a: [M,K] (K-major) or [K,M] when a_mn; b: [N,K] (K-major) or [K,N] when b_mn.
     out: bf16 or fp32 [M,N]. kernel: "1cta" (128x{128,256} tile per CTA), "2cta" (256x256 tile per
-    CTA pair, tcgen05 cta_group::2), "2cta_accpf" (candidate: as "2cta", bf16 `accumulate` reads the old C
-    tile ahead of the accumulators) or None = GEMM_KERNEL default ("2cta" for M, N >= 256).
+    CTA pair, tcgen05 cta_group::2), "2cta_accpf" (another name of "2cta", whose epilogue requests the old C tile of a
+    bf16 `accumulate` ahead of the accumulators) or None = GEMM_KERNEL default ("2cta" for M, N >= 256).
     """
     _bf16(a, "a"); _bf16(b, "b")
     # shapes, strides and types are read once each: this function runs for every product of a step
@@ -193,10 +191,9 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, a_mn: bool = Fa
         flags |= GEMM_RELU
     kern = kernel or GEMM_KERNEL
     if kern in ("2cta", "2cta_accpf") and bn == 0 and M >= 256 and N >= 256:
-        accpf = kern == "2cta_accpf" or (GEMM_ACC_PREFETCH and accumulate)
         # a long reduction whose last wave of tiles would leave most of the GPU idle is cut up there (below this length
         # it never is: see the kernel's plan)
-        ws_bytes = _gemm2_workspace(M, N, K, a.device.index) if K > 3000 and max_ctas == 0 and not accpf else 0
+        ws_bytes = _gemm2_workspace(M, N, K, a.device.index) if K > 3000 and max_ctas == 0 else 0
         if ws_bytes:
             ws = torch.empty(ws_bytes, dtype=torch.uint8, device=a.device)
             rc = lib().zb_gemm2_split_bf16(_a(a), _a(b), _a(out), M, N, K, lda, ldb, ldc,
@@ -205,8 +202,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor, *, a_mn: bool = Fa
                                            _a(status_word(a.device)), _stream())
             _check(rc, "gemm2_split")
             return out
-        fn = lib().zb_gemm2_accpf_bf16 if accpf else lib().zb_gemm2_bf16
-        rc = fn(_a(a), _a(b), _a(out), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn),
+        rc = lib().zb_gemm2_bf16(_a(a), _a(b), _a(out), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn),
                                  _a(bias), _a(addend), 0 if addend is None else addend.stride(0),
                                  flags, max_ctas, _a(status_word(a.device)), _stream())
         _check(rc, "gemm2")
