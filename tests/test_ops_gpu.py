@@ -285,10 +285,10 @@ def test_colsum(k):
     _close(out, dy.float().sum(0), atol=1e-2, rtol=1e-3)
 
 
-@pytest.mark.parametrize("T", [1, 7, 9, 300, 4100])
-@pytest.mark.parametrize("N,width", [(8, 8), (264, 264), (260, 260), (512, 1536), (5120, 5120)])
+@pytest.mark.parametrize("T", [1, 7, 9, 300, 4100, 8192, 8193, 9000])
+@pytest.mark.parametrize("N,width", [(8, 8), (264, 264), (260, 260), (512, 1536), (4096, 4096), (4104, 4104), (5120, 5120)])
 def test_colsum_sizes(k, T, N, width):
-    """Sizes at the edges of the split over CTAs and rows; 260 columns take the kernel for unaligned rows, 512 of 1536 a
+    """Sizes at the edges of the split over CTAs and rows and of the rule for one launch (8192 rows, 4096 columns); 260 columns take the kernel for unaligned rows, 512 of 1536 a
     strided matrix.  Bound: fp32 sums of T bf16 values of unit variance, any order; half an ulp of a bf16 result, doubled
     for the rounding of the comparison."""
     dy = _rand(T, width, seed=T + N).cuda()[:, :N]
@@ -484,10 +484,10 @@ def test_flash_fwd(k, B, S, Hq, Hkv, D, causal, window, version, flags):
 
 
 def test_flash_default_versions_on_a_large_problem(k):
-    """The size-based default picks the two-tile forward here (20 heads x 8 pairs of query tiles >= 148 CTAs);
+    """The size-based default picks the two-tile forward here (20 heads x 8 pairs of query tiles, 160 CTAs);
     forward and backward defaults against the fp32 oracle, grouped-query heads, 2048 tokens."""
     B, S, Hq, Hkv, D = 1, 2048, 20, 4, 128
-    assert k._auto_fwd_version(B, S, Hq) == 4 and k._auto_fwd_version(1, 1000, 8) == 1
+    assert k._auto_fwd_version(B, S, Hq, D) == 4
     qkv = _rand(B * S, (Hq + 2 * Hkv) * D, seed=11)
     do = _rand(B * S, Hq * D, seed=12)
     q = qkv.float().requires_grad_(True)
@@ -498,6 +498,31 @@ def test_flash_default_versions_on_a_large_problem(k):
     k.check_status()
     _close(out, want_o.detach(), atol=2e-2, rtol=2e-2)
     _close(got, want, atol=4e-2, rtol=3e-2)
+
+
+def test_flash_fwd_version_rule(k):
+    """Both sides of both thresholds: CTAs of two query tiles, 64 at head size 128 and 148 at 64."""
+    assert k._auto_fwd_version(1, 1000, 16, 128) == 4 and k._auto_fwd_version(1, 1024, 16, 128) == 4      # 64 CTAs
+    assert k._auto_fwd_version(1, 768, 21, 128) == 1 and k._auto_fwd_version(9, 256, 7, 128) == 1         # 63
+    assert k._auto_fwd_version(1, 1000, 37, 64) == 4 and k._auto_fwd_version(4, 256, 37, 64) == 4         # 148
+    assert k._auto_fwd_version(1, 768, 49, 64) == 1 and k._auto_fwd_version(1, 1000, 16, 64) == 1         # 147, 64
+
+
+@pytest.mark.parametrize("B,S,Hq,Hkv,causal,window", [(1, 1000, 16, 4, True, 0), (2, 600, 12, 12, True, 200), (1, 900, 20, 20, False, 0),
+                                                      (3, 300, 16, 8, True, 0), (1, 1030, 25, 5, True, 0)])
+def test_flash_fwd_default_at_few_ctas(k, B, S, Hq, Hkv, causal, window):
+    """Head size 128 at 64 to 125 CTAs of two query tiles, where the default is the two-tile kernel: output and log-sum-exp
+    through the default dispatch, ragged lengths, one of them (300 and 1030 tokens) with an empty or nearly empty second
+    tile.  Bounds as in test_flash_fwd."""
+    D = 128
+    assert 64 <= B * Hq * ((S + 255) // 256) < 148 and k._auto_fwd_version(B, S, Hq, D) == 4
+    qkv = _rand(B * S, (Hq + 2 * Hkv) * D, seed=51).cuda()
+    out, lse = k.flash_fwd(qkv, B, S, Hq, Hkv, D, causal, window)
+    one, lse1 = k.flash_fwd(qkv, B, S, Hq, Hkv, D, causal, window, version=1)
+    k.check_status()
+    _close(out, ref.attention(qkv.float(), B, S, Hq, Hkv, D, causal, window), atol=2e-2, rtol=2e-2)
+    _close(lse, lse1, atol=1e-3, rtol=1e-4)       # both fp32 sums of the same exponentials, in another order
+    _close(out, one, atol=2e-2, rtol=2e-2)
 
 
 BWD_VERSIONS = [1, 2, 3]

@@ -358,7 +358,7 @@ ATTN_FWD_VERSION = int(os.environ.get("ZORSE_ATTN_FWD", "0"))
 ATTN_FWD4_FLAGS = int(os.environ.get("ZORSE_ATTN_FWD4_FLAGS", "1"))
 
 
-def _auto_fwd_version(B: int, S: int, Hq: int, D: int = 64) -> int:
+def _auto_fwd_version(B: int, S: int, Hq: int, D: int) -> int:
     # d = 128: one CTA for two query tiles beats two CTAs long before that fills the GPU (32 heads of 1000 tokens, 128 CTAs:
     # 38 -> 23 us; 32 heads of 512, 64 CTAs: 16.2 -> 15.2).  d = 64 stays at one CTA per SM: the two versions differ in the
     # last bit, which steps of the narrow twelve-layer models amplify, for 10 us of 44 (12 heads of 2048 tokens).
