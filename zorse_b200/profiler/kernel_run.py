@@ -2,8 +2,9 @@
 `ncu` captures (`ncu --set full --clock-control none -k regex:<name> -c 2 python -m
 zorse_b200.profiler.kernel_run <case>`).  Holds well under a few GB on the device.
 
-cases: gemm_fwd | gemm_dgrad | gemm_wgrad | flash_fwd1 | flash_fwd2 | flash_fwd4 | flash_fwd4p | flash_fwd4q | flash_bwd | flash_bwd2 |
-       flash_bwd3 | flash_bwd3_dkv | flash_bwd3_dq | rmsnorm | rmsnorm_bwd | layernorm_bwd | rope | swiglu_fwd | swiglu_bwd |
+cases: gemm_fwd | gemm_dgrad | gemm_wgrad | flash_fwd1 | flash_fwd2 | flash_fwd4 | flash_fwd4p | flash_fwd4q | flash_bwd1 | flash_bwd2 |
+       flash_bwd | flash_bwd3 | flash_bwd3_dkv | flash_bwd3_dq (flash_bwd: the default version; the last three also as
+       flash64_bwd3... on grouped heads of 64) | rmsnorm | rmsnorm_bwd | layernorm_bwd | rope | swiglu_fwd | swiglu_bwd |
        embedding_fwd | embedding_bwd | adam | ce
 Prints the median CUDA-event time of the repetitions (a 256 MB write between them keeps operands out of L2).
 """
@@ -31,7 +32,8 @@ def main(argv=None):
         fn = {"gemm_fwd": lambda: k.gemm(a, w, out), "gemm_dgrad": lambda: k.gemm(dy, w, dx, b_mn=True),
               "gemm_wgrad": lambda: k.gemm(dy, a, gw, a_mn=True, b_mn=True, accumulate=True)}[case]
     elif case.startswith("flash"):
-        B, S, Hq, Hkv, D = 1, 4096, 32, 32, 128   # qkv 100 MB
+        B, S, Hq, Hkv, D = (4, 4096, 32, 8, 64) if case.startswith("flash64") else (1, 4096, 32, 32, 128)   # qkv 100 MB
+        case = case.replace("flash64", "flash")
         qkv, do = rnd(B * S, (Hq + 2 * Hkv) * D), rnd(B * S, Hq * D)
         out, lse = k.flash_fwd(qkv, B, S, Hq, Hkv, D, True, 0)
         fn = {"flash_fwd1": lambda: k.flash_fwd(qkv, B, S, Hq, Hkv, D, True, 0, version=1),
@@ -39,7 +41,8 @@ def main(argv=None):
               "flash_fwd4": lambda: k.flash_fwd(qkv, B, S, Hq, Hkv, D, True, 0, version=4, flags=0),
               "flash_fwd4p": lambda: k.flash_fwd(qkv, B, S, Hq, Hkv, D, True, 0, version=4, flags=1),
               "flash_fwd4q": lambda: k.flash_fwd(qkv, B, S, Hq, Hkv, D, True, 0, version=4, flags=2),
-              "flash_bwd": lambda: k.flash_bwd(do, qkv, out, lse, B, S, Hq, Hkv, D, True, 0, version=1),
+              "flash_bwd": lambda: k.flash_bwd(do, qkv, out, lse, B, S, Hq, Hkv, D, True, 0),
+              "flash_bwd1": lambda: k.flash_bwd(do, qkv, out, lse, B, S, Hq, Hkv, D, True, 0, version=1),
               "flash_bwd2": lambda: k.flash_bwd(do, qkv, out, lse, B, S, Hq, Hkv, D, True, 0, version=2),
               "flash_bwd3": lambda: k.flash_bwd(do, qkv, out, lse, B, S, Hq, Hkv, D, True, 0, version=3),
               "flash_bwd3_dkv": lambda: k._flash_bwd3(do, qkv, out, lse, B, S, Hq, Hkv, D, True, 0, None, parts=1),
@@ -93,7 +96,7 @@ def main(argv=None):
         torch.cuda.synchronize()
         ts.append(ev0.elapsed_time(ev1))
     k.check_status()
-    print("ok", case, f"median {sorted(ts)[len(ts) // 2]:.4f} ms over {reps} runs")
+    print("ok", (argv or sys.argv[1:])[0], f"median {sorted(ts)[len(ts) // 2]:.4f} ms over {reps} runs")
 
 
 if __name__ == "__main__":
