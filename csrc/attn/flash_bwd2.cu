@@ -2,8 +2,8 @@
 // Same interface, scratch buffers and memory layouts as flash_bwd.cu.
 //
 // One CTA per (batch, kv head, 128-key tile); K and V stay in shared memory, Q / dO tiles of the
-// query heads of the GQA group stream through TWO shared-memory stages.  Scores are computed
-// transposed, keys on the TMEM lanes, so that P^T and dS^T feed the dV / dK products straight
+// query heads of the GQA group stream through two (d = 128) or four (d = 64) shared-memory stages, Q and
+// dO with barriers of their own.  Scores are computed transposed, keys on the TMEM lanes, so that P^T and dS^T feed the dV / dK products straight
 // from tensor memory:
 //     A  S^T  = K Q^T             SS   -> R_S  [0,128)      (columns = queries)
 //     B  dP^T = V dO^T            SS   -> R_dP [128,256)
@@ -87,7 +87,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   constexpr int BM = 128, BN = 128, QS = Cfg::QS, DB = D / 64;
   // With d = 64 tensor memory has room for a second S^T (without the dQ part): the scores of the next step are then formed
   // ahead of this step's P^T, and the compute warps go from one step's dS^T to the next step's exponentials without
-  // waiting for dV and S^T.  32 / 8 heads of 8192 tokens 795 -> 693 us, 2 x 4096 tokens 449 -> 407.
+  // waiting for dV and S^T.  32 / 8 heads of 8192 tokens 718 -> 660 us, 2 x 4096 tokens 398 -> 365 (statistics included).
   constexpr int NSB = (D == 64 && !DQ) ? 2 : 1;
   constexpr int BLK = 128 * 128;  // bytes of one [128 rows x 64 cols] bf16 block
   extern __shared__ uint8_t smem_raw[];
@@ -224,9 +224,10 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   } else if (warp == 9) {
     // ------------------------------ MMA issuer ------------------------------
     // The whole warp walks the loop, one elected lane issues (operands stay in uniform registers).  With that, P^T
-    // announced ahead of dS^T and fp32 P in registers the dK / dV kernel takes, for 4096 tokens, 32 heads, d = 128,
-    // 294 instead of 388 us, and for 2048 tokens, 32 / 8 heads, d = 64, 126 instead of 179 us (clocks per step of the
-    // first: 1460 exponentials, 630 dS^T, 1020 waiting for S^T and dP^T; the tensor pipe is busy for about 2260 of 3110).
+    // announced ahead of dS^T and fp32 P in registers the dK / dV kernel and the statistics take, for 4096 tokens, 32
+    // heads, d = 128, 272 instead of 390 us, and for 2048 tokens, 32 / 8 heads, d = 64, 108 instead of 181 us with one CTA
+    // per key tile (clocks per step of the first: 1460 exponentials, 630 dS^T, 1020 waiting for S^T and dP^T; the tensor
+    // pipe is busy for about 2260 of 3110).
     if (n_iters > 0) {
       const bool elected = elect_one();
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, false, false);  // K-major A and B
@@ -798,9 +799,10 @@ static int launch_bwd2(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const
 }
 
 // CTAs per key tile of the dK / dV kernel.  Splitting pays where one CTA per tile leaves SMs idle or waiting for the
-// longest: 2048 tokens, 32 / 8 heads (128 CTAs) with d = 64 118 -> 81 us, with d = 128 159 -> 112; 512 tokens, d = 128
-// (32 CTAs) 52 -> 38 with two and 32 with four.  From two waves on the second prologue and the sum at the end cost more:
-// 4608 tokens, d = 128 (288 CTAs) 339 -> 357 us, 8 x 512, d = 64 (256 CTAs) 91 -> 95.
+// longest.  One / two / four CTAs, us from cold caches with the statistics: 2048 tokens, 32 / 8 heads (128 tiles), d = 64
+// 108 / 70 / 91, d = 128 152 / 95 / 124; 512 tokens, d = 128 (32 tiles) 46 / 36 / 30.  From two waves on the second prologue
+// and the sum at the end cost as much or more: 4608 tokens, d = 128 (288 tiles) 294 / 314 / 386, 8 x 512, d = 64 (256 tiles)
+// 69 / 73 / 106, 8192 tokens, d = 64 (512 tiles) 662 / 650 / 816.
 static int bwd_cluster(int B, int S, int Hq, int Hkv) {
   const int rep = Hq / Hkv;
   const long ctas = long(Hkv) * ((S + 127) / 128) * B;
