@@ -363,7 +363,9 @@ def main():
             beat()
         tr.synchronize(); tr.barrier()
         t = torch.tensor([(time.perf_counter() - t0) / args.steps * 1e3], device=tr.device)
-        bts = torch.tensor([float(h2d_bytes), 4.0 if loss is not None else 0.0], device=tr.device)
+        # fp32 loss where there is one, and the kernels' 4-byte status word that the call fetches with it
+        d2h_bytes = (4.0 if loss is not None else 0.0) + (4.0 if tr._status_host is not None else 0.0)
+        bts = torch.tensor([float(h2d_bytes), d2h_bytes], device=tr.device)
         if world > 1:
             dist.all_reduce(t, op=dist.ReduceOp.MAX)
             dist.all_reduce(bts)
