@@ -674,13 +674,14 @@ static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, 
   CUtensorMap ta, tb;
   Gemm2Extra ex = {};
   // TMA epilogue: 16-byte aligned rows that do not overlap (a broadcast addend has a row stride of 0, which no tensor map
-  // takes), and at most one tensor to add to a bf16 output
+  // takes), rows of C that end on a 16-byte boundary (a store writes whole 16-byte pieces: it would clear what follows the
+  // last column of a wider matrix), and at most one tensor to add to a bf16 output
   CUtensorMap tc = {}, tx = {}, tw = {};
   const bool f32 = (p.flags & GEMM_OUT_F32) != 0, acc = (p.flags & GEMM_ACCUMULATE) != 0, add = p.addend != nullptr;
   auto rows_ok = [&](const void* base, long ld, int size) {
     return (reinterpret_cast<uintptr_t>(base) & 15) == 0 && ld * size % 16 == 0 && ld >= p.N;
   };
-  if (std::is_same<Params, GemmParams>::value && rows_ok(p.C, p.ldc, f32 ? 4 : 2) &&
+  if (std::is_same<Params, GemmParams>::value && rows_ok(p.C, p.ldc, f32 ? 4 : 2) && p.N % (f32 ? 4 : 8) == 0 &&
       !(f32 ? add : (add && acc)) && (!add || rows_ok(p.addend, p.ld_addend, 2))) {
     ex.ep = f32 ? EP_F32 : EP_BF16;
     ex.ep_load = !f32 && (acc || add);

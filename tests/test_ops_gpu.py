@@ -134,6 +134,25 @@ def test_gemm_split_last_wave(k, M, N, K, a_mn, b_mn):
     k.check_status()
 
 
+@pytest.mark.parametrize("M,K", [(300, 256), (1100, 2056), (300, 8200)])
+@pytest.mark.parametrize("N", [1029, 1030, 1032, 1036])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gemm_writes_only_its_columns(k, M, N, K, dtype):
+    """An output that is the left part of a wider matrix, its rows ending on a 16-byte boundary or not: what follows the last
+    column, and the last row, stays as it was.  Plain, accumulated, with an addend; whole tiles and a split last wave."""
+    a, b = _rand(M, K, seed=1).cuda(), _rand(N, K, seed=2).cuda()
+    want = a.double() @ b.double().t()
+    rtol = 0.0 if dtype == torch.float32 else 2.0 ** -8
+    atol = K * math.sqrt(K) * 2.0 ** -24 + 1e-5
+    add = _rand(M, 1040, seed=3).cuda()[:, :N]
+    for kw, more in (({}, 0.0), ({"accumulate": True}, 3.0), ({"addend": add}, add.double())):
+        full = torch.full((M + 1, 1048), 3.0, dtype=dtype, device="cuda")
+        k.gemm(a, b, full[:M, :N], kernel="2cta", **kw)
+        k.check_status()
+        _close(full[:M, :N], want + more, atol=atol, rtol=rtol)
+        assert bool((full[:M, N:] == 3.0).all()) and bool((full[M] == 3.0).all())
+
+
 @pytest.mark.parametrize("M,N,K", [(300, 520, 8200), (2500, 2040, 4104)])
 @pytest.mark.parametrize("room", [-16, -4, 0])
 def test_gemm_split_stays_inside_its_workspace(k, M, N, K, room):
@@ -644,23 +663,24 @@ def test_a_wait_that_runs_out_reports_and_leaves_the_context_usable(k):
 
 @pytest.mark.parametrize("M,N,K,a_mn,b_mn", [(512, 768, 1024, True, True), (304, 520, 256, True, True),
                                               (512, 512, 512, False, False), (256, 1000, 384, False, True),
-                                              (300, 1030, 2056, False, False)])
+                                              (300, 1032, 2056, False, False)])
 def test_accumulate_prefetch_gemm_matches_the_default(k, M, N, K, a_mn, b_mn):
     """The epilogue that requests the old C tile ahead of the accumulators by TMA gives the bits of the one that reads it
     from global memory, which rows that are not 16-byte aligned take (same arithmetic, same order), ragged edges included,
-    twice in a row."""
+    twice in a row; columns behind the last one stay as they were."""
     g = torch.Generator(device="cuda").manual_seed(M + N)
     a = torch.randn((K, M) if a_mn else (M, K), device="cuda", generator=g).to(torch.bfloat16)
     b = torch.randn((K, N) if b_mn else (N, K), device="cuda", generator=g).to(torch.bfloat16)
     c0 = torch.randn(M, N, device="cuda", generator=g).to(torch.bfloat16)
-    got = torch.empty(M, (N + 7) // 8 * 8, dtype=torch.bfloat16, device="cuda")[:, :N].copy_(c0)
+    rows = torch.full((M, (N + 15) // 8 * 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    got = rows[:, :N].copy_(c0)
     want = torch.empty(M, N + 9 + N % 2, dtype=torch.bfloat16, device="cuda")[:, 3:3 + N].copy_(c0)
     assert want.stride(0) % 2 == 1 and got.stride(0) % 8 == 0
     for _ in range(2):
         k.gemm(a, b, want, a_mn=a_mn, b_mn=b_mn, accumulate=True, kernel="2cta")
         k.gemm(a, b, got, a_mn=a_mn, b_mn=b_mn, accumulate=True, kernel="2cta")
     k.check_status()
-    assert torch.equal(got, want)
+    assert torch.equal(got, want) and bool((rows[:, N:] == 7.0).all())
 
 
 def test_checking_build_gives_the_same_results_and_a_clean_status():
