@@ -706,9 +706,10 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 // 4096 tokens, d = 128 32 -> 12 us, 32 heads of 2048, d = 64 15 -> 4 us (one warp per token and head, four-byte loads).
 template <int D>
 __global__ void __launch_bounds__(256)
-attn_bwd2_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                       const float* __restrict__ lse, float* __restrict__ stats, int S, int Hq, int s_pad, int o_vec) {
+attn_bwd2_stats_kernel(const __nv_bfloat16* o, const __nv_bfloat16* d_o,
+                       const float* lse, float* stats, int S, int Hq, int s_pad, int o_vec) {
   chain_trigger();
+  chain_wait();
   constexpr int LANES = D / 8, GROUPS = 256 / LANES, N = 64 / GROUPS;   // lanes per token, tokens at a time, tokens per group
   __shared__ float sm[64];
   const int s0 = blockIdx.x * 64, h = blockIdx.y, b = blockIdx.z;
@@ -720,9 +721,9 @@ attn_bwd2_stats_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16*
     x[i] = y[i] = make_uint4(0u, 0u, 0u, 0u);
     if (s < S) {
       const size_t at = ((size_t(b) * S + s) * Hq + h) * D + l * 8;
-      y[i] = ld_nc_v4(d_o + at);
+      y[i] = ld_v4(d_o + at);
       if (o_vec) {
-        x[i] = ld_nc_v4(o + at);
+        x[i] = ld_v4(o + at);
       } else {
         const uint32_t* p = reinterpret_cast<const uint32_t*>(o + at);
         x[i] = make_uint4(p[0], p[1], p[2], p[3]);
@@ -757,8 +758,9 @@ static int launch_stats(const __nv_bfloat16* o, const __nv_bfloat16* d_o, const 
   const dim3 grid((S + 63) / 64, Hq, B);
   const int o_vec = (reinterpret_cast<uintptr_t>(o) & 15) == 0;   // (dO is fetched by TMA and aligned anyway)
   if (reinterpret_cast<uintptr_t>(d_o) & 15) ZB_FAIL(-4, "attention: dO not 16-byte aligned");
-  if (D == 128) attn_bwd2_stats_kernel<128><<<grid, 256, 0, stream>>>(o, d_o, lse, stats, S, Hq, s_pad, o_vec);
-  else attn_bwd2_stats_kernel<64><<<grid, 256, 0, stream>>>(o, d_o, lse, stats, S, Hq, s_pad, o_vec);
+  if (D == 128) ZB_CUDA_OK(launch_pass(attn_bwd2_stats_kernel<128>, grid, 256, 0, stream, o, d_o, lse, stats, S, Hq, s_pad,
+                                       o_vec));
+  else ZB_CUDA_OK(launch_pass(attn_bwd2_stats_kernel<64>, grid, 256, 0, stream, o, d_o, lse, stats, S, Hq, s_pad, o_vec));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -130,6 +130,15 @@ inline cudaError_t launch_chained(void (*kern)(KArgs...), dim3 grid, int threads
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 
+// The same for the passes over memory (norms, activations, RoPE, column sums, loss): `kern` starts with chain_trigger and
+// chain_wait and reads its inputs with coherent loads.  A plain launch leaves about 2 us between two kernels, and a
+// block's backward has eleven of these.  Steps: BERT 10.22 -> 9.80 ms, ViT 13.69 -> 13.21, GPT of 512 21.1 -> 20.2; the large
+// models, whose clock follows their power, gain nothing.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pass(void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t stream, Args&&... args) {
+  return launch_chained(kern, grid, threads, smem, stream, 0, static_cast<Args&&>(args)...);
+}
+
 inline int num_sms() {
   static int n[64] = {0};
   int dev = 0;

@@ -409,6 +409,14 @@ __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
                : "l"(p));
   return v;
 }
+// The same through the coherent path, for kernels that may begin while their input is still being written (chain_wait).
+__device__ __forceinline__ uint4 ld_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
 // Peer (or any coherent) 16-byte load that must not use the non-coherent path.
 __device__ __forceinline__ uint4 ld_v4_relaxed_sys(const void* p) {
   uint4 v;

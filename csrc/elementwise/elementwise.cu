@@ -25,9 +25,10 @@ __device__ __forceinline__ uint4 pack8e(const float* f) {
 // buf: [T, row_stride] bf16; heads 0..nheads-1 of width d start at column 0 (q heads then
 // k heads in the packed QKV layout). cs: [S, d] fp32 = cos(d/2) | sin(d/2) per position.
 // position of token t = (t % S). sign = +1 forward, -1 backward (transpose rotation).
-__global__ void rope_kernel(__nv_bfloat16* __restrict__ buf, const float* __restrict__ cs, int T,
+__global__ void rope_kernel(__nv_bfloat16* buf, const float* cs, int T,
                             int S, int nheads, int d, int row_stride, float sign) {
   chain_trigger();
+  chain_wait();
   const int half = d >> 1;
   const int cpr = half >> 3;  // 16-byte chunks per half head
   const long total = long(T) * nheads * cpr;
@@ -60,9 +61,10 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ buf, const float* __rest
 
 // ------------------------------- SwiGLU -------------------------------
 // gu: [T, 2F] (gate | up), out: [T, F] = silu(gate) * up
-__global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
+__global__ void swiglu_fwd_kernel(const __nv_bfloat16* gu, __nv_bfloat16* out,
                                   long T, int F) {
   chain_trigger();
+  chain_wait();
   const int cpr = F >> 3;
   const long total = T * cpr;
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
@@ -70,17 +72,18 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfl
     const int c = int(i % cpr);
     const __nv_bfloat16* g = gu + t * 2 * F + c * 8;
     float a[8], b[8], o[8];
-    unpack8e(ld_nc_v4(g), a);
-    unpack8e(ld_nc_v4(g + F), b);
+    unpack8e(ld_v4(g), a);
+    unpack8e(ld_v4(g + F), b);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = a[j] / (1.f + __expf(-a[j])) * b[j];
     *reinterpret_cast<uint4*>(out + t * F + c * 8) = pack8e(o);
   }
 }
 // dgu: [T, 2F]: dgate = dout * up * silu'(gate), dup = dout * silu(gate)
-__global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __nv_bfloat16* __restrict__ dout,
-                                  __nv_bfloat16* __restrict__ dgu, long T, int F) {
+__global__ void swiglu_bwd_kernel(const __nv_bfloat16* gu, const __nv_bfloat16* dout,
+                                  __nv_bfloat16* dgu, long T, int F) {
   chain_trigger();
+  chain_wait();
   const int cpr = F >> 3;
   const long total = T * cpr;
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
@@ -88,9 +91,9 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
     const int c = int(i % cpr);
     const __nv_bfloat16* g = gu + t * 2 * F + c * 8;
     float a[8], b[8], d[8], da[8], db[8];
-    unpack8e(ld_nc_v4(g), a);
-    unpack8e(ld_nc_v4(g + F), b);
-    unpack8e(ld_nc_v4(dout + t * F + c * 8), d);
+    unpack8e(ld_v4(g), a);
+    unpack8e(ld_v4(g + F), b);
+    unpack8e(ld_v4(dout + t * F + c * 8), d);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       float sg = 1.f / (1.f + __expf(-a[j]));
@@ -122,23 +125,25 @@ __device__ __forceinline__ float act_bwd(float x, int kind) {
   float th = tanhf(u);
   return 0.5f * (1.f + th) + 0.5f * x * (1.f - th * th) * k0 * (1.f + 3.f * k1 * x * x);
 }
-__global__ void act_fwd_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y, long n8, int kind) {
+__global__ void act_fwd_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, long n8, int kind) {
   chain_trigger();
+  chain_wait();
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < n8; i += long(gridDim.x) * blockDim.x) {
     float a[8], o[8];
-    unpack8e(ld_nc_v4(x + i * 8), a);
+    unpack8e(ld_v4(x + i * 8), a);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = act_fwd(a[j], kind);
     *reinterpret_cast<uint4*>(y + i * 8) = pack8e(o);
   }
 }
-__global__ void act_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy,
-                               __nv_bfloat16* __restrict__ dx, long n8, int kind) {
+__global__ void act_bwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* dy,
+                               __nv_bfloat16* dx, long n8, int kind) {
   chain_trigger();
+  chain_wait();
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < n8; i += long(gridDim.x) * blockDim.x) {
     float a[8], d[8], o[8];
-    unpack8e(ld_nc_v4(x + i * 8), a);
-    unpack8e(ld_nc_v4(dy + i * 8), d);
+    unpack8e(ld_v4(x + i * 8), a);
+    unpack8e(ld_v4(dy + i * 8), d);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = d[j] * act_bwd(a[j], kind);
     *reinterpret_cast<uint4*>(dx + i * 8) = pack8e(o);
@@ -147,10 +152,11 @@ __global__ void act_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_b
 
 // ------------------------------- embedding -------------------------------
 // out[t, :] = table[ids[t], :] (+ pos_table[(t % S) + pos_offset, :])
-__global__ void embedding_fwd_kernel(const long* __restrict__ ids, const __nv_bfloat16* __restrict__ table,
-                                     const __nv_bfloat16* __restrict__ pos_table, __nv_bfloat16* __restrict__ out,
+__global__ void embedding_fwd_kernel(const long* ids, const __nv_bfloat16* table,
+                                     const __nv_bfloat16* pos_table, __nv_bfloat16* out,
                                      int T, int H, int V, int S, int pos_offset) {
   chain_trigger();
+  chain_wait();
   const int cpr = H >> 3;
   const long total = long(T) * cpr;
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
@@ -196,16 +202,18 @@ __device__ __forceinline__ void red_add8(__nv_bfloat16* p, const uint4& u) {
 }
 // VEC: both tables 16-byte aligned
 template <typename GT, bool VEC>
-__global__ void embedding_bwd_kernel(const long* __restrict__ ids, const __nv_bfloat16* __restrict__ dout,
-                                     GT* __restrict__ dtable, GT* __restrict__ dpos, int T, int H, int V,
+__global__ void embedding_bwd_kernel(const long* ids, const __nv_bfloat16* dout,
+                                     GT* dtable, GT* dpos, int T, int H, int V,
                                      int S, int pos_offset) {
+  chain_trigger();
+  chain_wait();
   const int cpr = H >> 3;
   const long total = long(T) * cpr;
   for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < total; i += long(gridDim.x) * blockDim.x) {
     const int t = int(i / cpr), c = int(i % cpr);
     long id = ids[t];
     id = id < 0 ? 0 : (id >= V ? V - 1 : id);
-    const uint4 u = ld_nc_v4(dout + size_t(t) * H + c * 8);
+    const uint4 u = ld_v4(dout + size_t(t) * H + c * 8);
     GT* dst = dtable + id * H + c * 8;
     if constexpr (VEC) {
       red_add8(dst, u);
@@ -229,9 +237,10 @@ __global__ void embedding_bwd_kernel(const long* __restrict__ ids, const __nv_bf
 // as a GEMM operand).  One thread writes 16 bytes; with p a multiple of 8 its eight values are one row segment.  A pure
 // copy: reads of the image and writes of the operand, both in order within a patch row.  8 images of 3 x 384 x 384, p = 16:
 // 712 us with torch unfold, transpose and conversion, 19 us so.
-__global__ void patches_kernel(const float* __restrict__ img, __nv_bfloat16* __restrict__ out, int C, int Hi, int Wi, int p,
+__global__ void patches_kernel(const float* img, __nv_bfloat16* out, int C, int Hi, int Wi, int p,
                                int kdim, long total) {
   chain_trigger();
+  chain_wait();
   const int cpr = kdim >> 3, nx = Wi / p, ny = Hi / p, pp = p * p;
   for (long w = blockIdx.x * long(blockDim.x) + threadIdx.x; w < total; w += long(gridDim.x) * blockDim.x) {
     const int k0 = int(w % cpr) * 8;
@@ -243,15 +252,16 @@ __global__ void patches_kernel(const float* __restrict__ img, __nv_bfloat16* __r
     for (int u = 0; u < 8; ++u) {
       const int k = k0 + u;
       const int c = k / pp, r = k - c * pp, i = r / p, j = r - i * p;
-      f[u] = c < C ? __ldg(img + ((b * C + c) * Hi + py * p + i) * long(Wi) + px * p + j) : 0.f;
+      f[u] = c < C ? img[((b * C + c) * Hi + py * p + i) * long(Wi) + px * p + j] : 0.f;
     }
     *reinterpret_cast<uint4*>(out + w * 8) = pack8e(f);
   }
 }
 // p a multiple of 8, Wi of 4, no padding: two 16-byte loads per thread
-__global__ void patches8_kernel(const float* __restrict__ img, __nv_bfloat16* __restrict__ out, int C, int Hi, int Wi, int p,
+__global__ void patches8_kernel(const float* img, __nv_bfloat16* out, int C, int Hi, int Wi, int p,
                                 long total) {
   chain_trigger();
+  chain_wait();
   const int pp = p * p, cpr = C * pp >> 3, nx = Wi / p, ny = Hi / p;
   for (long w = blockIdx.x * long(blockDim.x) + threadIdx.x; w < total; w += long(gridDim.x) * blockDim.x) {
     const int k = int(w % cpr) * 8;
@@ -260,7 +270,7 @@ __global__ void patches8_kernel(const float* __restrict__ img, __nv_bfloat16* __
     const long b = tok / (long(nx) * ny);
     const int c = k / pp, r = k - c * pp, i = r / p, j = r - i * p;
     const float4* src = reinterpret_cast<const float4*>(img + ((b * C + c) * Hi + py * p + i) * long(Wi) + px * p + j);
-    const float4 a = __ldg(src), d = __ldg(src + 1);
+    const float4 a = src[0], d = src[1];
     const float f[8] = {a.x, a.y, a.z, a.w, d.x, d.y, d.z, d.w};
     *reinterpret_cast<uint4*>(out + w * 8) = pack8e(f);
   }
@@ -282,8 +292,8 @@ int zb_rope(void* buf, const float* cs, int T, int S, int nheads, int d, int row
   if (d % 16 != 0 || row_stride % 8 != 0) ZB_FAIL(-1, "rope: head dim %d / stride %d unsupported", d, row_stride);
   if (T <= 0 || nheads <= 0) return 0;
   long total = long(T) * nheads * (d / 16);
-  rope_kernel<<<grid_for(total, 256), 256, 0, stream>>>(static_cast<__nv_bfloat16*>(buf), cs, T, S, nheads, d,
-                                                       row_stride, backward ? -1.f : 1.f);
+  ZB_CUDA_OK(launch_pass(rope_kernel, grid_for(total, 256), 256, 0, stream, static_cast<__nv_bfloat16*>(buf), cs, T, S,
+                         nheads, d, row_stride, backward ? -1.f : 1.f));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -292,8 +302,8 @@ int zb_swiglu_fwd(const void* gu, void* out, long T, int F, cudaStream_t stream)
   using namespace zb;
   if (F % 8 != 0) ZB_FAIL(-1, "swiglu: F=%d not a multiple of 8", F);
   if (T <= 0) return 0;
-  swiglu_fwd_kernel<<<grid_for(T * (F / 8), 256), 256, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), T, F);
+  ZB_CUDA_OK(launch_pass(swiglu_fwd_kernel, grid_for(T * (F / 8), 256), 256, 0, stream,
+                         static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), T, F));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -301,9 +311,9 @@ int zb_swiglu_bwd(const void* gu, const void* dout, void* dgu, long T, int F, cu
   using namespace zb;
   if (F % 8 != 0) ZB_FAIL(-1, "swiglu: F=%d not a multiple of 8", F);
   if (T <= 0) return 0;
-  swiglu_bwd_kernel<<<grid_for(T * (F / 8), 256), 256, 0, stream>>>(
-      static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dout),
-      static_cast<__nv_bfloat16*>(dgu), T, F);
+  ZB_CUDA_OK(launch_pass(swiglu_bwd_kernel, grid_for(T * (F / 8), 256), 256, 0, stream,
+                         static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dout),
+                         static_cast<__nv_bfloat16*>(dgu), T, F));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -311,8 +321,8 @@ int zb_act_fwd(const void* x, void* y, long n, int kind, cudaStream_t stream) {
   using namespace zb;
   if (n % 8 != 0) ZB_FAIL(-1, "act: n=%ld not a multiple of 8", n);
   if (n <= 0) return 0;
-  act_fwd_kernel<<<grid_for(n / 8, 256), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x),
-                                                          static_cast<__nv_bfloat16*>(y), n / 8, kind);
+  ZB_CUDA_OK(launch_pass(act_fwd_kernel, grid_for(n / 8, 256), 256, 0, stream, static_cast<const __nv_bfloat16*>(x),
+                         static_cast<__nv_bfloat16*>(y), n / 8, kind));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -320,9 +330,8 @@ int zb_act_bwd(const void* x, const void* dy, void* dx, long n, int kind, cudaSt
   using namespace zb;
   if (n % 8 != 0) ZB_FAIL(-1, "act: n=%ld not a multiple of 8", n);
   if (n <= 0) return 0;
-  act_bwd_kernel<<<grid_for(n / 8, 256), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x),
-                                                          static_cast<const __nv_bfloat16*>(dy),
-                                                          static_cast<__nv_bfloat16*>(dx), n / 8, kind);
+  ZB_CUDA_OK(launch_pass(act_bwd_kernel, grid_for(n / 8, 256), 256, 0, stream, static_cast<const __nv_bfloat16*>(x),
+                         static_cast<const __nv_bfloat16*>(dy), static_cast<__nv_bfloat16*>(dx), n / 8, kind));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -334,9 +343,9 @@ int zb_patches(const float* img, void* out, int B, int C, int Hi, int Wi, int p,
   if (total <= 0) return 0;
   auto O = static_cast<__nv_bfloat16*>(out);
   if (p % 8 == 0 && Wi % 4 == 0 && kdim == C * p * p && (reinterpret_cast<uintptr_t>(img) & 15) == 0)
-    patches8_kernel<<<grid_for(total, 256), 256, 0, stream>>>(img, O, C, Hi, Wi, p, total);
+    ZB_CUDA_OK(launch_pass(patches8_kernel, grid_for(total, 256), 256, 0, stream, img, O, C, Hi, Wi, p, total));
   else
-    patches_kernel<<<grid_for(total, 256), 256, 0, stream>>>(img, O, C, Hi, Wi, p, kdim, total);
+    ZB_CUDA_OK(launch_pass(patches_kernel, grid_for(total, 256), 256, 0, stream, img, O, C, Hi, Wi, p, kdim, total));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -345,9 +354,9 @@ int zb_embedding_fwd(const long* ids, const void* table, const void* pos_table, 
   using namespace zb;
   if (H % 8 != 0) ZB_FAIL(-1, "embedding: H=%d not a multiple of 8", H);
   if (T <= 0) return 0;
-  embedding_fwd_kernel<<<grid_for(long(T) * (H / 8), 256), 256, 0, stream>>>(
-      ids, static_cast<const __nv_bfloat16*>(table), static_cast<const __nv_bfloat16*>(pos_table),
-      static_cast<__nv_bfloat16*>(out), T, H, V, S, pos_offset);
+  ZB_CUDA_OK(launch_pass(embedding_fwd_kernel, grid_for(long(T) * (H / 8), 256), 256, 0, stream, ids,
+                         static_cast<const __nv_bfloat16*>(table), static_cast<const __nv_bfloat16*>(pos_table),
+                         static_cast<__nv_bfloat16*>(out), T, H, V, S, pos_offset));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -359,15 +368,16 @@ int zb_embedding_bwd(const long* ids, const void* dout, void* dtable, void* dpos
   const int g = grid_for(long(T) * (H / 8), 256);
   const bool vec = ((reinterpret_cast<uintptr_t>(dtable) | reinterpret_cast<uintptr_t>(dpos)) & 15) == 0;
   auto D = static_cast<const __nv_bfloat16*>(dout);
-  auto launch = [&](auto* table, auto* pos) {
+  auto launch = [&](auto* table, auto* pos) -> int {
     using GT = std::remove_pointer_t<decltype(table)>;
-    if (vec) embedding_bwd_kernel<GT, true><<<g, 256, 0, stream>>>(ids, D, table, pos, T, H, V, S, pos_offset);
-    else embedding_bwd_kernel<GT, false><<<g, 256, 0, stream>>>(ids, D, table, pos, T, H, V, S, pos_offset);
+    if (vec) ZB_CUDA_OK(launch_pass(embedding_bwd_kernel<GT, true>, g, 256, 0, stream, ids, D, table, pos, T, H, V, S,
+                                    pos_offset));
+    else ZB_CUDA_OK(launch_pass(embedding_bwd_kernel<GT, false>, g, 256, 0, stream, ids, D, table, pos, T, H, V, S,
+                                pos_offset));
+    return 0;
   };
-  if (grad_f32) launch(static_cast<float*>(dtable), static_cast<float*>(dpos));
-  else launch(static_cast<__nv_bfloat16*>(dtable), static_cast<__nv_bfloat16*>(dpos));
-  ZB_CUDA_OK(cudaGetLastError());
-  return 0;
+  return grad_f32 ? launch(static_cast<float*>(dtable), static_cast<float*>(dpos))
+                  : launch(static_cast<__nv_bfloat16*>(dtable), static_cast<__nv_bfloat16*>(dpos));
 }
 
 }  // extern "C"

@@ -569,8 +569,9 @@ static TileOrder gemm2_tile_order(int M, int N, int K) {
 // One thread per 8 columns of a row; rows of C and of the addend are 16-byte aligned.
 template <int BN>
 __global__ void __launch_bounds__(256)
-gemm2_fixup_kernel(const float* __restrict__ ws, const GemmParams p, const TileOrder order, int first_tile, int splits) {
+gemm2_fixup_kernel(const float* ws, const GemmParams p, const TileOrder order, int first_tile, int splits) {
   chain_trigger();
+  chain_wait();
   constexpr int CHUNKS = 256 * BN / 8;
   const int w = blockIdx.x * 256 + threadIdx.x;
   const int t = w / CHUNKS, e = w - t * CHUNKS;
@@ -740,7 +741,8 @@ static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, 
   }
   if constexpr (std::is_same<Params, GemmParams>::value) {
     if (ex.splits > 1) {
-      gemm2_fixup_kernel<BN><<<(tiles - ex.full) * (BN / 8), 256, 0, stream>>>(ws, p, ex.order, ex.full, ex.splits);
+      ZB_CUDA_OK(launch_pass(gemm2_fixup_kernel<BN>, (tiles - ex.full) * (BN / 8), 256, 0, stream, ws, p, ex.order, ex.full,
+                             ex.splits));
       ZB_CUDA_OK(cudaGetLastError());
     }
   }

@@ -17,10 +17,11 @@ __device__ __forceinline__ void ce_unpack8(const uint4& u, float* f) {
 }
 
 __global__ void __launch_bounds__(CE_THREADS)
-ce_fwd_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const long* __restrict__ targets,
-                  __nv_bfloat16* __restrict__ dlogits, float* __restrict__ loss_rows, int T, int V,
+ce_fwd_bwd_kernel(const __nv_bfloat16* logits, const long* targets,
+                  __nv_bfloat16* dlogits, float* loss_rows, int T, int V,
                   long ld, float grad_scale, long ignore_index) {
   chain_trigger();
+  chain_wait();
   __shared__ float red_m[CE_THREADS / 32], red_s[CE_THREADS / 32];
   __shared__ float bc[3];
   const int row = blockIdx.x;
@@ -112,9 +113,8 @@ extern "C" int zb_cross_entropy(const void* logits, const long* targets, void* d
                                 cudaStream_t stream) {
   using namespace zb;
   if (T <= 0) return 0;
-  ce_fwd_bwd_kernel<<<T, CE_THREADS, 0, stream>>>(static_cast<const __nv_bfloat16*>(logits), targets,
-                                                  static_cast<__nv_bfloat16*>(dlogits), loss_rows, T, V, ld,
-                                                  grad_scale, ignore_index);
+  ZB_CUDA_OK(launch_pass(ce_fwd_bwd_kernel, T, CE_THREADS, 0, stream, static_cast<const __nv_bfloat16*>(logits), targets,
+                         static_cast<__nv_bfloat16*>(dlogits), loss_rows, T, V, ld, grad_scale, ignore_index));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -20,10 +20,11 @@ namespace zb {
 // 21.2 -> 11.0 us, 4096 x 4096 22.5 -> 18.4 us (operands not in L2).
 template <bool LN, int RW>
 __global__ void __launch_bounds__(NORM_THREADS)
-norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
-                float* __restrict__ stats /* [T,2]: mean, rstd */, int T, int H, float eps) {
+norm_fwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* w,
+                const __nv_bfloat16* b, __nv_bfloat16* y,
+                float* stats /* [T,2]: mean, rstd */, int T, int H, float eps) {
   chain_trigger();
+  chain_wait();
   constexpr int TEAM = NORM_THREADS / RW, A = NORM_GROUPS<RW>;
   __shared__ float red[2][RW * 8];
   const int team = threadIdx.x / TEAM, tt = threadIdx.x % TEAM;
@@ -186,8 +187,9 @@ __global__ void colsum_accumulate_kernel(const float* __restrict__ part, int P, 
 // warps takes 256 columns, and every thread has four rows in flight; with one column and one row per thread the
 // sums were bound by the latency of two-byte loads: 2048 x 20480 91 -> 30 us, 4616 x 3072 48 -> 17 us, finish included.
 __global__ void __launch_bounds__(256)
-colsum_partial8_kernel(const __nv_bfloat16* __restrict__ dy, int T, int N, int ld, float* __restrict__ part) {
+colsum_partial8_kernel(const __nv_bfloat16* dy, int T, int N, int ld, float* part) {
   chain_trigger();
+  chain_wait();
   __shared__ float sm[8][256 + 8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = blockIdx.x * 256 + lane * 8;
@@ -204,11 +206,11 @@ colsum_partial8_kernel(const __nv_bfloat16* __restrict__ dy, int T, int N, int l
     for (; r + 3 * step < T; r += 4 * step) {
       uint4 u[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) u[k] = ld_nc_v4(dy + size_t(r + k * step) * ld + col);
+      for (int k = 0; k < 4; ++k) u[k] = ld_v4(dy + size_t(r + k * step) * ld + col);
 #pragma unroll
       for (int k = 0; k < 4; ++k) add(u[k]);
     }
-    for (; r < T; r += step) add(ld_nc_v4(dy + size_t(r) * ld + col));
+    for (; r < T; r += step) add(ld_v4(dy + size_t(r) * ld + col));
   }
 #pragma unroll
   for (int j = 0; j < 8; ++j) sm[warp][lane * 8 + j] = s[j];
@@ -228,8 +230,9 @@ colsum_partial8_kernel(const __nv_bfloat16* __restrict__ dy, int T, int N, int l
 // 8192 x 2048 12.5 -> 13.5 for one launch less; wider, two CTAs of this size per SM are too few: 2048 x 20480 21 -> 26.
 template <typename OutT>
 __global__ void __launch_bounds__(1024)
-colsum_one_kernel(const __nv_bfloat16* __restrict__ dy, int T, int N, int ld, OutT* __restrict__ out, int accumulate) {
+colsum_one_kernel(const __nv_bfloat16* dy, int T, int N, int ld, OutT* out, int accumulate) {
   chain_trigger();
+  chain_wait();
   __shared__ float sm[32][33];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + (lane & 3) * 8;
@@ -246,13 +249,13 @@ colsum_one_kernel(const __nv_bfloat16* __restrict__ dy, int T, int N, int ld, Ou
     for (; r + 3 * 256 < T; r += 4 * 256) {
       uint4 u[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) u[k] = ld_nc_v4(p + size_t(r + k * 256) * ld);
+      for (int k = 0; k < 4; ++k) u[k] = ld_v4(p + size_t(r + k * 256) * ld);
 #pragma unroll
       for (int k = 0; k < 4; ++k) add(u[k]);
     }
     uint4 u[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) u[k] = r + k * 256 < T ? ld_nc_v4(p + size_t(r + k * 256) * ld) : make_uint4(0u, 0u, 0u, 0u);
+    for (int k = 0; k < 3; ++k) u[k] = r + k * 256 < T ? ld_v4(p + size_t(r + k * 256) * ld) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
     for (int k = 0; k < 3; ++k) add(u[k]);
   }
@@ -275,9 +278,10 @@ colsum_one_kernel(const __nv_bfloat16* __restrict__ dy, int T, int N, int ld, Ou
 
 // The same for rows that are not 16-byte aligned (one column per thread).
 __global__ void __launch_bounds__(256)
-colsum_partial_kernel(const __nv_bfloat16* __restrict__ dy, int T, int N, int ld,
-                      float* __restrict__ part) {
+colsum_partial_kernel(const __nv_bfloat16* dy, int T, int N, int ld,
+                      float* part) {
   chain_trigger();
+  chain_wait();
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= N) return;
   float s = 0.f;
@@ -315,8 +319,8 @@ int zb_norm_fwd(const void* x, const void* w, const void* b, void* y, float* sta
 #define ZB_NORM_FWD(RW_)                                                                                           \
   do {                                                                                                             \
     const int blocks = (T + RW_ - 1) / RW_;                                                                        \
-    if (ln) norm_fwd_kernel<true, RW_><<<blocks, NORM_THREADS, 0, stream>>>(X, W, B, Y, stats, T, H, eps);         \
-    else norm_fwd_kernel<false, RW_><<<blocks, NORM_THREADS, 0, stream>>>(X, W, B, Y, stats, T, H, eps);           \
+    if (ln) ZB_CUDA_OK(launch_pass(norm_fwd_kernel<true, RW_>, blocks, NORM_THREADS, 0, stream, X, W, B, Y, stats, T, H, eps));         \
+    else ZB_CUDA_OK(launch_pass(norm_fwd_kernel<false, RW_>, blocks, NORM_THREADS, 0, stream, X, W, B, Y, stats, T, H, eps));           \
   } while (0)
   switch (norm_rows_per_cta(H)) {
     case 8: ZB_NORM_FWD(8); break;
@@ -351,17 +355,21 @@ int zb_colsum(const void* dy, int T, int N, int ld, float* part, void* out, int 
   int P = T < 64 ? T : 64;
   if (vec && N <= 4096 && T <= 8192) {
     auto DY = static_cast<const __nv_bfloat16*>(dy);
-    if (grad_f32) colsum_one_kernel<float><<<(N + 31) / 32, 1024, 0, stream>>>(DY, T, N, ld, static_cast<float*>(out), accumulate);
-    else colsum_one_kernel<__nv_bfloat16><<<(N + 31) / 32, 1024, 0, stream>>>(DY, T, N, ld, static_cast<__nv_bfloat16*>(out), accumulate);
+    if (grad_f32) ZB_CUDA_OK(launch_pass(colsum_one_kernel<float>, (N + 31) / 32, 1024, 0, stream, DY, T, N, ld,
+                                         static_cast<float*>(out), accumulate));
+    else ZB_CUDA_OK(launch_pass(colsum_one_kernel<__nv_bfloat16>, (N + 31) / 32, 1024, 0, stream, DY, T, N, ld,
+                                static_cast<__nv_bfloat16*>(out), accumulate));
     ZB_CUDA_OK(cudaGetLastError());
     return 0;
   }
   if (vec) {
     // about three CTAs per SM, and at least one row per warp
     P = std::min(P, std::max(1, std::min(3 * num_sms() / nb, (T + 7) / 8)));
-    colsum_partial8_kernel<<<dim3(nb, P), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(dy), T, N, ld, part);
+    ZB_CUDA_OK(launch_pass(colsum_partial8_kernel, dim3(nb, P), 256, 0, stream, static_cast<const __nv_bfloat16*>(dy), T, N,
+                           ld, part));
   } else {
-    colsum_partial_kernel<<<dim3(nb, P), 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(dy), T, N, ld, part);
+    ZB_CUDA_OK(launch_pass(colsum_partial_kernel, dim3(nb, P), 256, 0, stream, static_cast<const __nv_bfloat16*>(dy), T, N,
+                           ld, part));
   }
   ZB_CUDA_OK(cudaGetLastError());
   return colsum_finish(part, P, N, out, nullptr, nullptr, grad_f32, accumulate, stream);

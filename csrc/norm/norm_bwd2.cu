@@ -37,11 +37,12 @@ struct NormBwdCfg {
 
 template <bool LN, int RW, int NV>
 __global__ void __launch_bounds__(NORM_THREADS, 2)
-norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                 const __nv_bfloat16* __restrict__ w, const float* __restrict__ stats,
-                 const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                 float* __restrict__ part_dw, float* __restrict__ part_db, int T, int H) {
+norm_bwd2_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
+                 const __nv_bfloat16* w, const float* stats,
+                 const __nv_bfloat16* dres, __nv_bfloat16* dx,
+                 float* part_dw, float* part_db, int T, int H) {
   chain_trigger();
+  chain_wait();
   using Cfg = NormBwdCfg<NV>;
   constexpr int TEAM = NORM_THREADS / RW, NS = Cfg::STAGES, A = NORM_GROUPS<RW>;
   extern __shared__ __align__(128) uint8_t ring[];
@@ -150,7 +151,7 @@ norm_bwd2_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
   }
   // column sums of this CTA: teams in order, through shared memory (the ring: every copy into it has landed)
   cp_async_wait<0>();
-  auto finish = [&](auto& acc, float* __restrict__ part) {
+  auto finish = [&](auto& acc, float* part) {
     float* sm = reinterpret_cast<float*>(ring);
     float* out = part + size_t(blockIdx.x) * H;
     if (RW > 1) __syncthreads();
@@ -192,7 +193,8 @@ static int launch_norm_bwd2(const __nv_bfloat16* dy, const __nv_bfloat16* x, con
     ZB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, NormBwdCfg<NV>::SMEM_BYTES));
     attr_set = true;
   }
-  kern<<<blocks, NORM_THREADS, NormBwdCfg<NV>::SMEM_BYTES, stream>>>(dy, x, w, stats, dres, dx, part_dw, part_db, T, H);
+  ZB_CUDA_OK(launch_pass(kern, blocks, NORM_THREADS, NormBwdCfg<NV>::SMEM_BYTES, stream, dy, x, w, stats, dres, dx, part_dw,
+                         part_db, T, H));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }
@@ -202,12 +204,13 @@ static int launch_norm_bwd2(const __nv_bfloat16* dy, const __nv_bfloat16* x, con
 // blockIdx.y selects one of two such sums (weight and bias gradient in one launch).
 template <typename OutT>
 __global__ void __launch_bounds__(1024)
-colsum_accumulate2_kernel(const float* __restrict__ part0, const float* __restrict__ part1, int P, int H,
-                          OutT* __restrict__ out0, OutT* __restrict__ out1, int accumulate) {
+colsum_accumulate2_kernel(const float* part0, const float* part1, int P, int H,
+                          OutT* out0, OutT* out1, int accumulate) {
   chain_trigger();
+  chain_wait();
   __shared__ float sm[32][33];
-  const float* __restrict__ part = blockIdx.y ? part1 : part0;
-  OutT* __restrict__ out = blockIdx.y ? out1 : out0;
+  const float* part = blockIdx.y ? part1 : part0;
+  OutT* out = blockIdx.y ? out1 : out0;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int h = blockIdx.x * 32 + tx;
   float s = 0.f;
@@ -232,11 +235,11 @@ int colsum_finish(const float* part0, int P, int H, void* out0, const float* par
                   int accumulate, cudaStream_t stream) {
   const dim3 grid((H + 31) / 32, out1 != nullptr ? 2 : 1);
   if (grad_f32)
-    colsum_accumulate2_kernel<float><<<grid, 1024, 0, stream>>>(part0, part1, P, H, static_cast<float*>(out0),
-                                                               static_cast<float*>(out1), accumulate);
+    ZB_CUDA_OK(launch_pass(colsum_accumulate2_kernel<float>, grid, 1024, 0, stream, part0, part1, P, H,
+                           static_cast<float*>(out0), static_cast<float*>(out1), accumulate));
   else
-    colsum_accumulate2_kernel<__nv_bfloat16><<<grid, 1024, 0, stream>>>(
-        part0, part1, P, H, static_cast<__nv_bfloat16*>(out0), static_cast<__nv_bfloat16*>(out1), accumulate);
+    ZB_CUDA_OK(launch_pass(colsum_accumulate2_kernel<__nv_bfloat16>, grid, 1024, 0, stream, part0, part1, P, H,
+                           static_cast<__nv_bfloat16*>(out0), static_cast<__nv_bfloat16*>(out1), accumulate));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;
 }

@@ -132,6 +132,34 @@ def test_kernels_that_start_early_use_coherent_loads():
     assert not re.search(r"__ldg|ld_nc|__restrict__", main[:len(main) - len(plain)])
 
 
+def test_passes_that_start_early_wait_first_and_use_coherent_loads():
+    """Every kernel launched with launch_pass begins while its predecessor may still write: chain_wait stands before its
+    first access, and it has no non-coherent load (nor a __restrict__ from which the compiler makes one)."""
+    import pathlib
+    import re
+
+    root = pathlib.Path(__file__).resolve().parent.parent / "csrc"
+    seen = set()
+    for f in root.rglob("*.cu"):
+        text = f.read_text()
+        names = set(re.findall(r"launch_pass\(\s*(\w+)", text))
+        if "kern" in names:                                # a template instance picked a line before
+            names = names - {"kern"} | set(re.findall(r"auto kern = (\w+)<", text))
+        for name in names:
+            at = re.search(r"__global__[^;{]*?\b" + name + r"\(", text).end()
+            start = text.index("{", at)
+            end, depth = start + 1, 1
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[end], 0)
+                end += 1
+            body = text[start + 1:end]
+            assert body.split()[:2] == ["chain_trigger();", "chain_wait();"], name
+            assert not re.search(r"__ldg|ld_nc|ld\.global\.nc|__restrict__", text[at:end]), name
+            seen.add(name)
+    assert {"norm_fwd_kernel", "norm_bwd2_kernel", "rope_kernel", "swiglu_fwd_kernel", "act_bwd_kernel", "colsum_one_kernel",
+            "gemm2_fixup_kernel", "attn_bwd2_stats_kernel", "ce_fwd_bwd_kernel"} <= seen
+
+
 def bf(*shape):
     return torch.zeros(*shape, dtype=torch.bfloat16)
 
