@@ -700,7 +700,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 }
 
 // stats[(b, h)][0][s] = -lse * log2(e), stats[(b, h)][1][s] = -sum_d dO * O; rows padded to s_pad
-// entries that this kernel never writes (they must have been zeroed once).  A CTA takes 64 tokens of one head: D / 8 lanes
+// entries, zeros behind the last query.  A CTA takes 64 tokens of one head: D / 8 lanes
 // read a token's row in 16-byte pieces, all rows of a thread in flight at once, and the 64 results leave as two row
 // segments. 32 heads of
 // 4096 tokens, d = 128 32 -> 12 us, 32 heads of 2048, d = 64 15 -> 4 us (one warp per token and head, four-byte loads).
@@ -745,17 +745,17 @@ attn_bwd2_stats_kernel(const __nv_bfloat16* o, const __nv_bfloat16* d_o,
   }
   __syncthreads();
   const int s = s0 + int(threadIdx.x);
-  if (threadIdx.x < 64 && s < S) {
+  if (threadIdx.x < 64) {   // (the padding too: its P is masked, but 0 times what lies there has to be 0)
     const size_t bh = size_t(b) * Hq + h;
     float* row = stats + bh * 2 * size_t(s_pad);
-    row[s] = lse[bh * S + s] * -1.4426950408889634f;
+    row[s] = s < S ? lse[bh * S + s] * -1.4426950408889634f : 0.f;
     row[s_pad + s] = -sm[threadIdx.x];
   }
 }
 
 static int launch_stats(const __nv_bfloat16* o, const __nv_bfloat16* d_o, const float* lse, float* stats, int B, int S, int Hq,
                         int D, int s_pad, cudaStream_t stream) {
-  const dim3 grid((S + 63) / 64, Hq, B);
+  const dim3 grid(s_pad / 64, Hq, B);
   const int o_vec = (reinterpret_cast<uintptr_t>(o) & 15) == 0;   // (dO is fetched by TMA and aligned anyway)
   if (reinterpret_cast<uintptr_t>(d_o) & 15) ZB_FAIL(-4, "attention: dO not 16-byte aligned");
   if (D == 128) ZB_CUDA_OK(launch_pass(attn_bwd2_stats_kernel<128>, grid, 256, 0, stream, o, d_o, lse, stats, S, Hq, s_pad,
@@ -824,8 +824,7 @@ int zb_flash_bwd2_trace_warps() { return zb::BWD2_WARPS; }
 
 int zb_flash_bwd2_stats_floats(int B, int S, int Hq) { return B * Hq * 2 * ((S + 127) / 128 * 128); }
 
-// Scratch: stats fp32 [zb_flash_bwd2_stats_floats(B, S, Hq)], zeroed once by the caller (rows are padded to a
-// multiple of 128 and the padding is never written); dq_acc fp32 [B*S*Hq*D], zero on entry (left zero).
+// Scratch: stats fp32 [zb_flash_bwd2_stats_floats(B, S, Hq)]; dq_acc fp32 [B*S*Hq*D], zero on entry (left zero).
 // trace: nullptr, or a zeroed device buffer of trace_ctas * warps * events 64-bit words.
 int zb_flash_bwd2(const void* d_o, const void* qkv, const void* o, const float* lse, void* dqkv, float* stats,
                   float* dq_acc, int B, int S, int Hq, int Hkv, int D, int causal, int window, float softmax_scale,
@@ -859,7 +858,7 @@ int zb_flash_bwd2(const void* d_o, const void* qkv, const void* o, const float* 
 
 // Two-kernel backward without atomics: statistics pass, then dK / dV per key tile (this file's kernel without
 // its dQ part) and dQ per query tile (flash_bwd_dq.cu); the two main kernels are independent of each other.
-// Scratch: stats fp32 [zb_flash_bwd2_stats_floats(B, S, Hq)], zeroed once by the caller.
+// Scratch: stats fp32 [zb_flash_bwd2_stats_floats(B, S, Hq)].
 int zb_flash_bwd3(const void* d_o, const void* qkv, const void* o, const float* lse, void* dqkv, float* stats,
                   int B, int S, int Hq, int Hkv, int D, int causal, int window, float softmax_scale, int* status,
                   int parts, unsigned long long* trace, int trace_ctas, cudaStream_t stream) {

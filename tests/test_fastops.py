@@ -1,0 +1,177 @@
+"""The native calls of csrc/host/fastops.cpp against the wrappers of ops/sm100.py: same results, bit for bit, for every form
+of argument they take, and everything else declined (the wrapper then takes or refuses it)."""
+import pytest
+import torch
+
+from zorse_b200.ops import build
+from zorse_b200.ops import sm100 as k
+
+
+def _module():
+    import importlib.util
+
+    spec = importlib.util.spec_from_file_location("zorse_fastops", build.build_fast())
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    return mod
+
+
+def test_declines_what_is_not_on_a_gpu():
+    m = _module()
+    x, w = torch.zeros(4, 8, dtype=torch.bfloat16), torch.zeros(16, 8, dtype=torch.bfloat16)
+    g, v = torch.zeros(16, 8), torch.zeros(8)
+    calls = [(m.linear_fwd, (x, w, None, None)), (m.linear_dgrad, (x, x, None)), (m.linear_wgrad, (x, x, g, None)),
+             (m.norm_fwd, (x, v, None, 1e-5, False)), (m.norm_bwd, (x, x, v, g, None, v, None, False)),
+             (m.rope, (x, g, 4, 1, 8, False)), (m.swiglu_fwd, (x,)), (m.swiglu_bwd, (x, x)), (m.act_fwd, (x, 0)),
+             (m.act_bwd, (x, x, 0)), (m.attn_fwd, (x, 1, 4, 1, 1, 64, True, 0, 1)),
+             (m.attn_bwd, (x, x, x, g, 1, 4, 1, 1, 64, True, 0))]
+    for fn, args in calls:
+        assert fn(*args) is None
+        assert fn(*[None] * len(args)) is None and fn(*["x"] * len(args)) is None
+        with pytest.raises(TypeError):
+            fn(*args, None)
+    with pytest.raises(ValueError):
+        m.init((1, 2), RuntimeError)
+
+
+def test_entry_points_stand_in_the_order_of_the_table():
+    """`init` fills the table by position: as many names as members, each member named like its entry point."""
+    import re
+
+    src = build.FAST_SRC.read_text()
+    body = src[src.index("struct Entry {"):src.index("Entry lib;")]
+    members = re.findall(r"\(\*(\w+)\)", body)
+    names = [n[len("zb_"):] for n in k._FAST_ENTRIES]
+    same = {"gemm_bf16": "gemm", "gemm2_bf16": "gemm2", "gemm2_split_bf16": "gemm2_split",
+            "flash_bwd2_stats_floats": "flash_stats_floats"}
+    assert [same.get(n, n) for n in names] == members
+    # and each member takes what the C function takes
+    for name, member in zip(k._FAST_ENTRIES, members):
+        if name not in k._SIGNATURES:
+            continue
+        params = re.search(r"\(\*" + member + r"\)\(([^)]*)\)", body).group(1).split(",")
+        kinds = "".join("p" if "*" in p or "cudaStream_t" in p else {"int": "i", "long": "l", "float": "f"}[p.split()[-1]]
+                        for p in params)
+        assert kinds == k._SIGNATURES[name], name
+
+
+@pytest.fixture
+def ops():
+    from zorse_b200.ops.api import get_ops
+
+    o = get_ops("sm100")
+    k.status_word(0)
+    return o
+
+
+def _rand(*shape, seed=0, dtype=torch.bfloat16):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(dtype).cuda()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,K,N", [(300, 512, 768), (64, 264, 72), (1018, 512, 1544), (300, 8200, 520), (1, 8, 8)])
+@pytest.mark.parametrize("wide", [False, True])      # rows of a wider matrix
+def test_linear(ops, T, K, N, wide):
+    pad = 8 if wide else 0
+    x, w = _rand(T, K + pad, seed=1)[:, :K], _rand(N, K + pad, seed=2)[:, :K]
+    b, add = _rand(N, seed=3), _rand(T, N + pad, seed=4)[:, :N]
+    dy = _rand(T, N + pad, seed=5)[:, :N]
+
+    def wrap(a, c, M, n, **kw):
+        return k.gemm(a, c, torch.empty(M, n, dtype=torch.bfloat16, device="cuda"), **kw)
+
+    before = k.launch_count()
+    assert k._fast.linear_fwd(x, w, b, add) is not None and k.launch_count() > before
+    for bias in (None, b):
+        for addend in (None, add):
+            assert torch.equal(ops.linear_fwd(x, w, bias, addend), wrap(x, w, T, N, bias=bias, addend=addend))
+    addk = _rand(T, K, seed=6)
+    for addend in (None, addk):
+        assert torch.equal(ops.linear_dgrad(dy, w, addend), wrap(dy, w, T, K, b_mn=True, addend=addend))
+    for dt in (torch.float32, torch.bfloat16):
+        for bias in (False, True):
+            g = [torch.ones(N, K, dtype=dt, device="cuda") for _ in range(2)]
+            gb = [torch.ones(N, dtype=dt, device="cuda") for _ in range(2)]
+            assert k._fast.linear_wgrad(dy, x, g[0], gb[0] if bias else None) is True
+            k.gemm(dy, x, g[1], a_mn=True, b_mn=True, accumulate=True)
+            if bias:
+                k.colsum_accumulate(dy, gb[1])
+            assert torch.equal(g[0], g[1]) and torch.equal(gb[0], gb[1])
+    k.check_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,H", [(1, 8), (300, 512), (33, 1032), (5, 8192)])
+@pytest.mark.parametrize("ln", [False, True])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_norms(ops, T, H, ln, dt):
+    x, dy, w, b = _rand(T, H, seed=1), _rand(T, H, seed=2), _rand(H, seed=3), _rand(H, seed=4)
+    y, st = ops.norm_fwd(x, w, b if ln else None, 1e-5, ln)
+    y2, st2 = k.norm_fwd(x, w, b if ln else None, 1e-5, ln)
+    assert torch.equal(y, y2) and torch.equal(st, st2)
+    for dres in (None, _rand(T, H, seed=5)):
+        g = [torch.ones(4, H, dtype=dt, device="cuda") for _ in range(1)][0]
+        assert k._fast.norm_bwd(dy, x, w, st, dres, g[0], g[1] if ln else None, ln) is not None
+        dx2 = k.norm_bwd(dy, x, w, st, dres, g[2], g[3] if ln else None, ln)
+        assert torch.equal(g[0], g[2]) and torch.equal(g[1], g[3])
+        assert torch.equal(ops.norm_bwd(dy, x, w, st, dres, g[0], g[1] if ln else None, ln), dx2)
+    k.check_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,S,Hq,Hkv,D,causal,window", [(2, 150, 8, 8, 64, True, 0), (1, 600, 4, 2, 128, True, 200),
+                                                        (3, 129, 2, 1, 64, False, 0), (1, 1, 1, 1, 128, True, 5)])
+def test_attention(ops, B, S, Hq, Hkv, D, causal, window):
+    """The backward's statistics live in memory as the allocator hands it out: their padding is written by the kernel (NaN in
+    what the allocator will hand out next would show)."""
+    qkv, do = _rand(B * S, (Hq + 2 * Hkv) * D, seed=1), _rand(B * S, Hq * D, seed=2)
+    out, lse = k.flash_fwd(qkv, B, S, Hq, Hkv, D, causal, window, version=4)
+    got = k._fast.attn_fwd(qkv, B, S, Hq, Hkv, D, causal, window, k.ATTN_FWD4_FLAGS)
+    assert torch.equal(got[0], out) and torch.equal(got[1], lse)
+    want = k.flash_bwd(do, qkv, out, lse, B, S, Hq, Hkv, D, causal, window)
+    for _ in range(3):
+        for n in (2 * B * Hq * ((S + 127) // 128 * 128), qkv.numel() // 2):
+            torch.full((n,), float("nan"), device="cuda")
+        assert torch.equal(k._fast.attn_bwd(do, qkv, out, lse, B, S, Hq, Hkv, D, causal, window), want)
+    k.check_status()
+
+
+@pytest.mark.gpu
+def test_passes(ops):
+    q, h = _rand(300, 1536, seed=1), _rand(300, 768, seed=2)
+    cs = ops.rope_table(150, 64, 1e4, "cuda")
+    for backward in (False, True):
+        assert torch.equal(ops.rope_(q.clone(), cs, 150, 16, 64, backward), k.rope_(q.clone(), cs, 150, 16, 64, backward))
+    assert torch.equal(ops.swiglu_fwd(q), k.swiglu_fwd(q)) and torch.equal(ops.swiglu_bwd(q, h), k.swiglu_bwd(q, h))
+    for name, kind in (("gelu", 0), ("relu", 1), ("gelu_erf", 2)):
+        assert torch.equal(ops.act_fwd(h, name), k.act_fwd(h, kind)) and torch.equal(ops.act_bwd(h, h + 1, name), k.act_bwd(h, h + 1, kind))
+
+
+@pytest.mark.gpu
+def test_what_is_declined_and_what_is_refused(ops):
+    x, w = _rand(64, 512), _rand(256, 512)
+    f = k._fast
+    for args in ((x.float(), w, None, None), (x, w.t(), None, None), (x.t(), w, None, None), (x, w.cpu(), None, None),
+                 (x[0], w, None, None), (x, w, w[0], None), (x, w, None, x), (x[:0], w, None, None)):
+        assert f.linear_fwd(*args) is None
+    with pytest.raises(AssertionError):
+        ops.linear_fwd(x, w.t())
+    with pytest.raises(TypeError):
+        ops.linear_fwd(x.float(), w)
+    with pytest.raises(k.KernelError, match="H=12 unsupported"):
+        ops.norm_fwd(_rand(4, 12), _rand(12), None, 1e-5, False)
+
+    class Marked(torch.Tensor):
+        pass
+
+    assert f.swiglu_fwd(_rand(8, 64).as_subclass(Marked)) is None
+    assert f.rope(_rand(8, 64), torch.zeros(4, 64, device="cuda"), 8, 1, 64, False) is None      # a table of fewer positions
+    out = torch.empty(8, 64, dtype=torch.bfloat16, device="cuda")
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):                       # launches follow the current stream
+        a = _rand(4096, 4096, seed=7)
+        for _ in range(20):
+            a = ops.linear_fwd(a, _rand(4096, 4096, seed=8)) * 0.01
+        b = ops.linear_fwd(a, w.repeat(1, 8))
+    side.synchronize()
+    assert torch.equal(b, ops.linear_fwd(a, w.repeat(1, 8))) and out.shape == (8, 64)

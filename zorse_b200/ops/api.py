@@ -139,8 +139,16 @@ class RefOps:
             g.zero_()
 
 
+def _decline(*args):
+    """Stands for a native call that is switched off: as if it had declined its arguments."""
+    return None
+
+
 class Sm100Ops:
-    """Hand-written sm_100a kernels only. Requires bf16 CUDA tensors."""
+    """Hand-written sm_100a kernels only. Requires bf16 CUDA tensors.
+
+    The calls a step makes for every layer and microbatch go to the native module first (`sm100._fast`, 3 - 5 us of host
+    time against 7 - 16); what it declines with None goes through the wrappers."""
     name = "sm100"
 
     def __init__(self):
@@ -148,10 +156,25 @@ class Sm100Ops:
 
         self.k = sm100
         self.k.lib()
+        fast = sm100._fast
+        if fast is not None and sm100.GEMM_KERNEL == "2cta":
+            self._linear_fwd, self._linear_dgrad, self._linear_wgrad = fast.linear_fwd, fast.linear_dgrad, fast.linear_wgrad
+        else:
+            self._linear_fwd = self._linear_dgrad = self._linear_wgrad = _decline
+        default = fast is not None
+        self._norm_fwd = fast.norm_fwd if default and sm100.NORM_FWD_VERSION == 1 else _decline
+        self._norm_bwd = fast.norm_bwd if default and sm100.NORM_BWD_VERSION == 2 else _decline
+        self._attn_fwd = fast.attn_fwd if default and sm100.ATTN_FWD_VERSION == 0 else _decline
+        self._attn_bwd = fast.attn_bwd if default and sm100.ATTN_BWD_VERSION == 0 else _decline
+        for name in ("rope", "swiglu_fwd", "swiglu_bwd", "act_fwd", "act_bwd"):
+            setattr(self, "_" + name, getattr(fast, name) if default else _decline)
 
     def linear_fwd(self, x, w, bias=None, addend=None):
-        y = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)
-        return self.k.gemm(x, w, y, bias=bias, addend=addend)
+        y = self._linear_fwd(x, w, bias, addend)
+        if y is None:
+            y = torch.empty(x.shape[0], w.shape[0], dtype=x.dtype, device=x.device)
+            self.k.gemm(x, w, y, bias=bias, addend=addend)
+        return y
 
     def linear_fwd_gather(self, x, name, ag, bias=None):
         """Forward GEMM that also all-gathers the unit's parameters (see engine/fused.py)."""
@@ -162,44 +185,62 @@ class Sm100Ops:
                               epoch=ag.epoch, version_flags=ag.version_flags, need_version=ag.need_version, bias=bias)
 
     def linear_dgrad(self, dy, w, addend=None):
-        dx = torch.empty(dy.shape[0], w.shape[1], dtype=dy.dtype, device=dy.device)
-        return self.k.gemm(dy, w, dx, b_mn=True, addend=addend)
+        dx = self._linear_dgrad(dy, w, addend)
+        if dx is None:
+            dx = torch.empty(dy.shape[0], w.shape[1], dtype=dy.dtype, device=dy.device)
+            self.k.gemm(dy, w, dx, b_mn=True, addend=addend)
+        return dx
 
     def linear_wgrad(self, dy, x, gw, gb=None):
         # gw[N,K] += dy^T[N,T] @ x[T,K]: both operands contiguous along the non-reduced dim
-        self.k.gemm(dy, x, gw, a_mn=True, b_mn=True, accumulate=True)
-        if gb is not None:
-            self.k.colsum_accumulate(dy, gb)
+        if self._linear_wgrad(dy, x, gw, gb) is None:
+            self.k.gemm(dy, x, gw, a_mn=True, b_mn=True, accumulate=True)
+            if gb is not None:
+                self.k.colsum_accumulate(dy, gb)
 
     def norm_fwd(self, x, w, b, eps, ln):
-        return self.k.norm_fwd(x, w, b, eps, ln)
+        r = self._norm_fwd(x, w, b, eps, ln)
+        return self.k.norm_fwd(x, w, b, eps, ln) if r is None else r
 
     def norm_bwd(self, dy, x, w, stats, dres, gw, gb, ln):
-        return self.k.norm_bwd(dy, x, w, stats, dres, gw, gb, ln)
+        dx = self._norm_bwd(dy, x, w, stats, dres, gw, gb, ln)
+        return self.k.norm_bwd(dy, x, w, stats, dres, gw, gb, ln) if dx is None else dx
 
     def rope_table(self, S, d, theta, device):
         return ref.rope_table(S, d, theta, device)
 
     def rope_(self, qkv, cs, S, nheads, d, backward=False):
-        return self.k.rope_(qkv, cs, S, nheads, d, backward)
+        if self._rope(qkv, cs, S, nheads, d, backward) is None:
+            self.k.rope_(qkv, cs, S, nheads, d, backward)
+        return qkv
 
     def attn_fwd(self, qkv, B, S, Hq, Hkv, D, causal=True, window=0):
-        return self.k.flash_fwd(qkv, B, S, Hq, Hkv, D, causal, window)
+        k = self.k
+        if k._auto_fwd_version(B, S, Hq, D) == 4:
+            r = self._attn_fwd(qkv, B, S, Hq, Hkv, D, causal, window, k.ATTN_FWD4_FLAGS)
+            if r is not None:
+                return r
+        return k.flash_fwd(qkv, B, S, Hq, Hkv, D, causal, window)
 
     def attn_bwd(self, do, qkv, o, lse, B, S, Hq, Hkv, D, causal=True, window=0):
-        return self.k.flash_bwd(do, qkv, o, lse, B, S, Hq, Hkv, D, causal, window)
+        dqkv = self._attn_bwd(do, qkv, o, lse, B, S, Hq, Hkv, D, causal, window)
+        return self.k.flash_bwd(do, qkv, o, lse, B, S, Hq, Hkv, D, causal, window) if dqkv is None else dqkv
 
     def swiglu_fwd(self, gu):
-        return self.k.swiglu_fwd(gu)
+        y = self._swiglu_fwd(gu)
+        return self.k.swiglu_fwd(gu) if y is None else y
 
     def swiglu_bwd(self, gu, dout):
-        return self.k.swiglu_bwd(gu, dout)
+        dgu = self._swiglu_bwd(gu, dout)
+        return self.k.swiglu_bwd(gu, dout) if dgu is None else dgu
 
     def act_fwd(self, x, kind):
-        return self.k.act_fwd(x, _ACT_KINDS[kind])
+        y = self._act_fwd(x, _ACT_KINDS[kind])
+        return self.k.act_fwd(x, _ACT_KINDS[kind]) if y is None else y
 
     def act_bwd(self, x, dy, kind):
-        return self.k.act_bwd(x, dy, _ACT_KINDS[kind])
+        dx = self._act_bwd(x, dy, _ACT_KINDS[kind])
+        return self.k.act_bwd(x, dy, _ACT_KINDS[kind]) if dx is None else dx
 
     def patches(self, img, patch, kdim):
         return self.k.patches(img, patch, kdim)

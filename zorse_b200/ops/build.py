@@ -1,4 +1,5 @@
-"""Builds the sm_100a kernel library in-tree with nvcc (no torch headers involved).
+"""Builds the sm_100a kernel library in-tree with nvcc (no torch headers involved), and beside it the Python module that
+calls it without Python in between (`csrc/host/fastops.cpp`, g++ with torch's headers).
 
 Every `.cu` file under `csrc/` is compiled to an object with
 `-gencode arch=compute_100a,code=sm_100a` and linked into
@@ -12,9 +13,11 @@ from __future__ import annotations
 
 import argparse
 import os
+import importlib.util
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -64,6 +67,31 @@ def _compile_one(nvcc: str, src: Path, obj: Path, verbose: bool, extra=()) -> st
 
 
 DEBUG_LIB = OUT_DIR / "libzorse_sm100_dbg.so"
+FAST_SRC = CSRC / "host" / "fastops.cpp"
+FAST = OUT_DIR / "zorse_fastops.so"
+
+
+def build_fast(force: bool = False) -> Path:
+    """The module `zorse_fastops` for this interpreter and this torch."""
+    if not force and FAST.exists() and FAST.stat().st_mtime >= FAST_SRC.stat().st_mtime:
+        return FAST
+    torch_dir = Path(importlib.util.find_spec("torch").origin).parent
+    cxx = os.environ.get("CXX") or shutil.which("g++")
+    if not cxx:
+        raise RuntimeError("g++ not found; the host module cannot be built")
+    cuda = Path(find_nvcc()).resolve().parents[1]
+    OUT_DIR.mkdir(parents=True, exist_ok=True)
+    tmp = FAST.with_suffix(f".{os.getpid()}.tmp")
+    libs = ["torch_python", "torch", "torch_cpu", "torch_cuda", "c10", "c10_cuda"]
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", *(f"-I{d}" for d in (
+        torch_dir / "include", torch_dir / "include/torch/csrc/api/include", cuda / "include",
+        sysconfig.get_paths()["include"])), str(FAST_SRC), "-o", str(tmp), f"-L{torch_dir / 'lib'}", "-Wl,--no-as-needed",
+        *(f"-l{x}" for x in libs)]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"{FAST_SRC.name} does not build:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, FAST)
+    return FAST
 
 
 def build(force: bool = False, verbose: bool = False, debug_bounds: bool = False) -> Path:
@@ -73,6 +101,7 @@ def build(force: bool = False, verbose: bool = False, debug_bounds: bool = False
     library when ZORSE_DEBUG_BOUNDS=1."""
     if debug_bounds:
         return _build(force, verbose, OUT_DIR / "obj_dbg", DEBUG_LIB, ["-DZB_DEBUG_BOUNDS=1"], write_log=False)
+    build_fast(force)
     return _build(force, verbose, OBJ_DIR, LIB, [], write_log=True)
 
 

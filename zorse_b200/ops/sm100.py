@@ -79,11 +79,35 @@ def lib():
             getattr(_lib, name).argtypes = [_CTYPES[c] for c in sig]
         if "ZORSE_RS_ADAM_VARIANT" in os.environ:      # 0 / 1 select a peer-load kernel (1 is the library default)
             _lib.zb_set_rs_adam_variant(c_int(int(os.environ["ZORSE_RS_ADAM_VARIANT"])))
+        _load_fast()
     return _lib
 
 
+# The module csrc/host/fastops.cpp: the same entry points for the calls of a training step, without Python in between.  It
+# answers None to arguments it was not written for; the wrappers below take those.  None until the library is loaded.
+_fast = None
+_FAST_ENTRIES = ("zb_gemm_bf16", "zb_gemm2_bf16", "zb_gemm2_split_bf16", "zb_gemm2_workspace", "zb_norm_fwd", "zb_norm_bwd2",
+                 "zb_norm_partial_rows", "zb_colsum", "zb_rope", "zb_swiglu_fwd", "zb_swiglu_bwd", "zb_act_fwd", "zb_act_bwd",
+                 "zb_flash_fwd4", "zb_flash_bwd3", "zb_flash_bwd2_stats_floats", "zb_last_error")   # the order of its `Entry`
+
+
+def _load_fast() -> None:
+    global _fast
+    import importlib.util
+
+    from . import build as _build
+
+    spec = importlib.util.spec_from_file_location("zorse_fastops", _build.build_fast())
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    mod.init(tuple(ctypes.cast(getattr(_lib, n), c_void_p).value for n in _FAST_ENTRIES), KernelError)
+    for dev, word in _status.items():
+        mod.set_status(dev, word.data_ptr())
+    _fast = mod
+
+
 def launch_count() -> int:
-    return _launches
+    return _launches + (_fast.launch_count() if _fast is not None else 0)
 
 
 def _stream() -> c_void_p:
@@ -108,6 +132,8 @@ def status_word(device=None) -> torch.Tensor:
         dev = torch.cuda.current_device() if device is None else torch.device(device).index
     if dev not in _status:
         _status[dev] = torch.zeros(1, dtype=torch.int32, device=f"cuda:{dev}")
+        if _fast is not None:
+            _fast.set_status(dev, _status[dev].data_ptr())
     return _status[dev]
 
 
