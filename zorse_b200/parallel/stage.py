@@ -266,9 +266,13 @@ class PipelineStage:
         self.loss_sum = v if self.loss_sum is None else self.loss_sum + v
 
     # -- one layer, one microbatch ---------------------------------------------------
-    def forward_layer(self, li: int, mbl: int, x, targets, recompute: bool, want_loss: bool = True):
-        """Runs layer li on microbatch mbl. With recompute only the layer input is stashed."""
+    def forward_layer(self, li: int, mbl: int, x, targets, recompute: bool):
+        """Runs layer li on microbatch mbl. With recompute only the layer input is stashed, and the head does not run at
+        all: nothing but the loss comes out of it, and the backward pass forms its logits and the loss again."""
         layer = self.layers[li]
+        if recompute and layer.kind == "head":
+            self.stash.put((li, mbl), x)
+            return None
         c = self.ctx(mbl, targets if layer.kind == "head" else None)
         with phase("fwd." + layer.kind):
             if recompute:
@@ -279,8 +283,7 @@ class PipelineStage:
                 y = layer.forward(x, c, self.ops, sv)
                 self.saved[(li, mbl)] = sv
         if layer.kind == "head":
-            if want_loss:
-                self.add_loss(y)
+            self.add_loss(y)
             return None
         return y
 
@@ -293,7 +296,9 @@ class PipelineStage:
             x = self.stash.get((li, mbl))
             sv: dict = {}
             with phase("recompute." + layer.kind):
-                layer.forward(x, c, self.ops, sv)
+                y = layer.forward(x, c, self.ops, sv)
+            if layer.kind == "head":
+                self.add_loss(y)
             if self.cfg.sync_after_recompute and self.device.type == "cuda":
                 # `"skip_compute_sync": false` in the config: the host waits for the recomputed forward, which
                 # lets the caching allocator reuse freed blocks sooner (fewer allocation retries when memory is
