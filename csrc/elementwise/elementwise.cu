@@ -6,6 +6,7 @@
 // (models/gpt_simple.py:119-134) and nn.Embedding (models/llama_simple.py:550-552).
 #include "../common/host.h"
 #include "../common/ptx.cuh"
+#include "act_math.cuh"
 #include <type_traits>
 
 namespace zb {
@@ -75,7 +76,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* gu, __nv_bfloat16* out,
     unpack8e(ld_v4(g), a);
     unpack8e(ld_v4(g + F), b);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = a[j] / (1.f + __expf(-a[j])) * b[j];
+    for (int j = 0; j < 8; ++j) o[j] = swiglu_fwd(a[j], b[j]);
     *reinterpret_cast<uint4*>(out + t * F + c * 8) = pack8e(o);
   }
 }
@@ -95,36 +96,13 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* gu, const __nv_bfloat16* 
     unpack8e(ld_v4(g + F), b);
     unpack8e(ld_v4(dout + t * F + c * 8), d);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float sg = 1.f / (1.f + __expf(-a[j]));
-      float silu = a[j] * sg;
-      da[j] = d[j] * b[j] * (sg * (1.f + a[j] * (1.f - sg)));
-      db[j] = d[j] * silu;
-    }
+    for (int j = 0; j < 8; ++j) swiglu_bwd(a[j], b[j], d[j], da[j], db[j]);
     *reinterpret_cast<uint4*>(dgu + t * 2 * F + c * 8) = pack8e(da);
     *reinterpret_cast<uint4*>(dgu + t * 2 * F + F + c * 8) = pack8e(db);
   }
 }
 
 // ------------------------------- GELU / ReLU -------------------------------
-// kind: 0 = tanh GELU ("gelu_new"), 1 = ReLU, 2 = erf GELU
-__device__ __forceinline__ float act_fwd(float x, int kind) {
-  if (kind == 1) return fmaxf(x, 0.f);
-  if (kind == 2) return 0.5f * x * (1.f + erff(x * 0.7071067811865476f));
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  return 0.5f * x * (1.f + tanhf(k0 * (x + k1 * x * x * x)));
-}
-__device__ __forceinline__ float act_bwd(float x, int kind) {
-  if (kind == 1) return x > 0.f ? 1.f : 0.f;
-  if (kind == 2) {
-    float cdf = 0.5f * (1.f + erff(x * 0.7071067811865476f));
-    return cdf + x * 0.3989422804014327f * __expf(-0.5f * x * x);
-  }
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  float u = k0 * (x + k1 * x * x * x);
-  float th = tanhf(u);
-  return 0.5f * (1.f + th) + 0.5f * x * (1.f - th * th) * k0 * (1.f + 3.f * k1 * x * x);
-}
 __global__ void act_fwd_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, long n8, int kind) {
   chain_trigger();
   chain_wait();
@@ -132,7 +110,11 @@ __global__ void act_fwd_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, long n8
     float a[8], o[8];
     unpack8e(ld_v4(x + i * 8), a);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = act_fwd(a[j], kind);
+    for (int j = 0; j < 8; j += 2) {
+      const float2 v = act_fwd2(make_float2(a[j], a[j + 1]), kind);
+      o[j] = v.x;
+      o[j + 1] = v.y;
+    }
     *reinterpret_cast<uint4*>(y + i * 8) = pack8e(o);
   }
 }
@@ -145,7 +127,11 @@ __global__ void act_bwd_kernel(const __nv_bfloat16* x, const __nv_bfloat16* dy,
     unpack8e(ld_v4(x + i * 8), a);
     unpack8e(ld_v4(dy + i * 8), d);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) o[j] = d[j] * act_bwd(a[j], kind);
+    for (int j = 0; j < 8; j += 2) {
+      const float2 v = act_bwd2(make_float2(a[j], a[j + 1]), kind);
+      o[j] = d[j] * v.x;
+      o[j + 1] = d[j + 1] * v.y;
+    }
     *reinterpret_cast<uint4*>(dx + i * 8) = pack8e(o);
   }
 }

@@ -175,3 +175,82 @@ def test_what_is_declined_and_what_is_refused(ops):
         b = ops.linear_fwd(a, w.repeat(1, 8))
     side.synchronize()
     assert torch.equal(b, ops.linear_fwd(a, w.repeat(1, 8))) and out.shape == (8, 64)
+
+
+def _mlp_reference(x, w, b, act, pre=None, d=None):
+    """The pre-activations and the activation in fp64, or the gradient of the pre-activations for `d`."""
+    h = (x.double() @ w.double().t() + (0 if b is None else b.double())).bfloat16() if pre is None else pre
+    h = h.double().requires_grad_(True)
+    f = torch.nn.functional
+    a = {"swiglu": lambda: f.silu(h[:, :h.shape[1] // 2]) * h[:, h.shape[1] // 2:], "relu": lambda: f.relu(h),
+         "gelu": lambda: f.gelu(h, approximate="tanh"), "gelu_erf": lambda: f.gelu(h)}[act]()
+    if d is None:
+        return a.detach(), h.detach()
+    return torch.autograd.grad(a, h, d.double())[0]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,K,F", [(256, 512, 256), (300, 512, 1376), (1018, 264, 520), (2500, 768, 3080), (520, 4104, 1032),
+                                   (4104, 2048, 2056)])
+@pytest.mark.parametrize("act", ["swiglu", "gelu", "relu", "gelu_erf"])
+def test_activation_in_the_epilogue(ops, T, K, F, act):
+    """Both directions at ragged edges of the tiles (rows, columns, columns of one half of a gated unit), both tile widths and
+    both splits of shared memory (K below and from 2048 on).  The product is rounded to bf16 ahead of the activation, as a pass
+    of its own would find it, and the result once more: 2^-8 of the value covers a flip of the first rounding (a slope of at
+    most 1.13) and the second; the absolute part the same for values near a zero of the activation, whose argument is off by
+    2^-9 of its size, and the fast exponentials and tanh (2^-11 of 1)."""
+    rows = 2 * F if act == "swiglu" else F
+    x, w = _rand(T, K, seed=1), (_rand(rows, K, seed=2).float() / K ** 0.5).bfloat16()
+    b = None if act == "swiglu" else _rand(rows, seed=3)
+    kind = {"gelu": 0, "relu": 1, "gelu_erf": 2, "swiglu": 3}[act]
+    both, keep = k._fast.act_linear_fwd(x, w, b, kind, False), k._fast.act_linear_fwd(x, w, b, kind, True)
+    assert both[1] is None and torch.equal(both[0], keep[0])
+    a, pre = keep
+    assert torch.equal(pre, ops.linear_fwd(x, w, b))
+    plain = k.swiglu_fwd(pre) if act == "swiglu" else k.act_fwd(pre, kind)
+    want, _ = _mlp_reference(x, w, b, act, pre=None)
+    torch.testing.assert_close(a.double(), plain.double(), rtol=2.0 ** -7, atol=1e-6)
+    torch.testing.assert_close(a.double(), want, rtol=2.0 ** -6, atol=0.04)
+    down = (_rand(512, F, seed=4).float() / 512 ** 0.5).bfloat16()
+    dy = _rand(T, 512, seed=5)
+    got = k._fast.act_linear_dgrad(dy, down, pre, kind)
+    da = ops.linear_dgrad(dy, down)
+    plain = k.swiglu_bwd(pre, da) if act == "swiglu" else k.act_bwd(pre, da, kind)
+    torch.testing.assert_close(got.double(), plain.double(), rtol=2.0 ** -7, atol=1e-6)
+    torch.testing.assert_close(got.double(), _mlp_reference(x, w, b, act, pre=pre, d=da), rtol=2.0 ** -6, atol=0.02)
+    k.check_status()
+
+
+@pytest.mark.gpu
+def test_activation_products_that_are_not_for_the_epilogue(ops):
+    """Few rows, few or odd columns: declined, and the two calls they stand for give the result."""
+    for T, K, F in ((255, 512, 512), (300, 512, 248), (300, 512, 516)):
+        x, w = _rand(T, K, seed=1), (_rand(F, K, seed=2).float() / K ** 0.5).bfloat16()
+        assert k._fast.act_linear_fwd(x, w, None, 1, True) is None
+        if F % 8 == 0:
+            a, pre = ops.act_linear_fwd(x, w, None, "relu", True)
+            assert torch.equal(pre, ops.linear_fwd(x, w)) and torch.equal(a, pre.clamp(min=0))
+            d = ops.act_linear_dgrad(_rand(T, 512, seed=3), _rand(512, F, seed=4), pre, "relu")
+            assert d.shape == pre.shape
+    x = _rand(300, 512)
+    assert k._fast.act_linear_fwd(x, _rand(512, 512), _rand(512), 3, True) is None         # a gated unit with a bias
+    assert k._fast.act_linear_dgrad(x, _rand(512, 512), _rand(300, 512), 3) is None        # pre-activations of half the width
+
+
+@pytest.mark.gpu
+def test_gelu_erf_over_all_arguments(ops):
+    """Every bf16 argument against 64 bits.  In fp32 the value is off by a few 2^-24 of itself (the tail is never a difference
+    of larger numbers; the derivative has a zero near -0.75 and is off by a few 2^-24 there), so what is left is the rounding
+    to bf16: half a unit of 8 bits, 2^-8 of the value at most."""
+    x = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).cuda()
+    xd = x.double()
+    phi = torch.exp(-xd * xd / 2) / (2 * torch.pi) ** 0.5
+    cdf = 0.5 * torch.erfc(-xd / 2 ** 0.5)
+    y, dy = k.act_fwd(x, 2), k.act_bwd(x, torch.ones_like(x), 2)
+    for got, want in ((y, xd * cdf), (dy, cdf + xd * phi)):
+        m = torch.isfinite(xd) & torch.isfinite(want) & (want.abs() > 1e-30)
+        assert bool(((got.double() - want).abs()[m] <= (2.0 ** -8 + 1e-6) * want.abs()[m] + 2e-7 * (want.abs()[m] < 0.5)).all())
+    at = lambda t, bits: float(t[bits])
+    assert at(y, 0x7f80) == float("inf") and at(y, 0x0000) == 0.0 and at(y, 0x7f7f) == float(x[0x7f7f]) and at(y, 0xff7f) == 0.0
+    assert torch.isnan(y[0x7fc0]) and torch.isnan(y[0xff80]) and torch.isnan(dy[0x7fc0])       # as before: -inf times 0
+    assert at(dy, 0x0000) == 0.5 and at(dy, 0x7f7f) == 1.0 and at(dy, 0xff7f) == 0.0
