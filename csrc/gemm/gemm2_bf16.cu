@@ -13,6 +13,7 @@
 // Operand layouts and epilogue options are those of gemm_bf16.cu.
 #include "../common/host.h"
 #include "../common/ptx.cuh"
+#include "../elementwise/act_math.cuh"
 #include "gemm_common.cuh"
 #include <algorithm>
 #include <type_traits>
@@ -97,15 +98,15 @@ struct Gemm2Cfg {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int TMEM_COLS = 2 * BN;
   static constexpr int EP_BYTES = 32 * 128;    // epilogue box: 32 rows x 128 bytes
-  // Shared memory is split at launch: 6 operand stages and 2 epilogue boxes per epilogue warp, or 5 and 4.  The sixth
-  // stage is worth 3 - 5 % of the main loop (4096 x 22016 x 4096: 486 -> 472 us), two more boxes shorten the epilogue
-  // of a tile whose old C tile has to be read (load, add, store in flight at once).  The epilogue of a tile runs under
-  // the main loop of the next one, so the boxes only count where that loop is short: K < 2048.
-  // Tiles of 128 columns have stages of 24 KB instead of 32: 8 and 2, or 6 and 4.
-  static constexpr int MAX_STAGES = 8, MAX_EP_BUFS = 4;
-  static constexpr int STAGES_2 = BN == 256 ? 6 : 8, STAGES_4 = BN == 256 ? 5 : 6;   // with 2 / with 4 boxes
-  static constexpr int RING_BYTES = STAGES_2 * STAGE_BYTES + 4 * 2 * EP_BYTES;
-  static_assert(STAGES_4 * STAGE_BYTES + 4 * 4 * EP_BYTES <= RING_BYTES, "both splits fit the same space");
+  // Shared memory is split at launch: 32 KB of epilogue boxes (EP_SMALL) and 6 operand stages, or 64 KB and 5.  The sixth
+  // stage is worth 3 - 5 % of the main loop (4096 x 22016 x 4096: 486 -> 472 us), two boxes per epilogue warp instead of one
+  // shorten the epilogue of a tile (load, add, store in flight at once).  The epilogue of a tile runs under the main loop of
+  // the next one, so the boxes only count where that loop is short: K < 2048.
+  // Tiles of 128 columns have stages of 24 KB instead of 32: 8, or 6.
+  static constexpr int MAX_STAGES = 8, EP_SMALL = 8, EP_LARGE = 16;   // boxes
+  static constexpr int STAGES_S = BN == 256 ? 6 : 8, STAGES_L = BN == 256 ? 5 : 6;
+  static constexpr int RING_BYTES = STAGES_S * STAGE_BYTES + EP_SMALL * EP_BYTES;
+  static_assert(STAGES_L * STAGE_BYTES + EP_LARGE * EP_BYTES <= RING_BYTES, "both splits fit the same space");
   static constexpr int SMEM_BYTES = RING_BYTES + 1024 + 512;
 };
 
@@ -135,16 +136,22 @@ struct Gemm2Extra {
 // FUSED_AG (Params = GemmAgParams): four more warps per CTA pull the peers' parameter shards into the local
 // unsharded buffer while the tiles whose B rows are already present run; each CTA's producer waits for the
 // chunks that cover its own 128 rows of B.
-template <bool A_MN, bool B_MN, typename Params, int BN, int EP_BUFS>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(std::is_same<Params, GemmAgParams>::value ? 320 : 192, 1)
+// EP_WARPS: 4, or 8 in two groups that take the tile's boxes in turns.  A box takes a warp about 0.5 us (accumulators out of
+// tensor memory, conversion, shared memory, fence, store), so with four the end of a product's last tiles lasted 2 us, and
+// at K < 1000 the epilogue of a tile (with an activation above all) was longer than the main loop it has to hide under.
+template <bool A_MN, bool B_MN, typename Params, int BN, int EP_WARPS, int EP_BUFS>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + 32 * EP_WARPS + (std::is_same<Params, GemmAgParams>::value ? 128 : 0), 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                   const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_x,
                   const __grid_constant__ CUtensorMap tmap_w, const Params p, const Gemm2Extra ex) {
   using Cfg = Gemm2Cfg<BN>;
   constexpr bool SCATTER = std::is_same<Params, GemmScatterParams>::value;
   constexpr bool FUSED_AG = std::is_same<Params, GemmAgParams>::value;
+  constexpr int FE = FusedEp<Params>::value;
   constexpr int BK = Cfg::BK, MAXS = Cfg::MAX_STAGES, HALF_N = BN / 2;
-  constexpr int STAGES = EP_BUFS == 2 ? Cfg::STAGES_2 : Cfg::STAGES_4;
+  constexpr int STAGES = EP_WARPS * EP_BUFS == Cfg::EP_SMALL ? Cfg::STAGES_S : Cfg::STAGES_L;
+  static_assert(EP_WARPS * EP_BUFS == Cfg::EP_SMALL || EP_WARPS * EP_BUFS == Cfg::EP_LARGE, "a split of shared memory");
+  constexpr int EP_GROUPS = EP_WARPS / 4;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sE = smem + STAGES * Cfg::STAGE_BYTES;   // epilogue boxes, EP_BUFS per epilogue warp
@@ -152,9 +159,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   uint64_t* full = bars;                          // leader's copy is the one in use
   uint64_t* empty = bars + MAXS;                  // each CTA waits on its own
   uint64_t* tmem_full = bars + 2 * MAXS;          // [2], each CTA waits on its own
-  uint64_t* tmem_empty = bars + 2 * MAXS + 2;     // [2], leader's copy, 8 arrivals
-  uint64_t* x_full = bars + 2 * MAXS + 4;         // [4 warps][MAX_EP_BUFS]: a box of tmap_x has landed
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(x_full + 4 * Cfg::MAX_EP_BUFS);
+  uint64_t* tmem_empty = bars + 2 * MAXS + 2;     // [2], leader's copy, one arrival per epilogue warp of both CTAs
+  uint64_t* x_full = bars + 2 * MAXS + 4;         // [EP_WARPS][EP_BUFS]: a box of tmap_x has landed
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(x_full + Cfg::EP_LARGE);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -183,10 +190,12 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&tmem_full[i], 1);
-      mbar_init(&tmem_empty[i], 8);
+      mbar_init(&tmem_empty[i], 2 * EP_WARPS);
     }
-    for (int i = 0; i < 4 * Cfg::MAX_EP_BUFS; ++i) mbar_init(&x_full[i], 1);
+    for (int i = 0; i < EP_WARPS * EP_BUFS; ++i) mbar_init(&x_full[i], 1);
     mbar_fence_init();
+    tma_prefetch_desc(&tmap_a);   // (parameters of the kernel: nothing the kernel before this one writes)
+    tma_prefetch_desc(&tmap_b);
   }
   if (warp == 1) {
     tmem_alloc_pair(tmem_slot, Cfg::TMEM_COLS);
@@ -205,10 +214,6 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     // ------------------------------ TMA producer (both CTAs) ------------------------------
     {
       const bool elected = elect_one();
-      if (elected) {
-        tma_prefetch_desc(&tmap_a);
-        tma_prefetch_desc(&tmap_b);
-      }
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -218,9 +223,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         kb_range(item, kb0, kb1);
         tile_at(ex.order, tile, tm, tn);
         const int m0 = tm * Cfg::BM + int(cta) * 128;
-        const int n0 = tn * BN + int(cta) * HALF_N;
+        // (a gated unit's tile: rows of the gate's weights in the first CTA, the same rows of the other half in the second)
+        const int n0 = FE == FE_GLU_FWD ? tn * HALF_N + int(cta) * p.N : tn * BN + int(cta) * HALF_N;
         // (the second CTA's half may start past the edge of a ragged tile: its loads then read the fill value)
-        if (!zb_in_bounds(m0 - int(cta) * 128 < p.M && n0 - int(cta) * HALF_N < p.N && tile >= 0, p.status, 1)) break;
+        if (!zb_in_bounds(m0 - int(cta) * 128 < p.M && tn * (FE == FE_GLU_FWD ? HALF_N : BN) < p.N && tile >= 0, p.status, 1)) break;
         if constexpr (FUSED_AG) {
           if (p.gate_flags != nullptr && n0 < p.N) {
             // rows [n0, n0 + HALF_N) of B inside the flat buffer: wait for every chunk of a peer's shard they touch
@@ -307,14 +313,16 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         __syncwarp();
       }
     }
-  } else if (warp < 6) {
+  } else if (warp < 2 + EP_WARPS) {
     // ------------------------------ epilogue (own 128 rows) ------------------------------
-    const int q = warp & 3;
+    const int q = warp & 3;                        // which 32 rows (the lanes of tensor memory this warp may read)
+    const int h = EP_GROUPS > 1 ? (warp - 2) >> 2 : 0;   // boxes h, h + EP_GROUPS, ... of a tile
     const EpilogueCfg ecfg = epilogue_cfg(p);
-    uint8_t* my_boxes = sE + q * EP_BUFS * Cfg::EP_BYTES;
-    uint64_t* my_full = x_full + q * Cfg::MAX_EP_BUFS;
-    const uint32_t slot_mask = uint32_t(EP_BUFS) - 1, phase_shift = EP_BUFS == 4 ? 2 : 1;
-    const int ahead = EP_BUFS == 4 ? 2 : 1;   // boxes of tmap_x requested ahead of the one being added
+    uint8_t* my_boxes = sE + (warp - 2) * EP_BUFS * Cfg::EP_BYTES;
+    uint64_t* my_full = x_full + (warp - 2) * EP_BUFS;
+    static_assert(EP_BUFS == 2 || EP_BUFS == 4, "a power of two");
+    constexpr uint32_t slot_mask = uint32_t(EP_BUFS) - 1, phase_shift = EP_BUFS == 4 ? 2 : 1;
+    auto mine = [&](int n) { return n > h ? (n - h + EP_GROUPS - 1) / EP_GROUPS : 0; };   // of a tile's n boxes
     uint32_t ep_count = 0;   // boxes this warp has stored: slot and barrier phase of the next one
     int local = 0;
     for (int item = pair; item < num_items; item += num_pairs, ++local) {
@@ -325,20 +333,206 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const int n0 = tn * BN;
       const int buf = local & 1;
       const uint32_t use = uint32_t(local >> 1);
-      if (!SCATTER && ex.ep != EP_DIRECT) {
+      if constexpr (FE != FE_NONE) {
+        // ---- activation in the epilogue: groups of 64 columns, each one to three boxes ----
+        constexpr int COLS = FE == FE_GLU_FWD ? HALF_N : BN;
+        constexpr int LOADS = FE == FE_ACT_BWD ? 1 : FE == FE_GLU_BWD ? 2 : 0;
+        const int row0 = m0 + q * 32, c0 = tn * COLS;
+        const int groups = mine(row0 < p.M ? min(COLS / 64, (p.N - c0 + 63) / 64) : 0);
+        auto col_of = [&](int g) { return c0 + (h + g * EP_GROUPS) * 64; };
+        const int per_group = LOADS > 0 ? LOADS : p.keep ? (FE == FE_GLU_FWD ? 3 : 2) : 1;
+        auto box_of = [&](uint32_t k) { return my_boxes + (k & slot_mask) * Cfg::EP_BYTES; };
+        auto load_group = [&](int g) {   // the pre-activations of group g (lane 0)
+#pragma unroll
+          for (int u = 0; u < LOADS; ++u) {
+            const uint32_t k = ep_count + uint32_t(g * LOADS + u);
+            mbar_expect_tx(&my_full[k & slot_mask], Cfg::EP_BYTES);
+            if (FE == FE_GLU_BWD) tma_load_3d(box_of(k), &tmap_x, &my_full[k & slot_mask], col_of(g), u, row0);
+            else tma_load_2d(box_of(k), &tmap_x, &my_full[k & slot_mask], col_of(g), row0);
+          }
+        };
+        static_assert(EP_BUFS == 2, "a group has two boxes at a time");
+        const TileBias bias(p, c0, COLS, lane);
+        constexpr int DEPTH = LOADS > 0 ? EP_BUFS / LOADS : 1;   // groups whose loads the boxes hold
+        if (LOADS > 0 && lane == 0) {
+          bulk_wait_read<0>();
+          for (int g = 0; g < DEPTH && g < groups; ++g) load_group(g);
+        }
+        if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full[buf], use & 1, wctx, ST_TIMEOUT_TMEM_FULL))) break;
+        tc_fence_after();
+        auto release_tmem = [&] {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(&tmem_empty[buf], 0);
+        };
+        bool ok = true;
+        if (groups == 0) release_tmem();
+#pragma unroll 1
+        for (int g = 0; g < groups; ++g) {
+          const uint32_t k = ep_count + uint32_t(g * per_group);
+          const uint32_t row_off = uint32_t(lane) * 128, sw = uint32_t(lane & 7);
+          const uint32_t box0 = smem_u32(box_of(k)) + row_off, box1 = smem_u32(box_of(k + 1)) + row_off;
+          const int col = col_of(g);
+          const uint32_t t_addr = tmem_base + (uint32_t(q * 32) << 16) + uint32_t(buf * BN + col - c0);
+          uint32_t r[32], s[32];
+          tmem_ld32(t_addr, r);
+          tmem_ld32(t_addr + (FE == FE_GLU_FWD ? uint32_t(HALF_N) : 32u), s);
+          if (lane == 0) {
+            if (LOADS > 0) {
+              if (g > 0 && g - 1 + DEPTH < groups) {   // the boxes of group g - 1 take the loads of group g - 1 + DEPTH
+                bulk_wait_read<0>();
+                load_group(g - 1 + DEPTH);
+              }
+            } else if (per_group == 1) {
+              bulk_wait_read<EP_BUFS - 1>();
+            } else {
+              bulk_wait_read<0>();   // two or three boxes: all
+            }
+          }
+          tmem_wait_ld();
+          if constexpr (FE == FE_GLU_FWD) {
+            uint4 a[8];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              if (c == 1) {
+                tmem_ld32(t_addr + 32u, r);
+                tmem_ld32(t_addr + uint32_t(HALF_N) + 32u, s);
+                tmem_wait_ld();
+                if (g == groups - 1) release_tmem();
+              } else {
+                __syncwarp();
+              }
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const uint4 x = pack_f32x8(r, 8 * j), y = pack_f32x8(s, 8 * j);
+                const uint32_t off = (uint32_t(c * 4 + j) ^ sw) << 4;
+                if (p.keep) {
+                  st_shared_v4(box0 + off, x.x, x.y, x.z, x.w);
+                  st_shared_v4(box1 + off, y.x, y.y, y.z, y.w);
+                }
+                // of the values as they are stored, like a pass over them would see them
+                const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+                uint32_t o[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  const float2 gate = unpack_bf16x2(xs[u]), up = unpack_bf16x2(ys[u]);
+                  o[u] = pack_bf16x2(swiglu_fwd(gate.x, up.x), swiglu_fwd(gate.y, up.y));
+                }
+                a[c * 4 + j] = make_uint4(o[0], o[1], o[2], o[3]);
+              }
+            }
+            uint8_t* last = box_of(k + uint32_t(per_group - 1));
+            if (p.keep) {
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                if (zb_in_bounds(row0 >= 0 && row0 < p.M && col >= 0 && col < p.N, p.status, 2)) {
+                  tma_store_3d(&tmap_c, box_of(k), col, 0, row0);
+                  tma_store_3d(&tmap_c, box_of(k + 1), col, 1, row0);
+                }
+                bulk_commit();
+                bulk_wait_read<0>();   // the third box takes the place of the first
+              }
+              __syncwarp();
+            }
+            const uint32_t at = smem_u32(last) + row_off;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) st_shared_v4(at + ((uint32_t(j) ^ sw) << 4), a[j].x, a[j].y, a[j].z, a[j].w);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (zb_in_bounds(row0 >= 0 && row0 < p.M && col >= 0 && col < p.N, p.status, 2)) tma_store_2d(&tmap_w, last, col, row0);
+              bulk_commit();
+            }
+          } else {
+            if (g == groups - 1) release_tmem();
+            if constexpr (FE == FE_ACT_FWD) {
+              bias.add(p, col - c0, r);
+              bias.add(p, col - c0 + 32, s);
+              __syncwarp();
+            } else {
+              __syncwarp();
+#pragma unroll
+              for (int u = 0; u < LOADS; ++u)
+                ok = ok && __all_sync(0xffffffffu, mbar_wait(&my_full[(k + u) & slot_mask], ((k + u) >> phase_shift) & 1, wctx, ST_TIMEOUT_FULL));
+              if (!ok) break;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const uint4 x = j < 4 ? pack_f32x8(r, 8 * j) : pack_f32x8(s, 8 * (j - 4));   // h, or the gradient of the activation
+              const uint32_t off = (uint32_t(j) ^ sw) << 4;
+              const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+              uint32_t o[4], o2[4];
+              if constexpr (FE == FE_ACT_FWD) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  const float2 a = act_fwd2(unpack_bf16x2(xs[u]), p.act);
+                  o[u] = pack_bf16x2(a.x, a.y);
+                }
+                if (p.keep) st_shared_v4(box0 + off, x.x, x.y, x.z, x.w);
+                st_shared_v4((p.keep ? box1 : box0) + off, o[0], o[1], o[2], o[3]);
+              } else if constexpr (FE == FE_ACT_BWD) {
+                const uint4 h = ld_shared_v4(box0 + off);
+                const uint32_t hs[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  const float2 d = unpack_bf16x2(xs[u]), slope = act_bwd2(unpack_bf16x2(hs[u]), p.act);
+                  o[u] = pack_bf16x2(d.x * slope.x, d.y * slope.y);
+                }
+                st_shared_v4(box0 + off, o[0], o[1], o[2], o[3]);
+              } else {
+                const uint4 gv = ld_shared_v4(box0 + off), uv = ld_shared_v4(box1 + off);
+                const uint32_t gs[4] = {gv.x, gv.y, gv.z, gv.w}, us[4] = {uv.x, uv.y, uv.z, uv.w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  const float2 d = unpack_bf16x2(xs[u]), gate = unpack_bf16x2(gs[u]), up = unpack_bf16x2(us[u]);
+                  float dg0, dg1, du0, du1;
+                  swiglu_bwd(gate.x, up.x, d.x, dg0, du0);
+                  swiglu_bwd(gate.y, up.y, d.y, dg1, du1);
+                  o[u] = pack_bf16x2(dg0, dg1);
+                  o2[u] = pack_bf16x2(du0, du1);
+                }
+                st_shared_v4(box0 + off, o[0], o[1], o[2], o[3]);
+                st_shared_v4(box1 + off, o2[0], o2[1], o2[2], o2[3]);
+              }
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              const bool in = zb_in_bounds(row0 >= 0 && row0 < p.M && col >= 0 && col < p.N, p.status, 2);
+              if constexpr (FE == FE_ACT_FWD) {
+                if (p.keep) {
+                  if (in) tma_store_2d(&tmap_c, box_of(k), col, row0);
+                  bulk_commit();
+                }
+                if (in) tma_store_2d(&tmap_w, box_of(k + uint32_t(per_group - 1)), col, row0);
+              } else if constexpr (FE == FE_ACT_BWD) {
+                if (in) tma_store_2d(&tmap_c, box_of(k), col, row0);
+              } else {
+                if (in) tma_store_3d(&tmap_c, box_of(k), col, 0, row0);
+                if (in) tma_store_3d(&tmap_c, box_of(k + 1), col, 1, row0);
+              }
+              bulk_commit();
+            }
+          }
+        }
+        ep_count += uint32_t(groups * per_group);
+        if (!ok) break;
+      } else if (!SCATTER && ex.ep != EP_DIRECT) {
         const bool f32 = split || ex.ep == EP_F32;
         const int row0 = m0 + q * 32;
         const int wide = f32 ? 32 : 64;                    // columns of a box
-        const int boxes = split ? BN / 32 : row0 < p.M ? min(BN / wide, (p.N - n0 + wide - 1) / wide) : 0;
-        auto load_box = [&](int c) {   // box c of this tile -> its ring slot (lane 0)
-          const uint32_t k = ep_count + uint32_t(c);
+        const int boxes = mine(split ? BN / 32 : row0 < p.M ? min(BN / wide, (p.N - n0 + wide - 1) / wide) : 0);
+        auto col_of = [&](int i) { return n0 + (h + i * EP_GROUPS) * wide; };   // this warp's i-th box
+        auto load_box = [&](int i) {   // old C or addend -> its ring slot (lane 0)
+          const uint32_t k = ep_count + uint32_t(i);
           mbar_expect_tx(&my_full[k & slot_mask], Cfg::EP_BYTES);
-          tma_load_2d(my_boxes + (k & slot_mask) * Cfg::EP_BYTES, &tmap_x, &my_full[k & slot_mask], n0 + c * 64, row0);
+          tma_load_2d(my_boxes + (k & slot_mask) * Cfg::EP_BYTES, &tmap_x, &my_full[k & slot_mask], col_of(i), row0);
         };
+        const TileBias bias(p, n0, BN, lane);
         if (ex.ep_load && !split && lane == 0) {
-          bulk_wait_read<0>();   // stores of earlier boxes (issued a main loop ago) still hold the slots of boxes 0 and 1
-          if (boxes > 0) load_box(0);
-          if (boxes > 1) load_box(1);
+          bulk_wait_read<0>();   // stores of earlier boxes (issued a main loop ago) still hold the slots
+          for (int i = 0; i < EP_BUFS && i < boxes; ++i) load_box(i);
         }
         if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full[buf], use & 1, wctx, ST_TIMEOUT_TMEM_FULL))) break;
         tc_fence_after();
@@ -347,24 +541,21 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(&tmem_empty[buf], 0);
         };
-        auto wait_slot = [&] {      // the store of box k - EP_BUFS has left the slot of box k
-          if (EP_BUFS == 4) bulk_wait_read<3>();
-          else bulk_wait_read<1>();
-        };
+        auto wait_slot = [&] { bulk_wait_read<EP_BUFS - 1>(); };   // the store of box k - EP_BUFS has left the slot of box k
         bool ok = true;
         if (boxes == 0) release_tmem();
         for (int c = 0; c < boxes; ++c) {
           const uint32_t k = ep_count + uint32_t(c);
           const uint32_t box = smem_u32(my_boxes + (k & slot_mask) * Cfg::EP_BYTES) + uint32_t(lane) * 128;
-          const int col0 = n0 + c * wide;
-          const uint32_t t_addr = tmem_base + (uint32_t(q * 32) << 16) + uint32_t(buf * BN + c * wide);
+          const int col0 = col_of(c);
+          const uint32_t t_addr = tmem_base + (uint32_t(q * 32) << 16) + uint32_t(buf * BN + col0 - n0);
           if (f32) {
             uint32_t r[32];
             tmem_ld32(t_addr, r);
             if (lane == 0) wait_slot();
             tmem_wait_ld();
             if (c == boxes - 1) release_tmem();
-            if (!split) epilogue_bias_act(p, col0, r);
+            if (!split) { bias.add(p, col0 - n0, r); epilogue_act(p, r); }
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < 8; ++j)
@@ -376,17 +567,17 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             if (lane == 0) {
               if (!ex.ep_load) {
                 wait_slot();
-              } else if (c + ahead >= 2 && c + ahead < boxes) {
-                // box k + ahead takes the slot of box k - ahead, which has to have left
-                if (ahead == 2) bulk_wait_read<1>();
-                else bulk_wait_read<0>();
-                load_box(c + ahead);
+              } else if (c > 0 && c - 1 + EP_BUFS < boxes) {
+                bulk_wait_read<0>();   // box c - 1 has left: its slot takes the next one
+                load_box(c - 1 + EP_BUFS);
               }
             }
             tmem_wait_ld();
             if (c == boxes - 1) release_tmem();
-            epilogue_bias_act(p, col0, r);
-            epilogue_bias_act(p, col0 + 32, s);
+            bias.add(p, col0 - n0, r);
+            bias.add(p, col0 - n0 + 32, s);
+            epilogue_act(p, r);
+            epilogue_act(p, s);
             __syncwarp();
             if (ex.ep_load) {
               ok = __all_sync(0xffffffffu, mbar_wait(&my_full[k & slot_mask], (k >> phase_shift) & 1, wctx, ST_TIMEOUT_FULL));
@@ -409,7 +600,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (lane == 0) {
             const void* src = my_boxes + (k & slot_mask) * Cfg::EP_BYTES;
             if (split) {
-              tma_store_2d(&tmap_w, src, c * 32, (item - ex.full) * Cfg::BM + int(cta) * 128 + q * 32);
+              tma_store_2d(&tmap_w, src, col0 - n0, (item - ex.full) * Cfg::BM + int(cta) * 128 + q * 32);
             } else if (zb_in_bounds(row0 >= 0 && row0 < p.M && col0 >= 0 && col0 < p.N, p.status, 2)) {
               if (ex.ep == EP_F32 && ecfg.accum) tma_reduce_add_2d(&tmap_c, src, col0, row0);
               else tma_store_2d(&tmap_c, src, col0, row0);
@@ -430,7 +621,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         crow = static_cast<__nv_bfloat16*>(p.sc_dst[owner]) + size_t(row - owner * p.sc_rows) * p.ldc;
       }
 #pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
+      for (int c = h; c < BN / 32; c += EP_GROUPS) {
         const int col0 = n0 + c * 32;
         if (col0 >= p.N) break;
         uint32_t r[32];
@@ -445,14 +636,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       if (lane == 0) mbar_arrive_cluster(&tmem_empty[buf], 0);
       }
     }
-    if (lane == 0) bulk_wait_all();
     if constexpr (SCATTER) __threadfence_system();   // this thread's rows are visible to their owners before the flags
   }
 
-  if constexpr (FUSED_AG) if (warp >= 6) {
+  if constexpr (FUSED_AG) if (warp >= 2 + EP_WARPS) {
     // ------------------------------ all-gather copy warps ------------------------------
     const AgParams& ag = p.ag;
-    const int ct = threadIdx.x - 192;  // 0..127
+    const int ct = threadIdx.x - (64 + 32 * EP_WARPS);  // 0..127
     __shared__ int s_peer_ok;
     const int total = (ag.R - 1) * ag.cps;
     const long chunk16 = ag.chunk_bytes / 16;
@@ -517,7 +707,14 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
   }
   tc_fence_before();
-  cluster_sync_all();  // the leader's MMAs read the peer's shared memory: leave together
+  // The leader's MMAs read the peer's shared memory: leave together.  Where nothing written before is read behind this
+  // barrier it need not order memory: a releasing arrival waits for the epilogue's own writes, 0.7 us at the end of every
+  // product.  The stores of the last boxes are still being read meanwhile (their writes are complete when the grid is).
+  if constexpr (SCATTER || FUSED_AG) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+  else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  if (warp >= 2 && lane == 0) bulk_wait_read<0>();
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
@@ -711,11 +908,13 @@ static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, 
   else if (p.N % 64 == 0) { rc = make_tmap_mn3d(&tb, B, p.K, p.N, ldb, BN / 128); ex.b_3d = 1; }
   else rc = make_tmap_2d_bf16(&tb, B, p.K, p.N, ldb, 64, 64);
   if (rc) return rc;
-  // fewer stages and four boxes where the tile's epilogue is not hidden by a long main loop (comment at Gemm2Cfg)
-  const bool short_k = std::is_same<Params, GemmParams>::value && ex.ep != EP_DIRECT && p.K < 2048;
-  auto kern = gemm2_bf16_kernel<A_MN, B_MN, Params, BN, 2>;
-  if constexpr (std::is_same<Params, GemmParams>::value) {
-    if (short_k) kern = gemm2_bf16_kernel<A_MN, B_MN, Params, BN, 4>;
+  // fewer stages and two boxes per warp where the tile's epilogue is not hidden by a long main loop (comment at Gemm2Cfg)
+  constexpr bool PLAIN = std::is_same<Params, GemmParams>::value;
+  constexpr int WARPS = 4;
+  const bool short_k = PLAIN && ex.ep != EP_DIRECT && p.K < 2048;
+  auto kern = gemm2_bf16_kernel<A_MN, B_MN, Params, BN, WARPS, Gemm2Cfg<BN>::EP_SMALL / WARPS>;
+  if constexpr (PLAIN) {
+    if (short_k) kern = gemm2_bf16_kernel<A_MN, B_MN, Params, BN, WARPS, Gemm2Cfg<BN>::EP_LARGE / WARPS>;
   }
   static bool attr_set[2] = {false, false};
   if (!attr_set[short_k]) {
@@ -734,9 +933,9 @@ static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, 
   }
   if (ex.items < pairs) pairs = ex.items;
   if constexpr (std::is_same<Params, GemmParams>::value) {
-    ZB_CUDA_OK(launch_chained(kern, dim3(2 * pairs), 192, Cfg::SMEM_BYTES, stream, 0, ta, tb, tc, tx, tw, p, ex));
+    ZB_CUDA_OK(launch_chained(kern, dim3(2 * pairs), 64 + 32 * WARPS, Cfg::SMEM_BYTES, stream, 0, ta, tb, tc, tx, tw, p, ex));
   } else {
-    kern<<<2 * pairs, std::is_same<Params, GemmAgParams>::value ? 320 : 192, Cfg::SMEM_BYTES, stream>>>(ta, tb, tc, tx, tw, p, ex);
+    kern<<<2 * pairs, 64 + 32 * WARPS + (std::is_same<Params, GemmAgParams>::value ? 128 : 0), Cfg::SMEM_BYTES, stream>>>(ta, tb, tc, tx, tw, p, ex);
     ZB_CUDA_OK(cudaGetLastError());
   }
   if constexpr (std::is_same<Params, GemmParams>::value) {
@@ -747,6 +946,82 @@ static int launch_gemm2(const void* A, const void* B, const Params& p, int lda, 
     }
   }
   return 0;
+}
+
+// [rows][2][F] view of a gated unit's pre-activations (gate | up): boxes of 32 rows x 64 columns of one half, clipped at F
+static int make_tmap_halves(CUtensorMap* out, const void* base, uint64_t rows, uint64_t F) {
+  uint64_t dims[3] = {F, 2, rows};
+  uint64_t strides[2] = {F * 2, F * 4};
+  uint32_t box[3] = {64, 1, 32};
+  return make_tmap_nd_bf16(out, base, 3, dims, strides, box);
+}
+
+// Products with an activation in the epilogue.  FE_ACT_FWD: act(A B^T + bias) -> out, A B^T + bias -> pre.  FE_GLU_FWD: the
+// same for a gated unit (B: gate and up weights, N = F).  FE_ACT_BWD / FE_GLU_BWD: (A B) times the activation's derivative
+// at `pre` -> out.  All matrices but A and B are dense.
+//
+// As passes of their own the activations read and write everything once more (4096 x 11008, gated: 47 us forward, 79
+// backward) and cost a launch each; here the forward one works on accumulators, and the backward one fetches only what it
+// needs, under the main loop of the next tile.
+template <int FE, int BN>
+static int launch_gemm2_fused(const void* A, const void* B, void* pre, void* out, const GemmFusedParams<FE>& p, int lda, int ldb,
+                              cudaStream_t stream) {
+  using Cfg = Gemm2Cfg<BN>;
+  using Params = GemmFusedParams<FE>;
+  constexpr bool FWD = FE == FE_ACT_FWD || FE == FE_GLU_FWD, GLU = FE == FE_GLU_FWD || FE == FE_GLU_BWD;
+  const int cols = FE == FE_GLU_FWD ? 2 * p.N : p.N;   // of the accumulators
+  int pairs = num_sms() / 2;
+  if (BN == 256 && gemm2_plan(p.M, cols, p.K, pairs, false).bn == 128)
+    return launch_gemm2_fused<FE, 128>(A, B, pre, out, p, lda, ldb, stream);
+  CUtensorMap ta, tb, tc = {}, tx = {}, tw = {};
+  Gemm2Extra ex = {};
+  ex.ep = EP_BF16;
+  int rc = make_tmap_2d_bf16(&ta, A, p.M, p.K, lda, 128, 64);
+  if (rc) return rc;
+  if (FWD) rc = make_tmap_2d_bf16(&tb, B, cols, p.K, ldb, BN / 2, 64);
+  else if (p.N % 64 == 0) { rc = make_tmap_mn3d(&tb, B, p.K, p.N, ldb, BN / 128); ex.b_3d = 1; }
+  else rc = make_tmap_2d_bf16(&tb, B, p.K, p.N, ldb, 64, 64);
+  if (rc) return rc;
+  if (FWD) {
+    if ((rc = make_tmap_2d_out(&tw, out, p.M, p.N, p.N, false, 32))) return rc;
+    if (p.keep) {
+      rc = GLU ? make_tmap_halves(&tc, pre, p.M, p.N) : make_tmap_2d_out(&tc, pre, p.M, p.N, p.N, false, 32);
+      if (rc) return rc;
+    }
+  } else {
+    rc = GLU ? make_tmap_halves(&tx, pre, p.M, p.N) : make_tmap_2d_out(&tx, pre, p.M, p.N, p.N, false, 32);
+    if (rc) return rc;
+    rc = GLU ? make_tmap_halves(&tc, out, p.M, p.N) : make_tmap_2d_out(&tc, out, p.M, p.N, p.N, false, 32);
+    if (rc) return rc;
+  }
+  // two boxes per warp: eight warps and fewer stages where the main loop is short, four and the full ring elsewhere
+  const bool short_k = p.K < 2048;
+  auto kern = short_k ? gemm2_bf16_kernel<false, !FWD, Params, BN, 8, 2> : gemm2_bf16_kernel<false, !FWD, Params, BN, 4, 2>;
+  static bool attr_set[2] = {false, false};
+  if (!attr_set[short_k]) {
+    ZB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+    attr_set[short_k] = true;
+  }
+  ex.order = gemm2_tile_order<Params, BN>(p.M, cols, p.K);
+  ex.items = ex.full = ex.order.tiles_m * ex.order.tiles_n;
+  ex.splits = 1;
+  if (ex.items < pairs) pairs = ex.items;
+  ZB_CUDA_OK(launch_chained(kern, dim3(2 * pairs), short_k ? 320 : 192, Cfg::SMEM_BYTES, stream, 0, ta, tb, tc, tx, tw, p, ex));
+  return 0;
+}
+
+template <int FE>
+static int gemm2_fused_entry(const void* A, const void* B, const void* bias, void* pre, void* out, int M, int N, int K, int lda,
+                             int ldb, int act, int keep, int* status, cudaStream_t stream) {
+  GemmFusedParams<FE> p = {};
+  p.C = out;
+  p.bias = static_cast<const __nv_bfloat16*>(bias);
+  p.M = M; p.N = N; p.K = K;
+  p.ldc = N;
+  p.status = status;
+  p.act = act;
+  p.keep = keep;
+  return launch_gemm2_fused<FE, 256>(A, B, pre, out, p, lda, ldb, stream);
 }
 
 static int gemm2_entry(const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
@@ -795,6 +1070,30 @@ extern "C" int zb_gemm2_split_bf16(const void* A, const void* B, void* C, int M,
                                    int flags, void* workspace, long workspace_bytes, int* status, cudaStream_t stream) {
   return zb::gemm2_entry(A, B, C, M, N, K, lda, ldb, ldc, a_mn_major, b_mn_major, bias, addend, ld_addend, flags, 0,
                          static_cast<float*>(workspace), workspace_bytes, status, stream);
+}
+// MLP up-projection and activation: out = act(x w^T + bias).  act 0, 1, 2: as zb_act_fwd, w [N, K]; act 3: gated unit, w
+// [2N, K] = gate | up, no bias.  pre: the pre-activations ([M, N], act 3 [M, 2N]) are stored there, nullptr: not at all.
+// Returns 1, with nothing done, where the pair kernel or TMA cannot take it (fewer than 256 rows or columns, N % 8).
+extern "C" int zb_gemm2_act_fwd(const void* x, const void* w, const void* bias, void* pre, void* out, int M, int N, int K, int lda,
+                                int ldb, int act, int* status, cudaStream_t stream) {
+  using namespace zb;
+  if (M < 256 || N < 256 || K <= 0 || N % 8 || act < 0 || act > 3 || (act == 3 && bias != nullptr) ||
+      ((reinterpret_cast<uintptr_t>(pre) | reinterpret_cast<uintptr_t>(out)) & 15))
+    return 1;
+  if (act == 3) return gemm2_fused_entry<FE_GLU_FWD>(x, w, nullptr, pre, out, M, N, K, lda, ldb, 0, pre != nullptr, status, stream);
+  return gemm2_fused_entry<FE_ACT_FWD>(x, w, bias, pre, out, M, N, K, lda, ldb, act, pre != nullptr, status, stream);
+}
+// Gradient of the pre-activations: dpre = (dy w) act'(pre), w [K, N] (K: columns of dy); act 3: pre and dpre [M, 2N].
+// Returns 1 as zb_gemm2_act_fwd.
+extern "C" int zb_gemm2_act_bwd(const void* dy, const void* w, const void* pre, void* dpre, int M, int N, int K, int lda, int ldb,
+                                int act, int* status, cudaStream_t stream) {
+  using namespace zb;
+  if (M < 256 || N < 256 || K <= 0 || N % 8 || act < 0 || act > 3 ||
+      ((reinterpret_cast<uintptr_t>(pre) | reinterpret_cast<uintptr_t>(dpre)) & 15))
+    return 1;
+  void* h = const_cast<void*>(pre);
+  if (act == 3) return gemm2_fused_entry<FE_GLU_BWD>(dy, w, nullptr, h, dpre, M, N, K, lda, ldb, 0, 0, status, stream);
+  return gemm2_fused_entry<FE_ACT_BWD>(dy, w, nullptr, h, dpre, M, N, K, lda, ldb, act, 0, status, stream);
 }
 // C = A @ B^T (b_mn_major: A @ B) with the output rows scattered for a row-wise reduce-scatter over
 // R ranks: rows [q * M / R, (q + 1) * M / R) go to dst_ptrs[q] (this rank's bf16 staging slot in rank

@@ -48,6 +48,8 @@ struct Entry {
   int (*flash_bwd3)(const void*, const void*, const void*, const float*, void*, float*, int, int, int, int, int, int, int, float,
                     int*, int, unsigned long long*, int, cudaStream_t);
   int (*flash_stats_floats)(int, int, int);
+  int (*gemm2_act_fwd)(const void*, const void*, const void*, void*, void*, int, int, int, int, int, int, int*, cudaStream_t);
+  int (*gemm2_act_bwd)(const void*, const void*, const void*, void*, int, int, int, int, int, int, int*, cudaStream_t);
   const char* (*last_error)();
 };
 Entry lib;
@@ -204,6 +206,65 @@ PyObject* linear_wgrad(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
       return nullptr;
   }
   Py_RETURN_TRUE;
+  END_HANDLE_TH_ERRORS
+}
+
+constexpr int64_t ACT_SWIGLU = 3;   // the activation kinds of zb_gemm2_act_fwd: 0 - 2 as in act_fwd
+
+// act_linear_fwd(x, w, bias | None, kind, keep) -> (act(x w^T + bias), pre-activations | None)
+PyObject* act_linear_fwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  ZB_ARGS(5)
+  const Tensor *x = tensor_of(args[0]), *w = tensor_of(args[1]), *bias;
+  int64_t kind;
+  if (!optional_tensor(args[2], bias) || !matrix(x, BF16) || !matrix(w, BF16) || !int_arg(args[3], kind) || kind < 0 ||
+      kind > ACT_SWIGLU || !on(w, *x) || !on(bias, *x))
+    Py_RETURN_NONE;
+  const int64_t M = x->size(0), K = x->size(1), W = w->size(0), N = kind == ACT_SWIGLU ? W / 2 : W;
+  int* status = status_of(*x);
+  if (status == nullptr || w->size(1) != K || !fits(M) || !fits(W) || !fits(K) || !fits(x->stride(0)) || !fits(w->stride(0)) ||
+      (kind == ACT_SWIGLU && (bias != nullptr || W % 2)) || M < 256 || N < 256 || N % 8)
+    Py_RETURN_NONE;
+  if (bias != nullptr && !(dense(bias, BF16) && bias->dim() == 1 && bias->size(0) == W)) Py_RETURN_NONE;
+  Tensor out = empty({M, N}, *x, BF16), pre;
+  if (truth(args[4])) pre = empty({M, W}, *x, BF16);
+  void* pp = pre.defined() ? pre.data_ptr() : nullptr;
+  const cudaStream_t s = stream();
+  if (!launch("gemm2_act_fwd", 1, [&] {
+        return lib.gemm2_act_fwd(ptr(x), ptr(w), ptr(bias), pp, out.data_ptr(), int(M), int(N), int(K), int(x->stride(0)),
+                                 int(w->stride(0)), int(kind), status, s);
+      }))
+    return nullptr;
+  PyObject* r = PyTuple_New(2);
+  if (r == nullptr) return nullptr;
+  PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(std::move(out)));
+  PyTuple_SET_ITEM(r, 1, pp != nullptr ? THPVariable_Wrap(std::move(pre)) : Py_NewRef(Py_None));
+  return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// act_linear_dgrad(dy, w, pre, kind) -> (dy w) act'(pre)
+PyObject* act_linear_dgrad(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  ZB_ARGS(4)
+  const Tensor *dy = tensor_of(args[0]), *w = tensor_of(args[1]), *pre = tensor_of(args[2]);
+  int64_t kind;
+  if (!matrix(dy, BF16) || !matrix(w, BF16) || !dense(pre, BF16) || pre->dim() != 2 || !int_arg(args[3], kind) || kind < 0 ||
+      kind > ACT_SWIGLU || !on(w, *dy) || !on(pre, *dy))
+    Py_RETURN_NONE;
+  const int64_t M = dy->size(0), K = dy->size(1), N = w->size(1);
+  int* status = status_of(*dy);
+  if (status == nullptr || w->size(0) != K || pre->size(0) != M || pre->size(1) != (kind == ACT_SWIGLU ? 2 * N : N) || !fits(M) ||
+      !fits(2 * N) || !fits(K) || !fits(dy->stride(0)) || !fits(w->stride(0)) || M < 256 || N < 256 || N % 8)
+    Py_RETURN_NONE;
+  Tensor dpre = empty(pre->sizes(), *dy, BF16);
+  const cudaStream_t s = stream();
+  if (!launch("gemm2_act_bwd", 1, [&] {
+        return lib.gemm2_act_bwd(ptr(dy), ptr(w), ptr(pre), dpre.data_ptr(), int(M), int(N), int(K), int(dy->stride(0)),
+                                 int(w->stride(0)), int(kind), status, s);
+      }))
+    return nullptr;
+  return THPVariable_Wrap(std::move(dpre));
   END_HANDLE_TH_ERRORS
 }
 
@@ -448,7 +509,7 @@ PyObject* launch_count(PyObject*, PyObject* const*, Py_ssize_t) { return PyLong_
 
 #define ZB_FN(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {ZB_FN(init), ZB_FN(set_status), ZB_FN(launch_count), ZB_FN(linear_fwd), ZB_FN(linear_dgrad),
-                         ZB_FN(linear_wgrad), ZB_FN(norm_fwd), ZB_FN(norm_bwd), ZB_FN(rope), ZB_FN(swiglu_fwd),
+                         ZB_FN(linear_wgrad), ZB_FN(act_linear_fwd), ZB_FN(act_linear_dgrad), ZB_FN(norm_fwd), ZB_FN(norm_bwd), ZB_FN(rope), ZB_FN(swiglu_fwd),
                          ZB_FN(swiglu_bwd), ZB_FN(act_fwd), ZB_FN(act_bwd), ZB_FN(attn_fwd), ZB_FN(attn_bwd),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "zorse_fastops", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

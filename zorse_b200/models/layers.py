@@ -196,8 +196,7 @@ class TransformerBlock(Layer):
 
     def _mlp_fwd(self, xin, resid, ops, sv):
         p = self.p
-        hpre = ops.linear_fwd(xin, p["up_w"], p.get("up_b"))
-        a = ops.swiglu_fwd(hpre) if self.act == "swiglu" else ops.act_fwd(hpre, self.act)
+        a, hpre = ops.act_linear_fwd(xin, p["up_w"], p.get("up_b"), self.act, sv is not None)
         out = ops.linear_fwd(a, p["down_w"], p.get("down_b"), addend=resid)
         if sv is not None:
             sv.update(hpre=hpre, mlp_a=a)
@@ -205,9 +204,8 @@ class TransformerBlock(Layer):
 
     def _mlp_bwd(self, dout, xin, ops, sv, dres):
         p, g = self.p, self.g
-        da = ops.linear_dgrad(dout, p["down_w"])
+        dh = ops.act_linear_dgrad(dout, p["down_w"], sv["hpre"], self.act)
         ops.linear_wgrad(dout, sv["mlp_a"], g["down_w"], g.get("down_b"))
-        dh = ops.swiglu_bwd(sv["hpre"], da) if self.act == "swiglu" else ops.act_bwd(sv["hpre"], da, self.act)
         dxin = ops.linear_dgrad(dh, p["up_w"], addend=dres)
         ops.linear_wgrad(dh, xin, g["up_w"], g.get("up_b"))
         return dxin

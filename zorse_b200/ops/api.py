@@ -16,9 +16,25 @@ import torch
 from . import ref
 
 _ACT_KINDS = {"gelu": 0, "gelu_new": 0, "gelu_tanh": 0, "relu": 1, "gelu_erf": 2}
+_FUSED_ACT_KINDS = {**_ACT_KINDS, "swiglu": 3}   # of the products with an activation in their epilogue
 
 
-class RefOps:
+class _MlpOps:
+    """The two products of an MLP that have its activation beside them, for ops that have no single kernel for a call.
+    `act`: "swiglu" (w holds the gate's rows, then the up projection's) or a name of `act_fwd`."""
+
+    def act_linear_fwd(self, x, w, bias, act, keep):
+        """act(x w^T + bias), and the pre-activations if `keep` (else None)."""
+        pre = self.linear_fwd(x, w, bias)
+        return self.swiglu_fwd(pre) if act == "swiglu" else self.act_fwd(pre, act), pre if keep else None
+
+    def act_linear_dgrad(self, dy, w, pre, act):
+        """(dy w) times the derivative of the activation at `pre`."""
+        da = self.linear_dgrad(dy, w)
+        return self.swiglu_bwd(pre, da) if act == "swiglu" else self.act_bwd(pre, da, act)
+
+
+class RefOps(_MlpOps):
     name = "ref"
 
     # ---- linear -----------------------------------------------------------------
@@ -144,7 +160,7 @@ def _decline(*args):
     return None
 
 
-class Sm100Ops:
+class Sm100Ops(_MlpOps):
     """Hand-written sm_100a kernels only. Requires bf16 CUDA tensors.
 
     The calls a step makes for every layer and microbatch go to the native module first (`sm100._fast`, 3 - 5 us of host
@@ -159,8 +175,10 @@ class Sm100Ops:
         fast = sm100._fast
         if fast is not None and sm100.GEMM_KERNEL == "2cta":
             self._linear_fwd, self._linear_dgrad, self._linear_wgrad = fast.linear_fwd, fast.linear_dgrad, fast.linear_wgrad
+            self._act_linear_fwd, self._act_linear_dgrad = fast.act_linear_fwd, fast.act_linear_dgrad
         else:
             self._linear_fwd = self._linear_dgrad = self._linear_wgrad = _decline
+            self._act_linear_fwd = self._act_linear_dgrad = _decline
         default = fast is not None
         self._norm_fwd = fast.norm_fwd if default and sm100.NORM_FWD_VERSION == 1 else _decline
         self._norm_bwd = fast.norm_bwd if default and sm100.NORM_BWD_VERSION == 2 else _decline
@@ -197,6 +215,14 @@ class Sm100Ops:
             self.k.gemm(dy, x, gw, a_mn=True, b_mn=True, accumulate=True)
             if gb is not None:
                 self.k.colsum_accumulate(dy, gb)
+
+    def act_linear_fwd(self, x, w, bias, act, keep):
+        r = self._act_linear_fwd(x, w, bias, _FUSED_ACT_KINDS[act], keep)
+        return super().act_linear_fwd(x, w, bias, act, keep) if r is None else r
+
+    def act_linear_dgrad(self, dy, w, pre, act):
+        r = self._act_linear_dgrad(dy, w, pre, _FUSED_ACT_KINDS[act])
+        return super().act_linear_dgrad(dy, w, pre, act) if r is None else r
 
     def norm_fwd(self, x, w, b, eps, ln):
         r = self._norm_fwd(x, w, b, eps, ln)
