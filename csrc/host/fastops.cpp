@@ -36,7 +36,7 @@ struct Entry {
   int (*norm_fwd)(const void*, const void*, const void*, void*, float*, int, int, float, int, cudaStream_t);
   int (*norm_bwd2)(const void*, const void*, const void*, const float*, const void*, void*, float*, float*, void*, void*, int, int,
                    int, int, int, cudaStream_t);
-  int (*norm_partial_rows)(int);
+  int (*norm_bwd2_rows)(int, int);
   int (*colsum)(const void*, int, int, int, float*, void*, int, int, cudaStream_t);
   int (*rope)(void*, const float*, int, int, int, int, int, int, cudaStream_t);
   int (*swiglu_fwd)(const void*, void*, long, int, cudaStream_t);
@@ -50,6 +50,7 @@ struct Entry {
   int (*flash_stats_floats)(int, int, int);
   int (*gemm2_act_fwd)(const void*, const void*, const void*, void*, void*, int, int, int, int, int, int, int*, cudaStream_t);
   int (*gemm2_act_bwd)(const void*, const void*, const void*, void*, int, int, int, int, int, int, int*, cudaStream_t);
+  int (*column_sums)(const long*, int, cudaStream_t);
   const char* (*last_error)();
 };
 Entry lib;
@@ -154,6 +155,17 @@ int gemm(const Tensor* a, const Tensor* b, const Tensor& out, bool a_mn, bool b_
   }) ? 1 : -1;
 }
 
+// Whether column_sums takes this bf16 matrix.
+bool summable(const Tensor& t) {
+  return t.size(1) % 8 == 0 && t.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+}
+bool later(PyObject* sums, PyObject* entry) {   // (takes over `entry`)
+  if (entry == nullptr) return false;
+  const int rc = PyList_Append(sums, entry);
+  Py_DECREF(entry);
+  return rc == 0;
+}
+
 PyObject* forward_like(PyObject* const* args, bool b_mn, PyObject* bias_o, PyObject* add_o) {
   const Tensor *x = tensor_of(args[0]), *w = tensor_of(args[1]), *bias, *add;
   if (!optional_tensor(bias_o, bias) || !optional_tensor(add_o, add) || !matrix(x, BF16) || !matrix(w, BF16)) Py_RETURN_NONE;
@@ -182,10 +194,11 @@ PyObject* linear_dgrad(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   return forward_like(args, true, Py_None, args[2]);
   END_HANDLE_TH_ERRORS
 }
-// linear_wgrad(dy, x, gw, gb | None): gw += dy^T x, gb += column sums of dy.  True when done.
+// linear_wgrad(dy, x, gw, gb | None, sums | None): gw += dy^T x, gb += column sums of dy.  With a list `sums` the second is
+// left to column_sums, (dy, gb) appended.  True when done.
 PyObject* linear_wgrad(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  ZB_ARGS(4)
+  ZB_ARGS(5)
   const Tensor *dy = tensor_of(args[0]), *x = tensor_of(args[1]), *gw = tensor_of(args[2]), *gb;
   if (!optional_tensor(args[3], gb) || !matrix(dy, BF16) || !matrix(x, BF16)) Py_RETURN_NONE;
   if (!(matrix(gw, F32) || matrix(gw, BF16)) || !on(x, *dy) || !on(gw, *dy) || !on(gb, *dy)) Py_RETURN_NONE;
@@ -195,6 +208,7 @@ PyObject* linear_wgrad(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int done = gemm(dy, x, *gw, true, true, nullptr, nullptr, true, status);
   if (done < 0) return nullptr;
   if (done == 0) Py_RETURN_NONE;
+  if (gb != nullptr && PyList_Check(args[4]) && summable(*dy)) return later(args[4], PyTuple_Pack(2, args[0], args[3])) ? Py_NewRef(Py_True) : nullptr;
   if (gb != nullptr) {
     const int64_t T = dy->size(0), N = dy->size(1);
     const Tensor part = empty({T < 64 ? T : 64, N}, *dy, F32);
@@ -294,10 +308,11 @@ PyObject* norm_fwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// norm_bwd(dy, x, w, stats, dres | None, dw, db | None, layernorm) -> dx (+ dres); dw, db are added to
+// norm_bwd(dy, x, w, stats, dres | None, dw, db | None, layernorm, sums | None) -> dx (+ dres); dw, db are added to, or, with
+// a list `sums`, left to column_sums as (partial sums, dw, db | None)
 PyObject* norm_bwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  ZB_ARGS(8)
+  ZB_ARGS(9)
   const Tensor *dy = tensor_of(args[0]), *x = tensor_of(args[1]), *w = tensor_of(args[2]), *stats = tensor_of(args[3]);
   const Tensor *dres, *dw = tensor_of(args[5]), *db;
   if (!optional_tensor(args[4], dres) || !optional_tensor(args[6], db) || !dense(dy, BF16) || !dense(x, BF16) ||
@@ -312,18 +327,75 @@ PyObject* norm_bwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (!on(dy, *x) || !on(w, *x) || !on(stats, *x) || !on(dres, *x) || !on(dw, *x) || !on(db, *x)) Py_RETURN_NONE;
   if (status_of(*x) == nullptr) Py_RETURN_NONE;
   const bool bias = ln && db != nullptr;
-  const int64_t P = lib.norm_partial_rows(int(T));
+  const bool defer = PyList_Check(args[8]);
+  const int64_t P = lib.norm_bwd2_rows(int(T), int(H));
   Tensor dx = empty({T, H}, *x, BF16);
-  const Tensor part = empty({bias ? 2 : 1, P, H}, *x, F32);
+  Tensor part = empty({bias ? 2 : 1, P, H}, *x, F32);
   float* part_dw = static_cast<float*>(part.data_ptr());
   float* part_db = bias ? part_dw + P * H : nullptr;
   const cudaStream_t s = stream();
   if (!launch("norm_bwd", 1, [&] {
         return lib.norm_bwd2(ptr(dy), ptr(x), ptr(w), static_cast<const float*>(ptr(stats)), ptr(dres), dx.data_ptr(), part_dw,
-                             part_db, ptr(dw), ptr(db), int(T), int(H), ln, dw->scalar_type() == F32, 1, s);
+                             part_db, defer ? nullptr : ptr(dw), defer ? nullptr : ptr(db), int(T), int(H), ln,
+                             dw->scalar_type() == F32, 1, s);
       }))
     return nullptr;
+  if (defer) {
+    PyObject* sums = THPVariable_Wrap(std::move(part));
+    if (sums == nullptr) return nullptr;
+    PyObject* entry = PyTuple_Pack(3, sums, args[5], bias ? args[6] : Py_None);
+    Py_DECREF(sums);
+    if (!later(args[8], entry)) return nullptr;
+  }
   return THPVariable_Wrap(std::move(dx));
+  END_HANDLE_TH_ERRORS
+}
+
+// column_sums(sums): what linear_wgrad and norm_bwd have left in the list, which is emptied.
+PyObject* column_sums(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  ZB_ARGS(1)
+  if (!PyList_Check(args[0]) || !ready) {
+    PyErr_SetString(PyExc_TypeError, "column_sums takes the list that linear_wgrad and norm_bwd have filled");
+    return nullptr;
+  }
+  constexpr int MAX = 8;   // sums per launch
+  long desc[MAX][7];
+  int n = 0;
+  const cudaStream_t s = stream();
+  auto run = [&] {
+    const bool ok = n == 0 || launch("column_sums", 1, [&] { return lib.column_sums(desc[0], n, s); });
+    n = 0;
+    return ok;
+  };
+  auto add = [&](const Tensor& src, int64_t offset, int64_t rows, int64_t cols, int64_t ld, const Tensor& out) {
+    if (n == MAX && !run()) return false;
+    const bool f32 = src.scalar_type() == F32;
+    const long d[7] = {reinterpret_cast<long>(src.data_ptr()) + long(offset * (f32 ? 4 : 2)), reinterpret_cast<long>(out.data_ptr()),
+                       long(rows), long(cols), long(ld), f32, out.scalar_type() == F32};
+    memcpy(desc[n++], d, sizeof(d));
+    return true;
+  };
+  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(args[0]); ++i) {
+    PyObject* e = PyList_GET_ITEM(args[0], i);
+    const Py_ssize_t k = PyTuple_Check(e) ? PyTuple_GET_SIZE(e) : 0;
+    const Tensor *src = k > 0 ? tensor_of(PyTuple_GET_ITEM(e, 0)) : nullptr, *out = k > 1 ? tensor_of(PyTuple_GET_ITEM(e, 1)) : nullptr;
+    const Tensor* second = nullptr;
+    if (src == nullptr || out == nullptr || (k == 3 && !optional_tensor(PyTuple_GET_ITEM(e, 2), second)) ||
+        (k == 3) != (src->dim() == 3)) {
+      PyErr_SetString(PyExc_TypeError, "column_sums: an entry that linear_wgrad or norm_bwd did not make");
+      return nullptr;
+    }
+    if (k == 2) {
+      if (!add(*src, 0, src->size(0), src->size(1), src->stride(0), *out)) return nullptr;
+    } else {
+      const int64_t P = src->size(1), H = src->size(2);
+      if (!add(*src, 0, P, H, H, *out) || (second != nullptr && !add(*src, P * H, P, H, H, *second))) return nullptr;
+    }
+  }
+  if (!run()) return nullptr;
+  if (PyList_SetSlice(args[0], 0, PyList_GET_SIZE(args[0]), nullptr) != 0) return nullptr;
+  Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }
 
@@ -509,7 +581,7 @@ PyObject* launch_count(PyObject*, PyObject* const*, Py_ssize_t) { return PyLong_
 
 #define ZB_FN(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {ZB_FN(init), ZB_FN(set_status), ZB_FN(launch_count), ZB_FN(linear_fwd), ZB_FN(linear_dgrad),
-                         ZB_FN(linear_wgrad), ZB_FN(act_linear_fwd), ZB_FN(act_linear_dgrad), ZB_FN(norm_fwd), ZB_FN(norm_bwd), ZB_FN(rope), ZB_FN(swiglu_fwd),
+                         ZB_FN(linear_wgrad), ZB_FN(act_linear_fwd), ZB_FN(act_linear_dgrad), ZB_FN(norm_fwd), ZB_FN(norm_bwd), ZB_FN(column_sums), ZB_FN(rope), ZB_FN(swiglu_fwd),
                          ZB_FN(swiglu_bwd), ZB_FN(act_fwd), ZB_FN(act_bwd), ZB_FN(attn_fwd), ZB_FN(attn_bwd),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "zorse_fastops", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -246,6 +246,12 @@ int colsum_finish(const float* part0, int P, int H, void* out0, const float* par
 
 }  // namespace zb
 
+// Rows of partial sums that zb_norm_bwd2 writes (of the zb_norm_partial_rows(T) it has room for).
+extern "C" int zb_norm_bwd2_rows(int T, int H) {
+  const int rw = zb::norm_rows_per_cta(H), groups = (T + rw - 1) / rw, cap = zb_norm_partial_rows(T);
+  return groups < cap ? groups : cap;
+}
+
 extern "C" int zb_norm_bwd2(const void* dy, const void* x, const void* w, const float* stats, const void* dres,
                             void* dx, float* part_dw, float* part_db, void* dw, void* db, int T, int H, int ln,
                             int grad_f32, int accumulate, cudaStream_t stream) {
@@ -258,8 +264,7 @@ extern "C" int zb_norm_bwd2(const void* dy, const void* x, const void* w, const 
   auto DR = static_cast<const __nv_bfloat16*>(dres);
   auto DX = static_cast<__nv_bfloat16*>(dx);
   const int rw = norm_rows_per_cta(H), nv = (H / 8 + NORM_THREADS / rw - 1) / (NORM_THREADS / rw);
-  const int groups = (T + rw - 1) / rw, cap = zb_norm_partial_rows(T);   // two CTAs per SM, a row of partial sums each
-  const int P = groups < cap ? groups : cap;
+  const int P = zb_norm_bwd2_rows(T, H);   // two CTAs per SM, a row of partial sums each
   int rc = 0;
 #define ZB_NORM_BWD(RW_, NV_)                                                                                        \
   rc = ln ? launch_norm_bwd2<true, RW_, NV_>(DY, X, W, stats, DR, DX, part_dw, part_db, T, H, P, stream)              \

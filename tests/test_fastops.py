@@ -20,8 +20,8 @@ def test_declines_what_is_not_on_a_gpu():
     m = _module()
     x, w = torch.zeros(4, 8, dtype=torch.bfloat16), torch.zeros(16, 8, dtype=torch.bfloat16)
     g, v = torch.zeros(16, 8), torch.zeros(8)
-    calls = [(m.linear_fwd, (x, w, None, None)), (m.linear_dgrad, (x, x, None)), (m.linear_wgrad, (x, x, g, None)),
-             (m.norm_fwd, (x, v, None, 1e-5, False)), (m.norm_bwd, (x, x, v, g, None, v, None, False)),
+    calls = [(m.linear_fwd, (x, w, None, None)), (m.linear_dgrad, (x, x, None)), (m.linear_wgrad, (x, x, g, None, None)),
+             (m.norm_fwd, (x, v, None, 1e-5, False)), (m.norm_bwd, (x, x, v, g, None, v, None, False, None)),
              (m.rope, (x, g, 4, 1, 8, False)), (m.swiglu_fwd, (x,)), (m.swiglu_bwd, (x, x)), (m.act_fwd, (x, 0)),
              (m.act_bwd, (x, x, 0)), (m.attn_fwd, (x, 1, 4, 1, 1, 64, True, 0, 1)),
              (m.attn_bwd, (x, x, x, g, 1, 4, 1, 1, 64, True, 0))]
@@ -92,7 +92,7 @@ def test_linear(ops, T, K, N, wide):
         for bias in (False, True):
             g = [torch.ones(N, K, dtype=dt, device="cuda") for _ in range(2)]
             gb = [torch.ones(N, dtype=dt, device="cuda") for _ in range(2)]
-            assert k._fast.linear_wgrad(dy, x, g[0], gb[0] if bias else None) is True
+            assert k._fast.linear_wgrad(dy, x, g[0], gb[0] if bias else None, None) is True
             k.gemm(dy, x, g[1], a_mn=True, b_mn=True, accumulate=True)
             if bias:
                 k.colsum_accumulate(dy, gb[1])
@@ -111,11 +111,49 @@ def test_norms(ops, T, H, ln, dt):
     assert torch.equal(y, y2) and torch.equal(st, st2)
     for dres in (None, _rand(T, H, seed=5)):
         g = [torch.ones(4, H, dtype=dt, device="cuda") for _ in range(1)][0]
-        assert k._fast.norm_bwd(dy, x, w, st, dres, g[0], g[1] if ln else None, ln) is not None
+        assert k._fast.norm_bwd(dy, x, w, st, dres, g[0], g[1] if ln else None, ln, None) is not None
         dx2 = k.norm_bwd(dy, x, w, st, dres, g[2], g[3] if ln else None, ln)
         assert torch.equal(g[0], g[2]) and torch.equal(g[1], g[3])
         assert torch.equal(ops.norm_bwd(dy, x, w, st, dres, g[0], g[1] if ln else None, ln), dx2)
     k.check_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,widths", [(1, [8, 512]), (7, [72, 64, 520]), (300, [768, 3072, 768, 2304]), (2503, [1032, 8, 200]),
+                                      (4616, [768] * 6)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_column_sums_of_a_layer_in_one_launch(ops, T, widths, dt):
+    """Bias gradients of matrices of several widths (one a slice of wider rows) and the gradients of two norms: fewer and more
+    than fit one launch, against 64 bits, and the same bits each time.  Bounds: fp32 sums of T terms in chains of at most T / 256
+    + 40 additions, of numbers whose absolute sum is `mass`; bf16 gradients round once more."""
+    H = 512
+    x, dyn, w = _rand(T, H, seed=1), _rand(T, H, seed=2), _rand(H, seed=3)
+    _, st = k.norm_fwd(x, w, w, 1e-5, True)
+    dys = [_rand(T, n + 8 * (i == 1), seed=10 + i)[:, :n] for i, n in enumerate(widths)]
+
+    def run():
+        sums, outs = ops.new_sums(), [torch.ones(n, dtype=dt, device="cuda") for n in widths]
+        gw = [torch.zeros(n, 16, dtype=dt, device="cuda") for n in widths]
+        norm = [torch.ones(H, dtype=dt, device="cuda") for _ in range(4)]
+        before = k.launch_count()
+        for dy, g, o in zip(dys, gw, outs):
+            ops.linear_wgrad(dy, x[:, :16].contiguous(), g, o, sums=sums)
+        for i in (0, 2):
+            ops.norm_bwd(dyn, x, w, st, None, norm[i], norm[i + 1], True, sums)
+        assert len(sums) == len(widths) + 2 and all(bool((o == 1).all()) for o in outs + norm)
+        ops.finish_sums(sums)
+        assert not sums and k.launch_count() - before == len(widths) + 2 + -(-(len(widths) + 4) // 8)
+        return outs + norm
+
+    got, again = run(), run()
+    k.check_status()
+    xh = (x.double() - st[:, :1].double()) * st[:, 1:].double()
+    srcs = [d.double() for d in dys] + [dyn.double() * xh, dyn.double()] * 2
+    for o, o2, src in zip(got, again, srcs):
+        assert torch.equal(o, o2)
+        mass = 1 + src.abs().sum(0)
+        tol = mass * (T / 256 + 40) * 2.0 ** -24 + (0 if dt == torch.float32 else 2.0 ** -8) * (1 + src.sum(0)).abs()
+        assert bool(((o.double() - 1 - src.sum(0)).abs() <= tol + 1e-6).all())
 
 
 @pytest.mark.gpu

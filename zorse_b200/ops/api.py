@@ -34,7 +34,19 @@ class _MlpOps:
         return self.swiglu_bwd(pre, da) if act == "swiglu" else self.act_bwd(pre, da, act)
 
 
-class RefOps(_MlpOps):
+class _SumOps:
+    """Column sums (bias gradients, norm gradients) of a layer's backward pass may be collected and done in one launch:
+    `sums = ops.new_sums()`, passed to `linear_wgrad` and `norm_bwd`, and `ops.finish_sums(sums)` at the end, before anything
+    else reads the gradients.  None, or ops that ignore it: each sum is done where it is asked for."""
+
+    def new_sums(self):
+        return None
+
+    def finish_sums(self, sums):
+        pass
+
+
+class RefOps(_MlpOps, _SumOps):
     name = "ref"
 
     # ---- linear -----------------------------------------------------------------
@@ -50,7 +62,7 @@ class RefOps(_MlpOps):
         dx = dy @ w
         return dx if addend is None else dx + addend
 
-    def linear_wgrad(self, dy, x, gw, gb=None):
+    def linear_wgrad(self, dy, x, gw, gb=None, sums=None):
         gw.add_((dy.float().t() @ x.float()).to(gw.dtype))
         if gb is not None:
             gb.add_(dy.float().sum(0).to(gb.dtype))
@@ -66,7 +78,7 @@ class RefOps(_MlpOps):
             y = y + b.float()
         return y.to(x.dtype), torch.stack([mean, rstd], dim=1)
 
-    def norm_bwd(self, dy, x, w, stats, dres, gw, gb, ln):
+    def norm_bwd(self, dy, x, w, stats, dres, gw, gb, ln, sums=None):
         xf, dyf = x.float(), dy.float()
         mean, rstd = stats[:, 0:1], stats[:, 1:2]
         xh = (xf - mean) * rstd
@@ -160,7 +172,7 @@ def _decline(*args):
     return None
 
 
-class Sm100Ops(_MlpOps):
+class Sm100Ops(_MlpOps, _SumOps):
     """Hand-written sm_100a kernels only. Requires bf16 CUDA tensors.
 
     The calls a step makes for every layer and microbatch go to the native module first (`sm100._fast`, 3 - 5 us of host
@@ -180,6 +192,7 @@ class Sm100Ops(_MlpOps):
             self._linear_fwd = self._linear_dgrad = self._linear_wgrad = _decline
             self._act_linear_fwd = self._act_linear_dgrad = _decline
         default = fast is not None
+        self._column_sums = fast.column_sums if default else None
         self._norm_fwd = fast.norm_fwd if default and sm100.NORM_FWD_VERSION == 1 else _decline
         self._norm_bwd = fast.norm_bwd if default and sm100.NORM_BWD_VERSION == 2 else _decline
         self._attn_fwd = fast.attn_fwd if default and sm100.ATTN_FWD_VERSION == 0 else _decline
@@ -209,9 +222,9 @@ class Sm100Ops(_MlpOps):
             self.k.gemm(dy, w, dx, b_mn=True, addend=addend)
         return dx
 
-    def linear_wgrad(self, dy, x, gw, gb=None):
+    def linear_wgrad(self, dy, x, gw, gb=None, sums=None):
         # gw[N,K] += dy^T[N,T] @ x[T,K]: both operands contiguous along the non-reduced dim
-        if self._linear_wgrad(dy, x, gw, gb) is None:
+        if self._linear_wgrad(dy, x, gw, gb, sums) is None:
             self.k.gemm(dy, x, gw, a_mn=True, b_mn=True, accumulate=True)
             if gb is not None:
                 self.k.colsum_accumulate(dy, gb)
@@ -228,8 +241,15 @@ class Sm100Ops(_MlpOps):
         r = self._norm_fwd(x, w, b, eps, ln)
         return self.k.norm_fwd(x, w, b, eps, ln) if r is None else r
 
-    def norm_bwd(self, dy, x, w, stats, dres, gw, gb, ln):
-        dx = self._norm_bwd(dy, x, w, stats, dres, gw, gb, ln)
+    def new_sums(self):
+        return [] if self._column_sums is not None else None
+
+    def finish_sums(self, sums):
+        if sums:
+            self._column_sums(sums)
+
+    def norm_bwd(self, dy, x, w, stats, dres, gw, gb, ln, sums=None):
+        dx = self._norm_bwd(dy, x, w, stats, dres, gw, gb, ln, sums)
         return self.k.norm_bwd(dy, x, w, stats, dres, gw, gb, ln) if dx is None else dx
 
     def rope_table(self, S, d, theta, device):
@@ -241,11 +261,12 @@ class Sm100Ops(_MlpOps):
         return qkv
 
     def attn_fwd(self, qkv, B, S, Hq, Hkv, D, causal=True, window=0):
+        # the two-tile kernel at every size: where it leaves most of the GPU idle its steps are still shorter (d = 64: 2 x 8
+        # heads of 128 tokens 10.5 -> 5.0 us, of 509 14.7 -> 11.4, 12 heads of 2048 44.8 -> 31.2)
         k = self.k
-        if k._auto_fwd_version(B, S, Hq, D) == 4:
-            r = self._attn_fwd(qkv, B, S, Hq, Hkv, D, causal, window, k.ATTN_FWD4_FLAGS)
-            if r is not None:
-                return r
+        r = self._attn_fwd(qkv, B, S, Hq, Hkv, D, causal, window, k.ATTN_FWD4_FLAGS)
+        if r is not None:
+            return r
         return k.flash_fwd(qkv, B, S, Hq, Hkv, D, causal, window)
 
     def attn_bwd(self, do, qkv, o, lse, B, S, Hq, Hkv, D, causal=True, window=0):

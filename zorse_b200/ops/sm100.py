@@ -87,9 +87,9 @@ def lib():
 # answers None to arguments it was not written for; the wrappers below take those.  None until the library is loaded.
 _fast = None
 _FAST_ENTRIES = ("zb_gemm_bf16", "zb_gemm2_bf16", "zb_gemm2_split_bf16", "zb_gemm2_workspace", "zb_norm_fwd", "zb_norm_bwd2",
-                 "zb_norm_partial_rows", "zb_colsum", "zb_rope", "zb_swiglu_fwd", "zb_swiglu_bwd", "zb_act_fwd", "zb_act_bwd",
+                 "zb_norm_bwd2_rows", "zb_colsum", "zb_rope", "zb_swiglu_fwd", "zb_swiglu_bwd", "zb_act_fwd", "zb_act_bwd",
                  "zb_flash_fwd4", "zb_flash_bwd3", "zb_flash_bwd2_stats_floats", "zb_gemm2_act_fwd",
-                 "zb_gemm2_act_bwd", "zb_last_error")   # the order of its `Entry`
+                 "zb_gemm2_act_bwd", "zb_column_sums", "zb_last_error")   # the order of its `Entry`
 
 
 def _load_fast() -> None:
@@ -386,9 +386,7 @@ ATTN_FWD4_FLAGS = int(os.environ.get("ZORSE_ATTN_FWD4_FLAGS", "1"))
 
 
 def _auto_fwd_version(B: int, S: int, Hq: int, D: int) -> int:
-    # d = 128: one CTA for two query tiles beats two CTAs long before that fills the GPU (32 heads of 1000 tokens, 128 CTAs:
-    # 38 -> 23 us; 32 heads of 512, 64 CTAs: 16.2 -> 15.2).  d = 64 stays at one CTA per SM: the two versions differ in the
-    # last bit, which steps of the narrow twelve-layer models amplify, for 10 us of 44 (12 heads of 2048 tokens).
+    # the two-tile kernel where it fills the GPU (d = 64) or nearly half of it (d = 128)
     return 4 if B * Hq * ((S + 255) // 256) >= (64 if D == 128 else 148) else 1
 
 

@@ -102,6 +102,7 @@ class DeferredWgrad:
 
     def linear_wgrad(self, *a, **k):
         if self.active:
+            k.pop("sums", None)      # the layer finishes its sums before the queue is flushed
             self._queue.append((a, k))
         else:
             self._ops.linear_wgrad(*a, **k)
@@ -270,13 +271,12 @@ class PipelineStage:
         """Runs layer li on microbatch mbl. With recompute only the layer input is stashed, and the head does not run at
         all: nothing but the loss comes out of it, and the backward pass forms its logits and the loss again."""
         layer = self.layers[li]
-        if recompute and layer.kind == "head":
-            self.stash.put((li, mbl), x)
-            return None
         c = self.ctx(mbl, targets if layer.kind == "head" else None)
         with phase("fwd." + layer.kind):
             if recompute:
                 self.stash.put((li, mbl), x)
+                if layer.kind == "head":
+                    return None
                 y = layer.forward(x, c, self.ops, None)
             else:
                 sv: dict = {}
