@@ -81,6 +81,7 @@ template <int D, bool TRACE, bool DQ, int CL>
 __global__ void __launch_bounds__(32 * BWD2_WARPS, 1)
 flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                   const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
+                  const __grid_constant__ CUtensorMap tmap_dk, const __grid_constant__ CUtensorMap tmap_dv,
                   const AttnBwdParams p, const float* stats, int s_pad,
                   unsigned long long* trace, int trace_ctas) {
   using Cfg = AttnBwd2Cfg<D>;
@@ -98,8 +99,9 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   uint8_t* sDO = sQ + QS * Cfg::TILE_BYTES;           // QS tiles
   uint8_t* sDS = sDO + QS * Cfg::TILE_BYTES;          // dS^T: [128 keys][128 queries], two 64-query blocks
   uint64_t* bars = reinterpret_cast<uint64_t*>(sDS + Cfg::DS_BYTES);
-  uint64_t* kv_full = bars;             // 1
-  uint64_t* q_full = bars + 1;          // QS
+  uint64_t* k_full = bars;              // 1
+  uint64_t* v_full = bars + 1;          // 1
+  uint64_t* q_full = bars + 2;          // QS
   uint64_t* q_empty = q_full + QS;      // QS
   uint64_t* do_full = q_empty + QS;     // QS
   uint64_t* do_empty = do_full + QS;    // QS
@@ -142,7 +144,8 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    mbar_init(kv_full, 1);
+    mbar_init(k_full, 1);
+    mbar_init(v_full, 1);
     for (int i = 0; i < QS; ++i) {
       mbar_init(&q_full[i], 1);
       mbar_init(&q_empty[i], 1);
@@ -176,19 +179,19 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       tma_prefetch_desc(&tmap_k);
       tma_prefetch_desc(&tmap_v);
       tma_prefetch_desc(&tmap_do);
-      if (n_iters > 0) {   // nobody waits for K / V otherwise, and a copy must not outlive the CTA
-        mbar_expect_tx(kv_full, 2 * Cfg::TILE_BYTES);
+      // K and the first Q are all that the first scores need: they go ahead of V and dO (nobody waits for them without a
+      // step, and a copy must not outlive the CTA)
+      auto load_kv = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar) {
+        mbar_expect_tx(bar, Cfg::TILE_BYTES);
 #pragma unroll
-        for (int b = 0; b < DB; ++b) {
-          tma_load_4d(sK + b * BLK, &tmap_k, kv_full, b * 64, kv_head, kv0, batch);
-          tma_load_4d(sV + b * BLK, &tmap_v, kv_full, b * 64, kv_head, kv0, batch);
-        }
-      }
+        for (int b = 0; b < DB; ++b) tma_load_4d(dst + b * BLK, tm, bar, b * 64, kv_head, kv0, batch);
+      };
+      if (n_iters > 0) load_kv(sK, &tmap_k, k_full);
+      int head = head0, qt = i_lo;
       for (int it = 0; it < n_iters; ++it) {
         const int st = it % QS;
         const uint32_t ph = uint32_t(it / QS) & 1;
-        const int head = head0 + it / per_head;
-        const int q0 = (i_lo + it % per_head) * BM;
+        const int q0 = qt * BM;
         if (!zb_in_bounds(q0 >= 0 && q0 < p.S && head < p.Hq && kv0 < p.S, p.status, 8)) break;
         // Q and dO have their own barriers: dO_i is free once dV_i is done, Q_i only after dK_i, more than half a step
         // later, and the first S^T needs Q alone
@@ -217,8 +220,15 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
             tma_load_4d(sDO + st * Cfg::TILE_BYTES + b * BLK, &tmap_do, &do_full[st], b * 64, head, q0, batch);
           return true;
         };
-        if (it < QS ? !(load_q() && load_do()) : !(load_do() && load_q())) break;
+        if (it == 0) {
+          if (!load_q()) break;
+          load_kv(sV, &tmap_v, v_full);
+          if (!load_do()) break;
+        } else if (it < QS ? !(load_q() && load_do()) : !(load_do() && load_q())) {
+          break;
+        }
         tr(TB_TMA_ISSUED);
+        if (++qt == i_hi) { qt = i_lo; ++head; }
       }
     }
   } else if (warp == 9) {
@@ -237,7 +247,7 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       const uint32_t k_addr = smem_u32(sK), v_addr = smem_u32(sV), ds_addr = smem_u32(sDS);
       const uint32_t r_dp = tmem_base + Cfg::DP_COL;
       auto r_s = [&](int it) { return tmem_base + (NSB == 2 && (it & 1) ? uint32_t(Cfg::S1_COL) : 0u); };
-      bool ok = mbar_wait_warp(kv_full, 0, wctx, ST_TIMEOUT_FULL);
+      bool ok = mbar_wait_warp(k_full, 0, wctx, ST_TIMEOUT_FULL);
       auto issue_a = [&](int it) {  // S^T = K Q^T
         if (elected) {
           const uint32_t q_addr = smem_u32(sQ + (it % QS) * Cfg::TILE_BYTES), d = r_s(it);
@@ -265,8 +275,9 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       if (ok) {
         tc_fence_after();
         issue_a(0);
-        ok = mbar_wait_warp(&do_full[0], 0, wctx, ST_TIMEOUT_FULL);
+        ok = mbar_wait_warp(v_full, 0, wctx, ST_TIMEOUT_FULL);
       }
+      if (ok) ok = mbar_wait_warp(&do_full[0], 0, wctx, ST_TIMEOUT_FULL);
       if (ok) {
         tc_fence_after();
         issue_b(smem_u32(sDO));
@@ -387,9 +398,10 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     const bool key_ok = key < p.S;
     uint8_t* ds_row = sDS + half * BLK + t * 128;  // this thread's 128-byte row of its 64-query block
     bool ok = true;
+    int head = head0, qt = i_lo - 1;   // (counted along: two divisions per step otherwise)
     for (int it = 0; it < n_iters; ++it) {
-      const int head = head0 + it / per_head;
-      const int q0 = (i_lo + it % per_head) * BM;
+      if (++qt == i_hi) { qt = i_lo; ++head; }
+      const int q0 = qt * BM;
       const int qc0 = q0 + half * 64;            // first query column of this thread
       // statistics of the tile's queries: global rows indexed by the absolute query (one-kernel form), or the
       // copy the producer placed in shared memory with the stage
@@ -611,7 +623,6 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     }
     // ------------------------------ dK / dV write-out ------------------------------
     // the last dq_full arrival also covers every dK / dV MMA issued before it
-    const int width = (p.Hq + 2 * p.Hkv) * D;
     ok = __all_sync(0xffffffffu, ok);
     const uint32_t sums = smem_u32(sQ) + uint32_t(t) * 4;   // CL > 1: [which][column][key] fp32 over the Q / dO stages
     if constexpr (CL > 1) {
@@ -638,17 +649,19 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
       for (int q = 0; q < CL; ++q) ok = ok && ld_cluster_u32(abort_addr, q) == 0;
     }
+    // The tiles leave through the places of K and V, whose last readers are done, and TMA, which drops the rows behind the
+    // sequence.  Stores straight from the registers went to 32 rows per instruction, half a sector each: 1.9 us per CTA of
+    // 12.7 (d = 64, 577 tokens), 4.1 of 36 (d = 128, 4096 tokens).
 #pragma unroll 1
     for (int which = 0; which < 2; ++which) {
       if (CL == 2 && which != cl_rank) continue;           // rank 0 writes dK, rank 1 dV
-      if (CL == 4 && which != (cl_rank >> 1)) continue;    // ranks 0 and 1: alternate column blocks of dK, 2 and 3: of dV
+      if (CL == 4 && which != (cl_rank >> 1)) continue;    // ranks 0 and 1: alternate row halves of dK, 2 and 3: of dV
+      if (CL == 4 && ((warp & 3) >> 1) != (cl_rank & 1)) continue;
       const uint32_t col0 = which == 0 ? Cfg::DK_COL : Cfg::DV_COL;
       const float mul = !DQ && which == 0 ? p.scale : 1.f;   // the two-kernel form leaves dS unscaled
-      __nv_bfloat16* dst = p.dqkv + (size_t(batch) * p.S + key) * width +
-                           size_t(which == 0 ? (p.Hq + kv_head) : (p.Hq + p.Hkv + kv_head)) * D;
+      const uint32_t row = smem_u32(which == 0 ? sK : sV) + uint32_t(t) * 128;
 #pragma unroll 1
       for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
-        if (CL == 4 && (c & 1) != (cl_rank & 1)) continue;
         uint32_t r[32];
         if constexpr (CL > 1) {
 #pragma unroll
@@ -666,20 +679,42 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
           for (int k = 0; k < 32; ++k) r[k] = 0u;
         }
-        if (ok && key_ok) {
 #pragma unroll
-          for (int k = 0; k < 32; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * mul);
+        for (int k = 0; k < 32; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * mul);
+        // columns [32 c, 32 c + 32) of the tile: 16-byte pieces 4 (c & 1) ... of block c / 2
+        const uint32_t at = row + uint32_t(c >> 1) * BLK;
 #pragma unroll
-          for (int v4 = 0; v4 < 4; ++v4) {
-            uint4 u;
-            u.x = pack_bf16x2(__uint_as_float(r[v4 * 8 + 0]), __uint_as_float(r[v4 * 8 + 1]));
-            u.y = pack_bf16x2(__uint_as_float(r[v4 * 8 + 2]), __uint_as_float(r[v4 * 8 + 3]));
-            u.z = pack_bf16x2(__uint_as_float(r[v4 * 8 + 4]), __uint_as_float(r[v4 * 8 + 5]));
-            u.w = pack_bf16x2(__uint_as_float(r[v4 * 8 + 6]), __uint_as_float(r[v4 * 8 + 7]));
-            *reinterpret_cast<uint4*>(dst + c * 32 + v4 * 8) = u;
+        for (int v4 = 0; v4 < 4; ++v4)
+          st_shared_v4(at + ((uint32_t((c & 1) * 4 + v4) ^ uint32_t(t & 7)) << 4),
+                       pack_bf16x2(__uint_as_float(r[v4 * 8 + 0]), __uint_as_float(r[v4 * 8 + 1])),
+                       pack_bf16x2(__uint_as_float(r[v4 * 8 + 2]), __uint_as_float(r[v4 * 8 + 3])),
+                       pack_bf16x2(__uint_as_float(r[v4 * 8 + 4]), __uint_as_float(r[v4 * 8 + 5])),
+                       pack_bf16x2(__uint_as_float(r[v4 * 8 + 6]), __uint_as_float(r[v4 * 8 + 7])));
+      }
+    }
+    fence_proxy_async_smem();
+    asm volatile("bar.sync 1, 256;" ::: "memory");   // the compute warps
+    // (a warp that gave up has raised the abort word; with CL > 1 all ranks have seen each other's)
+    if (warp == 0 && ok && *abort_flag == 0) {
+      if (lane == 0) {
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {
+          if ((CL == 2 && which != cl_rank) || (CL == 4 && which != (cl_rank >> 1))) continue;
+          const uint8_t* tile = which == 0 ? sK : sV;
+          // boxes of 64 rows: CL = 4 stores one of the two
+#pragma unroll
+          for (int hr = 0; hr < 2; ++hr) {
+            if (CL == 4 && hr != (cl_rank & 1)) continue;
+            if (kv0 + hr * 64 >= p.S) continue;
+#pragma unroll
+            for (int b = 0; b < DB; ++b)
+              tma_store_4d(which == 0 ? &tmap_dk : &tmap_dv, tile + b * BLK + hr * 64 * 128, b * 64, kv_head, kv0 + hr * 64, batch);
           }
         }
+        bulk_commit();
+        bulk_wait_read<0>();
       }
+      __syncwarp();
     }
   }
 
@@ -765,10 +800,11 @@ static int launch_stats(const __nv_bfloat16* o, const __nv_bfloat16* d_o, const 
   return 0;
 }
 
-static int make_head_tmap_bwd2(CUtensorMap* out, const __nv_bfloat16* base, int B, int S, int heads, int D, int width) {
+static int make_head_tmap_bwd2(CUtensorMap* out, const __nv_bfloat16* base, int B, int S, int heads, int D, int width,
+                               uint32_t rows = 128) {
   uint64_t dims[4] = {uint64_t(D), uint64_t(heads), uint64_t(S), uint64_t(B)};
   uint64_t strides[3] = {uint64_t(D) * 2, uint64_t(width) * 2, uint64_t(width) * 2 * uint64_t(S)};
-  uint32_t box[4] = {64, 1, 128, 1};
+  uint32_t box[4] = {64, 1, rows, 1};
   return make_tmap_nd_bf16(out, base, 4, dims, strides, box);
 }
 
@@ -777,8 +813,10 @@ static int launch_bwd2(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const
                        int s_pad, unsigned long long* trace, int trace_ctas, cudaStream_t stream) {
   using Cfg = AttnBwd2Cfg<D>;
   const int width = (p.Hq + 2 * p.Hkv) * D;
-  CUtensorMap tq, tk, tv, tdo;
+  CUtensorMap tq, tk, tv, tdo, tdk, tdv;
   int rc;
+  if ((rc = make_head_tmap_bwd2(&tdk, p.dqkv + size_t(p.Hq) * D, p.B, p.S, p.Hkv, D, width, 64))) return rc;
+  if ((rc = make_head_tmap_bwd2(&tdv, p.dqkv + size_t(p.Hq + p.Hkv) * D, p.B, p.S, p.Hkv, D, width, 64))) return rc;
   if ((rc = make_head_tmap_bwd2(&tq, qkv, p.B, p.S, p.Hq, D, width))) return rc;
   if ((rc = make_head_tmap_bwd2(&tk, qkv + size_t(p.Hq) * D, p.B, p.S, p.Hkv, D, width))) return rc;
   if ((rc = make_head_tmap_bwd2(&tv, qkv + size_t(p.Hq + p.Hkv) * D, p.B, p.S, p.Hkv, D, width))) return rc;
@@ -791,10 +829,10 @@ static int launch_bwd2(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const
   }
   dim3 grid(p.Hkv * CL, (p.S + 127) / 128, p.B);
   if constexpr (!DQ) {
-    ZB_CUDA_OK(launch_chained(kern, grid, 32 * BWD2_WARPS, Cfg::SMEM_BYTES, stream, CL > 1 ? CL : 0, tq, tk, tv, tdo, p, stats,
+    ZB_CUDA_OK(launch_chained(kern, grid, 32 * BWD2_WARPS, Cfg::SMEM_BYTES, stream, CL > 1 ? CL : 0, tq, tk, tv, tdo, tdk, tdv, p, stats,
                               s_pad, trace, trace_ctas));
   } else {
-    kern<<<grid, 32 * BWD2_WARPS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, p, stats, s_pad, trace, trace_ctas);
+    kern<<<grid, 32 * BWD2_WARPS, Cfg::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, tdk, tdv, p, stats, s_pad, trace, trace_ctas);
     ZB_CUDA_OK(cudaGetLastError());
   }
   return 0;

@@ -44,7 +44,7 @@ template <int D>
 __global__ void __launch_bounds__(320, 1)
 flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
-                    const AttnBwdParams p, const float* stats, int s_pad) {
+                    const __grid_constant__ CUtensorMap tmap_dq, const AttnBwdParams p, const float* stats, int s_pad) {
   using Cfg = AttnDqCfg<D>;
   constexpr int BM = 128, BN = 128, NK = Cfg::NK, NV = Cfg::NV, DB = D / 64;
   constexpr int BLK = 128 * 128;  // bytes of one [128 rows x 64 cols] bf16 block
@@ -297,8 +297,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     if (ok && n > 0) ok = mbar_wait(dq_done, 0, wctx, ST_TIMEOUT_MISC);
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();
-    const int width = (p.Hq + 2 * p.Hkv) * D;
-    __nv_bfloat16* dst = p.dqkv + (size_t(batch) * p.S + row) * width + size_t(head) * D;
+    // through the place of Q, whose last reader is done, and TMA (see flash_bwd2.cu)
 #pragma unroll 1
     for (int c = half * (D / 64); c < (half + 1) * (D / 64); ++c) {
       uint32_t r[32];
@@ -309,19 +308,27 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 #pragma unroll
         for (int k = 0; k < 32; ++k) r[k] = 0u;
       }
-      if (ok && row_ok) {
 #pragma unroll
-        for (int k = 0; k < 32; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * p.scale);
+      for (int k = 0; k < 32; ++k) r[k] = __float_as_uint(__uint_as_float(r[k]) * p.scale);
+      const uint32_t at = smem_u32(sQ) + uint32_t(c >> 1) * BLK + uint32_t(t) * 128;
 #pragma unroll
-        for (int v4 = 0; v4 < 4; ++v4) {
-          uint4 u;
-          u.x = pack_bf16x2(__uint_as_float(r[v4 * 8 + 0]), __uint_as_float(r[v4 * 8 + 1]));
-          u.y = pack_bf16x2(__uint_as_float(r[v4 * 8 + 2]), __uint_as_float(r[v4 * 8 + 3]));
-          u.z = pack_bf16x2(__uint_as_float(r[v4 * 8 + 4]), __uint_as_float(r[v4 * 8 + 5]));
-          u.w = pack_bf16x2(__uint_as_float(r[v4 * 8 + 6]), __uint_as_float(r[v4 * 8 + 7]));
-          *reinterpret_cast<uint4*>(dst + c * 32 + v4 * 8) = u;
-        }
+      for (int v4 = 0; v4 < 4; ++v4)
+        st_shared_v4(at + ((uint32_t((c & 1) * 4 + v4) ^ uint32_t(t & 7)) << 4),
+                     pack_bf16x2(__uint_as_float(r[v4 * 8 + 0]), __uint_as_float(r[v4 * 8 + 1])),
+                     pack_bf16x2(__uint_as_float(r[v4 * 8 + 2]), __uint_as_float(r[v4 * 8 + 3])),
+                     pack_bf16x2(__uint_as_float(r[v4 * 8 + 4]), __uint_as_float(r[v4 * 8 + 5])),
+                     pack_bf16x2(__uint_as_float(r[v4 * 8 + 6]), __uint_as_float(r[v4 * 8 + 7])));
+    }
+    fence_proxy_async_smem();
+    asm volatile("bar.sync 1, 256;" ::: "memory");   // the compute warps
+    if (warp == 0 && ok && *abort_flag == 0) {
+      if (lane == 0) {
+#pragma unroll
+        for (int b = 0; b < DB; ++b) tma_store_4d(&tmap_dq, sQ + b * BLK, b * 64, head, q0, batch);
+        bulk_commit();
+        bulk_wait_read<0>();
       }
+      __syncwarp();
     }
   }
 
@@ -349,12 +356,13 @@ static int launch_dq(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const A
                      int s_pad, cudaStream_t stream) {
   using Cfg = AttnDqCfg<D>;
   const int width = (p.Hq + 2 * p.Hkv) * D;
-  CUtensorMap tq, tk, tv, tdo;
+  CUtensorMap tq, tk, tv, tdo, tdq;
   int rc;
   if ((rc = make_head_tmap_dq(&tq, qkv, p.B, p.S, p.Hq, D, width))) return rc;
   if ((rc = make_head_tmap_dq(&tk, qkv + size_t(p.Hq) * D, p.B, p.S, p.Hkv, D, width))) return rc;
   if ((rc = make_head_tmap_dq(&tv, qkv + size_t(p.Hq + p.Hkv) * D, p.B, p.S, p.Hkv, D, width))) return rc;
   if ((rc = make_head_tmap_dq(&tdo, d_o, p.B, p.S, p.Hq, D, p.Hq * D))) return rc;
+  if ((rc = make_head_tmap_dq(&tdq, p.dqkv, p.B, p.S, p.Hq, D, width))) return rc;
   auto kern = flash_bwd_dq_kernel<D>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -362,7 +370,7 @@ static int launch_dq(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const A
     attr_set = true;
   }
   dim3 grid(p.Hq, (p.S + 127) / 128, p.B);
-  ZB_CUDA_OK(launch_chained(kern, grid, 320, Cfg::SMEM_BYTES, stream, 0, tq, tk, tv, tdo, p, stats, s_pad));
+  ZB_CUDA_OK(launch_chained(kern, grid, 320, Cfg::SMEM_BYTES, stream, 0, tq, tk, tv, tdo, tdq, p, stats, s_pad));
   return 0;
 }
 

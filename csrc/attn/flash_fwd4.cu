@@ -82,7 +82,8 @@ enum : int {
 template <int D, bool TRACE, int MODE>
 __global__ void __launch_bounds__(32 * FWD4_WARPS, 1)
 flash_fwd4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                  const __grid_constant__ CUtensorMap tmap_v, const AttnFwd4Params p) {
+                  const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o,
+                  const AttnFwd4Params p) {
   using Cfg = AttnFwd4Cfg<D>;
   constexpr int BM = 128, BN = 128, NSLOT = Cfg::NSLOT, DB = D / 64, BLK = 128 * 128;
   constexpr bool PACKED = MODE >= 1;   // two-wide fp32 fma / add, three-input maximum
@@ -449,7 +450,8 @@ flash_fwd4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     tr(TR_EPI_BEGIN);
     tc_fence_after();
     const float inv_l = (l_run > 0.f) ? 1.f / l_run : 0.f;
-    __nv_bfloat16* orow = p.O + (size_t(batch) * p.S + row) * p.ldo + head * D;
+    // O leaves through the chain's Q tile, whose last reader is done, and TMA, which drops the rows behind the sequence
+    const uint32_t orow = smem_u32(sQ) + uint32_t(c) * Cfg::TILE_BYTES + uint32_t(t) * 128;
 #pragma unroll 1
     for (int ch = 0; ch < D / 32; ++ch) {
       uint32_t r[32];
@@ -460,23 +462,29 @@ flash_fwd4_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
         for (int k = 0; k < 32; ++k) r[k] = 0u;
       }
-      if (ok && row < p.S) {
+      const uint32_t at = orow + uint32_t(ch >> 1) * BLK;
 #pragma unroll
-        for (int v4 = 0; v4 < 4; ++v4) {
-          uint4 u;
-          u.x = pack_bf16x2(__uint_as_float(r[v4 * 8 + 0]) * inv_l, __uint_as_float(r[v4 * 8 + 1]) * inv_l);
-          u.y = pack_bf16x2(__uint_as_float(r[v4 * 8 + 2]) * inv_l, __uint_as_float(r[v4 * 8 + 3]) * inv_l);
-          u.z = pack_bf16x2(__uint_as_float(r[v4 * 8 + 4]) * inv_l, __uint_as_float(r[v4 * 8 + 5]) * inv_l);
-          u.w = pack_bf16x2(__uint_as_float(r[v4 * 8 + 6]) * inv_l, __uint_as_float(r[v4 * 8 + 7]) * inv_l);
-          *reinterpret_cast<uint4*>(orow + ch * 32 + v4 * 8) = u;
-        }
-      }
+      for (int v4 = 0; v4 < 4; ++v4)
+        st_shared_v4(at + ((uint32_t((ch & 1) * 4 + v4) ^ uint32_t(t & 7)) << 4),
+                     pack_bf16x2(__uint_as_float(r[v4 * 8 + 0]) * inv_l, __uint_as_float(r[v4 * 8 + 1]) * inv_l),
+                     pack_bf16x2(__uint_as_float(r[v4 * 8 + 2]) * inv_l, __uint_as_float(r[v4 * 8 + 3]) * inv_l),
+                     pack_bf16x2(__uint_as_float(r[v4 * 8 + 4]) * inv_l, __uint_as_float(r[v4 * 8 + 5]) * inv_l),
+                     pack_bf16x2(__uint_as_float(r[v4 * 8 + 6]) * inv_l, __uint_as_float(r[v4 * 8 + 7]) * inv_l));
+    }
+    fence_proxy_async_smem();
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + c) : "memory");   // the chain's four warps
+    if ((warp & 3) == 0 && lane == 0 && ok && *abort_flag == 0 && q0 < p.S) {
+#pragma unroll
+      for (int b = 0; b < DB; ++b)
+        tma_store_4d(&tmap_o, sQ + c * Cfg::TILE_BYTES + b * BLK, b * 64, head, q0, batch);
+      bulk_commit();
     }
     if (ok && row < p.S && p.lse != nullptr) {
       const float m_eff = (m_run == -INFINITY) ? 0.f : m_run;
       p.lse[(size_t(batch) * p.Hq + head) * p.S + row] =
           (l_run > 0.f) ? (m_eff * scale + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
     }
+    if ((warp & 3) == 0 && lane == 0) bulk_wait_read<0>();
     tr(TR_EPI_END);
   }
 
@@ -502,8 +510,9 @@ static int make_head_tmap4(CUtensorMap* out, const __nv_bfloat16* base, int B, i
 template <int D, bool TRACE, int MODE>
 static int launch_fwd4(const __nv_bfloat16* qkv, int width, const AttnFwd4Params& p, cudaStream_t stream) {
   using Cfg = AttnFwd4Cfg<D>;
-  CUtensorMap tq, tk, tv;
+  CUtensorMap tq, tk, tv, to;
   int rc;
+  if ((rc = make_head_tmap4(&to, p.O, p.B, p.S, p.Hq, D, p.ldo))) return rc;
   if ((rc = make_head_tmap4(&tq, qkv, p.B, p.S, p.Hq, D, width))) return rc;
   if ((rc = make_head_tmap4(&tk, qkv + size_t(p.Hq) * D, p.B, p.S, p.Hkv, D, width))) return rc;
   if ((rc = make_head_tmap4(&tv, qkv + size_t(p.Hq + p.Hkv) * D, p.B, p.S, p.Hkv, D, width))) return rc;
@@ -514,7 +523,7 @@ static int launch_fwd4(const __nv_bfloat16* qkv, int width, const AttnFwd4Params
     attr_set = true;
   }
   dim3 grid(p.Hq, (p.S + 255) / 256, p.B);
-  ZB_CUDA_OK(launch_chained(kern, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, 0, tq, tk, tv, p));
+  ZB_CUDA_OK(launch_chained(kern, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, 0, tq, tk, tv, to, p));
   return 0;
 }
 
