@@ -168,8 +168,8 @@ flash_bwd2_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   if constexpr (!DQ) {
-    chain_trigger();
     chain_wait();
+    chain_trigger();   // behind the wait: the dQ kernel starts on this, under the last CTAs here (chain_late in ptx.cuh)
   }
 
   if (warp == 8) {
@@ -851,7 +851,7 @@ static int bwd_cluster(int B, int S, int Hq, int Hkv) {
 }
 
 int attn_bwd_dq(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const AttnBwdParams& p, const float* stats, int s_pad,
-                int D, cudaStream_t stream);   // flash_bwd_dq.cu
+                int D, int late, cudaStream_t stream);   // flash_bwd_dq.cu
 
 }  // namespace zb
 
@@ -936,7 +936,7 @@ int zb_flash_bwd3(const void* d_o, const void* qkv, const void* o, const float* 
     rc = D == 128 ? run(std::integral_constant<int, 128>()) : run(std::integral_constant<int, 64>());
   }
   if (rc) return rc;
-  return (parts & 2) ? attn_bwd_dq(QKV, DO, p, stats, s_pad, D, stream) : 0;
+  return (parts & 2) ? attn_bwd_dq(QKV, DO, p, stats, s_pad, D, parts == 3, stream) : 0;
 }
 
 }  // extern "C"

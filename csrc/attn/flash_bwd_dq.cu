@@ -44,7 +44,8 @@ template <int D>
 __global__ void __launch_bounds__(320, 1)
 flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
-                    const __grid_constant__ CUtensorMap tmap_dq, const AttnBwdParams p, const float* stats, int s_pad) {
+                    const __grid_constant__ CUtensorMap tmap_dq, const AttnBwdParams p, const float* stats, int s_pad,
+                    const int late) {
   using Cfg = AttnDqCfg<D>;
   constexpr int BM = 128, BN = 128, NK = Cfg::NK, NV = Cfg::NV, DB = D / 64;
   constexpr int BLK = 128 * 128;  // bytes of one [128 rows x 64 cols] bf16 block
@@ -108,8 +109,10 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // The kernel before this one is the dK / dV kernel, of which nothing is needed here; it has waited for the statistics.
+  // 480 CTAs each (8 x 12 heads of 577 tokens) make 3.2 rounds on 148 SMs, so a quarter of its time most SMs idled.
+  if (!late) chain_wait();
   chain_trigger();
-  chain_wait();
 
   if (warp == 8) {
     // ------------------------------ TMA producer ------------------------------
@@ -342,6 +345,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
+  if (late) chain_wait();
 }
 
 static int make_head_tmap_dq(CUtensorMap* out, const __nv_bfloat16* base, int B, int S, int heads, int D, int width) {
@@ -353,7 +357,7 @@ static int make_head_tmap_dq(CUtensorMap* out, const __nv_bfloat16* base, int B,
 
 template <int D>
 static int launch_dq(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const AttnBwdParams& p, const float* stats,
-                     int s_pad, cudaStream_t stream) {
+                     int s_pad, int late, cudaStream_t stream) {
   using Cfg = AttnDqCfg<D>;
   const int width = (p.Hq + 2 * p.Hkv) * D;
   CUtensorMap tq, tk, tv, tdo, tdq;
@@ -370,16 +374,17 @@ static int launch_dq(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const A
     attr_set = true;
   }
   dim3 grid(p.Hq, (p.S + 127) / 128, p.B);
-  ZB_CUDA_OK(launch_chained(kern, grid, 320, Cfg::SMEM_BYTES, stream, 0, tq, tk, tv, tdo, tdq, p, stats, s_pad));
+  ZB_CUDA_OK(launch_chained(kern, grid, 320, Cfg::SMEM_BYTES, stream, 0, tq, tk, tv, tdo, tdq, p, stats, s_pad, late));
   return 0;
 }
 
 // dQ part of the two-kernel backward: writes the q columns of dqkv.  `stats` as written by the key-tile
 // kernel's statistics pass (lse in log2 units and delta per row, rows padded to s_pad).
+// late: the kernel in front in the stream is the key-tile kernel of the same call.
 int attn_bwd_dq(const __nv_bfloat16* qkv, const __nv_bfloat16* d_o, const AttnBwdParams& p, const float* stats, int s_pad,
-                int D, cudaStream_t stream) {
-  if (D == 128) return launch_dq<128>(qkv, d_o, p, stats, s_pad, stream);
-  return launch_dq<64>(qkv, d_o, p, stats, s_pad, stream);
+                int D, int late, cudaStream_t stream) {
+  if (D == 128) return launch_dq<128>(qkv, d_o, p, stats, s_pad, late, stream);
+  return launch_dq<64>(qkv, d_o, p, stats, s_pad, late, stream);
 }
 
 }  // namespace zb

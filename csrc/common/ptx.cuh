@@ -50,6 +50,11 @@ __device__ __forceinline__ bool zb_in_bounds(bool cond, int* status, int site) {
 // launched once every CTA of this one has got here (it only lets it take up idle resources early).  chain_wait: returns
 // when the kernel before this one has finished and its writes are visible; every thread of a kernel launched with
 // launch_chained calls it before it touches global memory.  Kernels that wait for other processes do neither.
+// chain_late: a kernel that reads nothing its predecessor writes need not wait for it at its start: it takes up SMs as those of
+// the predecessor become free, and waits at its end, so that whoever waits for it has waited for the predecessor too.  Its
+// inputs have to be complete by then: the first kernel in front of it that did wait has called chain_trigger behind its
+// chain_wait, so nothing behind that one starts before everything in front of that one is done.  A late kernel writes to no
+// memory that a kernel since then still uses (workspaces that went back to an allocator included).
 __device__ __forceinline__ void chain_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

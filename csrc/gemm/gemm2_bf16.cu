@@ -205,9 +205,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   cluster_sync_all();  // barriers of both CTAs are initialised before anyone signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const bool late = (p.flags & GEMM_LATE) != 0;
   if constexpr (!SCATTER && !FUSED_AG) {
+    if (!late) chain_wait();
     chain_trigger();
-    chain_wait();
   }
 
   if (warp == 0) {
@@ -715,6 +716,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   if (warp >= 2 && lane == 0) bulk_wait_read<0>();
   __syncwarp();
   asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  if constexpr (!SCATTER && !FUSED_AG) {
+    if (late) chain_wait();
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);

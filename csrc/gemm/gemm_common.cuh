@@ -11,6 +11,9 @@ enum : int {
   GEMM_ACCUMULATE = 2,  // C += result (read-modify-write in C's dtype, fp32 add)
   GEMM_GELU = 4,        // tanh-GELU applied after bias (forward of GPT-style MLPs)
   GEMM_RELU = 8,
+  // The kernel before this one in the stream writes nothing that this product reads, and that one's predecessors are known to
+  // be done when it starts: see chain_late in ptx.cuh
+  GEMM_LATE = 16,
 };
 
 struct GemmParams {

@@ -22,7 +22,7 @@ namespace {
 
 using at::Tensor;
 
-constexpr int GEMM_OUT_F32 = 1, GEMM_ACCUMULATE = 2;
+constexpr int GEMM_OUT_F32 = 1, GEMM_ACCUMULATE = 2, GEMM_LATE = 16;
 
 // Entry points of the kernel library, in the order `init` gets them.
 struct Entry {
@@ -50,7 +50,7 @@ struct Entry {
   int (*flash_stats_floats)(int, int, int);
   int (*gemm2_act_fwd)(const void*, const void*, const void*, void*, void*, int, int, int, int, int, int, int*, cudaStream_t);
   int (*gemm2_act_bwd)(const void*, const void*, const void*, void*, int, int, int, int, int, int, int*, cudaStream_t);
-  int (*column_sums)(const long*, int, cudaStream_t);
+  int (*column_sums)(const long*, int, int, cudaStream_t);
   const char* (*last_error)();
 };
 Entry lib;
@@ -121,16 +121,23 @@ bool truth(PyObject* o) { return PyObject_IsTrue(o) == 1; }
     return nullptr;                                                                         \
   }
 
-// out[M, N] (+)= A B^T; `out` as the caller prepared it.  1: done, 0: not for here, -1: error set.
-int gemm(const Tensor* a, const Tensor* b, const Tensor& out, bool a_mn, bool b_mn, const Tensor* bias, const Tensor* addend,
-         bool accumulate, int* status) {
+// Whether out[M, N] (+)= A B^T is a product for here.
+bool product(const Tensor* a, const Tensor* b, const Tensor& out, bool a_mn, bool b_mn) {
   const int64_t M = out.size(0), N = out.size(1), K = a->size(a_mn ? 0 : 1);
-  if (a->size(a_mn ? 1 : 0) != M || b->size(b_mn ? 1 : 0) != N || b->size(b_mn ? 0 : 1) != K) return 0;
-  if (!fits(M) || !fits(N) || !fits(K) || !fits(a->stride(0)) || !fits(b->stride(0)) || !fits(out.stride(0))) return 0;
+  return a->size(a_mn ? 1 : 0) == M && b->size(b_mn ? 1 : 0) == N && b->size(b_mn ? 0 : 1) == K && fits(M) && fits(N) && fits(K) &&
+         fits(a->stride(0)) && fits(b->stride(0)) && fits(out.stride(0));
+}
+
+// out[M, N] (+)= A B^T; `out` as the caller prepared it.  1: done, 0: not for here, -1: error set.
+// more: flags, GEMM_LATE for one that starts under the kernel before it; whole: no tiles cut along K (a workspace).
+int gemm(const Tensor* a, const Tensor* b, const Tensor& out, bool a_mn, bool b_mn, const Tensor* bias, const Tensor* addend,
+         bool accumulate, int* status, int more = 0, bool whole = false) {
+  const int64_t M = out.size(0), N = out.size(1), K = a->size(a_mn ? 0 : 1);
+  if (!product(a, b, out, a_mn, b_mn)) return 0;
   if (bias != nullptr && !(dense(bias, BF16) && bias->dim() == 1 && bias->size(0) == N)) return 0;
   if (addend != nullptr && !(matrix(addend, BF16) && addend->size(0) == M && addend->size(1) == N && fits(addend->stride(0))))
     return 0;
-  const int flags = (out.scalar_type() == F32 ? GEMM_OUT_F32 : 0) | (accumulate ? GEMM_ACCUMULATE : 0);
+  const int flags = (out.scalar_type() == F32 ? GEMM_OUT_F32 : 0) | (accumulate ? GEMM_ACCUMULATE : 0) | more;
   const int lda = int(a->stride(0)), ldb = int(b->stride(0)), ldc = int(out.stride(0));
   const int ldx = addend == nullptr ? 0 : int(addend->stride(0));
   const void *pa = ptr(a), *pb = ptr(b), *pbias = ptr(bias), *px = ptr(addend);
@@ -142,7 +149,7 @@ int gemm(const Tensor* a, const Tensor* b, const Tensor& out, bool a_mn, bool b_
       return lib.gemm(pa, pb, pc, m, n, k, lda, ldb, ldc, a_mn, b_mn, pbias, px, ldx, flags, 0, 0, status, s);
     }) ? 1 : -1;
   // (the same line as in the wrapper: shorter reductions are never cut)
-  const int ws_bytes = k > 3000 ? lib.gemm2_workspace(m, n, k) : 0;
+  const int ws_bytes = k > 3000 && !whole ? lib.gemm2_workspace(m, n, k) : 0;
   if (ws_bytes > 0) {
     const Tensor ws = empty({ws_bytes}, *a, at::kByte);
     void* pw = ws.data_ptr();
@@ -155,13 +162,13 @@ int gemm(const Tensor* a, const Tensor* b, const Tensor& out, bool a_mn, bool b_
   }) ? 1 : -1;
 }
 
-// Whether column_sums takes this bf16 matrix.
+// Whether zb_column_sums takes this bf16 matrix.
 bool summable(const Tensor& t) {
   return t.size(1) % 8 == 0 && t.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
 }
-bool later(PyObject* sums, PyObject* entry) {   // (takes over `entry`)
+bool later(PyObject* list, PyObject* entry) {   // (takes over `entry`)
   if (entry == nullptr) return false;
-  const int rc = PyList_Append(sums, entry);
+  const int rc = PyList_Append(list, entry);
   Py_DECREF(entry);
   return rc == 0;
 }
@@ -194,8 +201,8 @@ PyObject* linear_dgrad(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   return forward_like(args, true, Py_None, args[2]);
   END_HANDLE_TH_ERRORS
 }
-// linear_wgrad(dy, x, gw, gb | None, sums | None): gw += dy^T x, gb += column sums of dy.  With a list `sums` the second is
-// left to column_sums, (dy, gb) appended.  True when done.
+// linear_wgrad(dy, x, gw, gb | None, later | None): gw += dy^T x, gb += column sums of dy.  With a list `later` both are left
+// to finish, (dy, x, gw, gb | None) appended.  True when done.
 PyObject* linear_wgrad(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   ZB_ARGS(5)
@@ -205,10 +212,11 @@ PyObject* linear_wgrad(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (gb != nullptr && !(gradient(gb) && gb->dim() == 1 && gb->size(0) == dy->size(1))) Py_RETURN_NONE;
   int* status = status_of(*dy);
   if (status == nullptr) Py_RETURN_NONE;
+  if (PyList_Check(args[4]) && product(dy, x, *gw, true, true) && (gb == nullptr || summable(*dy)))
+    return later(args[4], PyTuple_Pack(4, args[0], args[1], args[2], args[3])) ? Py_NewRef(Py_True) : nullptr;
   const int done = gemm(dy, x, *gw, true, true, nullptr, nullptr, true, status);
   if (done < 0) return nullptr;
   if (done == 0) Py_RETURN_NONE;
-  if (gb != nullptr && PyList_Check(args[4]) && summable(*dy)) return later(args[4], PyTuple_Pack(2, args[0], args[3])) ? Py_NewRef(Py_True) : nullptr;
   if (gb != nullptr) {
     const int64_t T = dy->size(0), N = dy->size(1);
     const Tensor part = empty({T < 64 ? T : 64, N}, *dy, F32);
@@ -308,8 +316,8 @@ PyObject* norm_fwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// norm_bwd(dy, x, w, stats, dres | None, dw, db | None, layernorm, sums | None) -> dx (+ dres); dw, db are added to, or, with
-// a list `sums`, left to column_sums as (partial sums, dw, db | None)
+// norm_bwd(dy, x, w, stats, dres | None, dw, db | None, layernorm, later | None) -> dx (+ dres); dw, db are added to, or,
+// with a list `later`, left to finish as (partial sums, dw, db | None)
 PyObject* norm_bwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   ZB_ARGS(9)
@@ -351,20 +359,50 @@ PyObject* norm_bwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   END_HANDLE_TH_ERRORS
 }
 
-// column_sums(sums): what linear_wgrad and norm_bwd have left in the list, which is emptied.
-PyObject* column_sums(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+// finish(later): the products and column sums that linear_wgrad and norm_bwd have left in the list, which is emptied.
+//
+// No product reads what another one writes, so each but the first starts on the SMs that the one before it has done with,
+// where one after the other every one ended with most of the GPU idle (a BERT block's four weight gradients are 54, 18, 72 and
+// 72 tiles on 74 pairs), and the column sums run beside the last.  All operands stay in the list until everything is
+// launched, and only the last product may have a workspace of the allocator's: the rules of chain_late (ptx.cuh).
+PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   ZB_ARGS(1)
   if (!PyList_Check(args[0]) || !ready) {
-    PyErr_SetString(PyExc_TypeError, "column_sums takes the list that linear_wgrad and norm_bwd have filled");
+    PyErr_SetString(PyExc_TypeError, "finish takes the list that linear_wgrad and norm_bwd have filled");
     return nullptr;
+  }
+  auto refuse = [] {
+    PyErr_SetString(PyExc_TypeError, "finish: an entry that linear_wgrad or norm_bwd did not make");
+    return nullptr;
+  };
+  const Py_ssize_t entries = PyList_GET_SIZE(args[0]);
+  Py_ssize_t products = 0, launched = 0;
+  for (Py_ssize_t i = 0; i < entries; ++i) {
+    PyObject* e = PyList_GET_ITEM(args[0], i);
+    if (!PyTuple_Check(e) || (PyTuple_GET_SIZE(e) != 3 && PyTuple_GET_SIZE(e) != 4)) return refuse();
+    products += PyTuple_GET_SIZE(e) == 4;
   }
   constexpr int MAX = 8;   // sums per launch
   long desc[MAX][7];
   int n = 0;
+  bool late = false;       // a product has been launched here: what the sums read was complete before it
   const cudaStream_t s = stream();
+  for (Py_ssize_t i = 0; i < entries; ++i) {
+    PyObject* e = PyList_GET_ITEM(args[0], i);
+    if (PyTuple_GET_SIZE(e) != 4) continue;
+    const Tensor *dy = tensor_of(PyTuple_GET_ITEM(e, 0)), *x = tensor_of(PyTuple_GET_ITEM(e, 1)), *gw = tensor_of(PyTuple_GET_ITEM(e, 2));
+    if (dy == nullptr || x == nullptr || gw == nullptr) return refuse();
+    int* status = status_of(*dy);
+    if (status == nullptr) return refuse();
+    const bool first = launched == 0, last = ++launched == products;
+    const int done = gemm(dy, x, *gw, true, true, nullptr, nullptr, true, status, first ? 0 : GEMM_LATE, !last);
+    if (done < 0) return nullptr;
+    if (done == 0) return refuse();
+    late = true;
+  }
   auto run = [&] {
-    const bool ok = n == 0 || launch("column_sums", 1, [&] { return lib.column_sums(desc[0], n, s); });
+    const bool ok = n == 0 || launch("column_sums", 1, [&] { return lib.column_sums(desc[0], n, late, s); });
     n = 0;
     return ok;
   };
@@ -376,25 +414,23 @@ PyObject* column_sums(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     memcpy(desc[n++], d, sizeof(d));
     return true;
   };
-  for (Py_ssize_t i = 0; i < PyList_GET_SIZE(args[0]); ++i) {
+  for (Py_ssize_t i = 0; i < entries; ++i) {
     PyObject* e = PyList_GET_ITEM(args[0], i);
-    const Py_ssize_t k = PyTuple_Check(e) ? PyTuple_GET_SIZE(e) : 0;
-    const Tensor *src = k > 0 ? tensor_of(PyTuple_GET_ITEM(e, 0)) : nullptr, *out = k > 1 ? tensor_of(PyTuple_GET_ITEM(e, 1)) : nullptr;
-    const Tensor* second = nullptr;
-    if (src == nullptr || out == nullptr || (k == 3 && !optional_tensor(PyTuple_GET_ITEM(e, 2), second)) ||
-        (k == 3) != (src->dim() == 3)) {
-      PyErr_SetString(PyExc_TypeError, "column_sums: an entry that linear_wgrad or norm_bwd did not make");
-      return nullptr;
-    }
-    if (k == 2) {
-      if (!add(*src, 0, src->size(0), src->size(1), src->stride(0), *out)) return nullptr;
+    const Tensor* src = tensor_of(PyTuple_GET_ITEM(e, 0));
+    if (src == nullptr) return refuse();
+    if (PyTuple_GET_SIZE(e) == 4) {
+      const Tensor* gb;
+      if (!optional_tensor(PyTuple_GET_ITEM(e, 3), gb)) return refuse();
+      if (gb != nullptr && !add(*src, 0, src->size(0), src->size(1), src->stride(0), *gb)) return nullptr;
     } else {
+      const Tensor *out = tensor_of(PyTuple_GET_ITEM(e, 1)), *second;
+      if (out == nullptr || !optional_tensor(PyTuple_GET_ITEM(e, 2), second) || src->dim() != 3) return refuse();
       const int64_t P = src->size(1), H = src->size(2);
       if (!add(*src, 0, P, H, H, *out) || (second != nullptr && !add(*src, P * H, P, H, H, *second))) return nullptr;
     }
   }
   if (!run()) return nullptr;
-  if (PyList_SetSlice(args[0], 0, PyList_GET_SIZE(args[0]), nullptr) != 0) return nullptr;
+  if (PyList_SetSlice(args[0], 0, entries, nullptr) != 0) return nullptr;
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }
@@ -581,7 +617,7 @@ PyObject* launch_count(PyObject*, PyObject* const*, Py_ssize_t) { return PyLong_
 
 #define ZB_FN(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {ZB_FN(init), ZB_FN(set_status), ZB_FN(launch_count), ZB_FN(linear_fwd), ZB_FN(linear_dgrad),
-                         ZB_FN(linear_wgrad), ZB_FN(act_linear_fwd), ZB_FN(act_linear_dgrad), ZB_FN(norm_fwd), ZB_FN(norm_bwd), ZB_FN(column_sums), ZB_FN(rope), ZB_FN(swiglu_fwd),
+                         ZB_FN(linear_wgrad), ZB_FN(act_linear_fwd), ZB_FN(act_linear_dgrad), ZB_FN(norm_fwd), ZB_FN(norm_bwd), ZB_FN(finish), ZB_FN(rope), ZB_FN(swiglu_fwd),
                          ZB_FN(swiglu_bwd), ZB_FN(act_fwd), ZB_FN(act_bwd), ZB_FN(attn_fwd), ZB_FN(attn_bwd),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "zorse_fastops", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

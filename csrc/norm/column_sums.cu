@@ -22,12 +22,13 @@ struct ColSumItem {
 };
 struct ColSumItems {
   ColSumItem item[COLSUM_MAX];
+  int late;   // nothing that the kernel before this one writes is read here (chain_late in ptx.cuh)
 };
 
 __global__ void __cluster_dims__(COLSUM_RANKS, 1, 1) __launch_bounds__(256)
 column_sums_kernel(const __grid_constant__ ColSumItems p) {
   chain_trigger();
-  chain_wait();
+  if (!p.late) chain_wait();
   __shared__ float warp_sum[8][COLSUM_COLS], cta_sum[COLSUM_COLS];
   const int strip = blockIdx.x / COLSUM_RANKS, rank = blockIdx.x % COLSUM_RANKS;
   int i = 0;
@@ -114,17 +115,20 @@ column_sums_kernel(const __grid_constant__ ColSumItems p) {
   }
   // nobody leaves while its sums are read
   asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+  if (p.late) chain_wait();
 }
 
 }  // namespace zb
 
 // n <= 8 sums.  desc: per sum src, out, rows, cols, row distance in elements, 1 if src is fp32 (else bf16), 1 if out is.  Rows
 // of src start on 16-byte boundaries and cols is a multiple of 8 (bf16) or 4 (fp32).  Returns 1, with nothing done, otherwise.
-extern "C" int zb_column_sums(const long* desc, int n, cudaStream_t stream) {
+// late: the kernel in front of this one in the stream writes none of the sources (see chain_late in ptx.cuh).
+extern "C" int zb_column_sums(const long* desc, int n, int late, cudaStream_t stream) {
   using namespace zb;
   if (n <= 0) return 0;
   if (n > COLSUM_MAX) ZB_FAIL(-1, "column_sums: %d sums (at most %d)", n, COLSUM_MAX);
   ColSumItems p = {};
+  p.late = late;
   int strips = 0, used = 0;
   for (int i = 0; i < n; ++i, desc += 7) {
     ColSumItem& it = p.item[used];

@@ -122,7 +122,7 @@ def test_norms(ops, T, H, ln, dt):
 @pytest.mark.parametrize("T,widths", [(1, [8, 512]), (7, [72, 64, 520]), (300, [768, 3072, 768, 2304]), (2503, [1032, 8, 200]),
                                       (4616, [768] * 6)])
 @pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
-def test_column_sums_of_a_layer_in_one_launch(ops, T, widths, dt):
+def test_finish_of_a_layer_in_one_launch(ops, T, widths, dt):
     """Bias gradients of matrices of several widths (one a slice of wider rows) and the gradients of two norms: fewer and more
     than fit one launch, against 64 bits, and the same bits each time.  Bounds: fp32 sums of T terms in chains of at most T / 256
     + 40 additions, of numbers whose absolute sum is `mass`; bf16 gradients round once more."""
@@ -130,19 +130,20 @@ def test_column_sums_of_a_layer_in_one_launch(ops, T, widths, dt):
     x, dyn, w = _rand(T, H, seed=1), _rand(T, H, seed=2), _rand(H, seed=3)
     _, st = k.norm_fwd(x, w, w, 1e-5, True)
     dys = [_rand(T, n + 8 * (i == 1), seed=10 + i)[:, :n] for i, n in enumerate(widths)]
+    x16 = x[:, :16].contiguous()
 
     def run():
-        sums, outs = ops.new_sums(), [torch.ones(n, dtype=dt, device="cuda") for n in widths]
+        later, outs = ops.collect(), [torch.ones(n, dtype=dt, device="cuda") for n in widths]
         gw = [torch.zeros(n, 16, dtype=dt, device="cuda") for n in widths]
         norm = [torch.ones(H, dtype=dt, device="cuda") for _ in range(4)]
         before = k.launch_count()
         for dy, g, o in zip(dys, gw, outs):
-            ops.linear_wgrad(dy, x[:, :16].contiguous(), g, o, sums=sums)
+            ops.linear_wgrad(dy, x16, g, o, later=later)
         for i in (0, 2):
-            ops.norm_bwd(dyn, x, w, st, None, norm[i], norm[i + 1], True, sums)
-        assert len(sums) == len(widths) + 2 and all(bool((o == 1).all()) for o in outs + norm)
-        ops.finish_sums(sums)
-        assert not sums and k.launch_count() - before == len(widths) + 2 + -(-(len(widths) + 4) // 8)
+            ops.norm_bwd(dyn, x, w, st, None, norm[i], norm[i + 1], True, later)
+        assert len(later) == len(widths) + 2 and all(bool((o == 1).all()) for o in outs + norm)
+        ops.finish(later)
+        assert not later and k.launch_count() - before == len(widths) + 2 + -(-(len(widths) + 4) // 8)
         return outs + norm
 
     got, again = run(), run()
@@ -154,6 +155,44 @@ def test_column_sums_of_a_layer_in_one_launch(ops, T, widths, dt):
         mass = 1 + src.abs().sum(0)
         tol = mass * (T / 256 + 40) * 2.0 ** -24 + (0 if dt == torch.float32 else 2.0 ** -8) * (1 + src.sum(0)).abs()
         assert bool(((o.double() - 1 - src.sum(0)).abs() <= tol + 1e-6).all())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,sizes", [(300, [(1536, 512), (512, 512), (2048, 512), (512, 2048)]), (4616, [(2304, 768), (768, 768)]),
+                                     (3072, [(768, 768)]), (8200, [(520, 264), (264, 520), (1032, 1000)]), (64, [(304, 256), (72, 512)])])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_weight_gradients_that_start_under_one_another(ops, T, sizes, dt):
+    """A layer's products without a wait between them, behind a kernel that has just written their operands, several times into
+    the same gradients: the bits of the same products one after the other (whole tiles: the same sums in the same order; the
+    last one is cut along K as it would be alone), and bias gradients of operands written just before."""
+    dys = [torch.zeros(T, n, dtype=torch.bfloat16, device="cuda") for n, _ in sizes]
+    xs = [_rand(T, m, seed=20 + i) for i, (_, m) in enumerate(sizes)]
+    fresh = [[_rand(T, n, seed=40 + 10 * r + i) for i, (n, _) in enumerate(sizes)] for r in range(3)]
+    new = lambda *shape: [torch.zeros(*shape, dtype=dt, device="cuda") for _ in range(2)]
+    gw, gb = [new(n, m) for n, m in sizes], [new(n) for n, _ in sizes]
+    for r in range(3):
+        for i, dy in enumerate(dys):
+            k.lib().zb_act_fwd(fresh[r][i].data_ptr(), dy.data_ptr(), dy.numel(), 1, k._stream())   # relu, launched like a step's
+        later = ops.collect()
+        for i, dy in enumerate(dys):
+            ops.linear_wgrad(dy, xs[i], gw[i][0], gb[i][0], later=later)
+        ops.finish(later)
+    for r in range(3):
+        for i in range(len(sizes)):
+            dy = fresh[r][i].clamp(min=0)
+            torch.cuda.synchronize()
+            if i + 1 < len(sizes) and T > 3000 and min(sizes[i]) >= 256:      # not cut along K there
+                rc = k.lib().zb_gemm2_bf16(dy.data_ptr(), xs[i].data_ptr(), gw[i][1].data_ptr(), *sizes[i], T, sizes[i][0], sizes[i][1],
+                                           sizes[i][1], 1, 1, 0, 0, 0, k.GEMM_ACCUMULATE | (k.GEMM_OUT_F32 if dt == torch.float32 else 0),
+                                           0, k.status_word(0).data_ptr(), k._stream())
+                k._check(rc, "gemm2")
+            else:
+                k.gemm(dy, xs[i], gw[i][1], a_mn=True, b_mn=True, accumulate=True)
+            gb[i][1] += dy.double().sum(0).to(dt)
+    k.check_status()
+    for i in range(len(sizes)):
+        assert torch.equal(gw[i][0], gw[i][1]), i
+        torch.testing.assert_close(gb[i][0].double(), gb[i][1].double(), rtol=1e-5 if dt == torch.float32 else 2.0 ** -6, atol=1e-2)
 
 
 @pytest.mark.gpu

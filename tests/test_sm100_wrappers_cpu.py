@@ -153,11 +153,28 @@ def test_passes_that_start_early_wait_first_and_use_coherent_loads():
                 depth += {"{": 1, "}": -1}.get(text[end], 0)
                 end += 1
             body = text[start + 1:end]
-            assert body.split()[:2] == ["chain_trigger();", "chain_wait();"], name
+            # (a late kernel waits at its end instead)
+            assert re.match(r"\s*chain_trigger\(\);\s*(if \(!p\.late\) )?chain_wait\(\);", body), name
+            assert ("p.late" in body) == (re.search(r"if \(p\.late\) chain_wait\(\);\s*}?$", body) is not None), name
             assert not re.search(r"__ldg|ld_nc|ld\.global\.nc|__restrict__", text[at:end]), name
             seen.add(name)
     assert {"norm_fwd_kernel", "norm_bwd2_kernel", "rope_kernel", "swiglu_fwd_kernel", "act_bwd_kernel", "colsum_one_kernel",
             "gemm2_fixup_kernel", "attn_bwd2_stats_kernel", "ce_fwd_bwd_kernel"} <= seen
+
+
+def test_kernels_that_a_late_one_follows_trigger_behind_their_wait():
+    """A late kernel (chain_late in ptx.cuh) starts when every CTA of its predecessor has triggered, and takes that for a sign
+    that everything in front of the predecessor is done."""
+    import pathlib
+    import re
+
+    root = pathlib.Path(__file__).resolve().parent.parent / "csrc"
+    for name, wait in (("gemm/gemm2_bf16.cu", r"if \(!late\) chain_wait\(\);"), ("attn/flash_bwd_dq.cu", r"if \(!late\) chain_wait\(\);"),
+                       ("attn/flash_bwd2.cu", r"chain_wait\(\);")):
+        text = (root / name).read_text().split("attn_bwd2_stats_kernel")[0].split("gemm2_fixup_kernel(")[0]
+        assert len(re.findall(wait + r"\s*chain_trigger\(\);", text)) == 1 and text.count("chain_trigger();") == 1, name
+    for name in ("gemm/gemm2_bf16.cu", "attn/flash_bwd_dq.cu"):
+        assert (root / name).read_text().count("if (late) chain_wait();") == 1, name
 
 
 def bf(*shape):

@@ -180,18 +180,18 @@ class TransformerBlock(Layer):
             sv.update(qkv=qkv, att=att, lse=lse)
         return out
 
-    def _attn_bwd(self, dout, xin, ctx, ops, sv, dres, sums):
+    def _attn_bwd(self, dout, xin, ctx, ops, sv, dres, later):
         """dout: grad of the o-projection output; returns grad wrt xin (+ dres)."""
         p, g, B, S = self.p, self.g, ctx["B"], ctx["S"]
         datt = ops.linear_dgrad(dout, p["o_w"])
-        ops.linear_wgrad(dout, sv["att"], g["o_w"], g.get("o_b"), sums=sums)
+        ops.linear_wgrad(dout, sv["att"], g["o_w"], g.get("o_b"), later=later)
         dqkv = ops.attn_bwd(datt, sv["qkv"], sv["att"], sv["lse"], B, S, self.Hq, self.Hkv, self.D, self.causal,
                             self.window)
         cs = self._rope(ops, S, dout.device)
         if cs is not None:
             ops.rope_(dqkv, cs, S, self.Hq + self.Hkv, self.D, backward=True)
         dxin = ops.linear_dgrad(dqkv, p["qkv_w"], addend=dres)
-        ops.linear_wgrad(dqkv, xin, g["qkv_w"], g.get("qkv_b"), sums=sums)
+        ops.linear_wgrad(dqkv, xin, g["qkv_w"], g.get("qkv_b"), later=later)
         return dxin
 
     def _mlp_fwd(self, xin, resid, ops, sv):
@@ -202,12 +202,12 @@ class TransformerBlock(Layer):
             sv.update(hpre=hpre, mlp_a=a)
         return out
 
-    def _mlp_bwd(self, dout, xin, ops, sv, dres, sums):
+    def _mlp_bwd(self, dout, xin, ops, sv, dres, later):
         p, g = self.p, self.g
         dh = ops.act_linear_dgrad(dout, p["down_w"], sv["hpre"], self.act)
-        ops.linear_wgrad(dout, sv["mlp_a"], g["down_w"], g.get("down_b"), sums=sums)
+        ops.linear_wgrad(dout, sv["mlp_a"], g["down_w"], g.get("down_b"), later=later)
         dxin = ops.linear_dgrad(dh, p["up_w"], addend=dres)
-        ops.linear_wgrad(dh, xin, g["up_w"], g.get("up_b"), sums=sums)
+        ops.linear_wgrad(dh, xin, g["up_w"], g.get("up_b"), later=later)
         return dxin
 
     # ---- block ----------------------------------------------------------------------
@@ -232,18 +232,18 @@ class TransformerBlock(Layer):
     def backward(self, dy, ctx, ops, saved):
         p, g, sv = self.p, self.g, saved
         ln = self.norm == "ln"
-        sums = ops.new_sums()
+        later = ops.collect()
         if self.pre_norm:
-            dn2 = self._mlp_bwd(dy, sv["n2"], ops, sv, None, sums)
-            dh1 = ops.norm_bwd(dn2, sv["h1"], p["norm2_w"], sv["st2"], dy, g["norm2_w"], g.get("norm2_b"), ln, sums)
-            dn1 = self._attn_bwd(dh1, sv["n1"], ctx, ops, sv, None, sums)
-            dx = ops.norm_bwd(dn1, sv["x"], p["norm1_w"], sv["st1"], dh1, g["norm1_w"], g.get("norm1_b"), ln, sums)
+            dn2 = self._mlp_bwd(dy, sv["n2"], ops, sv, None, later)
+            dh1 = ops.norm_bwd(dn2, sv["h1"], p["norm2_w"], sv["st2"], dy, g["norm2_w"], g.get("norm2_b"), ln, later)
+            dn1 = self._attn_bwd(dh1, sv["n1"], ctx, ops, sv, None, later)
+            dx = ops.norm_bwd(dn1, sv["x"], p["norm1_w"], sv["st1"], dh1, g["norm1_w"], g.get("norm1_b"), ln, later)
         else:
-            dr2 = ops.norm_bwd(dy, sv["r2"], p["norm2_w"], sv["st2"], None, g["norm2_w"], g.get("norm2_b"), ln, sums)
-            dh1 = self._mlp_bwd(dr2, sv["h1"], ops, sv, dr2, sums)
-            dr1 = ops.norm_bwd(dh1, sv["r1"], p["norm1_w"], sv["st1"], None, g["norm1_w"], g.get("norm1_b"), ln, sums)
-            dx = self._attn_bwd(dr1, sv["x"], ctx, ops, sv, dr1, sums)
-        ops.finish_sums(sums)
+            dr2 = ops.norm_bwd(dy, sv["r2"], p["norm2_w"], sv["st2"], None, g["norm2_w"], g.get("norm2_b"), ln, later)
+            dh1 = self._mlp_bwd(dr2, sv["h1"], ops, sv, dr2, later)
+            dr1 = ops.norm_bwd(dh1, sv["r1"], p["norm1_w"], sv["st1"], None, g["norm1_w"], g.get("norm1_b"), ln, later)
+            dx = self._attn_bwd(dr1, sv["x"], ctx, ops, sv, dr1, later)
+        ops.finish(later)
         return dx
 
     def flops_per_token(self, S):

@@ -34,19 +34,20 @@ class _MlpOps:
         return self.swiglu_bwd(pre, da) if act == "swiglu" else self.act_bwd(pre, da, act)
 
 
-class _SumOps:
-    """Column sums (bias gradients, norm gradients) of a layer's backward pass may be collected and done in one launch:
-    `sums = ops.new_sums()`, passed to `linear_wgrad` and `norm_bwd`, and `ops.finish_sums(sums)` at the end, before anything
-    else reads the gradients.  None, or ops that ignore it: each sum is done where it is asked for."""
+class _LaterOps:
+    """The weight gradients of a layer's backward pass, and the column sums behind its bias and norm gradients, may be
+    collected and done together at its end: `later = ops.collect()`, passed to `linear_wgrad` and `norm_bwd`, whose operands
+    it keeps alive, and `ops.finish(later)` before anything else reads the gradients.  None, or ops that ignore it: each is
+    done where it is asked for."""
 
-    def new_sums(self):
+    def collect(self):
         return None
 
-    def finish_sums(self, sums):
+    def finish(self, later):
         pass
 
 
-class RefOps(_MlpOps, _SumOps):
+class RefOps(_MlpOps, _LaterOps):
     name = "ref"
 
     # ---- linear -----------------------------------------------------------------
@@ -62,7 +63,7 @@ class RefOps(_MlpOps, _SumOps):
         dx = dy @ w
         return dx if addend is None else dx + addend
 
-    def linear_wgrad(self, dy, x, gw, gb=None, sums=None):
+    def linear_wgrad(self, dy, x, gw, gb=None, later=None):
         gw.add_((dy.float().t() @ x.float()).to(gw.dtype))
         if gb is not None:
             gb.add_(dy.float().sum(0).to(gb.dtype))
@@ -78,7 +79,7 @@ class RefOps(_MlpOps, _SumOps):
             y = y + b.float()
         return y.to(x.dtype), torch.stack([mean, rstd], dim=1)
 
-    def norm_bwd(self, dy, x, w, stats, dres, gw, gb, ln, sums=None):
+    def norm_bwd(self, dy, x, w, stats, dres, gw, gb, ln, later=None):
         xf, dyf = x.float(), dy.float()
         mean, rstd = stats[:, 0:1], stats[:, 1:2]
         xh = (xf - mean) * rstd
@@ -172,7 +173,7 @@ def _decline(*args):
     return None
 
 
-class Sm100Ops(_MlpOps, _SumOps):
+class Sm100Ops(_MlpOps, _LaterOps):
     """Hand-written sm_100a kernels only. Requires bf16 CUDA tensors.
 
     The calls a step makes for every layer and microbatch go to the native module first (`sm100._fast`, 3 - 5 us of host
@@ -192,7 +193,7 @@ class Sm100Ops(_MlpOps, _SumOps):
             self._linear_fwd = self._linear_dgrad = self._linear_wgrad = _decline
             self._act_linear_fwd = self._act_linear_dgrad = _decline
         default = fast is not None
-        self._column_sums = fast.column_sums if default else None
+        self._finish = fast.finish if default else None
         self._norm_fwd = fast.norm_fwd if default and sm100.NORM_FWD_VERSION == 1 else _decline
         self._norm_bwd = fast.norm_bwd if default and sm100.NORM_BWD_VERSION == 2 else _decline
         self._attn_fwd = fast.attn_fwd if default and sm100.ATTN_FWD_VERSION == 0 else _decline
@@ -222,9 +223,9 @@ class Sm100Ops(_MlpOps, _SumOps):
             self.k.gemm(dy, w, dx, b_mn=True, addend=addend)
         return dx
 
-    def linear_wgrad(self, dy, x, gw, gb=None, sums=None):
+    def linear_wgrad(self, dy, x, gw, gb=None, later=None):
         # gw[N,K] += dy^T[N,T] @ x[T,K]: both operands contiguous along the non-reduced dim
-        if self._linear_wgrad(dy, x, gw, gb, sums) is None:
+        if self._linear_wgrad(dy, x, gw, gb, later) is None:
             self.k.gemm(dy, x, gw, a_mn=True, b_mn=True, accumulate=True)
             if gb is not None:
                 self.k.colsum_accumulate(dy, gb)
@@ -241,15 +242,15 @@ class Sm100Ops(_MlpOps, _SumOps):
         r = self._norm_fwd(x, w, b, eps, ln)
         return self.k.norm_fwd(x, w, b, eps, ln) if r is None else r
 
-    def new_sums(self):
-        return [] if self._column_sums is not None else None
+    def collect(self):
+        return [] if self._finish is not None else None
 
-    def finish_sums(self, sums):
-        if sums:
-            self._column_sums(sums)
+    def finish(self, later):
+        if later:
+            self._finish(later)
 
-    def norm_bwd(self, dy, x, w, stats, dres, gw, gb, ln, sums=None):
-        dx = self._norm_bwd(dy, x, w, stats, dres, gw, gb, ln, sums)
+    def norm_bwd(self, dy, x, w, stats, dres, gw, gb, ln, later=None):
+        dx = self._norm_bwd(dy, x, w, stats, dres, gw, gb, ln, later)
         return self.k.norm_bwd(dy, x, w, stats, dres, gw, gb, ln) if dx is None else dx
 
     def rope_table(self, S, d, theta, device):

@@ -102,7 +102,7 @@ class DeferredWgrad:
 
     def linear_wgrad(self, *a, **k):
         if self.active:
-            k.pop("sums", None)      # the layer finishes its sums before the queue is flushed
+            k.pop("later", None)      # the layer finishes its own list before the queue is flushed
             self._queue.append((a, k))
         else:
             self._ops.linear_wgrad(*a, **k)
