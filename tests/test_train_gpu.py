@@ -182,3 +182,39 @@ def test_smoke_entry():
     import __graft_entry__ as g
 
     g.smoke()
+
+
+@pytest.mark.parametrize("buffers", [1, 5])
+def test_backward_shards_come_from_the_masters(buffers, monkeypatch):
+    """A parked unit that is fetched again for its backward pass gets its bf16 shard from the landed fp32 master: the same
+    bits as the parked copy's (both are the master rounded to nearest), so the losses are those of a run that fetches every
+    shard, and the bf16 copies cross the link once.  With one landing buffer, which the unit above holds, they
+    are fetched as before."""
+    from zorse_b200.engine.zero import MasterLanding, ZeroUnit
+    from zorse_b200.trainer import Trainer, TrainerOptions
+
+    def run(from_master):
+        with monkeypatch.context() as m:
+            m.setattr(MasterLanding, "BUFFERS", buffers)
+            if not from_master:
+                m.setattr(ZeroUnit, "_shard_from_master", lambda self: False)
+            tr = Trainer(_cfg(gbs=4, mbs=2), TrainerOptions(schedule="layer_major", ops="sm100", optimizer_in_backward=True,
+                                                            offload_model_params=True))
+            batch = tr.synthetic_batch()
+            counters = tr.stages[0].engine.counters
+            losses = [tr.train_step_from_host(batch) for _ in range(3)]
+            before = counters.h2d_bytes
+            losses.append(tr.train_step_from_host(batch))
+            units = tr.stages[0].engine.units
+            tr.check_kernels()
+            torch.cuda.synchronize()
+            for u in units:
+                assert u.master_slot is None
+                assert torch.equal(u.host_p, u.host_master.to(torch.bfloat16))
+            return losses, counters.h2d_bytes - before, [u.host_p.numel() for u in units]
+
+    losses, moved, n = run(True)
+    want, every, _ = run(False)
+    assert losses == pytest.approx(want, rel=1e-3), (losses, want)
+    assert every == sum(n) * 6 + sum(n[:-1]) * 2             # every master and shard, all shards but the head's again
+    assert moved == every - (2 * sum(n[:-1]) if buffers == 5 else 0)

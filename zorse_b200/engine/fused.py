@@ -126,7 +126,7 @@ class FusedZeroUnit(ZeroUnit):
         dist.barrier(group=pg)
 
     # ------------------------------------------------------------------ parameters
-    def prefetch(self):
+    def prefetch(self, update_next: bool = False):
         return  # the gather rides on the unit's first GEMM
 
     def acquire(self) -> None:

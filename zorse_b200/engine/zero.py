@@ -135,16 +135,16 @@ class Streams:
 
 
 class MasterLanding:
-    """Device buffers in which parked fp32 masters land on their way to an optimizer inside the backward pass: three, of the
+    """Device buffers in which parked fp32 masters land on their way to an optimizer inside the backward pass: five, of the
     largest unit's size, kept for the life of the stage.  A buffer is taken when a copy into it is issued and given back
     with the event behind its last use, which the next copy into it waits for.  (A block per fetch from the caching
     allocator crosses streams and cannot be handed out again before the GPU has passed that point, while the host runs a
-    whole backward pass ahead: every master became resident.)  With two buffers the copy stream, which also brings the bf16
-    shards, waits for a write-back too often: OPT 125M step 41.1 ms against 39.7; a stream of their own lets the masters
-    take link bandwidth from the shards: 42.7; no copy ahead of the optimizer: 44.1.
+    whole backward pass ahead: every master became resident.)  With few buffers the copies to the GPU, which also bring what
+    the backward pass computes on, wait for write-backs: OPT 125M step 32.9 ms with three, 31.4 with four, 30.8 with five;
+    six and eight gain nothing more.  A stream of their own lets the masters take link bandwidth from the shards.
     `p16` takes the bf16 image of an update on its way to the host; only the communication stream touches it.  Nothing is
     then left for the first step of a stage to allocate there (two allocations while the GPU is busy, 1 to 60 ms each)."""
-    BUFFERS = 3
+    BUFFERS = 5
 
     def __init__(self, device: torch.device, streams: Streams, n: int, compute_dtype: torch.dtype):
         self.stream = streams.copy
@@ -242,9 +242,11 @@ class ZeroUnit:
         self.master = None
         self.p_shard = None
 
-    def _fetch_shard(self):
+    def _fetch_shard(self, update_next: bool = False):
         """H2D of the bf16 shard on the copy stream; the comm stream waits for it."""
         if self.p_shard is not None or self.host_p is None:
+            return
+        if update_next and self._shard_from_master():
             return
         if self.cuda:
             self.p_shard = torch.empty(self.shard_n, dtype=self.cfg.compute_dtype, device=self.device)
@@ -256,6 +258,24 @@ class ZeroUnit:
         else:
             self.p_shard = self.host_p.clone()
         self.counters.h2d_bytes += self.host_p.numel() * self.host_p.element_size()
+
+    def _shard_from_master(self) -> bool:
+        """The shard for the one backward pass between here and the unit's update: rounded on the device from the fp32 master,
+        which the optimizer behind that pass needs anyway, so the bf16 copy does not cross the link a second time (a quarter
+        of what goes to the GPU per step: OPT 125M 40.0 ms without this and with three landing buffers, 33 with this).  Not for
+        a pass with others behind it: it would hold a landing buffer that an earlier update needs.  False without one."""
+        self._fetch_master()
+        if self.master_slot is None:
+            return False
+        self.p_shard = torch.empty(self.shard_n, dtype=self.cfg.compute_dtype, device=self.device)
+        stream = self.landing.stream
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            self.p_shard.copy_(self.landing.bufs[self.master_slot][:self.shard_n])
+        self.p_shard.record_stream(stream)
+        if self.R > 1:                 # (the gather; the communication stream has the updates' write-backs to do otherwise)
+            self.streams.comm.wait_stream(stream)
+        return True
 
     def _fetch_master(self):
         """Starts the H2D copy of the parked fp32 master for an optimizer inside the backward pass, ahead of the gradient
@@ -284,11 +304,12 @@ class ZeroUnit:
             self.master_slot = None
 
     # ------------------------------------------------------------------ parameters
-    def prefetch(self):
-        """Issues the all-gather (no-op if the unsharded buffer exists or is in flight)."""
+    def prefetch(self, update_next: bool = False):
+        """Issues the all-gather (no-op if the unsharded buffer exists or is in flight).  `update_next`: only one backward
+        pass lies between here and the unit's update."""
         if self.full is not None:
             return
-        self._fetch_shard()
+        self._fetch_shard(update_next)
         if self.R == 1:
             if self.cuda and self.host_p is not None:
                 ev = torch.cuda.Event()
@@ -364,6 +385,7 @@ class ZeroUnit:
     def grad_views(self) -> None:
         if self.grad is None:
             self.grad = torch.zeros(self.n, dtype=self.cfg.reduce_dtype, device=self.device)
+            self._fetch_master()       # of a unit that has kept its shard since the forward pass: it comes under the backward
         if self.cuda:
             SC.wrote(("grad", id(self)))   # backward kernels on the current stream accumulate into it
         self.layer.bind(self.full, self.grad)

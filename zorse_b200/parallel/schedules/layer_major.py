@@ -90,9 +90,9 @@ class LayerMajorSchedule(ScheduleBase):
         handles = {} if st.is_last else self._recv_all(st, st.recv_bwd, reversed(range(M)), recv_mode)
         for li in reversed(range(L)):
             units[li].acquire()
+            units[li].grad_views()      # (ahead of the next fetch: a parked unit's master is needed first)
             if li > 0:
-                units[li - 1].prefetch()
-            units[li].grad_views()
+                units[li - 1].prefetch(update_next=True)     # all its microbatches, then the update
             deferred = []
             for mbl in reversed(range(M)):
                 if li == L - 1:
