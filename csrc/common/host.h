@@ -63,19 +63,20 @@ inline int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, 
   return 0;
 }
 
-// 2-D output tensor (bf16 or fp32, row stride `ld` elements) read and written in boxes of 128 bytes x `box_rows` rows,
-// 128-byte swizzle.
+// 2-D output tensor (bf16 or fp32, row stride `ld` elements) read and written in boxes of `row_bytes` (128 or 64) x `box_rows`
+// rows, swizzled over `row_bytes`.
 inline int make_tmap_2d_out(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, bool f32,
-                            uint32_t box_rows) {
+                            uint32_t box_rows, uint32_t row_bytes = 128) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) ZB_FAIL(-3, "cuTensorMapEncodeTiled entry point not available");
   const uint64_t es = f32 ? 4 : 2;
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {ld * es};
-  cuuint32_t box[2] = {cuuint32_t(128 / es), box_rows};
+  cuuint32_t box[2] = {cuuint32_t(row_bytes / es), box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(out, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base),
-                  dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  row_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) ZB_FAIL(-5, "cuTensorMapEncodeTiled failed with %d", int(r));
   return 0;

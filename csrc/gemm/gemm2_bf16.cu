@@ -335,12 +335,22 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       const int buf = local & 1;
       const uint32_t use = uint32_t(local >> 1);
       if constexpr (FE != FE_NONE) {
-        // ---- activation in the epilogue: groups of 64 columns, each one to three boxes ----
+        // ---- activation or rotation in the epilogue: groups of 64 columns, each one to three boxes ----
         constexpr int COLS = FE == FE_GLU_FWD ? HALF_N : BN;
+        // FE_ROPE: a group is 32 pairs of columns, half a head's width apart: a head of 64, or half of one of 128 (two boxes of
+        // 32 columns).  The cosines and sines of a thread's row for them stay in its registers: those of a head of 64 for all
+        // heads of the tile; the halves of wider heads go to the two warps of the rows, or come one after the other where
+        // there is one.
+        const int head = FE == FE_ROPE ? p.act : 64, halves = FE == FE_ROPE ? head / 64 : 1;
+        const bool half_each = FE == FE_ROPE && EP_GROUPS == 2 && halves == 2;
         constexpr int LOADS = FE == FE_ACT_BWD ? 1 : FE == FE_GLU_BWD ? 2 : 0;
         const int row0 = m0 + q * 32, c0 = tn * COLS;
-        const int groups = mine(row0 < p.M ? min(COLS / 64, (p.N - c0 + 63) / 64) : 0);
-        auto col_of = [&](int g) { return c0 + (h + g * EP_GROUPS) * 64; };
+        const int heads = row0 < p.M ? min(COLS / head, (p.N - c0 + head - 1) / head) : 0;
+        const int groups = mine(heads * halves);
+        auto half_of = [&](int g) { return halves == 1 ? 0 : half_each ? h : int(g >= heads); };
+        auto col_of = [&](int g) {
+          return halves == 1 ? c0 + (h + g * EP_GROUPS) * 64 : c0 + (half_each || g < heads ? g : g - heads) * 128 + half_of(g) * 32;
+        };
         const int per_group = LOADS > 0 ? LOADS : p.keep ? (FE == FE_GLU_FWD ? 3 : 2) : 1;
         auto box_of = [&](uint32_t k) { return my_boxes + (k & slot_mask) * Cfg::EP_BYTES; };
         auto load_group = [&](int g) {   // the pre-activations of group g (lane 0)
@@ -359,6 +369,21 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           bulk_wait_read<0>();
           for (int g = 0; g < DEPTH && g < groups; ++g) load_group(g);
         }
+        [[maybe_unused]] float co[FE == FE_ROPE ? 32 : 1], si[FE == FE_ROPE ? 32 : 1];
+        [[maybe_unused]] auto load_angles = [&](int c) {
+          if constexpr (FE == FE_ROPE) {
+            const float4* at = reinterpret_cast<const float4*>(p.cs + size_t((row0 + lane) % p.S) * head + 32 * c);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const uint4 a = ld_v4(at + j), b = ld_v4(at + (head >> 3) + j);
+              co[4 * j] = __uint_as_float(a.x); co[4 * j + 1] = __uint_as_float(a.y);
+              co[4 * j + 2] = __uint_as_float(a.z); co[4 * j + 3] = __uint_as_float(a.w);
+              si[4 * j] = __uint_as_float(b.x); si[4 * j + 1] = __uint_as_float(b.y);
+              si[4 * j + 2] = __uint_as_float(b.z); si[4 * j + 3] = __uint_as_float(b.w);
+            }
+          }
+        };
+        if (FE == FE_ROPE && groups > 0 && c0 < p.rope_cols) load_angles(half_of(0));   // under the main loop
         if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full[buf], use & 1, wctx, ST_TIMEOUT_TMEM_FULL))) break;
         tc_fence_after();
         auto release_tmem = [&] {
@@ -377,7 +402,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           const uint32_t t_addr = tmem_base + (uint32_t(q * 32) << 16) + uint32_t(buf * BN + col - c0);
           uint32_t r[32], s[32];
           tmem_ld32(t_addr, r);
-          tmem_ld32(t_addr + (FE == FE_GLU_FWD ? uint32_t(HALF_N) : 32u), s);
+          tmem_ld32(t_addr + (FE == FE_GLU_FWD ? uint32_t(HALF_N) : FE == FE_ROPE ? uint32_t(head >> 1) : 32u), s);
           if (lane == 0) {
             if (LOADS > 0) {
               if (g > 0 && g - 1 + DEPTH < groups) {   // the boxes of group g - 1 take the loads of group g - 1 + DEPTH
@@ -391,7 +416,56 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             }
           }
           tmem_wait_ld();
-          if constexpr (FE == FE_GLU_FWD) {
+          if constexpr (FE == FE_ROPE) {
+            const int far = head >> 1;   // from a column to the other of its pair
+            if (halves == 2 && !half_each && g == heads && c0 < p.rope_cols) load_angles(1);
+            if (g == groups - 1) release_tmem();
+            else __syncwarp();
+            bias.add(p, col - c0, r);
+            bias.add(p, col - c0 + far, s);
+            // the values as they would be stored, like a pass over them sees them
+            uint4 x[4], y[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              x[j] = pack_f32x8(r, 8 * j);
+              y[j] = pack_f32x8(s, 8 * j);
+              if (col < p.rope_cols) {
+                uint32_t xs[4] = {x[j].x, x[j].y, x[j].z, x[j].w}, ys[4] = {y[j].x, y[j].y, y[j].z, y[j].w};
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                  const float2 a = unpack_bf16x2(xs[u]), b = unpack_bf16x2(ys[u]);
+                  const int i = 8 * j + 2 * u;
+                  xs[u] = pack_bf16x2(a.x * co[i] - b.x * si[i], a.y * co[i + 1] - b.y * si[i + 1]);
+                  ys[u] = pack_bf16x2(b.x * co[i] + a.x * si[i], b.y * co[i + 1] + a.y * si[i + 1]);
+                }
+                x[j] = make_uint4(xs[0], xs[1], xs[2], xs[3]);
+                y[j] = make_uint4(ys[0], ys[1], ys[2], ys[3]);
+              }
+            }
+            if (halves == 1) {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                st_shared_v4(box0 + ((uint32_t(j) ^ sw) << 4), x[j].x, x[j].y, x[j].z, x[j].w);
+                st_shared_v4(box0 + ((uint32_t(4 + j) ^ sw) << 4), y[j].x, y[j].y, y[j].z, y[j].w);
+              }
+            } else {   // two boxes of 32 rows of 64 bytes, their 16-byte pieces swizzled by two bits of the row
+              const uint32_t at = smem_u32(box_of(k)) + uint32_t(lane) * 64, sw2 = uint32_t(lane >> 1) & 3;
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                st_shared_v4(at + ((uint32_t(j) ^ sw2) << 4), x[j].x, x[j].y, x[j].z, x[j].w);
+                st_shared_v4(at + uint32_t(Cfg::EP_BYTES / 2) + ((uint32_t(j) ^ sw2) << 4), y[j].x, y[j].y, y[j].z, y[j].w);
+              }
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (zb_in_bounds(row0 >= 0 && row0 < p.M && col >= 0 && col + far < p.N, p.status, 2)) {
+                tma_store_2d(&tmap_w, box_of(k), col, row0);
+                if (halves == 2) tma_store_2d(&tmap_w, box_of(k) + Cfg::EP_BYTES / 2, col + far, row0);
+              }
+              bulk_commit();
+            }
+          } else if constexpr (FE == FE_GLU_FWD) {
             uint4 a[8];
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
@@ -962,17 +1036,20 @@ static int make_tmap_halves(CUtensorMap* out, const void* base, uint64_t rows, u
 
 // Products with an activation in the epilogue.  FE_ACT_FWD: act(A B^T + bias) -> out, A B^T + bias -> pre.  FE_GLU_FWD: the
 // same for a gated unit (B: gate and up weights, N = F).  FE_ACT_BWD / FE_GLU_BWD: (A B) times the activation's derivative
-// at `pre` -> out.  All matrices but A and B are dense.
+// at `pre` -> out.  FE_ROPE: A B^T + bias with its first heads rotated -> out.  All matrices but A and B are dense.
 //
 // As passes of their own the activations read and write everything once more (4096 x 11008, gated: 47 us forward, 79
 // backward) and cost a launch each; here the forward one works on accumulators, and the backward one fetches only what it
 // needs, under the main loop of the next tile.
+// The rotation, one more pass over the projection, has both halves of its pairs in the accumulators.  As two calls, as one, and
+// the product alone: 8192 x 2560 x 2048, heads of 64, 69.1, 59.9 and 59.1 us; 3000 x 3072 x 1024, heads of 128, 23.0, 19.0
+// and 19.8; 1024 x 1536 x 512 8.3, 6.5 and 5.5.
 template <int FE, int BN>
 static int launch_gemm2_fused(const void* A, const void* B, void* pre, void* out, const GemmFusedParams<FE>& p, int lda, int ldb,
                               cudaStream_t stream) {
   using Cfg = Gemm2Cfg<BN>;
   using Params = GemmFusedParams<FE>;
-  constexpr bool FWD = FE == FE_ACT_FWD || FE == FE_GLU_FWD, GLU = FE == FE_GLU_FWD || FE == FE_GLU_BWD;
+  constexpr bool FWD = FE == FE_ACT_FWD || FE == FE_GLU_FWD || FE == FE_ROPE, GLU = FE == FE_GLU_FWD || FE == FE_GLU_BWD;
   const int cols = FE == FE_GLU_FWD ? 2 * p.N : p.N;   // of the accumulators
   int pairs = num_sms() / 2;
   if (BN == 256 && gemm2_plan(p.M, cols, p.K, pairs, false).bn == 128)
@@ -987,7 +1064,7 @@ static int launch_gemm2_fused(const void* A, const void* B, void* pre, void* out
   else rc = make_tmap_2d_bf16(&tb, B, p.K, p.N, ldb, 64, 64);
   if (rc) return rc;
   if (FWD) {
-    if ((rc = make_tmap_2d_out(&tw, out, p.M, p.N, p.N, false, 32))) return rc;
+    if ((rc = make_tmap_2d_out(&tw, out, p.M, p.N, p.N, false, 32, FE == FE_ROPE && p.act == 128 ? 64 : 128))) return rc;
     if (p.keep) {
       rc = GLU ? make_tmap_halves(&tc, pre, p.M, p.N) : make_tmap_2d_out(&tc, pre, p.M, p.N, p.N, false, 32);
       if (rc) return rc;
@@ -1016,7 +1093,8 @@ static int launch_gemm2_fused(const void* A, const void* B, void* pre, void* out
 
 template <int FE>
 static int gemm2_fused_entry(const void* A, const void* B, const void* bias, void* pre, void* out, int M, int N, int K, int lda,
-                             int ldb, int act, int keep, int* status, cudaStream_t stream) {
+                             int ldb, int act, int keep, int* status, cudaStream_t stream, const float* cs = nullptr, int S = 0,
+                             int rope_cols = 0) {
   GemmFusedParams<FE> p = {};
   p.C = out;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
@@ -1025,6 +1103,9 @@ static int gemm2_fused_entry(const void* A, const void* B, const void* bias, voi
   p.status = status;
   p.act = act;
   p.keep = keep;
+  p.cs = cs;
+  p.S = S;
+  p.rope_cols = rope_cols;
   return launch_gemm2_fused<FE, 256>(A, B, pre, out, p, lda, ldb, stream);
 }
 
@@ -1086,6 +1167,19 @@ extern "C" int zb_gemm2_act_fwd(const void* x, const void* w, const void* bias, 
     return 1;
   if (act == 3) return gemm2_fused_entry<FE_GLU_FWD>(x, w, nullptr, pre, out, M, N, K, lda, ldb, 0, pre != nullptr, status, stream);
   return gemm2_fused_entry<FE_ACT_FWD>(x, w, bias, pre, out, M, N, K, lda, ldb, act, pre != nullptr, status, stream);
+}
+// Projection to query, key and value heads with the rotation of the first `heads` (rotate-half within each head of d columns;
+// row m is position m % S of cs, [S, d] fp32 cosines | sines): out = rope(x w^T + bias), [M, N] dense.  Returns 1, with nothing
+// done, where it is not for this kernel: as zb_gemm2_act_fwd, heads of other widths than 64 and 128, and columns that are no
+// whole heads.  Products whose last wave the plain kernel cuts into parts are taken too: 2048 x 12288 x 4096 is 133 us cut and 14
+// for the pass, 147 as here.
+extern "C" int zb_gemm2_rope_fwd(const void* x, const void* w, const void* bias, const float* cs, void* out, int M, int N, int K,
+                                 int lda, int ldb, int S, int heads, int d, int* status, cudaStream_t stream) {
+  using namespace zb;
+  if (M < 256 || N < 256 || K <= 0 || (d != 64 && d != 128) || N % d || S <= 0 || heads <= 0 || heads > N / d ||
+      ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(cs)) & 15))
+    return 1;
+  return gemm2_fused_entry<FE_ROPE>(x, w, bias, nullptr, out, M, N, K, lda, ldb, d, 0, status, stream, cs, S, heads * d);
 }
 // Gradient of the pre-activations: dpre = (dy w) act'(pre), w [K, N] (K: columns of dy); act 3: pre and dpre [M, 2N].
 // Returns 1 as zb_gemm2_act_fwd.

@@ -72,13 +72,16 @@ struct GemmAgParams : GemmParams {
 };
 
 
-// Activation of an MLP in the epilogue (csrc/gemm/gemm2_bf16.cu): which one decides how the accumulators are used.
-enum : int { FE_NONE = 0, FE_ACT_FWD = 1, FE_GLU_FWD = 2, FE_ACT_BWD = 3, FE_GLU_BWD = 4 };
+// Activation of an MLP, or rotation of query and key heads, in the epilogue (csrc/gemm/gemm2_bf16.cu): which one decides how
+// the accumulators are used.
+enum : int { FE_NONE = 0, FE_ACT_FWD = 1, FE_GLU_FWD = 2, FE_ACT_BWD = 3, FE_GLU_BWD = 4, FE_ROPE = 5 };
 template <int FE_>
 struct GemmFusedParams : GemmParams {
   static constexpr int FE = FE_;
-  int act;    // FE_ACT_*: kind as in act_fwd / act_bwd
+  int act;    // FE_ACT_*: kind as in act_fwd / act_bwd; FE_ROPE: width of a head, 64 or 128
   int keep;   // forward: store the pre-activation too (the backward pass will need it)
+  const float* cs;     // FE_ROPE: [S, head] cosines | sines of a position; row m of the product is position m % S
+  int S, rope_cols;    // FE_ROPE: the columns ahead of rope_cols are rotated
 };
 template <typename P>
 struct FusedEp { static constexpr int value = FE_NONE; };

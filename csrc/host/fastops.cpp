@@ -50,6 +50,8 @@ struct Entry {
   int (*flash_stats_floats)(int, int, int);
   int (*gemm2_act_fwd)(const void*, const void*, const void*, void*, void*, int, int, int, int, int, int, int*, cudaStream_t);
   int (*gemm2_act_bwd)(const void*, const void*, const void*, void*, int, int, int, int, int, int, int*, cudaStream_t);
+  int (*gemm2_rope_fwd)(const void*, const void*, const void*, const float*, void*, int, int, int, int, int, int, int, int, int*,
+                        cudaStream_t);
   int (*column_sums)(const long*, int, int, cudaStream_t);
   const char* (*last_error)();
 };
@@ -262,6 +264,33 @@ PyObject* act_linear_fwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(std::move(out)));
   PyTuple_SET_ITEM(r, 1, pp != nullptr ? THPVariable_Wrap(std::move(pre)) : Py_NewRef(Py_None));
   return r;
+  END_HANDLE_TH_ERRORS
+}
+
+// linear_rope_fwd(x, w, bias | None, cs, S, heads, d) -> x w^T + bias with its first `heads` heads rotated
+PyObject* linear_rope_fwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  ZB_ARGS(7)
+  const Tensor *x = tensor_of(args[0]), *w = tensor_of(args[1]), *bias, *cs = tensor_of(args[3]);
+  int64_t S, heads, d;
+  if (!optional_tensor(args[2], bias) || !matrix(x, BF16) || !matrix(w, BF16) || !dense(cs, F32) || !int_arg(args[4], S) ||
+      !int_arg(args[5], heads) || !int_arg(args[6], d) || !on(w, *x) || !on(bias, *x) || !on(cs, *x))
+    Py_RETURN_NONE;
+  const int64_t M = x->size(0), K = x->size(1), N = w->size(0);
+  int* status = status_of(*x);
+  if (status == nullptr || w->size(1) != K || !fits(M) || !fits(N) || !fits(K) || !fits(x->stride(0)) || !fits(w->stride(0)) ||
+      !fits(S) || M < 256 || N < 256 || (d != 64 && d != 128) || N % d || S <= 0 || heads <= 0 || heads > N / d ||
+      cs->dim() != 2 || cs->size(0) < S || cs->size(1) != d || (reinterpret_cast<uintptr_t>(ptr(cs)) & 15))
+    Py_RETURN_NONE;
+  if (bias != nullptr && !(dense(bias, BF16) && bias->dim() == 1 && bias->size(0) == N)) Py_RETURN_NONE;
+  Tensor out = empty({M, N}, *x, BF16);
+  const cudaStream_t s = stream();
+  if (!launch("gemm2_rope_fwd", 1, [&] {
+        return lib.gemm2_rope_fwd(ptr(x), ptr(w), ptr(bias), static_cast<const float*>(ptr(cs)), out.data_ptr(), int(M), int(N),
+                                  int(K), int(x->stride(0)), int(w->stride(0)), int(S), int(heads), int(d), status, s);
+      }))
+    return nullptr;
+  return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }
 
@@ -617,7 +646,8 @@ PyObject* launch_count(PyObject*, PyObject* const*, Py_ssize_t) { return PyLong_
 
 #define ZB_FN(f) {#f, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(f)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {ZB_FN(init), ZB_FN(set_status), ZB_FN(launch_count), ZB_FN(linear_fwd), ZB_FN(linear_dgrad),
-                         ZB_FN(linear_wgrad), ZB_FN(act_linear_fwd), ZB_FN(act_linear_dgrad), ZB_FN(norm_fwd), ZB_FN(norm_bwd), ZB_FN(finish), ZB_FN(rope), ZB_FN(swiglu_fwd),
+                         ZB_FN(linear_wgrad), ZB_FN(act_linear_fwd), ZB_FN(act_linear_dgrad), ZB_FN(linear_rope_fwd),
+                         ZB_FN(norm_fwd), ZB_FN(norm_bwd), ZB_FN(finish), ZB_FN(rope), ZB_FN(swiglu_fwd),
                          ZB_FN(swiglu_bwd), ZB_FN(act_fwd), ZB_FN(act_bwd), ZB_FN(attn_fwd), ZB_FN(attn_bwd),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "zorse_fastops", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -315,6 +315,47 @@ def test_activation_products_that_are_not_for_the_epilogue(ops):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("T,K,S", [(256, 256, 256), (301, 520, 43), (1030, 2048, 515), (2500, 768, 2500), (4104, 2056, 1026)])
+@pytest.mark.parametrize("Hq,Hkv,d,bias", [(4, 4, 64, False), (5, 1, 64, True), (2, 1, 128, True), (9, 3, 128, False)])
+def test_rotation_in_the_epilogue(ops, T, K, S, Hq, Hkv, d, bias):
+    """Ragged rows and columns, rows that start again at position 0 inside a tile, value heads that stay as they are, both tile
+    widths and both splits of shared memory.  The product is rounded ahead of the rotation, as the pass it stands for finds it:
+    against that pass one flip of the second rounding (2^-7, or 2^-22 of the pair where its terms cancel); against 64 bits 2^-8
+    of either of a pair, then 2^-8 of the result."""
+    x, w = _rand(T, K, seed=1), (_rand((Hq + 2 * Hkv) * d, K, seed=2).float() / K ** 0.5).bfloat16()
+    b = _rand((Hq + 2 * Hkv) * d, seed=3) if bias else None
+    cs = ops.rope_table(S, d, 1e4, "cuda")
+    got = k._fast.linear_rope_fwd(x, w, b, cs, S, Hq + Hkv, d)
+    y = x.double() @ w.double().t() + (0 if b is None else b.double())
+    c, sn = cs.double()[torch.arange(T, device="cuda") % S].view(T, 1, 2, d // 2).unbind(2)
+    heads = y.view(T, -1, 2, d // 2)
+    lo, hi = heads[:, :Hq + Hkv].unbind(2)
+    rot = torch.stack((lo * c - hi * sn, hi * c + lo * sn), 2)
+    want = torch.cat((rot, heads[:, Hq + Hkv:]), 1).reshape(T, -1)
+    pair = heads.abs().sum(2, keepdim=True).expand(-1, -1, 2, -1).reshape(T, -1)
+    two = ops.rope_(ops.linear_fwd(x, w, b), cs, S, Hq + Hkv, d)
+    assert ((got.double() - two.double()).abs() <= 2.0 ** -7 * two.double().abs() + 2.0 ** -22 * pair).all()
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * 1.01 * (want.abs() + pair)).all()
+    assert torch.equal(got.view(T, -1, d)[:, Hq + Hkv:], two.view(T, -1, d)[:, Hq + Hkv:])
+    k.check_status()
+
+
+@pytest.mark.gpu
+def test_projections_whose_rotation_stays_a_pass(ops):
+    """Few rows, heads of other widths, columns that are no whole heads, more heads than columns, a table for other heads or
+    too few positions: declined; where the two calls take it, they give the result."""
+    x, w = _rand(300, 512), _rand(512, 512, seed=2)
+    cs = {d: ops.rope_table(300, d, 1e4, "cuda") for d in (32, 64, 128)}
+    f = k._fast.linear_rope_fwd
+    assert f(x[:255], w, None, cs[64], 300, 8, 64) is None and f(x, w[:248], None, cs[64], 300, 2, 64) is None
+    assert f(x, w, None, cs[32], 300, 8, 32) is None and f(x, w, None, cs[64], 300, 9, 64) is None
+    assert f(x, w[:320], None, cs[128], 300, 2, 128) is None
+    assert f(x, w, None, cs[128], 300, 8, 64) is None and f(x, w, None, cs[64], 301, 8, 64) is None
+    assert f(x, w, None, cs[64].bfloat16(), 300, 8, 64) is None
+    assert torch.equal(ops.linear_rope_fwd(x, w, None, cs[32], 300, 8, 32), ops.rope_(ops.linear_fwd(x, w), cs[32], 300, 8, 32))
+
+
+@pytest.mark.gpu
 def test_gelu_erf_over_all_arguments(ops):
     """Every bf16 argument against 64 bits.  In fp32 the value is off by a few 2^-24 of itself (the tail is never a difference
     of larger numbers; the derivative has a zero near -0.75 and is off by a few 2^-24 there), so what is left is the rounding

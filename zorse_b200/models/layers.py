@@ -167,13 +167,15 @@ class TransformerBlock(Layer):
     def _attn_fwd(self, xin, resid, ctx, ops, sv):
         p, B, S = self.p, ctx["B"], ctx["S"]
         ag = self.__dict__.pop("_ag", None)  # left by a fused ZeRO unit: gather the unit inside this GEMM
+        cs = self._rope(ops, S, xin.device)
         if ag is not None:
             qkv = ops.linear_fwd_gather(xin, "qkv_w", ag, p.get("qkv_b"))
+            if cs is not None:
+                ops.rope_(qkv, cs, S, self.Hq + self.Hkv, self.D)
+        elif cs is not None:
+            qkv = ops.linear_rope_fwd(xin, p["qkv_w"], p.get("qkv_b"), cs, S, self.Hq + self.Hkv, self.D)
         else:
             qkv = ops.linear_fwd(xin, p["qkv_w"], p.get("qkv_b"))
-        cs = self._rope(ops, S, xin.device)
-        if cs is not None:
-            ops.rope_(qkv, cs, S, self.Hq + self.Hkv, self.D)
         att, lse = ops.attn_fwd(qkv, B, S, self.Hq, self.Hkv, self.D, self.causal, self.window)
         out = ops.linear_fwd(att, p["o_w"], p.get("o_b"), addend=resid)
         if sv is not None:

@@ -19,8 +19,9 @@ _ACT_KINDS = {"gelu": 0, "gelu_new": 0, "gelu_tanh": 0, "relu": 1, "gelu_erf": 2
 _FUSED_ACT_KINDS = {**_ACT_KINDS, "swiglu": 3}   # of the products with an activation in their epilogue
 
 
-class _MlpOps:
-    """The two products of an MLP that have its activation beside them, for ops that have no single kernel for a call.
+class _EpilogueOps:
+    """Products with something elementwise beside them, as two calls, for ops that have no single kernel for a call: of an MLP
+    with its activation, of attention's input projection with the rotation.
     `act`: "swiglu" (w holds the gate's rows, then the up projection's) or a name of `act_fwd`."""
 
     def act_linear_fwd(self, x, w, bias, act, keep):
@@ -32,6 +33,10 @@ class _MlpOps:
         """(dy w) times the derivative of the activation at `pre`."""
         da = self.linear_dgrad(dy, w)
         return self.swiglu_bwd(pre, da) if act == "swiglu" else self.act_bwd(pre, da, act)
+
+    def linear_rope_fwd(self, x, w, bias, cs, S, nheads, d):
+        """x w^T + bias with its first `nheads` heads of d columns rotated (`rope_`)."""
+        return self.rope_(self.linear_fwd(x, w, bias), cs, S, nheads, d)
 
 
 class _LaterOps:
@@ -47,7 +52,7 @@ class _LaterOps:
         pass
 
 
-class RefOps(_MlpOps, _LaterOps):
+class RefOps(_EpilogueOps, _LaterOps):
     name = "ref"
 
     # ---- linear -----------------------------------------------------------------
@@ -173,7 +178,7 @@ def _decline(*args):
     return None
 
 
-class Sm100Ops(_MlpOps, _LaterOps):
+class Sm100Ops(_EpilogueOps, _LaterOps):
     """Hand-written sm_100a kernels only. Requires bf16 CUDA tensors.
 
     The calls a step makes for every layer and microbatch go to the native module first (`sm100._fast`, 3 - 5 us of host
@@ -189,9 +194,10 @@ class Sm100Ops(_MlpOps, _LaterOps):
         if fast is not None and sm100.GEMM_KERNEL == "2cta":
             self._linear_fwd, self._linear_dgrad, self._linear_wgrad = fast.linear_fwd, fast.linear_dgrad, fast.linear_wgrad
             self._act_linear_fwd, self._act_linear_dgrad = fast.act_linear_fwd, fast.act_linear_dgrad
+            self._linear_rope_fwd = fast.linear_rope_fwd
         else:
             self._linear_fwd = self._linear_dgrad = self._linear_wgrad = _decline
-            self._act_linear_fwd = self._act_linear_dgrad = _decline
+            self._act_linear_fwd = self._act_linear_dgrad = self._linear_rope_fwd = _decline
         default = fast is not None
         self._finish = fast.finish if default else None
         self._norm_fwd = fast.norm_fwd if default and sm100.NORM_FWD_VERSION == 1 else _decline
@@ -237,6 +243,10 @@ class Sm100Ops(_MlpOps, _LaterOps):
     def act_linear_dgrad(self, dy, w, pre, act):
         r = self._act_linear_dgrad(dy, w, pre, _FUSED_ACT_KINDS[act])
         return super().act_linear_dgrad(dy, w, pre, act) if r is None else r
+
+    def linear_rope_fwd(self, x, w, bias, cs, S, nheads, d):
+        y = self._linear_rope_fwd(x, w, bias, cs, S, nheads, d)
+        return super().linear_rope_fwd(x, w, bias, cs, S, nheads, d) if y is None else y
 
     def norm_fwd(self, x, w, b, eps, ln):
         r = self._norm_fwd(x, w, b, eps, ln)

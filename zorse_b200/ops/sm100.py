@@ -89,7 +89,7 @@ _fast = None
 _FAST_ENTRIES = ("zb_gemm_bf16", "zb_gemm2_bf16", "zb_gemm2_split_bf16", "zb_gemm2_workspace", "zb_norm_fwd", "zb_norm_bwd2",
                  "zb_norm_bwd2_rows", "zb_colsum", "zb_rope", "zb_swiglu_fwd", "zb_swiglu_bwd", "zb_act_fwd", "zb_act_bwd",
                  "zb_flash_fwd4", "zb_flash_bwd3", "zb_flash_bwd2_stats_floats", "zb_gemm2_act_fwd",
-                 "zb_gemm2_act_bwd", "zb_column_sums", "zb_last_error")   # the order of its `Entry`
+                 "zb_gemm2_act_bwd", "zb_gemm2_rope_fwd", "zb_column_sums", "zb_last_error")   # the order of its `Entry`
 
 
 def _load_fast() -> None:
