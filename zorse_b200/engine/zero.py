@@ -331,6 +331,8 @@ class ZeroUnit:
                 ev = torch.cuda.Event()
                 ev.record(self.streams.comm)
             full.record_stream(self.streams.comm)
+            if self.host_p is not None:
+                self.p_shard.record_stream(self.streams.comm)   # (let go below, while the gather may still read it)
             self.full_event = ev
         else:
             self._gather_into(full, self.p_shard)
