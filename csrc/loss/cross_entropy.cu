@@ -2,21 +2,63 @@
 //   loss[t]    = logsumexp(logits[t, :]) - logits[t, target[t]]
 //   dlogits    = (softmax(logits[t, :]) - onehot(target[t])) * grad_scale      (bf16)
 // One CTA per row; the row is read twice (the second read hits L2) and the gradient is
-// written once, in place if dlogits == logits.  Replaces F.cross_entropy + its autograd
-// (reference call site zorse_utils/pipeline_schedule_v2.py:182-184).
+// written once, in place if dlogits == logits.
+//
+// Two exponentials per logit: the exponential unit takes 117 us of the 160 that memory takes for 2048 x 128256, so what else is
+// done per logit has to stay small (packed differences and maxima) and several loads in flight.  With scalars and one load
+// at a time, and now: 2048 x 128256 265 -> 209 us, 4096 x 32000 111 -> 94, 3072 x 30528 86 -> 71, 1018 x 49152 46 -> 39, 256 x
+// 32000 13.7 -> 9.4.  The sums run in the order of the columns a thread has, one after the other: same results as then.
 #include "../common/host.h"
 #include "../common/ptx.cuh"
 
 namespace zb {
 
-constexpr int CE_THREADS = 512;
+constexpr int CE_THREADS = 512, CE_UNROLL = 4;   // 16-byte pieces of a thread in flight
 
-__device__ __forceinline__ void ce_unpack8(const uint4& u, float* f) {
-  float2 a = unpack_bf16x2(u.x), b = unpack_bf16x2(u.y), c = unpack_bf16x2(u.z), d = unpack_bf16x2(u.w);
-  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+// e^(x - m) of two values: the difference, then times log2(e), as __expf forms it
+__device__ __forceinline__ float2 ce_exp2(float2 x, float m) {
+  float a, b;
+  ffma2(a, b, x.x, x.y, 1.f, 1.f, -m, -m);
+  fmul2(a, b, a, b, 1.4426950408889634f, 1.4426950408889634f);
+  return make_float2(exp2f(a), exp2f(b));
+}
+__device__ __forceinline__ uint32_t ce_max2(uint32_t a, uint32_t b) {
+  asm("max.bf16x2 %0, %0, %1;" : "+r"(a) : "r"(b));
+  return a;
+}
+// The gradient of a row.
+__device__ __forceinline__ void ce_gradient(const uint4* xv, uint4* dv, int n, int hit, int target, float m, float inv, float gs) {
+  for (int c0 = threadIdx.x; c0 < n; c0 += CE_UNROLL * CE_THREADS) {
+    uint4 u[CE_UNROLL];
+#pragma unroll
+    for (int i = 0; i < CE_UNROLL; ++i)
+      if (c0 + i * CE_THREADS < n) u[i] = xv[c0 + i * CE_THREADS];
+#pragma unroll
+    for (int i = 0; i < CE_UNROLL; ++i) {
+      const int c = c0 + i * CE_THREADS;
+      if (c >= n) break;
+      const uint32_t w[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
+      float2 g[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        g[j] = ce_exp2(unpack_bf16x2(w[j]), m);
+        fmul2(g[j].x, g[j].y, g[j].x, g[j].y, inv, inv);
+      }
+      if (c == hit) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (2 * j == target) g[j].x -= gs;
+          if (2 * j + 1 == target) g[j].y -= gs;
+        }
+      }
+      dv[c] = make_uint4(pack_bf16x2(g[0].x, g[0].y), pack_bf16x2(g[1].x, g[1].y), pack_bf16x2(g[2].x, g[2].y),
+                         pack_bf16x2(g[3].x, g[3].y));
+    }
+  }
 }
 
-__global__ void __launch_bounds__(CE_THREADS)
+template <int CTAS>   // per SM
+__global__ void __launch_bounds__(CE_THREADS, CTAS)
 ce_fwd_bwd_kernel(const __nv_bfloat16* logits, const long* targets,
                   __nv_bfloat16* dlogits, float* loss_rows, int T, int V,
                   long ld, float grad_scale, long ignore_index) {
@@ -27,6 +69,7 @@ ce_fwd_bwd_kernel(const __nv_bfloat16* logits, const long* targets,
   const int row = blockIdx.x;
   const __nv_bfloat16* x = logits + row * ld;
   const bool vec = (V % 8 == 0) && (ld % 8 == 0);
+  const int n = V / 8;
   const long tgt = targets[row];
   const bool ignored = (tgt == ignore_index) || tgt < 0 || tgt >= V;
   // The target's logit is read ahead of the last barrier: behind it other threads may have written the gradient over it.
@@ -34,15 +77,27 @@ ce_fwd_bwd_kernel(const __nv_bfloat16* logits, const long* targets,
   float m = -INFINITY, s = 0.f;
   if (vec) {
     const uint4* xv = reinterpret_cast<const uint4*>(x);
-    for (int c = threadIdx.x; c < V / 8; c += CE_THREADS) {
-      float f[8];
-      ce_unpack8(xv[c], f);
-      float cm = f[0];
+    for (int c0 = threadIdx.x; c0 < n; c0 += CE_UNROLL * CE_THREADS) {
+      uint4 u[CE_UNROLL];
 #pragma unroll
-      for (int j = 1; j < 8; ++j) cm = fmaxf(cm, f[j]);
-      if (cm > m) { s *= __expf(m - cm); m = cm; }
+      for (int i = 0; i < CE_UNROLL; ++i) {
+        u[i] = make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // minus infinities add nothing
+        if (c0 + i * CE_THREADS < n) u[i] = xv[c0 + i * CE_THREADS];
+      }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) s += __expf(f[j] - m);
+      for (int i = 0; i < CE_UNROLL; ++i) {
+        const uint32_t w[4] = {u[i].x, u[i].y, u[i].z, u[i].w};
+        const float2 t = unpack_bf16x2(ce_max2(ce_max2(w[0], w[1]), ce_max2(w[2], w[3])));
+        const float cm = fmaxf(t.x, t.y);
+        if (cm > m) { s *= __expf(m - cm); m = cm; }
+        const float at = m == -INFINITY ? 0.f : m;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 e = ce_exp2(unpack_bf16x2(w[j]), at);
+          s += e.x;
+          s += e.y;
+        }
+      }
     }
   } else {
     for (int c = threadIdx.x; c < V; c += CE_THREADS) {
@@ -84,19 +139,8 @@ ce_fwd_bwd_kernel(const __nv_bfloat16* logits, const long* targets,
   if (vec) {
     const uint4* xv = reinterpret_cast<const uint4*>(x);
     uint4* dv = reinterpret_cast<uint4*>(dx);
-    for (int c = threadIdx.x; c < V / 8; c += CE_THREADS) {
-      float f[8];
-      ce_unpack8(xv[c], f);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        f[j] = __expf(f[j] - m) * inv;
-        if (c * 8 + j == tgt) f[j] -= gs;
-      }
-      uint4 o;
-      o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]);
-      o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
-      dv[c] = o;
-    }
+    const int hit = ignored ? -1 : int(tgt / 8), target = int(tgt % 8);   // the piece the target lies in, and where
+    ce_gradient(xv, dv, n, hit, target, m, inv, gs);
   } else {
     for (int c = threadIdx.x; c < V; c += CE_THREADS) {
       float f = __expf(__bfloat162float(x[c]) - m) * inv;
@@ -113,7 +157,12 @@ extern "C" int zb_cross_entropy(const void* logits, const long* targets, void* d
                                 cudaStream_t stream) {
   using namespace zb;
   if (T <= 0) return 0;
-  ZB_CUDA_OK(launch_pass(ce_fwd_bwd_kernel, T, CE_THREADS, 0, stream, static_cast<const __nv_bfloat16*>(logits), targets,
+  // Two CTAs per SM, with more registers for loads, where more rows than that are not there (256 x 32000: 9.9 us, with three 12.6)
+  // or would not stay in L2 until their second reading (2048 x 128256: 211 and 231 us; 2048 x 50272, 45 MB: 89 and 80).
+  const bool two = T <= 2 * num_sms() || 3L * num_sms() * V * 2 > 100'000'000L;
+  auto kern = ce_fwd_bwd_kernel<3>;
+  if (two) kern = ce_fwd_bwd_kernel<2>;
+  ZB_CUDA_OK(launch_pass(kern, T, CE_THREADS, 0, stream, static_cast<const __nv_bfloat16*>(logits), targets,
                          static_cast<__nv_bfloat16*>(dlogits), loss_rows, T, V, ld, grad_scale, ignore_index));
   ZB_CUDA_OK(cudaGetLastError());
   return 0;

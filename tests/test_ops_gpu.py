@@ -422,6 +422,25 @@ def test_cross_entropy(k, T, V):
     _close(d, lr.grad, atol=2e-3, rtol=2e-2)
 
 
+@pytest.mark.parametrize("T,V", [(3, 8), (700, 16376), (290, 16384), (300, 16392), (310, 120000)])
+def test_cross_entropy_against_64_bits(k, T, V):
+    """A row of one piece, rows that end inside, at and just behind a round of pieces, both numbers of CTAs per SM, logits of
+    minus infinity (whole rounds of a thread among them) and far below the others.  fp32 sums of V probabilities and two
+    exponentials: 2^-16 of the loss' terms; the gradient half a unit in the last of 8 bits on top of 2^-16 of the largest."""
+    logits = (torch.randn(T, V, device="cuda", generator=torch.Generator("cuda").manual_seed(V)) * 2).to(torch.bfloat16)
+    if V > 8:
+        logits[1, : V - 8] = -float("inf")
+        logits[2, : V // 2] = -200.0
+    tg = torch.randint(V - 8, V, (T,), device="cuda")
+    d = torch.empty_like(logits)
+    got = k.cross_entropy(logits, tg, 1.0, dlogits=d)
+    want = torch.logsumexp(logits.double(), 1) - logits.double().gather(1, tg[:, None])[:, 0]
+    torch.testing.assert_close(got.double(), want, rtol=2.0 ** -16, atol=2.0 ** -16 * 8)
+    grad = torch.softmax(logits.double(), 1)
+    grad.scatter_add_(1, tg[:, None], torch.full((T, 1), -1.0, device="cuda", dtype=torch.float64))
+    torch.testing.assert_close(d.double(), grad, rtol=2.0 ** -8, atol=2.0 ** -16)
+
+
 def test_cross_entropy_ignored_rows(k):
     """Rows whose target is the ignore index (-100) give zero loss and a zero gradient row."""
     T, V = 64, 1000
