@@ -290,7 +290,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         kb_range(item, kb0, kb1);
         const int buf = local & 1;
         const uint32_t use = uint32_t(local >> 1);
-        if (!mbar_wait_warp(&tmem_empty[buf], (use & 1) ^ 1, wctx, ST_TIMEOUT_TMEM_EMPTY)) break;
+        ok = mbar_wait_warp(&tmem_empty[buf], (use & 1) ^ 1, wctx, ST_TIMEOUT_TMEM_EMPTY);
+        if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + uint32_t(buf * BN);
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -313,6 +314,11 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         if (ok && elected) umma_commit_pair(&tmem_full[buf]);
         __syncwarp();
       }
+      // The second CTA's epilogue warps arrive on these barriers from another SM, and the last arrivals release accumulators
+      // that no tile wants any more: without a wait this CTA could be gone, and its shared memory another's, when one lands
+      // (the barrier at the end orders no memory).  The waits are those of two more tiles, one per buffer.
+      for (int i = 0; i < 2 && ok; ++i, ++local)
+        ok = mbar_wait_warp(&tmem_empty[local & 1], (uint32_t(local >> 1) & 1) ^ 1, wctx, ST_TIMEOUT_TMEM_EMPTY);
     }
   } else if (warp < 2 + EP_WARPS) {
     // ------------------------------ epilogue (own 128 rows) ------------------------------
@@ -784,7 +790,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   tc_fence_before();
   // The leader's MMAs read the peer's shared memory: leave together.  Where nothing written before is read behind this
   // barrier it need not order memory: a releasing arrival waits for the epilogue's own writes, 0.7 us at the end of every
-  // product.  The stores of the last boxes are still being read meanwhile (their writes are complete when the grid is).
+  // product.  Arrivals on the other CTA's barriers are no such writes: the issuer of the leader has waited for them above.
+  // The stores of the last boxes are still being read meanwhile (their writes are complete when the grid is).
   if constexpr (SCATTER || FUSED_AG) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
   else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   if (warp >= 2 && lane == 0) bulk_wait_read<0>();
