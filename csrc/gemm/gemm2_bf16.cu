@@ -272,6 +272,12 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
+      // The leader's commits arrive on the stage barriers of both CTAs: those of the last stages are waited for too, so that
+      // none is on its way to a CTA that has left.  The waits are those of one more round of loads.
+      for (int i = 0; i < STAGES && ok; ++i) {
+        ok = mbar_wait_warp(&empty[stage], phase ^ 1, wctx, ST_TIMEOUT_EMPTY);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA only) ------------------------------

@@ -60,3 +60,36 @@ def test_those_waits_end_exactly_when_every_arrival_has_landed(tiles, arrivals):
     for local in (tiles, tiles + 1):
         wait(local)
     assert landed == tiles * arrivals and not owed
+
+
+def test_the_producers_wait_for_the_last_release_of_the_stages():
+    producer = section("TMA producer (both CTAs)")
+    behind = producer[producer.index("tma_load_2d_pair(sb + j"):]
+    assert re.search(r"for \(int i = 0; i < STAGES && ok; \+\+i\) \{\s*"
+                     r"ok = mbar_wait_warp\(&empty\[stage\], phase \^ 1, [^;]*;\s*"
+                     r"if \(\+\+stage == STAGES\) \{ stage = 0; phase \^= 1; \}\s*\}", behind)
+
+
+@pytest.mark.parametrize("stages", [5, 6, 8])
+@pytest.mark.parametrize("blocks", [0, 1, 4, 5, 6, 7, 8, 13, 16, 24])
+def test_those_waits_end_exactly_when_every_commit_has_landed(stages, blocks):
+    bars, owed, landed = [Barrier(1) for _ in range(stages)], [], 0
+    stage = phase = 0
+
+    def step(load):
+        nonlocal stage, phase, landed
+        while not bars[stage].passed(phase ^ 1):
+            assert owed, "a wait that nothing ends"
+            bars[owed.pop(0)].arrive()
+            landed += 1
+        if load:
+            owed.append(stage)
+        stage += 1
+        if stage == stages:
+            stage, phase = 0, phase ^ 1
+
+    for _ in range(blocks):
+        step(True)
+    for _ in range(stages):
+        step(False)
+    assert landed == blocks and not owed
