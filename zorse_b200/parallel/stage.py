@@ -7,6 +7,7 @@ stages (interleaving), as in the reference (zorse_utils/pipeline.py:36-318).
 """
 from __future__ import annotations
 
+import itertools
 import os
 from typing import Optional
 
@@ -90,7 +91,10 @@ class DeferredWgrad:
     calls are queued with their arguments (the views into the bucket they accumulate into stay valid), and
     `flush()` runs them in order, so a schedule can send the input gradient first and do the weight gradients
     while the upstream stage is already working: the chain between stages gets shorter by the weight-gradient
-    time per stage.  Results are bit-identical: every bucket entry receives the same additions in the same order."""
+    time per stage.  What a layer collects for its `finish` (`later`) is collected again and finished together, layer by
+    layer and microbatch by microbatch.  Results are bit-identical: every bucket entry receives the same additions in the
+    same order, and each of them comes from the same kernels as without the queue (products that run together are not cut
+    along the reduction where one alone would be)."""
 
     def __init__(self, ops):
         self._ops = ops
@@ -102,15 +106,23 @@ class DeferredWgrad:
 
     def linear_wgrad(self, *a, **k):
         if self.active:
-            k.pop("later", None)      # the layer finishes its own list before the queue is flushed
-            self._queue.append((a, k))
+            later = a[4] if len(a) > 4 else k.pop("later", None)   # (finished by the layer long before the queue is flushed)
+            self._queue.append((later, a[:4], k))
         else:
             self._ops.linear_wgrad(*a, **k)
 
     def flush(self) -> None:
         q, self._queue = self._queue, []
-        for a, k in q:
-            self._ops.linear_wgrad(*a, **k)
+        for _, calls in itertools.groupby(q, key=lambda e: id(e[0])):   # (the queue keeps the lists: no two have one id)
+            calls = list(calls)
+            if calls[0][0] is None:
+                for _, a, k in calls:
+                    self._ops.linear_wgrad(*a, **k)
+                continue
+            later = self._ops.collect()
+            for _, a, k in calls:
+                self._ops.linear_wgrad(*a, **k, later=later)
+            self._ops.finish(later)
 
 
 class PipelineStage:
