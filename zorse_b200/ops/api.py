@@ -272,13 +272,14 @@ class Sm100Ops(_EpilogueOps, _LaterOps):
         return qkv
 
     def attn_fwd(self, qkv, B, S, Hq, Hkv, D, causal=True, window=0):
-        # the two-tile kernel at every size: where it leaves most of the GPU idle its steps are still shorter (d = 64: 2 x 8
-        # heads of 128 tokens 10.5 -> 5.0 us, of 509 14.7 -> 11.4, 12 heads of 2048 44.8 -> 31.2)
+        # The two-tile kernel at every size, by either way: where it leaves most of the GPU idle its steps are still shorter
+        # (d = 64: 2 x 8 heads of 128 tokens 10.5 -> 5.0 us, of 509 14.7 -> 11.4, 12 heads of 2048 44.8 -> 31.2).  Its results
+        # differ from the one-tile kernel's in last bits, with the same error against 64 bits (2 x 8 heads of 509: 1.996e-3).
         k = self.k
         r = self._attn_fwd(qkv, B, S, Hq, Hkv, D, causal, window, k.ATTN_FWD4_FLAGS)
         if r is not None:
             return r
-        return k.flash_fwd(qkv, B, S, Hq, Hkv, D, causal, window)
+        return k.flash_fwd(qkv, B, S, Hq, Hkv, D, causal, window, version=k.ATTN_FWD_VERSION or 4)
 
     def attn_bwd(self, do, qkv, o, lse, B, S, Hq, Hkv, D, causal=True, window=0):
         dqkv = self._attn_bwd(do, qkv, o, lse, B, S, Hq, Hkv, D, causal, window)

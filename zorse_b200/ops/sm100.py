@@ -377,8 +377,9 @@ def _window(window: int, S: int) -> int:
     return 0 if window >= S else window
 
 
-# 0 = by problem size: version 4 (two query tiles per CTA, 256 query rows), or version 1 (one 128-row tile per CTA) for
-# small problems; 1 / 2 / 4 force a version.
+# 1 / 2 / 4 force a version.  0: the op layer (`api.Sm100Ops`, what layers call) takes version 4 (two query tiles per CTA,
+# 256 query rows) at every size; `flash_fwd` called without a version takes it, or version 1 (one 128-row tile per CTA) for
+# small problems.
 ATTN_FWD_VERSION = int(os.environ.get("ZORSE_ATTN_FWD", "0"))
 
 
@@ -394,9 +395,9 @@ def flash_fwd(qkv, B: int, S: int, Hq: int, Hkv: int, D: int, causal: bool = Tru
               scale: Optional[float] = None, version: Optional[int] = None, flags: Optional[int] = None,
               trace: Optional[torch.Tensor] = None, trace_ctas: int = 0):
     """qkv: packed [B*S, (Hq+2Hkv)*D]. Returns (out [B*S, Hq*D], lse [B, Hq, S]).
-    version 1: one query tile per CTA, S double-buffered in TMEM, P staged through shared memory (default
+    version 1: one query tile per CTA, S double-buffered in TMEM, P staged through shared memory (default here
     for small problems); version 2: two query tiles per CTA, P kept in
-    TMEM; version 4 (default otherwise, 143 against 257 us on 32 heads of 4096 tokens, d = 128): two
+    TMEM; version 4 (the op layer's, and default otherwise, 143 against 257 us on 32 heads of 4096 tokens, d = 128): two
     query tiles, one MMA issuer, score rows in registers (`flags` 1: two-wide
     fp32 math, 2: also a quarter of the exponentials as a polynomial on the fma pipe; `trace`: zeroed int64 buffer from `flash_fwd4_trace_buffer` for a phase timeline)."""
     _bf16(qkv, "qkv")
