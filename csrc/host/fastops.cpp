@@ -17,6 +17,8 @@
 
 #include <cmath>
 #include <cstdint>
+#include <utility>
+#include <vector>
 
 namespace {
 
@@ -394,6 +396,7 @@ PyObject* norm_bwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 // where one after the other every one ended with most of the GPU idle (a BERT block's four weight gradients are 54, 18, 72 and
 // 72 tiles on 74 pairs), and the column sums run beside the last.  All operands stay in the list until everything is
 // launched, and only the last product may have a workspace of the allocator's: the rules of chain_late (ptx.cuh).
+// A product whose gradient lies in memory that an earlier one of the list writes (two calls for one parameter) waits for it.
 PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
   ZB_ARGS(1)
@@ -416,6 +419,19 @@ PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   long desc[MAX][7];
   int n = 0;
   bool late = false;       // a product has been launched here: what the sums read was complete before it
+  // Bytes that kernels launched here, or sums not launched yet, add to; `claim` answers whether none of them is in `out`,
+  // which else has to wait: then all of them are done, and the record starts anew.
+  std::vector<std::pair<uintptr_t, uintptr_t>> written;
+  auto claim = [&](const Tensor& out) {
+    const uintptr_t lo = reinterpret_cast<uintptr_t>(out.data_ptr());
+    const int64_t last = out.dim() == 2 ? (out.size(0) - 1) * out.stride(0) + out.size(1) : out.numel();
+    const uintptr_t hi = lo + uintptr_t(last) * out.element_size();
+    bool free = true;
+    for (const auto& w : written) free = free && (hi <= w.first || w.second <= lo);
+    if (!free) written.clear();
+    written.emplace_back(lo, hi);
+    return free;
+  };
   const cudaStream_t s = stream();
   for (Py_ssize_t i = 0; i < entries; ++i) {
     PyObject* e = PyList_GET_ITEM(args[0], i);
@@ -424,8 +440,8 @@ PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (dy == nullptr || x == nullptr || gw == nullptr) return refuse();
     int* status = status_of(*dy);
     if (status == nullptr) return refuse();
-    const bool first = launched == 0, last = ++launched == products;
-    const int done = gemm(dy, x, *gw, true, true, nullptr, nullptr, true, status, first ? 0 : GEMM_LATE, !last);
+    const bool first = launched == 0, last = ++launched == products, free = claim(*gw);
+    const int done = gemm(dy, x, *gw, true, true, nullptr, nullptr, true, status, first || !free ? 0 : GEMM_LATE, !last);
     if (done < 0) return nullptr;
     if (done == 0) return refuse();
     late = true;
@@ -437,6 +453,10 @@ PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   };
   auto add = [&](const Tensor& src, int64_t offset, int64_t rows, int64_t cols, int64_t ld, const Tensor& out) {
     if (n == MAX && !run()) return false;
+    if (!claim(out)) {
+      if (!run()) return false;
+      late = false;
+    }
     const bool f32 = src.scalar_type() == F32;
     const long d[7] = {reinterpret_cast<long>(src.data_ptr()) + long(offset * (f32 ? 4 : 2)), reinterpret_cast<long>(out.data_ptr()),
                        long(rows), long(cols), long(ld), f32, out.scalar_type() == F32};
