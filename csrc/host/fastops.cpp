@@ -132,10 +132,18 @@ bool product(const Tensor* a, const Tensor* b, const Tensor& out, bool a_mn, boo
          fits(a->stride(0)) && fits(b->stride(0)) && fits(out.stride(0));
 }
 
+// The workspace for a product whose last wave of tiles is to be cut along K; undefined where it is not.
+Tensor split_workspace(int64_t M, int64_t N, int64_t K, const Tensor& like) {
+  // (the same lines as in the wrapper: shorter reductions are never cut)
+  const int bytes = M >= 256 && N >= 256 && K > 3000 ? lib.gemm2_workspace(int(M), int(N), int(K)) : 0;
+  return bytes > 0 ? empty({bytes}, like, at::kByte) : Tensor();
+}
+
 // out[M, N] (+)= A B^T; `out` as the caller prepared it.  1: done, 0: not for here, -1: error set.
-// more: flags, GEMM_LATE for one that starts under the kernel before it; whole: no tiles cut along K (a workspace).
+// more: flags, GEMM_LATE for one that starts under the kernel before it; workspace: what split_workspace gave, nullptr: gemm
+// asks itself.
 int gemm(const Tensor* a, const Tensor* b, const Tensor& out, bool a_mn, bool b_mn, const Tensor* bias, const Tensor* addend,
-         bool accumulate, int* status, int more = 0, bool whole = false) {
+         bool accumulate, int* status, int more = 0, const Tensor* workspace = nullptr) {
   const int64_t M = out.size(0), N = out.size(1), K = a->size(a_mn ? 0 : 1);
   if (!product(a, b, out, a_mn, b_mn)) return 0;
   if (bias != nullptr && !(dense(bias, BF16) && bias->dim() == 1 && bias->size(0) == N)) return 0;
@@ -152,11 +160,10 @@ int gemm(const Tensor* a, const Tensor* b, const Tensor& out, bool a_mn, bool b_
     return launch("gemm", 1, [&] {
       return lib.gemm(pa, pb, pc, m, n, k, lda, ldb, ldc, a_mn, b_mn, pbias, px, ldx, flags, 0, 0, status, s);
     }) ? 1 : -1;
-  // (the same line as in the wrapper: shorter reductions are never cut)
-  const int ws_bytes = k > 3000 && !whole ? lib.gemm2_workspace(m, n, k) : 0;
-  if (ws_bytes > 0) {
-    const Tensor ws = empty({ws_bytes}, *a, at::kByte);
+  const Tensor ws = workspace != nullptr ? *workspace : split_workspace(m, n, k, *a);
+  if (ws.defined()) {
     void* pw = ws.data_ptr();
+    const long ws_bytes = ws.numel();
     return launch("gemm2_split", 1, [&] {
       return lib.gemm2_split(pa, pb, pc, m, n, k, lda, ldb, ldc, a_mn, b_mn, pbias, px, ldx, flags, pw, ws_bytes, status, s);
     }) ? 1 : -1;
@@ -395,7 +402,8 @@ PyObject* norm_bwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 // No product reads what another one writes, so each but the first starts on the SMs that the one before it has done with,
 // where one after the other every one ended with most of the GPU idle (a BERT block's four weight gradients are 54, 18, 72 and
 // 72 tiles on 74 pairs), and the column sums run beside the last.  All operands stay in the list until everything is
-// launched, and only the last product may have a workspace of the allocator's: the rules of chain_late (ptx.cuh).
+// launched, and only the last product may have a workspace of the allocator's, taken ahead of the first launch (meanwhile another
+// thread may launch on this stream and give back memory that its kernels still use): the rules of chain_late (ptx.cuh).
 // A product whose gradient lies in memory that an earlier one of the list writes (two calls for one parameter) waits for it.
 PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
@@ -410,10 +418,19 @@ PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   };
   const Py_ssize_t entries = PyList_GET_SIZE(args[0]);
   Py_ssize_t products = 0, launched = 0;
+  Tensor none, workspace;   // (of the last product)
   for (Py_ssize_t i = 0; i < entries; ++i) {
     PyObject* e = PyList_GET_ITEM(args[0], i);
     if (!PyTuple_Check(e) || (PyTuple_GET_SIZE(e) != 3 && PyTuple_GET_SIZE(e) != 4)) return refuse();
     products += PyTuple_GET_SIZE(e) == 4;
+  }
+  for (Py_ssize_t i = entries; products > 0 && i-- > 0;) {
+    PyObject* e = PyList_GET_ITEM(args[0], i);
+    if (PyTuple_GET_SIZE(e) != 4) continue;
+    const Tensor *dy = tensor_of(PyTuple_GET_ITEM(e, 0)), *gw = tensor_of(PyTuple_GET_ITEM(e, 2));
+    if (dy == nullptr || gw == nullptr || status_of(*dy) == nullptr || dy->dim() != 2 || gw->dim() != 2) return refuse();
+    workspace = split_workspace(gw->size(0), gw->size(1), dy->size(0), *dy);
+    break;
   }
   constexpr int MAX = 8;   // sums per launch
   long desc[MAX][7];
@@ -441,7 +458,7 @@ PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     int* status = status_of(*dy);
     if (status == nullptr) return refuse();
     const bool first = launched == 0, last = ++launched == products, free = claim(*gw);
-    const int done = gemm(dy, x, *gw, true, true, nullptr, nullptr, true, status, first || !free ? 0 : GEMM_LATE, !last);
+    const int done = gemm(dy, x, *gw, true, true, nullptr, nullptr, true, status, first || !free ? 0 : GEMM_LATE, last ? &workspace : &none);
     if (done < 0) return nullptr;
     if (done == 0) return refuse();
     late = true;
