@@ -268,6 +268,10 @@ static inline int grid_for(long work_items, int threads) {
   return int(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
+static bool aligned16(const void* a, const void* b = nullptr, const void* c = nullptr) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15) == 0;
+}
+
 }  // namespace zb
 
 extern "C" {
@@ -277,6 +281,7 @@ int zb_rope(void* buf, const float* cs, int T, int S, int nheads, int d, int row
   using namespace zb;
   if (d % 16 != 0 || row_stride % 8 != 0) ZB_FAIL(-1, "rope: head dim %d / stride %d unsupported", d, row_stride);
   if (T <= 0 || nheads <= 0) return 0;
+  if (!aligned16(buf, cs)) ZB_FAIL(-4, "rope: an operand is not 16-byte aligned");
   long total = long(T) * nheads * (d / 16);
   ZB_CUDA_OK(launch_pass(rope_kernel, grid_for(total, 256), 256, 0, stream, static_cast<__nv_bfloat16*>(buf), cs, T, S,
                          nheads, d, row_stride, backward ? -1.f : 1.f));
@@ -288,6 +293,7 @@ int zb_swiglu_fwd(const void* gu, void* out, long T, int F, cudaStream_t stream)
   using namespace zb;
   if (F % 8 != 0) ZB_FAIL(-1, "swiglu: F=%d not a multiple of 8", F);
   if (T <= 0) return 0;
+  if (!aligned16(gu, out)) ZB_FAIL(-4, "swiglu: an operand is not 16-byte aligned");
   ZB_CUDA_OK(launch_pass(swiglu_fwd_kernel, grid_for(T * (F / 8), 256), 256, 0, stream,
                          static_cast<const __nv_bfloat16*>(gu), static_cast<__nv_bfloat16*>(out), T, F));
   ZB_CUDA_OK(cudaGetLastError());
@@ -297,6 +303,7 @@ int zb_swiglu_bwd(const void* gu, const void* dout, void* dgu, long T, int F, cu
   using namespace zb;
   if (F % 8 != 0) ZB_FAIL(-1, "swiglu: F=%d not a multiple of 8", F);
   if (T <= 0) return 0;
+  if (!aligned16(gu, dout, dgu)) ZB_FAIL(-4, "swiglu: an operand is not 16-byte aligned");
   ZB_CUDA_OK(launch_pass(swiglu_bwd_kernel, grid_for(T * (F / 8), 256), 256, 0, stream,
                          static_cast<const __nv_bfloat16*>(gu), static_cast<const __nv_bfloat16*>(dout),
                          static_cast<__nv_bfloat16*>(dgu), T, F));
@@ -307,6 +314,7 @@ int zb_act_fwd(const void* x, void* y, long n, int kind, cudaStream_t stream) {
   using namespace zb;
   if (n % 8 != 0) ZB_FAIL(-1, "act: n=%ld not a multiple of 8", n);
   if (n <= 0) return 0;
+  if (!aligned16(x, y)) ZB_FAIL(-4, "act: an operand is not 16-byte aligned");
   ZB_CUDA_OK(launch_pass(act_fwd_kernel, grid_for(n / 8, 256), 256, 0, stream, static_cast<const __nv_bfloat16*>(x),
                          static_cast<__nv_bfloat16*>(y), n / 8, kind));
   ZB_CUDA_OK(cudaGetLastError());
@@ -316,6 +324,7 @@ int zb_act_bwd(const void* x, const void* dy, void* dx, long n, int kind, cudaSt
   using namespace zb;
   if (n % 8 != 0) ZB_FAIL(-1, "act: n=%ld not a multiple of 8", n);
   if (n <= 0) return 0;
+  if (!aligned16(x, dy, dx)) ZB_FAIL(-4, "act: an operand is not 16-byte aligned");
   ZB_CUDA_OK(launch_pass(act_bwd_kernel, grid_for(n / 8, 256), 256, 0, stream, static_cast<const __nv_bfloat16*>(x),
                          static_cast<const __nv_bfloat16*>(dy), static_cast<__nv_bfloat16*>(dx), n / 8, kind));
   ZB_CUDA_OK(cudaGetLastError());

@@ -97,15 +97,20 @@ Tensor empty(at::IntArrayRef sizes, const Tensor& like, at::ScalarType type) {
 }
 void* ptr(const Tensor* t) { return t == nullptr ? nullptr : t->data_ptr(); }
 
-// Runs `f` (the launches, 0 or an error code) without the GIL; counts `n` launches or raises KernelError.
+// Runs `f` (the launches, 0 or an error code) without the GIL; counts `n` launches or raises KernelError.  An entry point
+// answers 1, having done nothing, to what it was not written for: false without an error then where `declined` is given.
 template <typename F>
-bool launch(const char* what, int n, F&& f) {
+bool launch(const char* what, int n, F&& f, bool* declined = nullptr) {
   int rc;
   Py_BEGIN_ALLOW_THREADS
   rc = f();
   Py_END_ALLOW_THREADS
-  if (rc != 0) {   // (the error text is this thread's)
-    PyErr_Format(kernel_error, "%s: %s", what, lib.last_error());
+  if (rc == 1 && declined != nullptr) {
+    *declined = true;
+    return false;
+  }
+  if (rc != 0) {   // (the error text is this thread's, and of an earlier error where this entry point set none)
+    PyErr_Format(kernel_error, "%s: %s", what, rc == 1 ? "arguments it does not take" : lib.last_error());
     return false;
   }
   launches += n;
@@ -263,11 +268,14 @@ PyObject* act_linear_fwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (truth(args[4])) pre = empty({M, W}, *x, BF16);
   void* pp = pre.defined() ? pre.data_ptr() : nullptr;
   const cudaStream_t s = stream();
+  bool declined = false;
   if (!launch("gemm2_act_fwd", 1, [&] {
         return lib.gemm2_act_fwd(ptr(x), ptr(w), ptr(bias), pp, out.data_ptr(), int(M), int(N), int(K), int(x->stride(0)),
                                  int(w->stride(0)), int(kind), status, s);
-      }))
+      }, &declined)) {
+    if (declined) Py_RETURN_NONE;
     return nullptr;
+  }
   PyObject* r = PyTuple_New(2);
   if (r == nullptr) return nullptr;
   PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(std::move(out)));
@@ -294,11 +302,14 @@ PyObject* linear_rope_fwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (bias != nullptr && !(dense(bias, BF16) && bias->dim() == 1 && bias->size(0) == N)) Py_RETURN_NONE;
   Tensor out = empty({M, N}, *x, BF16);
   const cudaStream_t s = stream();
+  bool declined = false;
   if (!launch("gemm2_rope_fwd", 1, [&] {
         return lib.gemm2_rope_fwd(ptr(x), ptr(w), ptr(bias), static_cast<const float*>(ptr(cs)), out.data_ptr(), int(M), int(N),
                                   int(K), int(x->stride(0)), int(w->stride(0)), int(S), int(heads), int(d), status, s);
-      }))
+      }, &declined)) {
+    if (declined) Py_RETURN_NONE;
     return nullptr;
+  }
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }
@@ -319,11 +330,14 @@ PyObject* act_linear_dgrad(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     Py_RETURN_NONE;
   Tensor dpre = empty(pre->sizes(), *dy, BF16);
   const cudaStream_t s = stream();
+  bool declined = false;
   if (!launch("gemm2_act_bwd", 1, [&] {
         return lib.gemm2_act_bwd(ptr(dy), ptr(w), ptr(pre), dpre.data_ptr(), int(M), int(N), int(K), int(dy->stride(0)),
                                  int(w->stride(0)), int(kind), status, s);
-      }))
+      }, &declined)) {
+    if (declined) Py_RETURN_NONE;
     return nullptr;
+  }
   return THPVariable_Wrap(std::move(dpre));
   END_HANDLE_TH_ERRORS
 }
