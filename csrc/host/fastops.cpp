@@ -416,8 +416,13 @@ PyObject* norm_bwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 // No product reads what another one writes, so each but the first starts on the SMs that the one before it has done with,
 // where one after the other every one ended with most of the GPU idle (a BERT block's four weight gradients are 54, 18, 72 and
 // 72 tiles on 74 pairs), and the column sums run beside the last.  All operands stay in the list until everything is
-// launched, and only the last product may have a workspace of the allocator's, taken ahead of the first launch (meanwhile another
-// thread may launch on this stream and give back memory that its kernels still use): the rules of chain_late (ptx.cuh).
+// launched, and the workspaces are taken ahead of the first launch (what the allocator hands out behind it may have been given
+// back by another thread while kernels on this stream still use it): the rules of chain_late (ptx.cuh).
+// Long products are cut along K as they are alone, for the same bits and the same accuracy: what a tensor core adds to an
+// accumulator it truncates, so the error of an fp32 result grows with the tokens summed in one (9.1e-6 over 8192), and with
+// whole products in the list weights of 512 columns, all of whose tiles are cut alone (512 x 512: 4.8e-7), lost up to a
+// factor of 19.  But for the last, products with a side that is no multiple of 32, which no layer here has, stay whole: their
+// results in a list have been held to the bits of whole tiles.
 // A product whose gradient lies in memory that an earlier one of the list writes (two calls for one parameter) waits for it.
 PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
@@ -432,19 +437,20 @@ PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   };
   const Py_ssize_t entries = PyList_GET_SIZE(args[0]);
   Py_ssize_t products = 0, launched = 0;
-  Tensor none, workspace;   // (of the last product)
   for (Py_ssize_t i = 0; i < entries; ++i) {
     PyObject* e = PyList_GET_ITEM(args[0], i);
     if (!PyTuple_Check(e) || (PyTuple_GET_SIZE(e) != 3 && PyTuple_GET_SIZE(e) != 4)) return refuse();
     products += PyTuple_GET_SIZE(e) == 4;
   }
-  for (Py_ssize_t i = entries; products > 0 && i-- > 0;) {
+  std::vector<Tensor> workspaces;   // one per product, undefined for one that runs whole
+  for (Py_ssize_t i = 0; i < entries; ++i) {
     PyObject* e = PyList_GET_ITEM(args[0], i);
     if (PyTuple_GET_SIZE(e) != 4) continue;
     const Tensor *dy = tensor_of(PyTuple_GET_ITEM(e, 0)), *gw = tensor_of(PyTuple_GET_ITEM(e, 2));
     if (dy == nullptr || gw == nullptr || status_of(*dy) == nullptr || dy->dim() != 2 || gw->dim() != 2) return refuse();
-    workspace = split_workspace(gw->size(0), gw->size(1), dy->size(0), *dy);
-    break;
+    const int64_t M = gw->size(0), N = gw->size(1);
+    const bool last = Py_ssize_t(workspaces.size()) + 1 == products;
+    workspaces.push_back(last || (M % 32 == 0 && N % 32 == 0) ? split_workspace(M, N, dy->size(0), *dy) : Tensor());
   }
   constexpr int MAX = 8;   // sums per launch
   long desc[MAX][7];
@@ -471,8 +477,10 @@ PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (dy == nullptr || x == nullptr || gw == nullptr) return refuse();
     int* status = status_of(*dy);
     if (status == nullptr) return refuse();
-    const bool first = launched == 0, last = ++launched == products, free = claim(*gw);
-    const int done = gemm(dy, x, *gw, true, true, nullptr, nullptr, true, status, first || !free ? 0 : GEMM_LATE, last ? &workspace : &none);
+    const bool free = claim(*gw);
+    const int done = gemm(dy, x, *gw, true, true, nullptr, nullptr, true, status, launched == 0 || !free ? 0 : GEMM_LATE,
+                          &workspaces[launched]);
+    ++launched;
     if (done < 0) return nullptr;
     if (done == 0) return refuse();
     late = true;

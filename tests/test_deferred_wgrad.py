@@ -75,3 +75,31 @@ def test_held_back_gradients_of_blocks_are_the_same_bits(model, B, S, dt):
     k.check_status()
     for a, b in zip(*buckets):
         assert bool(a.any()) and torch.equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,sizes", [(8192, [(512, 1376), (2752, 512), (512, 512), (1536, 512)]), (5600, [(768, 3072), (768, 768), (2304, 768)]),
+                                     (6200, [(2048, 8192), (2048, 2048), (3072, 2048), (512, 512)]), (4600, [(4096, 3072), (6144, 4096), (512, 512)])])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_collected_products_are_cut_like_those_alone(T, sizes, dt):
+    """Reductions long enough to be cut for most of these: the bits of each product alone, behind kernels that have just written
+    the operands, twice into the same gradients."""
+    from zorse_b200.ops import sm100 as k
+    from zorse_b200.ops.api import get_ops
+
+    ops = get_ops("sm100")
+    rand = lambda *shape, seed: torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).bfloat16().cuda()
+    src, xs = [rand(T, n, seed=i) for i, (n, _) in enumerate(sizes)], [rand(T, m, seed=10 + i) for i, (_, m) in enumerate(sizes)]
+    got, want = ([torch.zeros(n, m, dtype=dt, device="cuda") for n, m in sizes] for _ in range(2))
+    for _ in range(2):
+        later, dys = ops.collect(), [ops.act_fwd(s, "relu") for s in src]
+        for dy, x, g in zip(dys, xs, got):
+            ops.linear_wgrad(dy, x, g, later=later)
+        ops.finish(later)
+        torch.cuda.synchronize()
+        for dy, x, g in zip(dys, xs, want):
+            ops.linear_wgrad(dy, x, g)
+    k.check_status()
+    assert any(k._gemm2_workspace(n, m, T, 0) for n, m in sizes[:-1])
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)
