@@ -4,9 +4,7 @@
 // Each of these sums reads a few megabytes that are still in L2, takes longer to launch than to read, and alone its strips of
 // columns make too few CTAs (768 columns: 24).  Together they fill the GPU: a cluster of eight CTAs takes 64 columns of one
 // matrix, each CTA an eighth of the rows with four 16-byte requests per thread in flight, and the eight partial sums are
-// added through distributed shared memory, in a fixed order, so results do not depend on timing.  The sums of warps and of
-// CTAs are added in pairs, as many additions deep as the kernels for one matrix have them: one after the other they were 4 to
-// 25 % further from 64 bits (8192 x 1024: 5.7e-8 of the sums; alone, and so, 4.9e-8).
+// added through distributed shared memory, in their order, so results do not depend on timing.
 // The four bias and four norm gradients of a BERT block (3072 tokens, 768 / 3072 wide): six launches 28 us, one launch 7.
 #include "../common/host.h"
 #include "../common/ptx.cuh"
@@ -26,10 +24,6 @@ struct ColSumItems {
   ColSumItem item[COLSUM_MAX];
   int late;   // nothing that the kernel before this one writes is read here (chain_late in ptx.cuh)
 };
-
-__device__ __forceinline__ float add8(const float (&v)[8]) {
-  return ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
-}
 
 __global__ void __cluster_dims__(COLSUM_RANKS, 1, 1) __launch_bounds__(256)
 column_sums_kernel(const __grid_constant__ ColSumItems p) {
@@ -92,22 +86,23 @@ column_sums_kernel(const __grid_constant__ ColSumItems p) {
   }
   __syncthreads();
   if (threadIdx.x < COLSUM_COLS) {
-    float v[8];
+    float t = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) v[w] = warp_sum[w][threadIdx.x];
-    cta_sum[threadIdx.x] = add8(v);
+    for (int w = 0; w < 8; ++w) t += warp_sum[w][threadIdx.x];
+    cta_sum[threadIdx.x] = t;
   }
   asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
   if (threadIdx.x < COLSUM_COLS / COLSUM_RANKS) {   // each CTA finishes eight of the columns
     const int c = rank * (COLSUM_COLS / COLSUM_RANKS) + int(threadIdx.x);
-    float v[COLSUM_RANKS];
+    float t = 0.f;
 #pragma unroll
     for (int q = 0; q < COLSUM_RANKS; ++q) {
       uint32_t a;
+      float v;
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(&cta_sum[c])), "r"(q));
-      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v[q]) : "r"(a) : "memory");
+      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+      t += v;
     }
-    const float t = add8(v);
     if (col0 + c < it.cols) {
       if (it.out_f32) {
         float* o = static_cast<float*>(it.out) + col0 + c;
