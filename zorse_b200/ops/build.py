@@ -12,8 +12,8 @@ Every `.cu` file under `csrc/` is compiled to an object with
 from __future__ import annotations
 
 import argparse
-import os
 import importlib.util
+import os
 import shutil
 import subprocess
 import sys
@@ -68,20 +68,39 @@ def _compile_one(nvcc: str, src: Path, obj: Path, verbose: bool, extra=()) -> st
 
 DEBUG_LIB = OUT_DIR / "libzorse_sm100_dbg.so"
 FAST_SRC = CSRC / "host" / "fastops.cpp"
-FAST = OUT_DIR / "zorse_fastops.so"
+
+
+class FastModuleUnavailable(RuntimeError):
+    """There is no module for this interpreter and this torch, nor a way to build one here."""
+
+
+def fast_path() -> Path:
+    """Where `zorse_fastops` lies.  It holds to one torch's C++ interface and one interpreter's, so both are in its name."""
+    import torch
+
+    return OUT_DIR / f"zorse_fastops-torch{torch.__version__}{sysconfig.get_config_var('EXT_SUFFIX')}"
 
 
 def build_fast(force: bool = False) -> Path:
-    """The module `zorse_fastops` for this interpreter and this torch."""
-    if not force and FAST.exists() and FAST.stat().st_mtime >= FAST_SRC.stat().st_mtime:
-        return FAST
+    """The module `zorse_fastops` for this interpreter and this torch; an installed copy, which has no `csrc/`, gets the one it
+    came with."""
+    out = fast_path()
+    if not FAST_SRC.exists():
+        if not out.exists():
+            raise FastModuleUnavailable(f"neither {out.name} nor {FAST_SRC} is there")
+        return out
+    if not force and out.exists() and out.stat().st_mtime >= FAST_SRC.stat().st_mtime:
+        return out
     torch_dir = Path(importlib.util.find_spec("torch").origin).parent
     cxx = os.environ.get("CXX") or shutil.which("g++")
     if not cxx:
-        raise RuntimeError("g++ not found; the host module cannot be built")
-    cuda = Path(find_nvcc()).resolve().parents[1]
+        raise FastModuleUnavailable("g++ not found; the host module cannot be built")
+    try:
+        cuda = Path(find_nvcc()).resolve().parents[1]
+    except RuntimeError as e:
+        raise FastModuleUnavailable(str(e)) from e
     OUT_DIR.mkdir(parents=True, exist_ok=True)
-    tmp = FAST.with_suffix(f".{os.getpid()}.tmp")
+    tmp = out.with_suffix(f".{os.getpid()}.tmp")
     libs = ["torch_python", "torch", "torch_cpu", "torch_cuda", "c10", "c10_cuda"]
     cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", *(f"-I{d}" for d in (
         torch_dir / "include", torch_dir / "include/torch/csrc/api/include", cuda / "include",
@@ -90,8 +109,8 @@ def build_fast(force: bool = False) -> Path:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"{FAST_SRC.name} does not build:\n{r.stdout}\n{r.stderr}")
-    os.replace(tmp, FAST)
-    return FAST
+    os.replace(tmp, out)
+    return out
 
 
 def build(force: bool = False, verbose: bool = False, debug_bounds: bool = False) -> Path:

@@ -12,6 +12,7 @@ import ctypes
 import functools
 import math
 import os
+import warnings
 from ctypes import c_float, c_int, c_long, c_void_p
 from pathlib import Path
 from typing import Optional
@@ -84,7 +85,8 @@ def lib():
 
 
 # The module csrc/host/fastops.cpp: the same entry points for the calls of a training step, without Python in between.  It
-# answers None to arguments it was not written for; the wrappers below take those.  None until the library is loaded.
+# answers None to arguments it was not written for; the wrappers below take those.  None until the library is loaded, and where
+# there is neither a module for this torch nor a way to build it (an installed copy): the wrappers then take every call.
 _fast = None
 _FAST_ENTRIES = ("zb_gemm_bf16", "zb_gemm2_bf16", "zb_gemm2_split_bf16", "zb_gemm2_workspace", "zb_norm_fwd", "zb_norm_bwd2",
                  "zb_norm_bwd2_rows", "zb_colsum", "zb_rope", "zb_swiglu_fwd", "zb_swiglu_bwd", "zb_act_fwd", "zb_act_bwd",
@@ -98,7 +100,12 @@ def _load_fast() -> None:
 
     from . import build as _build
 
-    spec = importlib.util.spec_from_file_location("zorse_fastops", _build.build_fast())
+    try:
+        path = _build.build_fast()
+    except _build.FastModuleUnavailable as e:
+        warnings.warn(f"no native call module, every launch goes through Python: {e}", RuntimeWarning, stacklevel=2)
+        return
+    spec = importlib.util.spec_from_file_location("zorse_fastops", path)
     mod = importlib.util.module_from_spec(spec)
     spec.loader.exec_module(mod)
     mod.init(tuple(ctypes.cast(getattr(_lib, n), c_void_p).value for n in _FAST_ENTRIES), KernelError)
