@@ -135,27 +135,37 @@ class Streams:
 
 
 class MasterLanding:
-    """Device buffers in which parked fp32 masters land on their way to an optimizer inside the backward pass: five, of the
-    largest unit's size, kept for the life of the stage.  A buffer is taken when a copy into it is issued and given back
+    """Device buffers in which parked fp32 masters land on their way to an optimizer inside the backward pass, of the largest
+    unit's size, kept for the life of the stage.  A buffer is taken when a copy into it is issued and given back
     with the event behind its last use, which the next copy into it waits for.  (A block per fetch from the caching
     allocator crosses streams and cannot be handed out again before the GPU has passed that point, while the host runs a
     whole backward pass ahead: every master became resident.)  With few buffers the copies to the GPU, which also bring what
     the backward pass computes on, wait for write-backs: OPT 125M step 32.9 ms with three, 31.4 with four, 30.8 with five;
     six and eight gain nothing more.  A stream of their own lets the masters take link bandwidth from the shards.
+    Parameters are parked to save device memory, so the fourth and fifth are there where they take at most EXTRA_BYTES
+    together (units of up to 134 million parameters: OPT 1.3B 0.9 GB; those of OPT 13B would take 2.5), and never more
+    buffers than units.
     `p16` takes the bf16 image of an update on its way to the host; only the communication stream touches it.  Nothing is
     then left for the first step of a stage to allocate there (two allocations while the GPU is busy, 1 to 60 ms each)."""
-    BUFFERS = 5
+    BUFFERS, FEW, EXTRA_BYTES = 5, 3, 1 << 30
 
-    def __init__(self, device: torch.device, streams: Streams, n: int, compute_dtype: torch.dtype):
+    @classmethod
+    def count(cls, n: int, units: int) -> int:
+        """Buffers for a stage of `units` units, the largest of n parameters."""
+        few = min(cls.FEW, cls.BUFFERS)
+        return min(units, cls.BUFFERS if (cls.BUFFERS - few) * 4 * n <= cls.EXTRA_BYTES else few)
+
+    def __init__(self, device: torch.device, streams: Streams, n: int, compute_dtype: torch.dtype, units: int):
         self.stream = streams.copy
-        self.bufs = [torch.empty(n, dtype=torch.float32, device=device) for _ in range(self.BUFFERS)]
+        buffers = self.count(n, units)
+        self.bufs = [torch.empty(n, dtype=torch.float32, device=device) for _ in range(buffers)]
         self.p16 = torch.empty(n, dtype=compute_dtype, device=device)
         for s in (streams.copy, streams.comm):
             s.wait_stream(torch.cuda.current_stream(device))   # the blocks may have been in use there
             for b in (*self.bufs, self.p16):                   # nor are they handed out before `s` has passed, in the end
                 b.record_stream(s)
-        self.used: list = [None] * self.BUFFERS
-        self.idle = deque(range(self.BUFFERS))
+        self.used: list = [None] * buffers
+        self.idle = deque(range(buffers))
 
     def take(self) -> Optional[int]:
         """A buffer, ready for work queued on `stream` from now on; None while all are waited for."""
@@ -566,7 +576,7 @@ class StageEngine:
         for lower, upper in zip(self.units, self.units[1:]):
             upper.below = lower
         if device.type == "cuda" and cfg.offload_params and cfg.optimizer_in_backward and self.units:
-            landing = MasterLanding(device, self.streams, max(u.shard_n for u in self.units), cfg.compute_dtype)
+            landing = MasterLanding(device, self.streams, max(u.shard_n for u in self.units), cfg.compute_dtype, len(self.units))
             for u in self.units:
                 u.landing = landing
 
