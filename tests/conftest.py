@@ -1,3 +1,4 @@
+import gc
 import os
 import sys
 
@@ -23,3 +24,11 @@ def pytest_collection_modifyitems(config, items):
     for item in items:
         if "gpu" in item.keywords:
             item.add_marker(skip)
+
+
+@pytest.fixture(autouse=True)
+def no_garbage_of_earlier_tests(request):
+    """Tests that compare the allocator's figures before and after a call must not see a collection, in between, of what other
+    tests have left in reference cycles."""
+    if "no_alloc" in request.node.nodeid:
+        gc.collect()

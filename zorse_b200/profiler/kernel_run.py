@@ -2,7 +2,8 @@
 `ncu` captures (`ncu --set full --clock-control none -k regex:<name> -c 2 python -m
 zorse_b200.profiler.kernel_run <case>`).  Holds well under a few GB on the device.
 
-cases: gemm_fwd | gemm_dgrad | gemm_wgrad | flash_fwd1 | flash_fwd2 | flash_fwd4 | flash_fwd4p | flash_fwd4q | flash_bwd1 | flash_bwd2 |
+cases: gemm_fwd | gemm_dgrad | gemm_wgrad | gemm_act_fwd | gemm_act_bwd | gemm_rope (products with an activation or a rotation in
+       the epilogue) | wgrad_list (a block's weight gradients, bias and norm gradients from one list) | flash_fwd1 | flash_fwd2 | flash_fwd4 | flash_fwd4p | flash_fwd4q | flash_bwd1 | flash_bwd2 |
        flash_bwd | flash_bwd3 | flash_bwd3_dkv | flash_bwd3_dq (flash_bwd: the default version; the last three also as
        flash64_bwd3... on grouped heads of 64) | rmsnorm | rmsnorm_bwd | layernorm_bwd | rope | swiglu_fwd | swiglu_bwd |
        embedding_fwd | embedding_bwd | adam | ce
@@ -24,7 +25,35 @@ def main(argv=None):
     dev = "cuda"
     g = torch.Generator(device=dev).manual_seed(0)
     rnd = lambda *s: (torch.randn(*s, device=dev, generator=g) * 0.5).to(torch.bfloat16)
-    if case.startswith("gemm"):
+    if case in ("gemm_act_fwd", "gemm_act_bwd", "gemm_rope", "wgrad_list"):
+        from zorse_b200.ops.api import get_ops
+
+        ops = get_ops("sm100")
+        k.status_word()
+        if case == "gemm_rope":
+            x, w = rnd(8192, 2048), rnd(2560, 2048)              # 34 + 10 MB, and 42 MB out
+            cs = ops.rope_table(2048, 64, 1e4, dev)
+            fn = lambda: ops.linear_rope_fwd(x, w, None, cs, 2048, 36, 64)
+        elif case == "wgrad_list":
+            T, shapes = 3072, [(768, 3072), (3072, 768), (768, 768), (2304, 768)]      # a BERT block
+            dys, xs = [rnd(T, n) for n, _ in shapes], [rnd(T, m) for _, m in shapes]
+            gws, gbs = [torch.zeros(n, m, device=dev) for n, m in shapes], [torch.zeros(n, device=dev) for n, _ in shapes]
+            nw, ng = rnd(768), torch.zeros(4, 768, device=dev)
+            _, st = ops.norm_fwd(xs[1], nw, nw, 1e-5, True)
+
+            def fn():
+                later = ops.collect()
+                for dy, x, gw, gb in zip(dys, xs, gws, gbs):
+                    ops.linear_wgrad(dy, x, gw, gb, later=later)
+                for i in (0, 2):
+                    ops.norm_bwd(dys[0], xs[1], nw, st, None, ng[i], ng[i + 1], True, later)
+                ops.finish(later)
+        else:
+            x, w, dn, dy = rnd(4096, 4096), rnd(22016, 4096), rnd(4096, 11008), rnd(4096, 4096)   # a 7B block: 180 MB of weights
+            _, pre = ops.act_linear_fwd(x, w, None, "swiglu", True)
+            fn = ((lambda: ops.act_linear_fwd(x, w, None, "swiglu", True)) if case == "gemm_act_fwd" else
+                  (lambda: ops.act_linear_dgrad(dy, dn, pre, "swiglu")))
+    elif case.startswith("gemm"):
         M, N, K = 4096, 11008, 4096          # 34 + 90 + 90 MB
         a, w, dy = rnd(M, K), rnd(N, K), rnd(M, N)
         out, dx = torch.empty(M, N, device=dev, dtype=torch.bfloat16), torch.empty(M, K, device=dev, dtype=torch.bfloat16)
