@@ -795,8 +795,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   }
   tc_fence_before();
   // The leader's MMAs read the peer's shared memory: leave together.  Where nothing written before is read behind this
-  // barrier it need not order memory: a releasing arrival waits for the epilogue's own writes, 0.7 us at the end of every
-  // product.  Arrivals on the other CTA's barriers are no such writes: the issuer of the leader has waited for them above.
+  // barrier it need not order memory: a releasing arrival waits for the epilogue's own writes, 0.5 us at the end of a short
+  // product (1018 x 2048 x 512 6.25 -> 5.75 us, 3072 x 768 x 768 7.24 -> 6.64, 3072 x 3072 x 768 13.3 -> 12.9).  Arrivals on the other CTA's barriers are no such writes: the issuer of the leader has waited for them above.
   // The stores of the last boxes are still being read meanwhile (their writes are complete when the grid is).
   if constexpr (SCATTER || FUSED_AG) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
   else asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");

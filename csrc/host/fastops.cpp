@@ -415,7 +415,8 @@ PyObject* norm_bwd(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 //
 // No product reads what another one writes, so each but the first starts on the SMs that the one before it has done with,
 // where one after the other every one ended with most of the GPU idle (a BERT block's four weight gradients are 54, 18, 72 and
-// 72 tiles on 74 pairs), and the column sums run beside the last.  All operands stay in the list until everything is
+// 72 tiles on 74 pairs), and the column sums take up SMs as the last product leaves them (such a list is 59 us, its products alone
+// 47: the sources have left L2 by then).  All operands stay in the list until everything is
 // launched, and the workspaces are taken ahead of the first launch (what the allocator hands out behind it may have been given
 // back by another thread while kernels on this stream still use it): the rules of chain_late (ptx.cuh).
 // Long products are cut along K as they are alone, for the same bits and the same accuracy: what a tensor core adds to an
