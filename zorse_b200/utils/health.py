@@ -34,13 +34,15 @@ class Heartbeat:
         self.store.set(f"hbin/{self.rank}", f"{step}:{self.clock():.3f}")
 
     def not_entered(self, step: int) -> list[int]:
-        """Ranks that have not reported entering step `step` (or any later one)."""
+        """Ranks that have not reported entering step `step` (or any later one), as a rank that has entered a step itself sees
+        it.  A store in which its own report is not to be found (read last) is gone, with the rank that hosts it, and knows
+        nothing of the others: none are named then."""
         out = []
         for r in range(self.world):
             hb = self.read(r, key="hbin")
             if hb is None or hb[0] < step:
                 out.append(r)
-        return out
+        return out if self.read(self.rank, key="hbin") is not None else []
 
     def read(self, rank: int, key: str = "hb"):
         try:
