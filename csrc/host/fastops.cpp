@@ -14,11 +14,11 @@
 
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/util/SmallVector.h>
 
 #include <cmath>
 #include <cstdint>
 #include <utility>
-#include <vector>
 
 namespace {
 
@@ -437,21 +437,20 @@ PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     return nullptr;
   };
   const Py_ssize_t entries = PyList_GET_SIZE(args[0]);
-  Py_ssize_t products = 0, launched = 0;
+  Py_ssize_t last = -1, launched = 0;
   for (Py_ssize_t i = 0; i < entries; ++i) {
     PyObject* e = PyList_GET_ITEM(args[0], i);
     if (!PyTuple_Check(e) || (PyTuple_GET_SIZE(e) != 3 && PyTuple_GET_SIZE(e) != 4)) return refuse();
-    products += PyTuple_GET_SIZE(e) == 4;
+    if (PyTuple_GET_SIZE(e) == 4) last = i;
   }
-  std::vector<Tensor> workspaces;   // one per product, undefined for one that runs whole
-  for (Py_ssize_t i = 0; i < entries; ++i) {
+  c10::SmallVector<Tensor, 8> workspaces;   // one per product, undefined for one that runs whole
+  for (Py_ssize_t i = 0; i <= last; ++i) {
     PyObject* e = PyList_GET_ITEM(args[0], i);
     if (PyTuple_GET_SIZE(e) != 4) continue;
     const Tensor *dy = tensor_of(PyTuple_GET_ITEM(e, 0)), *gw = tensor_of(PyTuple_GET_ITEM(e, 2));
-    if (dy == nullptr || gw == nullptr || status_of(*dy) == nullptr || dy->dim() != 2 || gw->dim() != 2) return refuse();
+    if (dy == nullptr || gw == nullptr || dy->dim() != 2 || gw->dim() != 2 || !dy->is_cuda()) return refuse();
     const int64_t M = gw->size(0), N = gw->size(1);
-    const bool last = Py_ssize_t(workspaces.size()) + 1 == products;
-    workspaces.push_back(last || (M % 32 == 0 && N % 32 == 0) ? split_workspace(M, N, dy->size(0), *dy) : Tensor());
+    workspaces.push_back(i == last || (M % 32 == 0 && N % 32 == 0) ? split_workspace(M, N, dy->size(0), *dy) : Tensor());
   }
   constexpr int MAX = 8;   // sums per launch
   long desc[MAX][7];
@@ -459,7 +458,7 @@ PyObject* finish(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   bool late = false;       // a product has been launched here: what the sums read was complete before it
   // Bytes that kernels launched here, or sums not launched yet, add to; `claim` answers whether none of them is in `out`,
   // which else has to wait: then all of them are done, and the record starts anew.
-  std::vector<std::pair<uintptr_t, uintptr_t>> written;
+  c10::SmallVector<std::pair<uintptr_t, uintptr_t>, 16> written;
   auto claim = [&](const Tensor& out) {
     const uintptr_t lo = reinterpret_cast<uintptr_t>(out.data_ptr());
     const int64_t last = out.dim() == 2 ? (out.size(0) - 1) * out.stride(0) + out.size(1) : out.numel();
