@@ -93,8 +93,8 @@ class DeferredWgrad:
     while the upstream stage is already working: the chain between stages gets shorter by the weight-gradient
     time per stage.  What a layer collects for its `finish` (`later`) is collected again and finished together, layer by
     layer and microbatch by microbatch.  Results are bit-identical: every bucket entry receives the same additions in the
-    same order, and each of them comes from the same kernels as without the queue (products that run together are not cut
-    along the reduction where one alone would be)."""
+    same order, and each of them comes from the same kernels as without the queue (a list's bias sums run in another order than
+    one alone)."""
 
     def __init__(self, ops):
         self._ops = ops
